@@ -7,6 +7,11 @@
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <string.h>
+
+#include <mutex>
+#include <set>
+#include <utility>
 
 #include "../../include/excalibur_b200.h"
 
@@ -50,6 +55,53 @@ inline int after_launch(const char* what) {
         return fail(EXB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
     return EXB_OK;
 }
+
+// The dynamic shared-memory limit is an attribute of the kernel function on a device, shared by every thread that
+// launches it: it is raised to the device's maximum once, never lowered, so that concurrent launches from several
+// host threads (one pipeline replica per thread) cannot undercut each other.  Occupancy follows the bytes a launch
+// actually asks for, not this limit.
+template <typename K>
+inline int raise_smem_limit(const exb_ctx* ctx, K kern) {
+    static std::mutex attr_mutex;
+    static std::set<std::pair<const void*, int>> raised;
+    std::lock_guard<std::mutex> lock(attr_mutex);
+    const auto key = std::make_pair(reinterpret_cast<const void*>(kern), ctx->device);
+    if (!raised.count(key)) {
+        cudaFuncAttributes fa;
+        EXB_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));      // static + dynamic shared memory share the device limit
+        EXB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_optin - (int)fa.sharedSizeBytes));
+        raised.insert(key);
+    }
+    return EXB_OK;
+}
+
+// Launch with programmatic stream serialization: the grid may be scheduled while the previous kernel of the stream
+// drains.  Every kernel launched this way calls pdl_wait() before it touches global memory that another kernel
+// writes or reads.
+template <typename... KArgs, typename... Args>
+inline int launch_pdl(const exb_ctx* ctx, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                      Args&&... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx->pdl ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return fail(EXB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
+    }
+    return after_launch(what);
+}
+// Let the next kernel of the stream be scheduled as soon as SMs free up / wait for the previous one's memory.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 

@@ -136,3 +136,34 @@ def test_dwconv_int8_in_out(ctx):
     # pre-rounding value sits on a rounding boundary.
     assert np.abs(y - ref).max() <= 1
     assert (y != ref).mean() < 1e-3
+
+
+# Edges of the streaming 3x3 kernel: maps smaller than a thread's four columns, one row, ragged column groups, channel
+# counts that do not fill (8, 24) or do not fit (264, 1240) one CTA, rows that end inside a stage, no padding; fp16 and
+# int8 results.
+@pytest.mark.parametrize("out_i8", [False, True])
+@pytest.mark.parametrize("case", [
+    # N, C, H, W, stride, pad, act
+    (1, 8, 1, 1, 1, 1, 103), (2, 8, 3, 3, 1, 0, 0), (3, 24, 5, 2, 1, 1, 1), (1, 264, 9, 33, 1, 1, 103), (2, 1240, 7, 6, 1, 1, 104),
+    (1, 8, 2, 2, 2, 1, 103), (1, 16, 3, 4, 2, 1, 1), (2, 264, 13, 12, 2, 1, 103), (1, 40, 31, 257, 2, 1, 0), (5, 96, 40, 11, 2, 0, 103),
+    (37, 32, 30, 31, 1, 1, 1), (64, 144, 14, 14, 1, 1, 103),
+])
+def test_dwconv_stream_edges(ctx, case, out_i8):
+    capi = _capi()
+    N, Cc, H, W, s, pad, act = case
+    r = rng(sum(case))
+    x = f16_round(r.standard_normal((N, Cc, H, W)))
+    w = (r.standard_normal((Cc, 1, 3, 3)) * 0.3).astype(np.float32)
+    b = (r.standard_normal(Cc) * 0.1).astype(np.float32)
+    ref = O.dwconv2d_f32(x, w, b, s, pad, act)
+    scale = np.float32(127.0 / 6.0)
+    d = capi.make_dw_desc(N, H, W, Cc, 3, s, pad, capi.EXB_F16, capi.EXB_I8 if out_i8 else capi.EXB_F16, act, out_scale=scale)
+    y = capi.dwconv2d(ctx, d, dev(to_nhwc(x).astype(np.float16)), capi.DwWeights(ctx, d, w, b))
+    ctx.sync_check()
+    y = to_nchw(host(y).astype(np.float32))
+    assert y.shape == ref.shape
+    if out_i8:
+        diff = np.abs(y - O.requantize_rne(ref, scale).astype(np.float32))
+        assert diff.max() <= 1 and (diff != 0).mean() < 1e-2
+    else:
+        np.testing.assert_allclose(y, ref, rtol=2e-3, atol=2e-3)
