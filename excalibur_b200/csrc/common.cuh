@@ -79,25 +79,38 @@ inline int raise_smem_limit(const exb_ctx* ctx, K kern) {
 // drains.  Every kernel launched this way calls pdl_wait() before it touches global memory that another kernel
 // writes or reads.
 template <typename... KArgs, typename... Args>
-inline int launch_pdl(const exb_ctx* ctx, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                      Args&&... args) {
+inline int launch_pdl_cluster(const exb_ctx* ctx, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, int cluster_z, size_t smem,
+                              cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (ctx->pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster_z > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = (unsigned)cluster_z;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = ctx->pdl ? 1 : 0;
+    cfg.numAttrs = n;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return fail(EXB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
     }
     return after_launch(what);
+}
+template <typename... KArgs, typename... Args>
+inline int launch_pdl(const exb_ctx* ctx, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                      Args&&... args) {
+    return launch_pdl_cluster(ctx, what, kern, grid, block, 1, smem, st, static_cast<Args&&>(args)...);
 }
 // Let the next kernel of the stream be scheduled as soon as SMs free up / wait for the previous one's memory.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -167,3 +167,37 @@ def test_dwconv_stream_edges(ctx, case, out_i8):
         assert diff.max() <= 1 and (diff != 0).mean() < 1e-2
     else:
         np.testing.assert_allclose(y, ref, rtol=2e-3, atol=2e-3)
+
+
+# Edges of the streaming pooling kernel: windows hanging over every border of maps smaller than a thread's four columns,
+# negative values next to padding (a maximum must not see the fill), channel counts around one CTA's, ceil mode, the
+# int8 second output; below 32 channels stride 2 takes the other kernel.
+@pytest.mark.parametrize("case", [
+    # N, C, H, W, type, k, s, pad, pad_mode, cip
+    (1, 8, 1, 1, 0, 5, 1, 2, 1, 0), (2, 264, 6, 3, 0, 5, 1, 2, 1, 0), (3, 40, 27, 33, 1, 5, 1, 2, 1, 1), (1, 520, 9, 5, 1, 3, 1, 1, 1, 0),
+    (2, 24, 5, 7, 0, 3, 1, 1, 1, 0), (2, 32, 2, 2, 0, 3, 2, 1, 1, 0), (1, 72, 37, 41, 0, 3, 2, 1, 0, 0), (2, 64, 30, 9, 1, 3, 2, 1, 0, 1),
+    (1, 32, 3, 5, 0, 2, 2, 0, 0, 0), (2, 136, 29, 31, 1, 2, 2, 0, 1, 0), (40, 64, 20, 20, 0, 5, 1, 2, 1, 0), (1, 16, 9, 9, 0, 3, 2, 1, 1, 0),
+])
+def test_pool_stream_edges(ctx, case):
+    capi = _capi()
+    N, Cc, H, W, type_, k, s, pad, pad_mode, cip = case
+    x = f16_round(rng(sum(case)).standard_normal((N, Cc, H, W)) - 3)
+    ref = O.pool2d_f32(x, type_, k, s, pad, False, pad_mode, cip)
+    q = np.float32(9.0)
+    d = capi.make_pool_desc(N, H, W, Cc, type_, k, s, pad, False, pad_mode, cip, capi.EXB_F16, capi.EXB_I8, q)
+    y, y2 = capi.pool2d(ctx, d, dev(to_nhwc(x).astype(np.float16)))
+    ctx.sync_check()
+    y = to_nchw(host(y).astype(np.float32))
+    assert y.shape == ref.shape
+    if type_ == 0:
+        np.testing.assert_array_equal(y, ref)
+        np.testing.assert_array_equal(to_nchw(host(y2)), O.requantize_rne(ref, q))
+    else:
+        np.testing.assert_allclose(y, ref, rtol=1e-3, atol=1e-3)
+
+
+# A map split over a cluster of CTAs, and channel counts that leave lanes of the last CTA without work.
+@pytest.mark.parametrize("type_", [0, 1])
+@pytest.mark.parametrize("shape", [(1, 8, 112, 111), (3, 264, 33, 29), (1, 64, 40, 40), (70, 272, 9, 9)])
+def test_global_pool_split(ctx, type_, shape):
+    test_global_pool(ctx, type_, shape)
