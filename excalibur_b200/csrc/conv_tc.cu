@@ -34,14 +34,8 @@
 // per-channel PReLU activation.
 // All mbarrier waits are bounded; when one runs out the kernel raises the context's error
 // word, every role leaves its loop, TMEM is freed and the launch returns normally.
-#include "conv_common.cuh"
+#include "conv_tc_host.cuh"
 #include "ptx_sm100.cuh"
-
-#include <cudaTypedefs.h>
-
-#include <mutex>
-#include <set>
-#include <utility>
 
 namespace exb {
 namespace {
@@ -50,7 +44,6 @@ constexpr int kMaxStages = 8;
 constexpr int kFirstEpiWarp = 2;   // warp 0 producer, warp 1 MMA issuer, epilogue warps from here on
 constexpr int kMaxAccBufs = 4;
 constexpr int kConstCh = 64;      // output channels of the pool epilogue (scale / bias travel as launch parameters)
-constexpr int kTileM = 128;
 constexpr uint32_t kMaxSpins = 1u << 21;  // tens of milliseconds at least; a legitimate wait is microseconds
 
 enum EpiKind { kEpiRow = 0, kEpiQuad = 1, kEpiPool = 2 };
@@ -917,6 +910,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
             const int tn = row / (p.TW * p.TH);
             const bool row_in_box = row < p.TW * p.TH * p.TN;
             const bool vec_ok = (p.e.cout_stride & 15) == 0;
+            const bool vec8_ok = (p.e.cout_stride & 7) == 0 && (p.e.y_pitch & 7) == 0 && p.e.out_dtype != EXB_I32;
             const int n_chunks = p.BN / 16;
             const bool lean = kInt8 && !kPrelu && vec_ok && p.e.out_dtype == EXB_I8 && p.e.out2_dtype < 0 &&
                               (p.e.act == EXB_ACT_NONE || p.e.act == EXB_ACT_RELU) && (p.BN & 31) == 0 && (p.e.cout_stride & 31) == 0 &&
@@ -1010,6 +1004,35 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                             bi[i] = reinterpret_cast<const float4*>(s_bias + cl)[i];
                         }
                         epi_row16<kInt8, kPrelu, 16, 2, 0>(p.e, sc, bi, cl, pix, do_res, rc, raw);
+                    } else if (vec8_ok) {
+                        // a multiple of 8 channels: the same in two halves, the second of the last chunk may be missing
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int c8 = cl + 8 * h;
+                            if (c8 >= p.e.cout_stride) break;
+                            float v[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) v[i] = epi_value<kInt8>(raw[8 * h + i], s_scale[c8 + i], s_bias[c8 + i]);
+                            if (p.has_res) {
+                                const uint4 rv = __ldg(reinterpret_cast<const uint4*>(p.e.residual + pix * p.e.cout_stride + c8));
+                                const __half2* rh = reinterpret_cast<const __half2*>(&rv);
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const float2 f = __half22float2(rh[i]);
+                                    v[2 * i] += f.x;
+                                    v[2 * i + 1] += f.y;
+                                }
+                            }
+                            if constexpr (kPrelu) {
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) v[i] = v[i] >= 0.f ? v[i] : v[i] * __ldg(p.e.slope + c8 + i);
+                            } else {
+                                apply_act_vec(v, p.e.act);
+                            }
+                            const int64_t off = pix * p.e.y_pitch + c8;
+                            epi_store_vec8(p.e.y, p.e.out_dtype, off, v, p.e.out_scale);
+                            if (p.e.out2_dtype >= 0) epi_store_vec8(p.e.y2, p.e.out2_dtype, off, v, p.e.out2_scale);
+                        }
                     } else {
                         // ragged channel count: element-wise stores, statically indexed so the
                         // accumulators stay in registers
@@ -1050,48 +1073,9 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
     }
 }
 
-// ---- host side ----------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    if (!fn) {
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(ptr);
-    }
-    return fn;
-}
-
-CUtensorMapSwizzle swizzle_for(int kb_bytes) {
-    return kb_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                           : (kb_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
-}
-
-int round_up(int a, int b) { return (a + b - 1) / b * b; }
-
-// Pick the pixel box (TW x TH x TN <= 128 rows) that wastes the fewest MMA rows; ties go to
-// the widest box (longest contiguous runs for the TMA unit), then the tallest.
-void choose_tile(int N, int OH, int OW, int& TW, int& TH, int& TN) {
-    double best = -1.0;
-    TW = 1; TH = 1; TN = 1;
-    for (int tw = 1; tw <= OW && tw <= kTileM; ++tw)
-        for (int th = 1; th <= OH && tw * th <= kTileM; ++th) {
-            int tn = kTileM / (tw * th);
-            if (tn > N) tn = N;
-            if (tn < 1) continue;
-            const int64_t tiles = (int64_t)((OW + tw - 1) / tw) * ((OH + th - 1) / th) * ((N + tn - 1) / tn);
-            const double eff = (double)OW * OH * N / ((double)tiles * kTileM);
-            const bool better = eff > best + 1e-9 ||
-                                (eff > best - 1e-9 && (tw > TW || (tw == TW && th > TH)));
-            if (better) {
-                best = eff;
-                TW = tw; TH = th; TN = tn;
-            }
-        }
-}
-
 }  // namespace
+
+// ---- host side ----------------------------------------------------------------------------
 
 bool conv_tc_pool_fusable(const ConvGeom& g) {
     const FoldPlan fold = conv_fold_plan(g);
@@ -1113,14 +1097,17 @@ bool conv_tc_eligible(const ConvGeom& g) {
 
 int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_conv_weights* w,
                    const void* residual, void* y, void* y2, cudaStream_t st) {
-    auto encode = get_encode_fn();
+    auto encode = tensor_map_encoder();
     if (!encode) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     const bool int8 = g.in_dtype == EXB_I8;
     const int es = int8 ? 1 : 2;
     ConvTcParams p;
     memset(&p, 0, sizeof(p));
     p.N = g.N; p.OH = g.OH; p.OW = g.OW;
-    choose_tile(g.N, g.OH, g.OW, p.TW, p.TH, p.TN);
+    {
+        const PixelBox b = choose_pixel_box(g.N, g.OH, g.OW);
+        p.TW = b.TW; p.TH = b.TH; p.TN = b.TN;
+    }
     p.tiles_w = (g.OW + p.TW - 1) / p.TW;
     p.tiles_h = (g.OH + p.TH - 1) / p.TH;
     p.tiles_nb = (g.N + p.TN - 1) / p.TN;
@@ -1325,10 +1312,8 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
 
     const CUtensorMapDataType dt = int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const CUtensorMapSwizzle sw = swizzle_for(p.kb_bytes);
-    // A: one view per input parity (only view 0 for stride 1).  Rows may be physically padded.
     const size_t px_bytes = (size_t)g.cin_stride * es;
     const size_t row_pitch = (size_t)g.w_pitch * px_bytes;
-    const int nviews = g.sh == 1 ? 1 : 4;
     if (patch) {
         // One map: whole padded rows as the innermost dimension, box = 24 pixels x patch_rows.
         cuuint64_t dims[3] = {(cuuint64_t)g.w_pitch * g.cin_stride, (cuuint64_t)g.H, (cuuint64_t)g.N};
@@ -1341,39 +1326,8 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled(patch) failed with %d", (int)r);
     }
-    for (int v = 0; v < (patch ? 0 : nviews); ++v) {
-        const int ph = v >> 1, pw = v & 1;
-        const int st_ = g.sh;
-        if (fold.on && pw) continue;   // the folded layout walks W inside the K row
-        // rows / columns of this view: indices ph, ph+st, ... < H
-        const int vh = (g.H - ph + st_ - 1) / st_;
-        const int vw = (g.W - pw + st_ - 1) / st_;
-        if (vh <= 0 || vw <= 0) return fail(EXB_ERR_UNSUPPORTED, "stride-2 convolution needs H and W of at least 2");
-        CUresult r;
-        if (fold.on) {
-            // dim0: F pixels x cin_stride channels (one K row), dim1: output columns, stepping
-            // stride_w pixels (windows of neighbouring columns overlap), dim2: rows of this parity.
-            cuuint64_t dims[4] = {(cuuint64_t)p.kb_elems, (cuuint64_t)g.OW, (cuuint64_t)vh, (cuuint64_t)g.N};
-            cuuint64_t strides[3] = {(cuuint64_t)g.sw * px_bytes, (cuuint64_t)st_ * row_pitch, (cuuint64_t)g.H * row_pitch};
-            cuuint32_t box[4] = {(cuuint32_t)p.kb_elems, (cuuint32_t)p.TW, (cuuint32_t)p.TH, (cuuint32_t)p.TN};
-            cuuint32_t estr[4] = {1, 1, 1, 1};
-            void* base = const_cast<char*>(static_cast<const char*>(x)) + (size_t)ph * row_pitch +
-                         (size_t)(g.w_pad - fold.pl_eff) * px_bytes;
-            r = encode(&p.tmA[v], dt, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        } else {
-            cuuint64_t dims[4] = {(cuuint64_t)g.cin_stride, (cuuint64_t)vw, (cuuint64_t)vh, (cuuint64_t)g.N};
-            cuuint64_t strides[3] = {(cuuint64_t)st_ * px_bytes, (cuuint64_t)st_ * row_pitch, (cuuint64_t)g.H * row_pitch};
-            cuuint32_t box[4] = {(cuuint32_t)p.kb_elems, (cuuint32_t)(p.rowbox ? p.TW + g.kw - 1 : p.TW), (cuuint32_t)p.TH,
-                                 (cuuint32_t)p.TN};
-            cuuint32_t estr[4] = {1, 1, 1, 1};
-            void* base = const_cast<char*>(static_cast<const char*>(x)) + (size_t)ph * row_pitch +
-                         (size_t)(pw + g.w_pad) * px_bytes;
-            r = encode(&p.tmA[v], dt, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        }
-        if (r != CUDA_SUCCESS) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled(A view %d) failed with %d", v, (int)r);
-    }
+    if (!patch)
+        if (int rc = encode_input_views(g, fold, x, p.kb_elems, sw, p.rowbox ? p.TW + g.kw - 1 : p.TW, p.TH, p.TN, p.tmA)) return rc;
     // Quad epilogue: N tiles of whole 32-channel blocks, every channel group of 8 either fully inside the output or
     // fully outside, weights stored in whole 32-row blocks (the permuting map walks rows 32 at a time).  Taken when
     // the epilogue moves fp16 / fp32 data (an fp16 output or residual): there its whole-sector accesses are worth
@@ -1435,23 +1389,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     else
         kern = int8 ? (two ? conv_tc_kernel<true, 8, kEpiRow, true> : conv_tc_kernel<true, 16, kEpiRow, true>)
                     : (two ? conv_tc_kernel<false, 8, kEpiRow, true> : conv_tc_kernel<false, 16, kEpiRow, true>);
-    // The dynamic shared-memory limit is an attribute of the kernel function on a device, shared by every thread that
-    // launches it: it is raised to the device's maximum once, never lowered, so that concurrent launches from several
-    // host threads (one pipeline replica per thread) cannot undercut each other.  Occupancy follows the bytes a launch
-    // actually asks for, not this limit.
-    {
-        static std::mutex attr_mutex;
-        static std::set<std::pair<const void*, int>> raised;
-        std::lock_guard<std::mutex> lock(attr_mutex);
-        const auto key = std::make_pair(reinterpret_cast<const void*>(kern), ctx->device);
-        if (!raised.count(key)) {
-            cudaFuncAttributes fa;
-            EXB_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));      // static + dynamic shared memory share the device limit
-            EXB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              ctx->smem_optin - (int)fa.sharedSizeBytes));
-            raised.insert(key);
-        }
-    }
+    if (int rc = raise_smem_limit(ctx, kern)) return rc;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)grid);
