@@ -79,7 +79,7 @@ inline int raise_smem_limit(const exb_ctx* ctx, K kern) {
 // drains.  Every kernel launched this way calls pdl_wait() before it touches global memory that another kernel
 // writes or reads.
 template <typename... KArgs, typename... Args>
-inline int launch_pdl_cluster(const exb_ctx* ctx, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, int cluster_z, size_t smem,
+inline int launch_pdl_cluster(const exb_ctx* ctx, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, dim3 cluster, size_t smem,
                               cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -93,10 +93,11 @@ inline int launch_pdl_cluster(const exb_ctx* ctx, const char* what, void (*kern)
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n++].val.programmaticStreamSerializationAllowed = 1;
     }
-    if (cluster_z > 1) {
+    if (cluster.x * cluster.y * cluster.z > 1) {
         attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = attr[n].val.clusterDim.y = 1;
-        attr[n++].val.clusterDim.z = (unsigned)cluster_z;
+        attr[n].val.clusterDim.x = cluster.x;
+        attr[n].val.clusterDim.y = cluster.y;
+        attr[n++].val.clusterDim.z = cluster.z;
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
@@ -110,7 +111,7 @@ inline int launch_pdl_cluster(const exb_ctx* ctx, const char* what, void (*kern)
 template <typename... KArgs, typename... Args>
 inline int launch_pdl(const exb_ctx* ctx, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                       Args&&... args) {
-    return launch_pdl_cluster(ctx, what, kern, grid, block, 1, smem, st, static_cast<Args&&>(args)...);
+    return launch_pdl_cluster(ctx, what, kern, grid, block, dim3(1), smem, st, static_cast<Args&&>(args)...);
 }
 // Let the next kernel of the stream be scheduled as soon as SMs free up / wait for the previous one's memory.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -221,7 +221,11 @@ extern "C" int exb_conv2d_fwd(exb_ctx* ctx, const exb_conv_desc* d, const void* 
         return fail(EXB_ERR_UNSUPPORTED, "fuse_pool is not available for this convolution (see exb_conv2d_pool_fusable)");
     if (g.y_pitch != g.cout_stride && !(d->impl != 1 && conv_tc_eligible(g)))
         return fail(EXB_ERR_UNSUPPORTED, "y_pitch needs the tensor-core kernel");
-    if (d->impl != 1 && conv_tc_eligible(g)) return conv_tc_launch(ctx, g, x, w, residual, y, y2, st);
+    if (d->impl != 1 && conv_tc_eligible(g)) {
+        if (d->impl == 0)
+            if (const ConvSplit sp = conv_split_plan(ctx, g, w); sp.splits) return conv_split_launch(ctx, g, sp, x, w, residual, y, y2, st);
+        return conv_tc_launch(ctx, g, x, w, residual, y, y2, st);
+    }
     return conv_direct_launch(ctx, g, x, w, residual, y, y2, st);
 }
 

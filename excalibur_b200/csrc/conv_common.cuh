@@ -200,6 +200,13 @@ int conv_direct_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb
                        const void* residual, void* y, void* y2, cudaStream_t st);
 int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_conv_weights* w,
                    const void* residual, void* y, void* y2, cudaStream_t st);
+// The split kernel (conv_split.cu): N tile and CTAs per tile of a launch, splits = 0 where the persistent kernel is used.
+struct ConvSplit {
+    int BN, splits;
+};
+ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w);
+int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, const void* x, const exb_conv_weights* w, const void* residual,
+                      void* y, void* y2, cudaStream_t st);
 // True when the tcgen05 kernel can run this geometry.
 bool conv_tc_eligible(const ConvGeom& g);
 // True when the tcgen05 kernel can also apply the 3x3/2 max pooling in its epilogue.

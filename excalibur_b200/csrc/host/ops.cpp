@@ -288,6 +288,9 @@ void operation_convolution<Dtype>::forward_nchw_f32(exb_ctx* h, const f32_list& 
     d.in_dtype = int8 ? EXB_I8 : EXB_F16;
     d.cin_stride = this->group_ == 1 ? round_up(C, int8 ? 32 : 16) : C;
     d.out_dtype = EXB_F32;
+    // Activation scales are taken from this path: one kernel, and so one order of the fp32 sums, whatever the batch - int8
+    // scales then do not depend on how many calibration images a forward holds.
+    if (!int8) d.impl = 2;
     d.act = exb_activation();
     int OH = 0, OW = 0;
     exb_check(exb_conv_out_dims(&d, &OH, &OW), "exb_conv_out_dims");

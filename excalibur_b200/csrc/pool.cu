@@ -412,8 +412,8 @@ int launch(exb_ctx* ctx, const exb_pool_desc* d, const PoolParams& p, const void
         while (splits < 8 && (int64_t)blocks * p.N * splits < 2 * ctx->sm_count && p.H * p.W >= 8 * rows * splits) splits *= 2;
         const dim3 grid(blocks, p.N, splits);
         const T* xi = static_cast<const T*>(x);
-        if (out2) return launch_pdl_cluster(ctx, "global_pool_kernel", global_pool_kernel<T, true>, grid, dim3(256), splits, 0, st, xi, static_cast<T*>(y), static_cast<int8_t*>(y2), p, cw, splits);
-        return launch_pdl_cluster(ctx, "global_pool_kernel", global_pool_kernel<T, false>, grid, dim3(256), splits, 0, st, xi, static_cast<T*>(y), nullptr, p, cw, splits);
+        if (out2) return launch_pdl_cluster(ctx, "global_pool_kernel", global_pool_kernel<T, true>, grid, dim3(256), dim3(1, 1, (unsigned)splits), 0, st, xi, static_cast<T*>(y), static_cast<int8_t*>(y2), p, cw, splits);
+        return launch_pdl_cluster(ctx, "global_pool_kernel", global_pool_kernel<T, false>, grid, dim3(256), dim3(1, 1, (unsigned)splits), 0, st, xi, static_cast<T*>(y), nullptr, p, cw, splits);
     }
     // The row stream needs rows of 64 bytes for its boxes where a window shares little with its neighbours (stride 2):
     // below 32 channels the kernel with a thread per output vector is 1.2-1.4 times as fast (64 maps @50x51, 16 and 24

@@ -173,7 +173,8 @@ typedef struct exb_conv_desc {
     int32_t act;            /* exb_act */
     float out_scale;        /* multiplier used when out_dtype == EXB_I8 */
     float out2_scale;       /* multiplier used when out2_dtype == EXB_I8 */
-    int32_t impl;           /* 0 = auto (tensor cores when eligible), 1 = force direct kernel */
+    int32_t impl;           /* 0 = auto (tensor cores when eligible), 1 = force direct kernel, 2 = the persistent
+                             * tensor-core kernel even where auto would divide tiles over clusters (few tiles) */
     /* Optional physically padded input rows: x is [N][H][x_w_pitch][cin_stride] and pixel 0 of a
      * row sits x_w_pad pixels in; the padding pixels hold zeros (exb_nchw_f32_to_nhwc_padded
      * writes this layout).  0 / 0 = dense rows.  With few input channels (a stem conv) this lets

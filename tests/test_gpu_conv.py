@@ -383,3 +383,62 @@ def test_conv_i8_residual_dual_output_shapes(ctx, case):
                             out_scale=nxt, out2_dtype=capi.EXB_F16)
     np.testing.assert_array_equal(q2, O.requantize_rne(v, nxt))
     np.testing.assert_array_equal(h2.astype(np.float32), f16_round(v))
+
+
+# The kernel for problems of few tiles: reductions of fewer K blocks than CTAs, K blocks that do not divide evenly, more of
+# them than the ring holds, channel counts that end inside a tile (multiples of 8), both strides, one pixel, maps
+# narrower than a box, every output form.  int8 equals the persistent kernel bit for bit, fp16 the oracle.
+SPLIT_CASES = [
+    # N, Cin, H, W, Cout, k, stride
+    (1, 512, 7, 7, 512, 3, 1), (1, 32, 1, 1, 8, 1, 1), (1, 64, 9, 5, 72, 3, 2), (2, 96, 14, 13, 40, 3, 1), (1, 512, 1, 1, 1000, 1, 1),
+    (3, 160, 7, 6, 264, 1, 1), (1, 256, 15, 15, 64, 3, 2), (1, 64, 56, 56, 64, 3, 1), (1, 1024, 4, 4, 32, 3, 1), (5, 32, 20, 3, 16, 5, 1),
+]
+
+
+@pytest.mark.parametrize("case", SPLIT_CASES)
+def test_conv_split_kernel(ctx, case):
+    import torch
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s = case
+    r = rng(sum(case) + 3)
+    xq = r.integers(-128, 128, (N, H, W, Cin)).astype(np.int8)
+    wq = r.integers(-127, 128, (Cout, Cin, k, k)).astype(np.int8)
+    b = r.standard_normal(Cout).astype(np.float32)
+    ws = r.uniform(500, 900, Cout).astype(np.float32)
+    got = {}
+    for impl in (0, 2):
+        for out, out2, res in ((capi.EXB_I8, -1, False), (capi.EXB_F16, capi.EXB_I8, True), (capi.EXB_F32, -1, False)):
+            d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8, out, out2, res=res, act=1, out_scale=9.0, out2_scale=9.0,
+                                    impl=impl)
+            oh, ow = capi.conv_out_dims(d)
+            skip = dev(rng(5).standard_normal((N, oh, ow, Cout)).astype(np.float16)) if res else None
+            ys = capi.conv2d(ctx, d, dev(xq), capi.ConvWeights(ctx, d, wq, b, ws, 40.0), residual=skip)
+            ctx.sync_check()
+            for i, y in enumerate(ys):
+                if y is not None:
+                    got.setdefault((out, i), []).append(y)
+    for key, (a, c) in got.items():
+        assert torch.equal(a, c), key
+    x = f16_round(r.uniform(-1, 1, (N, Cin, H, W)))
+    w = f16_round(r.standard_normal((Cout, Cin, k, k)) * np.sqrt(2.0 / (Cin * k * k)))
+    ref = O.conv2d_f32(x, w, b, s, k // 2, act=1)
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_F16, capi.EXB_F32, act=1)
+    y, _ = capi.conv2d(ctx, d, dev(to_nhwc(x).astype(np.float16)), capi.ConvWeights(ctx, d, w, b))
+    ctx.sync_check()
+    np.testing.assert_allclose(to_nchw(host(y)), ref, rtol=1e-4, atol=1e-4)
+
+
+# The persistent kernel on the small shapes of the tests above, which the automatic choice now gives to the split kernel;
+# channel counts that are multiples of 8 but not of 16 go through its two-halves epilogue.
+@pytest.mark.parametrize("case", I8_CASES + [(2, 96, 14, 13, 40, 3, 1, 1), (3, 64, 20, 20, 408, 1, 1, 0)])
+def test_conv_persistent_kernel_small(ctx, case):
+    capi = _capi()
+    N, Cin, H, W, Cout, k, stride, pad = case
+    r = rng(sum(case) + 21)
+    xq = r.integers(-128, 128, (N, Cin, H, W)).astype(np.int8)
+    wq = r.integers(-127, 128, (Cout, Cin, k, k)).astype(np.int8)
+    acc = O.conv2d_i8_acc(xq, wq, stride, pad).astype(np.float32)
+    y, _, _ = run_conv_i8(ctx, xq, wq, None, np.ones(Cout, np.float32), 1.0, stride, pad, capi.EXB_F32, act=1, impl=2)
+    np.testing.assert_array_equal(y, np.maximum(acc, 0))
+    q, _, _ = run_conv_i8(ctx, xq, wq, None, np.ones(Cout, np.float32), 1.0, stride, pad, capi.EXB_I8, act=1, out_scale=np.float32(1e-3), impl=2)
+    np.testing.assert_array_equal(q, O.requantize_rne(np.maximum(acc, 0), np.float32(1e-3)))
