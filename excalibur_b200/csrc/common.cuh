@@ -19,8 +19,8 @@ struct exb_ctx {
     int device;
     int sm_count;
     int smem_optin;          // max dynamic shared memory per block (opt-in)
-    int* d_error;            // device error word written by kernels whose bounded waits ran out
-    int* h_error;            // pinned host mirror
+    int* d_error;            // error word written by kernels whose bounded waits ran out: the device's view
+    int* h_error;            // and the host's of the same mapped word
     int pdl;                 // launch the conv kernel with programmatic stream serialization (default 1; EXB_PDL=0 turns it off)
 };
 

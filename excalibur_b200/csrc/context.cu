@@ -49,11 +49,12 @@ extern "C" int exb_ctx_create(int device, exb_ctx** out) {
         const char* e = getenv("EXB_PDL");   // EXB_PDL=0: plain stream-ordered launches of the conv kernel
         c->pdl = (e && e[0] == '0') ? 0 : 1;
     }
-    cudaError_t e = cudaMalloc(&c->d_error, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(c->d_error, 0, sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost(&c->h_error, sizeof(int));
+    // The error word lives in mapped host memory: kernels write it over the bus when they give up, and reading it after a
+    // synchronisation costs no copy.
+    cudaError_t e = cudaHostAlloc(&c->h_error, sizeof(int), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->d_error), c->h_error, 0);
     if (e != cudaSuccess) {
-        if (c->d_error) cudaFree(c->d_error);
+        if (c->h_error) cudaFreeHost(c->h_error);
         delete c;
         return fail(EXB_ERR_CUDA, "exb_ctx_create: %s", cudaGetErrorString(e));
     }
@@ -65,7 +66,6 @@ extern "C" int exb_ctx_create(int device, exb_ctx** out) {
 extern "C" int exb_ctx_destroy(exb_ctx* ctx) {
     if (!ctx) return EXB_OK;
     cudaSetDevice(ctx->device);
-    if (ctx->d_error) cudaFree(ctx->d_error);
     if (ctx->h_error) cudaFreeHost(ctx->h_error);
     delete ctx;
     return EXB_OK;
@@ -104,12 +104,10 @@ extern "C" int exb_selftest_bounded_wait(exb_ctx* ctx, int max_polls, void* stre
 extern "C" int exb_ctx_sync_check(exb_ctx* ctx, void* stream) {
     EXB_REQUIRE(ctx != nullptr, "exb_ctx_sync_check: null context");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    EXB_CUDA_TRY(cudaMemcpyAsync(ctx->h_error, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, st));
     EXB_CUDA_TRY(cudaStreamSynchronize(st));
-    const int word = *ctx->h_error;
+    const int word = *static_cast<volatile int*>(ctx->h_error);
     if (word != 0) {
-        EXB_CUDA_TRY(cudaMemsetAsync(ctx->d_error, 0, sizeof(int), st));
-        EXB_CUDA_TRY(cudaStreamSynchronize(st));
+        *static_cast<volatile int*>(ctx->h_error) = 0;
         return fail(EXB_ERR_TIMEOUT, "a kernel gave up a bounded wait (role code %d)", word);
     }
     return EXB_OK;

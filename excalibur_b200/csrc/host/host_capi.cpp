@@ -55,7 +55,7 @@ int copy_out(const std::shared_ptr<memory::tensor<float>>& t, float* out, int64_
         g_err = "output buffer too small";
         return EXB_ERR_BAD_ARG;
     }
-    std::memcpy(out, t->cpu_data(), sizeof(float) * (size_t)t->count());
+    host_copy(out, t->cpu_data(), sizeof(float) * (size_t)t->count());
     return EXB_OK;
 }
 

@@ -8,6 +8,7 @@
 #include <condition_variable>
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -42,6 +43,13 @@ private:
     uint16_t* dst_ = nullptr;
     size_t n_ = 0;
 };
+
+// memcpy by the process's host threads (at most 8, half of the machine's; started on first use, asleep in between) when
+// the block is worth waking them, by the caller alone when it is small or another caller has them.  `ready`, if given, is
+// called by the calling thread with the number of leading bytes that are complete, as they grow: a caller can send a
+// block on to a device while the next one is copied (the stores then bypass the caches).  One wake-up serves the whole
+// call; it costs some 10-50 us.
+void host_copy(void* dst, const void* src, size_t bytes, const std::function<void(size_t)>& ready = nullptr);
 
 }  // namespace excalibur
 }  // namespace glasssix

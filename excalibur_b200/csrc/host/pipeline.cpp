@@ -5,6 +5,8 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <cmath>
 #include <fstream>
 #include <functional>
 #include <set>
@@ -82,6 +84,8 @@ struct fmap_info {
     std::vector<float> extra_i8_scales;   // further int8 consumers with other scales
     std::shared_ptr<dev_buf> f16, i8, f32;
     std::vector<std::shared_ptr<dev_buf>> extra_i8;
+    // the device buffers of a feature map stay when its steps are laid out again for another division of the batch
+    void keep(const fmap_info& o) { f16 = o.f16; i8 = o.i8; f32 = o.f32; extra_i8 = o.extra_i8; }
     bool produced = false;
     bool f32_only = false;         // result of a Reshape / Transpose at the tail of the graph: fp32 NCHW only
 };
@@ -99,10 +103,12 @@ public:
                const std::vector<std::string>& inputs, const std::vector<std::string>& outputs, int device)
         : params_(params), ops_(ops), inputs_(inputs), outputs_(outputs), device_(device) {}
     ~fused_plan() {
-        if (host_f16_) cudaFreeHost(host_f16_);
-        if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
-        for (auto e : copied_) cudaEventDestroy(e);
+        programs_.clear();
+        if (pinned_in_) cudaFreeHost(pinned_in_);
+        for (auto e : half_free_)
+            if (e) cudaEventDestroy(e);
         if (copy_stream_) cudaStreamDestroy(copy_stream_);
+        if (out_stream_) cudaStreamDestroy(out_stream_);
         if (stream_) cudaStreamDestroy(stream_);
         if (ev0_) cudaEventDestroy(ev0_);
         if (ev1_) cudaEventDestroy(ev1_);
@@ -127,17 +133,26 @@ public:
     void build(int N, int C, int H, int W);
     bool built() const { return built_; }
     bool built_for(int N, int C, int H, int W) const { return built_ && N == N_ && C == C_ && H == H_ && W == W_; }
-    void run(const float* host_input, bool use_graph, bool profile, std::vector<trace_event>* trace);
+    // One forward: input to the device, kernels, results to host_out_.  chunks: 0 = as many sub-batches as pay (choose_slices),
+    // 1 = the whole batch at once, k = k equal ones; sub-batch c + 1 is copied to the device and sub-batch c - 1 back to the
+    // host while sub-batch c is computed.  host_threads > 0: the input is converted to fp16 on the host by that many
+    // threads before it is copied (half the PCIe bytes), when the ingest step can read fp16 planes.  host_f16 != nullptr:
+    // the caller's input is already fp16 NCHW.
+    void run(const float* host_input, int chunks, bool use_graph, int host_threads = 0, const uint16_t* host_f16 = nullptr);
+    void run_profiled(const float* host_input, std::vector<trace_event>* trace);
     std::shared_ptr<memory::tensor<float>> fetch(const std::string& name);
     double run_resident(int iters, bool use_graph);
-    // forward of k * N_ images: chunk c+1 is copied to the device while chunk c is computed.  host_threads > 0:
-    // each chunk is first converted to fp16 on the host by that many threads (half the PCIe bytes), when the
-    // plan's ingest step can read fp16 planes; otherwise the fp32 input is copied as it is.
-    // host_f16 != nullptr: the caller's input is already fp16 NCHW (pipeline<unsigned short>); it is copied as it is.
-    void run_chunked(const float* host_input, int k, bool use_graph, int host_threads = 0, const uint16_t* host_f16 = nullptr);
     bool host_f16_capable() const { return ingest_f16_capable_; }
     int launches() const { return launches_; }
-    double device_ms() const { return device_ms_; }
+    double device_ms() const {
+        if (times_pending_) {
+            float ms = 0;
+            cudaEventElapsedTime(&ms, ev0_, ev1_);
+            device_ms_ = ms;
+            times_pending_ = false;
+        }
+        return device_ms_;
+    }
     exb_ctx* ctx() { return ctx_; }
 
 private:
@@ -146,6 +161,7 @@ private:
         if (it != index_.end()) return it->second;
         fmap_info f;
         f.name = n;
+        if (auto k = kept_.find(n); k != kept_.end()) f.keep(k->second);
         f.root = (int)fmaps_.size();
         index_[n] = f.root;
         fmaps_.push_back(f);
@@ -161,20 +177,23 @@ private:
         return t;
     }
     void add_step(const std::string& name, std::function<void(cudaStream_t)> fn, int launches = 1) {
-        steps_.push_back({name, fn, launches});
+        emit_steps_->push_back({name, fn, launches});
     }
-    void* form_f16(fmap_info& f) {
-        if (!f.f16) f.f16 = std::make_shared<dev_buf>();
-        return f.f16->ensure((size_t)f.N * f.H * (f.w_pitch ? f.w_pitch : f.W) * f.cs * 2, device_);
+    // Device forms of a feature map hold the whole batch; while the steps of a sub-batch are laid out, the address is
+    // that of its first image.
+    void* form(std::shared_ptr<dev_buf>& b, const fmap_info& f, size_t per_image) {
+        if (!b) b = std::make_shared<dev_buf>();
+        if (f.N != emit_n_) uneven_ = true;      // a map whose first dimension is not the batch cannot be divided
+        const size_t images = f.N == emit_n_ ? (size_t)N_ : (size_t)f.N;
+        return static_cast<char*>(b->ensure(images * per_image, device_)) + (f.N == emit_n_ ? (size_t)emit_n0_ * per_image : 0);
     }
-    void* form_i8(fmap_info& f) {
-        if (!f.i8) f.i8 = std::make_shared<dev_buf>();
-        return f.i8->ensure((size_t)f.N * f.H * f.W * f.cs, device_);
+    void* form_f16(fmap_info& f) { return form(f.f16, f, (size_t)f.H * (f.w_pitch ? f.w_pitch : f.W) * f.cs * 2); }
+    void* form_i8(fmap_info& f) { return form(f.i8, f, (size_t)f.H * f.W * f.cs); }
+    void* form_extra_i8(fmap_info& f, size_t i) {
+        if (f.extra_i8.size() <= i) f.extra_i8.resize(i + 1);
+        return form(f.extra_i8[i], f, (size_t)f.H * f.W * f.cs);
     }
-    void* form_f32(fmap_info& f) {
-        if (!f.f32) f.f32 = std::make_shared<dev_buf>();
-        return f.f32->ensure((size_t)f.N * (f.f32_pitch ? f.f32_pitch : f.H * f.W * f.C) * 4, device_);
-    }
+    void* form_f32(fmap_info& f) { return form(f.f32, f, (size_t)(f.f32_pitch ? f.f32_pitch : f.H * f.W * f.C) * 4); }
     void set_shape(fmap_info& f, int N, int C, int H, int W) {
         f.N = N; f.C = C; f.H = H; f.W = W;
         f.cs = round_up(C, (f.need_i8 || C > 16) ? 32 : 16);
@@ -190,33 +209,80 @@ private:
     exb_ctx* ctx_ = nullptr;
     cudaStream_t stream_ = nullptr;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
-    cudaGraphExec_t graph_exec_ = nullptr;
     bool built_ = false;
     int N_ = 0, C_ = 0, H_ = 0, W_ = 0;
     std::vector<fmap_info> fmaps_;
     std::unordered_map<std::string, int> index_;
-    std::vector<plan_step> steps_;
-    dev_buf staging_in_;
+    std::unordered_map<std::string, fmap_info> kept_;
+    dev_buf staging_in_;                   // the input, as it crossed PCIe (fp32, or fp16 in the same bytes)
+    bool staged_f16_ = false;
     dev_buf norm_in_;                      // normalised fp32 input when the graph starts with an Input op
-    dev_buf chunk_stage_;                  // k chunks of fp32 input for run_chunked
-    const void* ingest_src_ = nullptr;     // what the ingest step (steps_[0]) reads; never part of the graph
-    bool ingest_src_f16_ = false;          // ingest_src_ holds fp16 planes (converted on the host)
     bool ingest_f16_capable_ = false;      // the ingest step has an fp16-source variant
-    void* host_f16_ = nullptr;             // pinned staging for the host-converted input
-    size_t host_f16_bytes_ = 0;
+
+    // A sub-batch: its kernels, replayed as one graph after a first eager run.
+    struct slice {
+        int n0 = 0, n = 0;
+        std::vector<plan_step> steps;
+        cudaGraphExec_t exec = nullptr;
+        bool warmed = false;
+        cudaEvent_t copied = nullptr, done = nullptr;
+        slice() = default;
+        slice(const slice&) = delete;
+        slice& operator=(const slice&) = delete;
+        ~slice() {
+            if (exec) cudaGraphExecDestroy(exec);
+            if (copied) cudaEventDestroy(copied);
+            if (done) cudaEventDestroy(done);
+        }
+    };
+    // A way to run the batch: its division, and whether the input arrives as fp16 planes.
+    struct program {
+        std::vector<int> sizes;
+        bool f16_src = false, uneven = false;
+        double flops_i8 = 0, flops_f16 = 0;      // dense convolutions
+        std::vector<std::unique_ptr<slice>> slices;
+        int launches() const {
+            int n = 0;
+            for (auto& s : slices)
+                for (auto& st : s->steps) n += st.launches;
+            return n;
+        }
+    };
+    std::vector<std::unique_ptr<program>> programs_;
+    program& program_for(const std::vector<int>& sizes, bool f16_src);
+    std::vector<int> choose_slices(bool f16_src);
+    void layout(slice& s, bool f16_src);   // the steps of images [s.n0, s.n0 + s.n)
+    int emit_n0_ = 0, emit_n_ = 0;
+    bool uneven_ = false;
+    std::vector<plan_step>* emit_steps_ = nullptr;
+    double body_flops_i8_ = 0, body_flops_f16_ = 0;
+    std::vector<int> auto_sizes_[2];       // choose_slices' answers
+
+    void launch(slice& s, bool use_graph);
+    void copy_results(const slice& s, cudaStream_t st);
+    void copy_input(const char* src, bool pageable, size_t offset, size_t bytes, cudaStream_t st);
+    void* pinned_in_ = nullptr;            // page-locked staging: host-converted input, or a pageable caller's
+    size_t pinned_bytes_ = 0;
+    void* pinned_in(size_t bytes) {
+        if (pinned_bytes_ < bytes) {
+            if (pinned_in_) cudaFreeHost(pinned_in_);
+            pinned_in_ = nullptr;
+            CUDA_CHECK(cudaHostAlloc(&pinned_in_, bytes, cudaHostAllocDefault));
+            pinned_bytes_ = bytes;
+        }
+        return pinned_in_;
+    }
+    int half_next_ = 0;
+    cudaEvent_t half_free_[2] = {};        // a half of the staging for pageable inputs has been read
     std::unique_ptr<convert_pool> pool_;
-    cudaStream_t copy_stream_ = nullptr;
-    std::vector<cudaEvent_t> copied_;
-    void launch_body(bool use_graph);
+    cudaStream_t copy_stream_ = nullptr, out_stream_ = nullptr;
     int launches_ = 0;
-    double device_ms_ = 0.0;
-    bool warmed_ = false;
+    mutable double device_ms_ = 0.0;
+    mutable bool times_pending_ = false;
 
 public:
     // results of the last run, by output feature map name
     std::unordered_map<std::string, std::shared_ptr<memory::tensor<float>>> host_out_;
-    // results of the last run_chunked (all k * N_ images)
-    std::unordered_map<std::string, std::shared_ptr<memory::tensor<float>>> chunk_out_;
 };
 
 void fused_plan::finish_forms(fmap_info& f, bool wrote_i8) {
@@ -232,11 +298,9 @@ void fused_plan::finish_forms(fmap_info& f, bool wrote_i8) {
             exb_check(exb_quantize_fwd(ctx, src, EXB_F16, static_cast<int8_t*>(dst), count, s, 1, st), "exb_quantize_fwd");
         });
     }
-    f.extra_i8.clear();
-    for (float s : f.extra_i8_scales) {
-        auto b = std::make_shared<dev_buf>();
-        void* dst = b->ensure((size_t)f.N * f.H * f.W * f.cs, device_);
-        f.extra_i8.push_back(b);
+    for (size_t i = 0; i < f.extra_i8_scales.size(); ++i) {
+        const float s = f.extra_i8_scales[i];
+        void* dst = form_extra_i8(f, i);
         void* src = form_f16(f);
         const int64_t count = (int64_t)f.N * f.H * f.W * f.cs;
         add_step("quantize " + f.name, [=](cudaStream_t st) {
@@ -246,9 +310,9 @@ void fused_plan::finish_forms(fmap_info& f, bool wrote_i8) {
 }
 
 const void* fused_plan::int8_form_for(fmap_info& f, float scale) {
-    if (f.i8 && f.i8_scale == scale) return f.i8->p;
+    if (f.i8 && f.i8_scale == scale) return form_i8(f);
     for (size_t i = 0; i < f.extra_i8_scales.size(); ++i)
-        if (f.extra_i8_scales[i] == scale) return f.extra_i8[i]->p;
+        if (f.extra_i8_scales[i] == scale) return form_extra_i8(f, i);
     LOG(FATAL) << "internal: no int8 form of " << f.name << " with scale " << scale;
     return nullptr;
 }
@@ -261,14 +325,62 @@ void fused_plan::build(int N, int C, int H, int W) {
         CUDA_CHECK(cudaEventCreate(&ev0_));
         CUDA_CHECK(cudaEventCreate(&ev1_));
     }
-    if (graph_exec_) {
-        cudaGraphExecDestroy(graph_exec_);
-        graph_exec_ = nullptr;
+    built_ = false;
+    programs_.clear();
+    fmaps_.clear();
+    kept_.clear();
+    times_pending_ = false;
+    for (auto& v : auto_sizes_) v.clear();
+    N_ = N; C_ = C; H_ = H; W_ = W;
+    program_for({N}, false);
+    host_out_.clear();
+    for (const auto& name : outputs_) {
+        fmap_info& f = fmaps_[root(fid(name))];
+        host_out_[name] = std::shared_ptr<memory::tensor<float>>(
+            new memory::tensor<float>(std::vector<int>{f.N, f.C, f.H, f.W}, device_, memory::NCHW, nullptr));
     }
-    steps_.clear();
+    built_ = true;
+}
+
+// The program for a division of the batch, laid out when it is first asked for.  A graph with a map whose first dimension
+// is not the batch runs undivided.
+fused_plan::program& fused_plan::program_for(const std::vector<int>& sizes, bool f16_src) {
+    for (auto& p : programs_)
+        if (p->sizes == sizes && p->f16_src == f16_src) return *p;
+    std::unique_ptr<program> p(new program);
+    p->sizes = sizes;
+    p->f16_src = f16_src;
+    int n0 = 0;
+    for (int n : sizes) {
+        std::unique_ptr<slice> s(new slice);
+        s->n0 = n0;
+        s->n = n;
+        n0 += n;
+        layout(*s, f16_src);
+        CUDA_CHECK(cudaStreamSynchronize(nullptr));      // clears of padding channels, on the default stream
+        p->uneven = uneven_;
+        p->flops_i8 += body_flops_i8_;
+        p->flops_f16 += body_flops_f16_;
+        if (uneven_ && sizes.size() > 1) break;
+        CUDA_CHECK(cudaEventCreateWithFlags(&s->copied, cudaEventDisableTiming));
+        CUDA_CHECK(cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming));
+        p->slices.push_back(std::move(s));
+    }
+    if (uneven_ && sizes.size() > 1) return program_for({N_}, f16_src);
+    programs_.push_back(std::move(p));
+    return *programs_.back();
+}
+
+void fused_plan::layout(slice& sl, bool f16_src) {
+    const int N = sl.n, C = C_, H = H_, W = W_;
+    emit_n0_ = sl.n0;
+    emit_n_ = sl.n;
+    emit_steps_ = &sl.steps;
+    uneven_ = false;
+    body_flops_i8_ = body_flops_f16_ = 0;
+    for (auto& f : fmaps_) kept_[f.name].keep(f);
     fmaps_.clear();
     index_.clear();
-    warmed_ = false;
     ingest_f16_capable_ = false;
     const size_t n_ops = ops_.size();
 
@@ -570,7 +682,10 @@ void fused_plan::build(int N, int C, int H, int W) {
         const int in_id = root(fid(inputs_[0]));
         fmap_info& in = fmaps_[in_id];
         set_shape(in, N, C, H, W);
-        ingest_src_ = static_cast<float*>(staging_in_.ensure((size_t)N * C * H * W * 4, device_));
+        const size_t per_image = (size_t)C * H * W;
+        char* staging = static_cast<char*>(staging_in_.ensure(N_ * per_image * 4, device_));
+        const float* src32 = reinterpret_cast<const float*>(staging + sl.n0 * per_image * 4);
+        const void* src16 = staging + sl.n0 * per_image * 2;
         // A few-channel image that feeds one fp16 convolution is stored as NHWC4 rows with zero
         // padding along W when that lets the tensor-core kernel fold the kw taps into K.
         bool padded = false;
@@ -608,7 +723,7 @@ void fused_plan::build(int N, int C, int H, int W) {
             void* yo = form_f16(fy);
             const int ocs = fy.cs;
             add_step("ingest+focus " + in.name, [=](cudaStream_t st) {
-                exb_check(exb_nchw_f32_focus_to_nhwc_f16(ctx, static_cast<const float*>(this->ingest_src_), yo, N, C, H, W, ocs, mul, add, st),
+                exb_check(exb_nchw_f32_focus_to_nhwc_f16(ctx, src32, yo, N, C, H, W, ocs, mul, add, st),
                           "exb_nchw_f32_focus_to_nhwc_f16");
             });
             absorbed[focus_op] = 1;
@@ -630,10 +745,10 @@ void fused_plan::build(int N, int C, int H, int W) {
         const bool image = !padded && C <= 4 && (direct_i8 ? (cs == 16 || cs == 32) : (cs == 8 || cs == 16));
         const float* ingest_fixed = nullptr;
         if (nmul && !quad && !image) {
-            float* norm = static_cast<float*>(norm_in_.ensure((size_t)N * C * H * W * 4, device_));
+            float* norm = static_cast<float*>(norm_in_.ensure(N_ * per_image * 4, device_)) + sl.n0 * per_image;
             ingest_fixed = norm;
             add_step(params_[input_norm_op].name_, [=](cudaStream_t st) {
-                exb_check(exb_channel_affine_fwd(ctx, static_cast<const float*>(this->ingest_src_), norm, nmul, nadd, N, C, 0,
+                exb_check(exb_channel_affine_fwd(ctx, src32, norm, nmul, nadd, N, C, 0,
                                                  (int64_t)H * W, EXB_F32, 0, EXB_ACT_NONE, st), "exb_channel_affine_fwd");
             });
         }
@@ -642,32 +757,31 @@ void fused_plan::build(int N, int C, int H, int W) {
         } else if (padded) {
             ingest_f16_capable_ = quad && !nmul;
             add_step("ingest " + in.name, [=](cudaStream_t st) {
-                if (this->ingest_src_f16_)
-                    exb_check(exb_nchw_f16_to_nhwc4_padded(ctx, this->ingest_src_, dst, N, C, H, W, w_pad, w_pitch, st),
+                if (f16_src)
+                    exb_check(exb_nchw_f16_to_nhwc4_padded(ctx, src16, dst, N, C, H, W, w_pad, w_pitch, st),
                               "exb_nchw_f16_to_nhwc4_padded");
                 else if (quad && nmul)
-                    exb_check(exb_nchw_f32_to_nhwc4_padded_norm(ctx, static_cast<const float*>(this->ingest_src_), dst, N, C, H, W,
+                    exb_check(exb_nchw_f32_to_nhwc4_padded_norm(ctx, src32, dst, N, C, H, W,
                                                                 w_pad, w_pitch, nmul, nadd, st),
                               "exb_nchw_f32_to_nhwc4_padded_norm");
                 else
-                    exb_check(exb_nchw_f32_to_nhwc_padded(ctx, ingest_fixed ? ingest_fixed : static_cast<const float*>(this->ingest_src_),
+                    exb_check(exb_nchw_f32_to_nhwc_padded(ctx, ingest_fixed ? ingest_fixed : src32,
                                                           dst, EXB_F16, N, C, H, W, cs, w_pad, w_pitch, 1.f, 1, st),
                               "exb_nchw_f32_to_nhwc_padded");
             });
         } else if (image) {
             add_step("ingest " + in.name, [=](cudaStream_t st) {
-                exb_check(exb_image_f32_to_nhwc_norm(ctx, static_cast<const float*>(this->ingest_src_), dst, direct_i8 ? EXB_I8 : EXB_F16,
+                exb_check(exb_image_f32_to_nhwc_norm(ctx, src32, dst, direct_i8 ? EXB_I8 : EXB_F16,
                                                      N, C, H, W, cs, nmul, nadd, direct_i8 ? s : 1.f, 1, st),
                           "exb_image_f32_to_nhwc_norm");
             });
         } else {
             // Both forms of a wide network input: the int8 form is quantised from the fp32 values themselves (as the
-            // reference's first int8 convolution does), not from their fp16 rounding.  One step, two launches: the
-            // ingest step is the only one that may read `ingest_src_`.
+            // reference's first int8 convolution does), not from their fp16 rounding.
             void* dst8 = (in.need_i8 && in.need_f16) ? form_i8(in) : nullptr;
             wrote_i8_from_f32 = dst8 != nullptr;
             add_step("ingest " + in.name, [=](cudaStream_t st) {
-                const float* src = ingest_fixed ? ingest_fixed : static_cast<const float*>(this->ingest_src_);
+                const float* src = ingest_fixed ? ingest_fixed : src32;
                 exb_check(exb_nchw_f32_to_nhwc(ctx, src, dst, direct_i8 ? EXB_I8 : EXB_F16, N, C, H, W, cs, direct_i8 ? s : 1.f, 1, st),
                           "exb_nchw_f32_to_nhwc");
                 if (dst8) exb_check(exb_nchw_f32_to_nhwc(ctx, src, dst8, EXB_I8, N, C, H, W, cs, s, 1, st), "exb_nchw_f32_to_nhwc");
@@ -782,6 +896,8 @@ void fused_plan::build(int N, int C, int H, int W) {
         auto* conv = dynamic_cast<operation_convolution<float>*>(ops_[i].get());
         CHECK_EQ(x.C, conv->in_channels()) << params_[i].name_ << ": input channels do not match the weights";
         const bool int8 = conv->is_int8() && conv->group_ == 1;
+        (int8 ? body_flops_i8_ : body_flops_f16_) += 2.0 * x.N * x.H * x.W / (conv->stride_h_ * conv->stride_w_) * conv->in_channels() *
+                                                     conv->output_channel_ / conv->group_ * conv->kernel_size_h_ * conv->kernel_size_w_;
         exb_conv_desc d = conv->base_desc(x.N, x.H, x.W);
         d.in_dtype = int8 ? EXB_I8 : EXB_F16;
         d.cin_stride = conv->group_ == 1 ? x.cs : x.C;
@@ -1275,13 +1391,9 @@ void fused_plan::build(int N, int C, int H, int W) {
     }
 
     // ---- 5. outputs: fp32 NCHW on the device, then one D2H each -------------------------------
-    host_out_.clear();
     for (const auto& name : outputs_) {
         fmap_info& f = fmaps_[root(fid(name))];
         CHECK(f.produced) << "output " << name << " is never produced";
-        auto t = std::shared_ptr<memory::tensor<float>>(
-            new memory::tensor<float>(std::vector<int>{f.N, f.C, f.H, f.W}, device_, memory::NCHW, nullptr));
-        host_out_[name] = t;
         if (f.need_f32 && f.f32 && f.H == 1 && f.W == 1 && !f.f32_only) continue;   // already fp32 [N][C]
         if (f.f32_only) continue;                                    // Reshape / Transpose results are fp32 NCHW already
         const void* src = form_f16(f);
@@ -1291,179 +1403,246 @@ void fused_plan::build(int N, int C, int H, int W) {
             exb_check(exb_nhwc_to_nchw_f32(ctx, src, EXB_F16, dst, n, c, h, w, cs, 1.f, st), "exb_nhwc_to_nchw_f32");
         });
     }
-    N_ = N; C_ = C; H_ = H; W_ = W;
-    built_ = true;
+    for (auto& f : fmaps_)
+        if (f.N == sl.n) f.N = N_;       // what fetch() and the results see is the whole batch
 }
 
-void fused_plan::run(const float* host_input, bool use_graph, bool profile, std::vector<trace_event>* trace) {
-    CUDA_CHECK(cudaSetDevice(device_));
-    const size_t in_bytes = (size_t)N_ * C_ * H_ * W_ * 4;
-    CUDA_CHECK(cudaMemcpyAsync(staging_in_.p, host_input, in_bytes, cudaMemcpyHostToDevice, stream_));
-    ingest_src_ = staging_in_.p;
-    ingest_src_f16_ = false;
-    launches_ = 0;
-    for (auto& s : steps_) launches_ += s.launches;
-    if (profile) {
-        // per-step device times; never replayed from the graph so every step can be bracketed
-        std::vector<cudaEvent_t> evs(steps_.size() + 1);
-        for (auto& e : evs) CUDA_CHECK(cudaEventCreate(&e));
-        CUDA_CHECK(cudaEventRecord(evs[0], stream_));
-        for (size_t i = 0; i < steps_.size(); ++i) {
-            steps_[i].run(stream_);
-            CUDA_CHECK(cudaEventRecord(evs[i + 1], stream_));
-        }
-        CUDA_CHECK(cudaStreamSynchronize(stream_));
-        if (trace) {
-            trace->clear();
-            for (size_t i = 0; i < steps_.size(); ++i) {
-                float b = 0, e = 0;
-                cudaEventElapsedTime(&b, evs[0], evs[i]);
-                cudaEventElapsedTime(&e, evs[0], evs[i + 1]);
-                trace->push_back({steps_[i].name, b, e});
-            }
-        }
-        float total = 0;
-        cudaEventElapsedTime(&total, evs[0], evs.back());
-        device_ms_ = total;
-        for (auto& e : evs) cudaEventDestroy(e);
-    } else {
-        CUDA_CHECK(cudaEventRecord(ev0_, stream_));
-        launch_body(use_graph);
-        CUDA_CHECK(cudaEventRecord(ev1_, stream_));
-    }
-    for (auto& kv : host_out_) {
-        fmap_info& f = fmaps_[root(index_[kv.first])];
-        if (f.f32_pitch)
-            CUDA_CHECK(cudaMemcpy2DAsync(kv.second->mutable_cpu_data(), (size_t)f.C * 4, f.f32->p, (size_t)f.f32_pitch * 4,
-                                         (size_t)f.C * 4, f.N, cudaMemcpyDeviceToHost, stream_));
-        else
-            CUDA_CHECK(cudaMemcpyAsync(kv.second->mutable_cpu_data(), f.f32->p, (size_t)f.N * f.C * f.H * f.W * 4,
-                                       cudaMemcpyDeviceToHost, stream_));
-    }
-    CUDA_CHECK(cudaStreamSynchronize(stream_));
-    if (!profile) {
-        float ms = 0;
-        cudaEventElapsedTime(&ms, ev0_, ev1_);
-        device_ms_ = ms;
-    }
-    exb_check(exb_ctx_sync_check(ctx_, stream_), "fused forward");
-}
-
-// The ingest step reads `ingest_src_` when it is launched and is therefore launched eagerly; the rest
-// of the plan runs eagerly the first time and as one CUDA graph afterwards.
-void fused_plan::launch_body(bool use_graph) {
-    steps_[0].run(stream_);
-    if (use_graph && warmed_ && steps_.size() > 1) {
-        if (!graph_exec_) {
+// The kernels of a sub-batch: eagerly the first time, as one CUDA graph afterwards.
+void fused_plan::launch(slice& s, bool use_graph) {
+    if (use_graph && s.warmed) {
+        if (!s.exec) {
             cudaGraph_t graph = nullptr;
             CUDA_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-            for (size_t i = 1; i < steps_.size(); ++i) steps_[i].run(stream_);
+            for (auto& st : s.steps) st.run(stream_);
             CUDA_CHECK(cudaStreamEndCapture(stream_, &graph));
-            CUDA_CHECK(cudaGraphInstantiate(&graph_exec_, graph, 0));
+            CUDA_CHECK(cudaGraphInstantiate(&s.exec, graph, 0));
             cudaGraphDestroy(graph);
         }
-        CUDA_CHECK(cudaGraphLaunch(graph_exec_, stream_));
+        CUDA_CHECK(cudaGraphLaunch(s.exec, stream_));
     } else {
-        for (size_t i = 1; i < steps_.size(); ++i) steps_[i].run(stream_);
-        warmed_ = true;
+        for (auto& st : s.steps) st.run(stream_);
+        s.warmed = true;
     }
+}
+
+void fused_plan::copy_results(const slice& s, cudaStream_t st) {
+    for (auto& kv : host_out_) {
+        fmap_info& f = fmaps_[root(index_[kv.first])];
+        const bool whole = f.N != N_;        // not divisible: the only sub-batch is the batch
+        const size_t first = whole ? 0 : s.n0, images = whole ? f.N : s.n, per = (size_t)f.C * f.H * f.W;
+        float* dst = kv.second->mutable_cpu_data() + first * per;
+        const float* src = static_cast<const float*>(f.f32->p) + first * (f.f32_pitch ? (size_t)f.f32_pitch : per);
+        if (f.f32_pitch)
+            CUDA_CHECK(cudaMemcpy2DAsync(dst, (size_t)f.C * 4, src, (size_t)f.f32_pitch * 4, (size_t)f.C * 4, images, cudaMemcpyDeviceToHost, st));
+        else
+            CUDA_CHECK(cudaMemcpyAsync(dst, src, images * per * 4, cudaMemcpyDeviceToHost, st));
+    }
+}
+
+// bytes [offset, offset + bytes) of the input to the device.  A pageable source is copied by the host threads into
+// page-locked memory, each stretch on its way as soon as it is complete: the driver's own staging is one thread (14-18
+// GB/s).
+void fused_plan::copy_input(const char* src, bool pageable, size_t offset, size_t bytes, cudaStream_t st) {
+    char* dst = static_cast<char*>(staging_in_.p) + offset;
+    src += offset;
+    if (!pageable || bytes < (256 << 10)) {
+        CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+        return;
+    }
+    constexpr size_t kHalf = 16 << 20, kLeast = 256 << 10;
+    char* pinned = static_cast<char*>(pinned_in(2 * kHalf));
+    for (size_t at = 0; at < bytes; at += kHalf) {      // large inputs go through two halves in turn
+        const int h = half_next_;
+        half_next_ ^= 1;
+        if (!half_free_[h]) CUDA_CHECK(cudaEventCreateWithFlags(&half_free_[h], cudaEventDisableTiming));
+        else CUDA_CHECK(cudaEventSynchronize(half_free_[h]));
+        char* half = pinned + h * kHalf;
+        const size_t n = std::min(kHalf, bytes - at);
+        size_t sent = 0;
+        host_copy(half, src + at, n, [&](size_t ready) {
+            if (ready - sent < kLeast && ready < n) return;
+            CUDA_CHECK(cudaMemcpyAsync(dst + at + sent, half + sent, ready - sent, cudaMemcpyHostToDevice, st));
+            sent = ready;
+        });
+        CUDA_CHECK(cudaEventRecord(half_free_[h], st));
+    }
+}
+
+void fused_plan::run(const float* host_input, int chunks, bool use_graph, int host_threads, const uint16_t* host_f16) {
+    CUDA_CHECK(cudaSetDevice(device_));
+    if (host_f16) CHECK(ingest_f16_capable_) << "this plan's ingest step cannot read fp16 planes";
+    const bool convert = !host_f16 && host_threads > 0 && ingest_f16_capable_;
+    const bool f16 = host_f16 != nullptr || convert;
+    const char* src = host_f16 ? reinterpret_cast<const char*>(host_f16) : reinterpret_cast<const char*>(host_input);
+    bool pageable = false;
+    if (!convert) {
+        cudaPointerAttributes at;
+        pageable = cudaPointerGetAttributes(&at, src) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+        (void)cudaGetLastError();
+    }
+    std::vector<int> sizes{N_};
+    if (chunks == 0) {
+        std::vector<int>& kept = auto_sizes_[f16];
+        if (kept.empty()) kept = choose_slices(f16);
+        sizes = kept;
+    } else if (chunks > 1 && N_ % chunks == 0) {
+        sizes.assign(chunks, N_ / chunks);
+    }
+    program& prog = program_for(sizes, f16);
+    launches_ = prog.launches();
+    staged_f16_ = f16;
+    const size_t image = (size_t)C_ * H_ * W_, image_bytes = image * (f16 ? 2 : 4);
+    const bool many = prog.slices.size() > 1;
+    if (many && !copy_stream_) {
+        CUDA_CHECK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
+        CUDA_CHECK(cudaStreamCreateWithFlags(&out_stream_, cudaStreamNonBlocking));
+    }
+    uint16_t* converted = nullptr;
+    if (convert) {
+        converted = static_cast<uint16_t*>(pinned_in(N_ * image * 2));
+        if (!pool_ || pool_->threads() != host_threads) pool_.reset(new convert_pool(host_threads));
+    }
+    cudaStream_t in_stream = many ? copy_stream_ : stream_, res_stream = many ? out_stream_ : stream_;
+    auto send = [&](slice& s) {
+        if (convert) pool_->run(host_input + s.n0 * image, converted + s.n0 * image, s.n * image);
+        copy_input(convert ? reinterpret_cast<const char*>(converted) : src, pageable, s.n0 * image_bytes, s.n * image_bytes, in_stream);
+        if (many) CUDA_CHECK(cudaEventRecord(s.copied, copy_stream_));
+    };
+    // Copies from page-locked memory return at once and are all queued first; where the host takes part in them, a
+    // sub-batch's kernels are queued before the host turns to the next one.
+    const bool ahead = many && !pageable && !convert;
+    if (ahead)
+        for (auto& s : prog.slices) send(*s);
+    CUDA_CHECK(cudaEventRecord(ev0_, stream_));
+    for (auto& s : prog.slices) {
+        if (!ahead) send(*s);
+        if (many) CUDA_CHECK(cudaStreamWaitEvent(stream_, s->copied, 0));
+        launch(*s, use_graph);
+        if (many) {
+            CUDA_CHECK(cudaEventRecord(s->done, stream_));
+            CUDA_CHECK(cudaStreamWaitEvent(out_stream_, s->done, 0));
+        }
+        if (s == prog.slices.back()) CUDA_CHECK(cudaEventRecord(ev1_, stream_));
+        copy_results(*s, res_stream);
+    }
+    if (many) CUDA_CHECK(cudaStreamSynchronize(out_stream_));
+    exb_check(exb_ctx_sync_check(ctx_, stream_), "fused forward");
+    times_pending_ = true;
+}
+
+void fused_plan::run_profiled(const float* host_input, std::vector<trace_event>* trace) {
+    // per-step device times; never replayed from the graph so every step can be bracketed
+    CUDA_CHECK(cudaSetDevice(device_));
+    program& prog = program_for({N_}, false);
+    slice& s = *prog.slices[0];
+    launches_ = prog.launches();
+    staged_f16_ = false;
+    CUDA_CHECK(cudaMemcpyAsync(staging_in_.p, host_input, (size_t)N_ * C_ * H_ * W_ * 4, cudaMemcpyHostToDevice, stream_));
+    std::vector<cudaEvent_t> evs(s.steps.size() + 1);
+    for (auto& e : evs) CUDA_CHECK(cudaEventCreate(&e));
+    CUDA_CHECK(cudaEventRecord(evs[0], stream_));
+    for (size_t i = 0; i < s.steps.size(); ++i) {
+        s.steps[i].run(stream_);
+        CUDA_CHECK(cudaEventRecord(evs[i + 1], stream_));
+    }
+    CUDA_CHECK(cudaStreamSynchronize(stream_));
+    s.warmed = true;
+    if (trace) {
+        trace->clear();
+        for (size_t i = 0; i < s.steps.size(); ++i) {
+            float b = 0, e = 0;
+            cudaEventElapsedTime(&b, evs[0], evs[i]);
+            cudaEventElapsedTime(&e, evs[0], evs[i + 1]);
+            trace->push_back({s.steps[i].name, b, e});
+        }
+    }
+    float total = 0;
+    cudaEventElapsedTime(&total, evs[0], evs.back());
+    device_ms_ = total;
+    times_pending_ = false;
+    for (auto& e : evs) cudaEventDestroy(e);
+    copy_results(s, stream_);
+    exb_check(exb_ctx_sync_check(ctx_, stream_), "fused forward");
 }
 
 double fused_plan::run_resident(int iters, bool use_graph) {
     if (!built_) return -1.0;
     CUDA_CHECK(cudaSetDevice(device_));
-    ingest_src_ = staging_in_.p;
-    ingest_src_f16_ = false;
-    if (!warmed_) launch_body(false);      // make sure every kernel has run eagerly once
+    program& prog = program_for({N_}, staged_f16_);
+    slice& s = *prog.slices[0];
+    launches_ = prog.launches();
+    if (!s.warmed) launch(s, false);      // make sure every kernel has run eagerly once
     CUDA_CHECK(cudaStreamSynchronize(stream_));
     CUDA_CHECK(cudaEventRecord(ev0_, stream_));
-    for (int i = 0; i < iters; ++i) launch_body(use_graph);
+    for (int i = 0; i < iters; ++i) launch(s, use_graph);
     CUDA_CHECK(cudaEventRecord(ev1_, stream_));
     CUDA_CHECK(cudaStreamSynchronize(stream_));
     float ms = 0;
     cudaEventElapsedTime(&ms, ev0_, ev1_);
+    device_ms_ = ms;
+    times_pending_ = false;
     exb_check(exb_ctx_sync_check(ctx_, stream_), "resident run");
     return ms;
 }
 
-void fused_plan::run_chunked(const float* host_input, int k, bool use_graph, int host_threads, const uint16_t* host_f16) {
-    CUDA_CHECK(cudaSetDevice(device_));
-    CHECK(built_ && k >= 1);
-    const size_t chunk_elems = (size_t)N_ * C_ * H_ * W_;
-    if (host_f16) CHECK(ingest_f16_capable_) << "this plan's ingest step cannot read fp16 planes";
-    const bool convert = !host_f16 && host_threads > 0 && ingest_f16_capable_;
-    const bool f16 = host_f16 != nullptr || convert;
-    float* stage = static_cast<float*>(chunk_stage_.ensure(chunk_elems * 4 * k, device_));
-    uint16_t* stage16 = reinterpret_cast<uint16_t*>(stage);
-    if (convert) {
-        if (host_f16_bytes_ < chunk_elems * 2 * k) {
-            if (host_f16_) cudaFreeHost(host_f16_);
-            host_f16_ = nullptr;
-            CUDA_CHECK(cudaHostAlloc(&host_f16_, chunk_elems * 2 * k, cudaHostAllocDefault));
-            host_f16_bytes_ = chunk_elems * 2 * k;
+// How a forward is divided when the caller leaves it open: the division whose modelled time is shortest.  Copies to the
+// device, kernels and copies back are three lanes that run side by side; a sub-batch passes through them one after the
+// other.  The kernels of n of N images are taken as launches * 4.6 us + body * (n / N)^0.8 (small sub-batches fill the
+// chip less), with the body from the plan's own traffic and arithmetic: within 15 % of the measured time of the
+// benchmark networks from 4 images on.  Copies move 53 GB/s.  Divisions are looked for among all ways to put 16 units
+// together in at most eight parts; one has to promise 3 % and 20 us to be taken.
+std::vector<int> fused_plan::choose_slices(bool f16_src) {
+    const program& prog = program_for({N_}, f16_src);
+    const std::vector<int> undivided{N_};
+    if (prog.uneven || N_ < 2) return undivided;
+    double bytes = 0, out_bytes = 0;
+    for (auto& f : fmaps_) {
+        const double px = (double)f.N * f.H * f.W;
+        if (f.f16) bytes += px * f.cs * 2;
+        if (f.i8) bytes += px * f.cs;
+        for (auto& e : f.extra_i8)
+            if (e) bytes += px * f.cs;
+        if (f.f32) bytes += px * f.C * 4;
+    }
+    for (auto& kv : host_out_) out_bytes += 4.0 * kv.second->count();
+    const double in_us = (double)N_ * C_ * H_ * W_ * (f16_src ? 2 : 4) / 53e3, out_us = out_bytes / 53e3;
+    const double fixed = 4.6 * prog.launches();
+    const double body = 2 * bytes / 4.5e6 + prog.flops_i8 / 1.2e9 + prog.flops_f16 / 0.6e9;
+    constexpr int kUnits = 16, kParts = 8;
+    double kernels[kUnits + 1];
+    for (int u = 0; u <= kUnits; ++u) kernels[u] = fixed + body * std::pow(u / (double)kUnits, 0.8);
+    const double whole = in_us + kernels[kUnits] + out_us;
+    double best = std::min(0.97 * whole, whole - 20.0);
+    std::vector<int> parts, best_parts;
+    const int step = N_ >= kUnits ? 1 : (kUnits + N_ - 1) / N_;      // a unit is at least one image
+    std::function<void(int, double, double, double)> walk = [&](int left, double in, double run, double out) {
+        if (out >= best) return;
+        if (left == 0) {
+            best = out;
+            best_parts = parts;
+            return;
         }
-        if (!pool_ || pool_->threads() != host_threads) pool_.reset(new convert_pool(host_threads));
-    }
-    if (!copy_stream_) CUDA_CHECK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
-    while ((int)copied_.size() < k) {
-        cudaEvent_t e;
-        CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        copied_.push_back(e);
-    }
-    for (auto& kv : host_out_) {
-        auto& t = chunk_out_[kv.first];
-        const std::vector<int> shp = kv.second->data_shape();
-        if (!t || t->num() != shp[0] * k)
-            t = std::shared_ptr<memory::tensor<float>>(
-                new memory::tensor<float>(std::vector<int>{shp[0] * k, shp[1], shp[2], shp[3]}, device_, memory::NCHW, nullptr));
-    }
-    launches_ = 0;
-    for (auto& s : steps_) launches_ += s.launches;
-    launches_ *= k;
-    // every copy is queued at once on its own stream; compute of chunk c waits for copy c only
-    if (!convert) {
-        for (int c = 0; c < k; ++c) {
-            if (host_f16)
-                CUDA_CHECK(cudaMemcpyAsync(stage16 + c * chunk_elems, host_f16 + c * chunk_elems, chunk_elems * 2,
-                                           cudaMemcpyHostToDevice, copy_stream_));
-            else
-                CUDA_CHECK(cudaMemcpyAsync(stage + c * chunk_elems, host_input + c * chunk_elems, chunk_elems * 4,
-                                           cudaMemcpyHostToDevice, copy_stream_));
-            CUDA_CHECK(cudaEventRecord(copied_[c], copy_stream_));
+        if ((int)parts.size() == kParts) return;
+        for (int u = step; u <= left; u += step) {
+            if (left - u > 0 && left - u < step) continue;
+            const double in2 = in + in_us * u / kUnits + 6.0, run2 = std::max(run, in2) + kernels[u] + 4.0;
+            const double out2 = std::max(out, run2) + out_us * u / kUnits + 6.0;
+            parts.push_back(u);
+            walk(left - u, in2, run2, out2);
+            parts.pop_back();
         }
+    };
+    walk(kUnits, 0, 0, 0);
+    if (best_parts.empty()) return undivided;
+    std::vector<int> sizes;
+    int units = 0, done = 0;
+    for (int u : best_parts) {
+        units += u;
+        const int upto = (int)((int64_t)N_ * units / kUnits);
+        if (upto > done) sizes.push_back(upto - done);
+        done = upto;
     }
-    CUDA_CHECK(cudaEventRecord(ev0_, stream_));
-    for (int c = 0; c < k; ++c) {
-        if (convert) {
-            // the host converts chunk c while the copy of chunk c-1 and the kernels of chunk c-2 run
-            uint16_t* h16 = static_cast<uint16_t*>(host_f16_) + c * chunk_elems;
-            pool_->run(host_input + c * chunk_elems, h16, chunk_elems);
-            CUDA_CHECK(cudaMemcpyAsync(stage16 + c * chunk_elems, h16, chunk_elems * 2, cudaMemcpyHostToDevice, copy_stream_));
-            CUDA_CHECK(cudaEventRecord(copied_[c], copy_stream_));
-        }
-        CUDA_CHECK(cudaStreamWaitEvent(stream_, copied_[c], 0));
-        ingest_src_ = f16 ? static_cast<const void*>(stage16 + c * chunk_elems) : static_cast<const void*>(stage + c * chunk_elems);
-        ingest_src_f16_ = f16;
-        launch_body(use_graph);
-        for (auto& kv : host_out_) {
-            fmap_info& f = fmaps_[root(index_[kv.first])];
-            const size_t per = (size_t)f.N * f.C * f.H * f.W;
-            float* dst = chunk_out_[kv.first]->mutable_cpu_data() + c * per;
-            if (f.f32_pitch)
-                CUDA_CHECK(cudaMemcpy2DAsync(dst, (size_t)f.C * 4, f.f32->p, (size_t)f.f32_pitch * 4, (size_t)f.C * 4, f.N,
-                                             cudaMemcpyDeviceToHost, stream_));
-            else
-                CUDA_CHECK(cudaMemcpyAsync(dst, f.f32->p, per * 4, cudaMemcpyDeviceToHost, stream_));
-        }
-    }
-    CUDA_CHECK(cudaEventRecord(ev1_, stream_));
-    CUDA_CHECK(cudaStreamSynchronize(stream_));
-    CUDA_CHECK(cudaStreamSynchronize(copy_stream_));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ev0_, ev1_);
-    device_ms_ = ms;
-    ingest_src_f16_ = false;
-    exb_check(exb_ctx_sync_check(ctx_, stream_), "chunked forward");
+    return sizes;
 }
 
 std::shared_ptr<memory::tensor<float>> fused_plan::fetch(const std::string& name_in) {
@@ -1594,7 +1773,6 @@ public:
         if (input_names_.empty()) LOG(FATAL) << "the graph has no input feature map";
     }
     ~impl() {
-        chunk_plan_.reset();
         plan_.reset();
         if (ctx_) exb_ctx_destroy(ctx_);
     }
@@ -1642,16 +1820,17 @@ public:
     int weights_mem_cost_ = 0;
     bool profile_ = false, fusion_ = true, graph_ = true;
     bool used_fused_ = false;
-    int h2d_chunks_ = 1;
+    int h2d_chunks_ = 0;            // 0: chosen by the plan
     int host_f16_threads_ = 0;
     std::string plan_refused_;      // why this graph's fused plan could not be built (then: op by op for good)
-    bool used_chunked_ = false;
-    std::unique_ptr<fused_plan> chunk_plan_;
     exb_ctx* ctx_ = nullptr;
     std::unique_ptr<fused_plan> plan_;
     std::vector<trace_event> trace_;
     int launches_ = 0;
-    double device_ms_ = 0.0;
+    double device_ms() const {
+        if (!used_fused_) return 0.0;
+        return inner_ ? inner_->device_ms() : (plan_ ? plan_->device_ms() : 0.0);
+    }
 };
 
 template <>
@@ -1740,23 +1919,10 @@ pipeline<float>::result_map pipeline<float>::impl::forward_gpu(const std::shared
         if (why.empty()) try {
             if (input->order() == memory::NHWC) input->convert_order();
             const int N = input->num(), C = input->channels(), H = input->height(), W = input->width();
-            used_chunked_ = false;
-            if ((h2d_chunks_ > 1 || host_f16_threads_ > 0) && !profile_ && N % h2d_chunks_ == 0) {
-                if (!chunk_plan_)
-                    chunk_plan_.reset(new fused_plan(op_params_, operations_, input_names_, output_names_, device_));
-                const int nc = N / h2d_chunks_;
-                if (!chunk_plan_->built_for(nc, C, H, W)) chunk_plan_->build(nc, C, H, W);
-                chunk_plan_->run_chunked(input->cpu_data(), h2d_chunks_, graph_, host_f16_threads_);
-                launches_ = chunk_plan_->launches();
-                device_ms_ = chunk_plan_->device_ms();
-                used_fused_ = true;
-                used_chunked_ = true;
-                return chunk_plan_->chunk_out_;
-            }
             if (!plan_->built_for(N, C, H, W)) plan_->build(N, C, H, W);
-            plan_->run(input->cpu_data(), graph_, profile_, &trace_);
+            if (profile_) plan_->run_profiled(input->cpu_data(), &trace_);
+            else plan_->run(input->cpu_data(), h2d_chunks_, graph_, host_f16_threads_);
             launches_ = plan_->launches();
-            device_ms_ = plan_->device_ms();
             used_fused_ = true;
             return plan_->host_out_;
         } catch (const plan_refusal& e) {
@@ -1764,7 +1930,6 @@ pipeline<float>::result_map pipeline<float>::impl::forward_gpu(const std::shared
             plan_refused_ = e.what();
             why = plan_refused_;
             plan_.reset();
-            chunk_plan_.reset();
         }
         LOG(WARNING) << "running op by op: " << why;
     }
@@ -1777,23 +1942,20 @@ bool pipeline<Dtype>::impl::forward_f16_input(const uint16_t*, int, int, int, in
 template <>
 bool pipeline<float>::impl::forward_f16_input(const uint16_t* host_f16, int N, int C, int H, int W, result_map& out) {
     if (!fusion_ || !plan_refused_.empty()) return false;
-    if (!chunk_plan_) chunk_plan_.reset(new fused_plan(op_params_, operations_, input_names_, output_names_, device_));
-    if (!chunk_plan_->unsupported_reason().empty()) return false;
-    const int k = (h2d_chunks_ > 1 && N % h2d_chunks_ == 0) ? h2d_chunks_ : 1;
+    if (!plan_) plan_.reset(new fused_plan(op_params_, operations_, input_names_, output_names_, device_));
+    if (!plan_->unsupported_reason().empty()) return false;
     try {
-        if (!chunk_plan_->built_for(N / k, C, H, W)) chunk_plan_->build(N / k, C, H, W);
+        if (!plan_->built_for(N, C, H, W)) plan_->build(N, C, H, W);
     } catch (const plan_refusal& e) {
         plan_refused_ = e.what();
-        chunk_plan_.reset();
+        plan_.reset();
         return false;
     }
-    if (!chunk_plan_->host_f16_capable()) return false;
-    chunk_plan_->run_chunked(nullptr, k, graph_, 0, host_f16);
-    launches_ = chunk_plan_->launches();
-    device_ms_ = chunk_plan_->device_ms();
+    if (!plan_->host_f16_capable()) return false;
+    plan_->run(nullptr, h2d_chunks_, graph_, 0, host_f16);
+    launches_ = plan_->launches();
     used_fused_ = true;
-    used_chunked_ = true;
-    out = chunk_plan_->chunk_out_;
+    out = plan_->host_out_;
     return true;
 }
 
@@ -1825,7 +1987,6 @@ pipeline<unsigned short>::result_map pipeline<unsigned short>::impl::forward_gpu
         pipeline<float>::result_map res;
         if (inner_->forward_f16_input(input->cpu_data(), input->num(), input->channels(), input->height(), input->width(), res)) {
             launches_ = inner_->launches_;
-            device_ms_ = inner_->device_ms_;
             used_fused_ = true;
             result_map out;
             for (auto& kv : res) {
@@ -1871,11 +2032,6 @@ std::shared_ptr<memory::tensor<Dtype>> pipeline<Dtype>::impl::get_featmap(std::s
 }
 template <>
 std::shared_ptr<memory::tensor<float>> pipeline<float>::impl::get_featmap(std::string_view name) {
-    if (used_fused_ && used_chunked_ && chunk_plan_) {
-        auto o = chunk_plan_->chunk_out_.find(std::string(name));
-        if (o != chunk_plan_->chunk_out_.end()) return o->second;
-        return chunk_plan_->fetch(std::string(name));
-    }
     if (used_fused_ && plan_) return plan_->fetch(std::string(name));
     auto it = featmap_index_.find(std::string(name));
     if (it == featmap_index_.end()) return nullptr;
@@ -1950,12 +2106,14 @@ template <typename Dtype> void pipeline<Dtype>::disable_profiler() { impl_->prof
 template <typename Dtype> int pipeline<Dtype>::device() const { return impl_->device_; }
 template <typename Dtype> void pipeline<Dtype>::set_fusion(bool on) { impl_->fusion_ = on; }
 template <typename Dtype> void pipeline<Dtype>::set_cuda_graph(bool on) { impl_->graph_ = on; }
-template <typename Dtype> void pipeline<Dtype>::set_h2d_chunks(int k) { impl_->h2d_chunks_ = k < 1 ? 1 : k; }
+template <typename Dtype> void pipeline<Dtype>::set_h2d_chunks(int k) { impl_->h2d_chunks_ = k < 0 ? 0 : k; }
 template <typename Dtype> void pipeline<Dtype>::set_host_f16_threads(int t) { impl_->host_f16_threads_ = t < 0 ? 0 : t; }
 template <typename Dtype> int pipeline<Dtype>::launches_last_forward() const { return impl_->launches_; }
 template <typename Dtype> double pipeline<Dtype>::run_resident(int iters) {
     if (!impl_->plan_ || !impl_->used_fused_ || !impl_->plan_->built()) return -1.0;
-    return impl_->plan_->run_resident(iters, impl_->graph_);
+    const double ms = impl_->plan_->run_resident(iters, impl_->graph_);
+    impl_->launches_ = impl_->plan_->launches();
+    return ms;
 }
 template <typename Dtype> int pipeline<Dtype>::trace_size() const { return (int)impl_->trace_.size(); }
 template <typename Dtype>
@@ -1966,7 +2124,7 @@ bool pipeline<Dtype>::trace_entry(int i, std::string& name, double& b, double& e
     e = impl_->trace_[i].end_ms;
     return true;
 }
-template <typename Dtype> double pipeline<Dtype>::device_ms_last_forward() const { return impl_->device_ms_; }
+template <typename Dtype> double pipeline<Dtype>::device_ms_last_forward() const { return impl_->device_ms(); }
 template <typename Dtype> std::vector<std::string> pipeline<Dtype>::input_names() const { return impl_->input_names_; }
 template <typename Dtype> std::vector<std::string> pipeline<Dtype>::output_names() const { return impl_->output_names_; }
 template <typename Dtype> std::string pipeline<Dtype>::version() { return exb_version(); }

@@ -47,9 +47,10 @@ public:
     int device() const;                  // the device id given at construction (-1 = none)
     void set_fusion(bool on);            // default on for pipeline<float> on a GPU
     void set_cuda_graph(bool on);        // replay the fused plan as a CUDA graph (default on)
-    // forward() of a batch divisible by k runs as k sub-batches: sub-batch c+1 is copied to the device
-    // while sub-batch c is computed (default 1 = whole batch at once).  Only the pipeline outputs
-    // cover the whole batch afterwards; get_featmap() of an inner map sees the last sub-batch.
+    // How forward() divides a batch: sub-batch c + 1 is copied to the device, and sub-batch c - 1 back to the host, while
+    // sub-batch c is computed.  0 (default): the division whose modelled time is shortest, the whole batch at once where
+    // none pays; 1: the whole batch; k: k equal sub-batches where k divides the batch.  Results and feature maps cover
+    // the whole batch either way.
     void set_h2d_chunks(int k);
     // t > 0: the forward converts the input to fp16 on the host with t threads before it is copied (half the
     // PCIe bytes, the same round-to-nearest-even as the device ingest kernel, so identical results); used

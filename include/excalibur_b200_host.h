@@ -38,8 +38,8 @@ EXB_API int exb_host_pipeline_create(const char* phai_text, const char* racy_pat
                                      void** out);
 EXB_API int exb_host_pipeline_destroy(void* p);
 /* key: "fusion" (fused NHWC plan, default 1), "cuda_graph" (default 1), "profile" (0/1 =
- * disable_profiler / enable_profiler, reference pipeline.hpp:38-39), "h2d_chunks" (k sub-batches whose
- * copies overlap the previous sub-batch's kernels, default 1), "host_f16_threads" (t > 0: the input is
+ * disable_profiler / enable_profiler, reference pipeline.hpp:38-39), "h2d_chunks" (k equal sub-batches whose
+ * copies overlap the kernels of their neighbours, 1 = the whole batch at once, default 0 = what pays), "host_f16_threads" (t > 0: the input is
  * converted to fp16 by t host threads before the copy - half the PCIe bytes, identical results; default 0). */
 EXB_API int exb_host_pipeline_set_option(void* p, const char* key, int value);
 /* The host-side fp32 -> fp16 conversion "host_f16_threads" uses (round to nearest even; F16C where the CPU

@@ -415,3 +415,29 @@ def test_pipeline_f16_falls_back_to_op_by_op():
     ref = O.conv2d_f32(f16_round(x), f16_round(w), b, 1, 1, act=1)
     assert out.shape == ref.shape
     assert_close_f16(out, ref, what="fp16 pipeline, op by op")
+
+
+def test_divided_forward_and_pageable_input():
+    """The division of a batch that forward() chooses by itself (uneven sub-batches), and inputs that are staged by the
+    host threads, give what the undivided forward gives; feature maps cover the whole batch."""
+    import torch
+    h = _host()
+    scales = {str(n): np.float32(s) for n, s in zip(G["resnet_scale_names"], G["resnet_scales"])}
+    g, _ = models.resnet18(2, act_scales=scales)
+    x = np.random.default_rng(12).uniform(0, 1, (201, 3, 160, 128)).astype(np.float32)       # 49 MB: several staging halves
+    pinned = torch.from_numpy(x).pin_memory()
+    p = h.Pipeline(g.phai_text(), g.racy_bytes(), 0, fusion=True)
+    p.set_option("h2d_chunks", 1)
+    p.forward_ptr(pinned.data_ptr(), *x.shape)
+    whole, fm, launches = p.get("logits"), p.get("s2b1_out"), p.stats()[0]
+    p.set_option("h2d_chunks", 0)
+    for src in (pinned.data_ptr(), x.ctypes.data):
+        for _ in range(3):      # eager, capture, replay
+            p.forward_ptr(src, *x.shape)
+            np.testing.assert_allclose(p.get("logits"), whole, rtol=2e-5, atol=2e-5)
+        assert p.stats()[0] > launches, "the batch was expected to be divided"
+        np.testing.assert_array_equal(p.get("s2b1_out"), fm)
+    assert p.run_resident(2) > 0 and p.stats()[0] == launches
+    small = np.ascontiguousarray(x[:3])      # one sub-batch from pageable memory, another shape
+    np.testing.assert_allclose(p.forward(small)["logits"], whole[:3], rtol=2e-5, atol=2e-5)
+    p.close()
