@@ -1449,15 +1449,17 @@ void fused_plan::copy_input(const char* src, bool pageable, size_t offset, size_
         CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
         return;
     }
-    constexpr size_t kHalf = 16 << 20, kLeast = 256 << 10;
-    char* pinned = static_cast<char*>(pinned_in(2 * kHalf));
-    for (size_t at = 0; at < bytes; at += kHalf) {      // large inputs go through two halves in turn
-        const int h = half_next_;
+    // large inputs go through two halves in turn; page-locking memory costs a millisecond for every few MB
+    constexpr size_t kMost = 8 << 20, kLeast = 256 << 10;
+    const size_t whole = (size_t)N_ * C_ * H_ * W_ * 4, half_bytes = std::min(kMost, whole);
+    char* pinned = static_cast<char*>(pinned_in(whole > half_bytes ? 2 * half_bytes : half_bytes));
+    for (size_t at = 0; at < bytes; at += half_bytes) {
+        const int h = whole > half_bytes ? half_next_ : 0;
         half_next_ ^= 1;
         if (!half_free_[h]) CUDA_CHECK(cudaEventCreateWithFlags(&half_free_[h], cudaEventDisableTiming));
         else CUDA_CHECK(cudaEventSynchronize(half_free_[h]));
-        char* half = pinned + h * kHalf;
-        const size_t n = std::min(kHalf, bytes - at);
+        char* half = pinned + h * half_bytes;
+        const size_t n = std::min(half_bytes, bytes - at);
         size_t sent = 0;
         host_copy(half, src + at, n, [&](size_t ready) {
             if (ready - sent < kLeast && ready < n) return;
