@@ -131,19 +131,30 @@ def last_error():
 
 
 # ---- torch plumbing ---------------------------------------------------------------------------
+# The operation helpers below are called once per layer by programs that keep their tensors on the device: what they do
+# in Python is paid on every call, so they look modules and types up once and pass plain addresses.
+_TORCH = None
+_DTYPES = {}       # exb dtype -> torch dtype, and back
+
+
 def _torch():
-    import torch
-    return torch
+    global _TORCH
+    if _TORCH is None:
+        import torch
+        _DTYPES.update({EXB_F16: torch.float16, EXB_I8: torch.int8, EXB_F32: torch.float32, EXB_I32: torch.int32})
+        _DTYPES.update({v: k for k, v in list(_DTYPES.items())})
+        _TORCH = torch
+    return _TORCH
 
 
 def torch_dtype(dt):
-    t = _torch()
-    return {EXB_F16: t.float16, EXB_I8: t.int8, EXB_F32: t.float32, EXB_I32: t.int32}[dt]
+    _torch()
+    return _DTYPES[dt]
 
 
 def exb_dtype_of(tensor):
-    t = _torch()
-    return {t.float16: EXB_F16, t.int8: EXB_I8, t.float32: EXB_F32, t.int32: EXB_I32}[tensor.dtype]
+    _torch()
+    return _DTYPES[tensor.dtype]
 
 
 def ptr(t):
@@ -152,6 +163,16 @@ def ptr(t):
 
 def cur_stream():
     return C.c_void_p(_torch().cuda.current_stream().cuda_stream)
+
+
+def _address(t):
+    return t.data_ptr() if t is not None else None
+
+
+def _stream():
+    """Handle of the current stream of the current device as an integer (the Stream object costs 2 us)."""
+    c = _torch()._C
+    return c._cuda_getCurrentRawStream(c._cuda_getDevice())
 
 
 def _np_ptr(a):
@@ -247,15 +268,18 @@ def conv_out_dims(desc):
 
 def conv2d(ctx, desc, x, weights, residual=None, y=None, y2=None):
     """x: NHWC torch tensor on the context's device.  Returns (y, y2)."""
-    t = _torch()
-    oh, ow = conv_out_dims(desc)
-    cs = desc.cout_stride or desc.Cout
-    if y is None:
-        y = t.empty((desc.N, oh, ow, cs), dtype=torch_dtype(desc.out_dtype), device=x.device)
-    if desc.out2_dtype != -1 and y2 is None:
-        y2 = t.empty((desc.N, oh, ow, cs), dtype=torch_dtype(desc.out2_dtype), device=x.device)
-    check(lib().exb_conv2d_fwd(ctx.handle, C.byref(desc), ptr(x), weights.handle, ptr(residual), ptr(y),
-                               ptr(y2), cur_stream()))
+    _torch()
+    two = desc.out2_dtype != -1
+    if y is None or (two and y2 is None):
+        oh, ow = conv_out_dims(desc)
+        shape = (desc.N, oh, ow, desc.cout_stride or desc.Cout)
+        if y is None:
+            y = x.new_empty(shape, dtype=_DTYPES[desc.out_dtype])
+        if two and y2 is None:
+            y2 = x.new_empty(shape, dtype=_DTYPES[desc.out2_dtype])
+    rc = lib().exb_conv2d_fwd(ctx._h, C.byref(desc), x.data_ptr(), weights._h, _address(residual), y.data_ptr(), _address(y2), _stream())
+    if rc:
+        check(rc)
     return y, y2
 
 
@@ -296,13 +320,15 @@ def make_dw_desc(N, H, W, Cc, k=3, stride=1, pad=1, in_dtype=EXB_F16, out_dtype=
 
 
 def dwconv2d(ctx, desc, x, weights, y=None):
-    t = _torch()
+    _torch()
     oh = (desc.H + desc.pad_t + desc.pad_b - desc.kh) // desc.stride_h + 1
     ow = (desc.W + desc.pad_l + desc.pad_r - desc.kw) // desc.stride_w + 1
     cs = desc.c_stride or desc.C
     if y is None:
-        y = t.empty((desc.N, oh, ow, cs), dtype=torch_dtype(desc.out_dtype), device=x.device)
-    check(lib().exb_dwconv2d_fwd(ctx.handle, C.byref(desc), ptr(x), weights.handle, ptr(y), cur_stream()))
+        y = x.new_empty((desc.N, oh, ow, cs), dtype=_DTYPES[desc.out_dtype])
+    rc = lib().exb_dwconv2d_fwd(ctx._h, C.byref(desc), x.data_ptr(), weights._h, y.data_ptr(), _stream())
+    if rc:
+        check(rc)
     return y
 
 
@@ -323,13 +349,17 @@ def pool_out_dims(desc):
 
 def pool2d(ctx, desc, x, y=None, y2=None):
     t = _torch()
-    ph, pw = pool_out_dims(desc)
-    cs = desc.c_stride or desc.C
-    if y is None:
-        y = t.empty((desc.N, ph, pw, cs), dtype=x.dtype, device=x.device)
-    if desc.out2_dtype != -1 and y2 is None:
-        y2 = t.empty((desc.N, ph, pw, cs), dtype=t.int8, device=x.device)
-    check(lib().exb_pool2d_fwd(ctx.handle, C.byref(desc), ptr(x), ptr(y), ptr(y2), cur_stream()))
+    two = desc.out2_dtype != -1
+    if y is None or (two and y2 is None):
+        ph, pw = pool_out_dims(desc)
+        shape = (desc.N, ph, pw, desc.c_stride or desc.C)
+        if y is None:
+            y = x.new_empty(shape)
+        if two and y2 is None:
+            y2 = x.new_empty(shape, dtype=t.int8)
+    rc = lib().exb_pool2d_fwd(ctx._h, C.byref(desc), x.data_ptr(), y.data_ptr(), _address(y2), _stream())
+    if rc:
+        check(rc)
     return y, y2
 
 
