@@ -113,9 +113,30 @@ inline int launch_pdl(const exb_ctx* ctx, const char* what, void (*kern)(KArgs..
                       Args&&... args) {
     return launch_pdl_cluster(ctx, what, kern, grid, block, dim3(1), smem, st, static_cast<Args&&>(args)...);
 }
+// The same where the caller checks with after_launch() itself.
+template <typename... KArgs, typename... Args>
+inline void launch_overlapped(const exb_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx->pdl ? 1 : 0;
+    (void)cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
 // Let the next kernel of the stream be scheduled as soon as SMs free up / wait for the previous one's memory.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Both, for kernels with nothing to do before the previous one is complete: they still gain the launch itself, 2 us of a
+// small kernel's 4-8.
+__device__ __forceinline__ void pdl_enter() {
+    pdl_launch_dependents();
+    pdl_wait();
+}
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 

@@ -21,6 +21,7 @@ struct ConcatArgs {
 // width, stride and offset is a multiple of 16 bytes, else one element).
 template <typename U>
 __global__ void __launch_bounds__(kThreads) concat_rows_kernel(ConcatArgs a, U* y, int64_t y_stride, int64_t rows) {
+    pdl_enter();
     const int64_t total = a.offset[a.n_in];
     const int64_t work = rows * total;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(kThreads) concat_rows_kernel(ConcatArgs a, U* 
 template <typename U>
 __global__ void __launch_bounds__(kThreads) interp_nearest_nhwc_kernel(const U* x, U* y, int N, int H, int W, int cs,
                                                                        int OH, int OW, float hs, float ws) {
+    pdl_enter();
     const int64_t work = (int64_t)N * OH * OW * cs;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < work; i += step) {
@@ -54,6 +56,7 @@ __global__ void __launch_bounds__(kThreads) interp_nearest_nhwc_kernel(const U* 
 
 __global__ void __launch_bounds__(kThreads) interp_nearest_nchw_kernel(const float* x, float* y, int planes, int H, int W,
                                                                        int OH, int OW, float hs, float ws) {
+    pdl_enter();
     const int64_t work = (int64_t)planes * OH * OW;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < work; i += step) {
@@ -71,6 +74,7 @@ __global__ void __launch_bounds__(kThreads) interp_nearest_nchw_kernel(const flo
 template <typename T>
 __global__ void __launch_bounds__(kThreads) focus_kernel(const T* __restrict__ x, T* __restrict__ y, int N, int C, int H,
                                                          int W, int in_stride, int out_stride, int channel_last) {
+    pdl_enter();
     const int OH = H / 2, OW = W / 2, OC = 4 * C;
     const int ocs = channel_last ? out_stride : OC;
     const int64_t work = (int64_t)N * OH * OW * ocs;
@@ -115,6 +119,7 @@ __global__ void __launch_bounds__(kThreads) channel_affine_kernel(const T* x, T*
                                                                   int64_t count, int C, int cs, int64_t inner,
                                                                   int channel_last, int act, const float* slope,
                                                                   int n_slope) {
+    pdl_enter();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) {
         const int c = channel_last ? (int)(i % cs) : (int)((i / inner) % C);
@@ -138,6 +143,7 @@ __global__ void __launch_bounds__(kThreads) channel_affine_nhwc_f16x8_kernel(con
                                                                              const float* add, const float* slope,
                                                                              int n_slope, int act, int64_t nvec, int C,
                                                                              int cs8) {
+    pdl_enter();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     const bool fixed = step % cs8 == 0;
     float m[8], a[8], sl[8];
@@ -202,6 +208,7 @@ __global__ void __launch_bounds__(kThreads) channel_affine_nhwc_f16x8_kernel(con
 __global__ void __launch_bounds__(kThreads) binary_bcast_nhwc_f16x8_kernel(const uint4* a, const uint4* b, uint4* y, int64_t nvec,
                                                                            int C, int cs8, int64_t vec_per_image, int op,
                                                                            int b_batch, int b_first) {
+    pdl_enter();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += step) {
         const int cv = (int)(i % cs8);
@@ -229,6 +236,7 @@ __global__ void __launch_bounds__(kThreads) binary_bcast_nhwc_f16x8_kernel(const
 template <typename T>
 __global__ void __launch_bounds__(kThreads) prelu_kernel(const T* x, T* y, const float* slope, int n_slope, int64_t count,
                                                          int C, int cs, int64_t inner, int channel_last) {
+    pdl_enter();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) {
         const int c = channel_last ? (int)(i % cs) : (int)((i / inner) % C);
@@ -246,6 +254,7 @@ __global__ void __launch_bounds__(kThreads) prelu_kernel(const T* x, T* y, const
 template <typename U>
 __global__ void __launch_bounds__(kThreads) depth_to_space_kernel(const U* __restrict__ x, U* __restrict__ y, int N, int H,
                                                                   int W, int rh, int rw, int C, int xs, int ys) {
+    pdl_enter();
     const int OH = H * rh, OW = W * rw;
     const int64_t work = (int64_t)N * OH * OW * ys;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -271,6 +280,7 @@ template <bool kGather>
 __global__ void __launch_bounds__(kThreads) depth_to_space_f16x8_kernel(const __half* __restrict__ x, uint4* __restrict__ y,
                                                                         int N, int H, int W, int rh, int rw, int C, int xs,
                                                                         int ys8) {
+    pdl_enter();
     const int OH = H * rh, OW = W * rw;
     const int64_t work = (int64_t)N * OH * OW * ys8;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -299,6 +309,7 @@ __global__ void __launch_bounds__(kThreads) depth_to_space_f16x8_kernel(const __
 // y[p][w][h] = x[p][h][w] for every plane p; 32x32 tiles through shared memory.
 __global__ void __launch_bounds__(256) transpose_planes_f32_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                                    int H, int W) {
+    pdl_enter();
     __shared__ float tile[32][33];
     const int64_t plane = blockIdx.z;
     const float* xp = x + plane * (int64_t)H * W;
@@ -319,6 +330,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) binary_bcast_kernel(const T* a, const T* b, T* y, int64_t count, int C, int cs,
                                                                 int64_t inner, int channel_last, int op, int b_batch,
                                                                 int b_first) {
+    pdl_enter();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     const int64_t per_image = channel_last ? inner * cs : inner * C;
     const int bcs = channel_last ? cs : C;
@@ -339,6 +351,7 @@ __global__ void __launch_bounds__(kThreads) binary_bcast_kernel(const T* a, cons
 // One thread per (n, p); C is small (class scores).  x may have a padded image stride.
 __global__ void __launch_bounds__(kThreads) softmax_channels_kernel(const float* __restrict__ x, float* __restrict__ y, int N,
                                                                     int C, int64_t inner, int64_t x_image_stride) {
+    pdl_enter();
     const int64_t total = (int64_t)N * inner;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
@@ -364,6 +377,7 @@ __global__ void __launch_bounds__(kThreads) softmax_channels_kernel(const float*
 // floats; channel -> (a, k) with a float reciprocal, exact for the few hundred channels of a head.
 __global__ void __launch_bounds__(kThreads) split_heads_kernel(const __half* __restrict__ x, float* __restrict__ y, int64_t rows,
                                                                int P, int cs, int A, int K) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const float inv_k = 1.0f / (float)K;
@@ -387,6 +401,7 @@ __global__ void __launch_bounds__(kThreads) split_heads_kernel(const __half* __r
 // value, the output column fastest: writes are contiguous, reads of neighbouring threads fall into the same pixel.
 __global__ void __launch_bounds__(kThreads) depth_to_space_nchw_f32_kernel(const __half* __restrict__ x, float* __restrict__ y,
                                                                            int N, int H, int W, int rh, int rw, int C, int xs) {
+    pdl_enter();
     const int OH = H * rh, OW = W * rw;
     const int64_t work = (int64_t)N * C * OH * OW;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -454,12 +469,12 @@ extern "C" int exb_concat_fwd(exb_ctx* ctx, int n_in, const void* const* xs, con
         for (int i = 0; i < n_in; ++i) { a.width[i] /= per; a.stride[i] /= per; a.offset[i] /= per; }
         for (int i = n_in; i <= kMaxConcatInputs; ++i) a.offset[i] = off / per;
         int grid = stream_grid(ctx, rows * (off / per), kThreads);
-        concat_rows_kernel<uint4><<<grid, kThreads, 0, st>>>(a, static_cast<uint4*>(y), y_stride / per, rows);
+        launch_overlapped(ctx, concat_rows_kernel<uint4>, grid, kThreads, st, a, static_cast<uint4*>(y), y_stride / per, rows);
     } else {
         int grid = stream_grid(ctx, rows * off, kThreads);
-        if (es == 1) concat_rows_kernel<uint8_t><<<grid, kThreads, 0, st>>>(a, static_cast<uint8_t*>(y), y_stride, rows);
-        else if (es == 2) concat_rows_kernel<uint16_t><<<grid, kThreads, 0, st>>>(a, static_cast<uint16_t*>(y), y_stride, rows);
-        else concat_rows_kernel<uint32_t><<<grid, kThreads, 0, st>>>(a, static_cast<uint32_t*>(y), y_stride, rows);
+        if (es == 1) launch_overlapped(ctx, concat_rows_kernel<uint8_t>, grid, kThreads, st, a, static_cast<uint8_t*>(y), y_stride, rows);
+        else if (es == 2) launch_overlapped(ctx, concat_rows_kernel<uint16_t>, grid, kThreads, st, a, static_cast<uint16_t*>(y), y_stride, rows);
+        else launch_overlapped(ctx, concat_rows_kernel<uint32_t>, grid, kThreads, st, a, static_cast<uint32_t*>(y), y_stride, rows);
     }
     return after_launch("exb_concat_fwd");
 }
@@ -478,7 +493,7 @@ extern "C" int exb_interp_nearest_fwd(exb_ctx* ctx, const void* x, void* y, int 
         const int64_t planes = (int64_t)N * C;
         EXB_REQUIRE(planes < (1ll << 31), "exb_interp_nearest_fwd: too many planes");
         int grid = stream_grid(ctx, planes * OH * OW, kThreads);
-        interp_nearest_nchw_kernel<<<grid, kThreads, 0, st>>>(static_cast<const float*>(x), static_cast<float*>(y),
+        launch_overlapped(ctx, interp_nearest_nchw_kernel, grid, kThreads, st, static_cast<const float*>(x), static_cast<float*>(y),
                                                               (int)planes, H, W, OH, OW, hs, ws);
         return after_launch("exb_interp_nearest_fwd");
     }
@@ -489,18 +504,18 @@ extern "C" int exb_interp_nearest_fwd(exb_ctx* ctx, const void* x, void* y, int 
     if ((cs * es) % 16 == 0 && aligned16(x) && aligned16(y)) {
         const int v = (int)(cs * es / 16);
         int grid = stream_grid(ctx, (int64_t)N * OH * OW * v, kThreads);
-        interp_nearest_nhwc_kernel<uint4><<<grid, kThreads, 0, st>>>(static_cast<const uint4*>(x), static_cast<uint4*>(y),
+        launch_overlapped(ctx, interp_nearest_nhwc_kernel<uint4>, grid, kThreads, st, static_cast<const uint4*>(x), static_cast<uint4*>(y),
                                                                      N, H, W, v, OH, OW, hs, ws);
     } else {
         int grid = stream_grid(ctx, (int64_t)N * OH * OW * cs, kThreads);
         if (es == 1)
-            interp_nearest_nhwc_kernel<uint8_t><<<grid, kThreads, 0, st>>>(static_cast<const uint8_t*>(x),
+            launch_overlapped(ctx, interp_nearest_nhwc_kernel<uint8_t>, grid, kThreads, st, static_cast<const uint8_t*>(x),
                                                                            static_cast<uint8_t*>(y), N, H, W, cs, OH, OW, hs, ws);
         else if (es == 2)
-            interp_nearest_nhwc_kernel<uint16_t><<<grid, kThreads, 0, st>>>(static_cast<const uint16_t*>(x),
+            launch_overlapped(ctx, interp_nearest_nhwc_kernel<uint16_t>, grid, kThreads, st, static_cast<const uint16_t*>(x),
                                                                             static_cast<uint16_t*>(y), N, H, W, cs, OH, OW, hs, ws);
         else
-            interp_nearest_nhwc_kernel<uint32_t><<<grid, kThreads, 0, st>>>(static_cast<const uint32_t*>(x),
+            launch_overlapped(ctx, interp_nearest_nhwc_kernel<uint32_t>, grid, kThreads, st, static_cast<const uint32_t*>(x),
                                                                             static_cast<uint32_t*>(y), N, H, W, cs, OH, OW, hs, ws);
     }
     return after_launch("exb_interp_nearest_fwd");
@@ -523,15 +538,15 @@ extern "C" int exb_focus_fwd(exb_ctx* ctx, const void* x, void* y, int N, int C,
     const int grid = stream_grid(ctx, work, kThreads);
     switch (dtype) {
     case EXB_F32:
-        focus_kernel<float><<<grid, kThreads, 0, st>>>(static_cast<const float*>(x), static_cast<float*>(y), N, C, H, W,
+        launch_overlapped(ctx, focus_kernel<float>, grid, kThreads, st, static_cast<const float*>(x), static_cast<float*>(y), N, C, H, W,
                                                        in_stride, out_stride, channel_last);
         break;
     case EXB_F16:
-        focus_kernel<uint16_t><<<grid, kThreads, 0, st>>>(static_cast<const uint16_t*>(x), static_cast<uint16_t*>(y), N, C, H,
+        launch_overlapped(ctx, focus_kernel<uint16_t>, grid, kThreads, st, static_cast<const uint16_t*>(x), static_cast<uint16_t*>(y), N, C, H,
                                                           W, in_stride, out_stride, channel_last);
         break;
     case EXB_I8:
-        focus_kernel<uint8_t><<<grid, kThreads, 0, st>>>(static_cast<const uint8_t*>(x), static_cast<uint8_t*>(y), N, C, H, W,
+        launch_overlapped(ctx, focus_kernel<uint8_t>, grid, kThreads, st, static_cast<const uint8_t*>(x), static_cast<uint8_t*>(y), N, C, H, W,
                                                          in_stride, out_stride, channel_last);
         break;
     default: return fail(EXB_ERR_UNSUPPORTED, "exb_focus_fwd: dtype %d", dtype);
@@ -556,16 +571,16 @@ static int channel_affine_impl(exb_ctx* ctx, const void* x, void* y, const float
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == EXB_F16 && channel_last && cs % 8 == 0 && aligned16(x) && aligned16(y)) {
         const int64_t nvec = count / 8;
-        channel_affine_nhwc_f16x8_kernel<<<slice_grid(ctx, nvec, cs / 8), kThreads, 0, st>>>(
+        launch_overlapped(ctx, channel_affine_nhwc_f16x8_kernel, slice_grid(ctx, nvec, cs / 8), kThreads, st, 
             static_cast<const uint4*>(x), static_cast<uint4*>(y), mul, add, slope, n_slope, act, nvec, C, cs / 8);
         return after_launch(what);
     }
     int grid = stream_grid(ctx, count, kThreads);
     if (dtype == EXB_F16)
-        channel_affine_kernel<__half><<<grid, kThreads, 0, st>>>(static_cast<const __half*>(x), static_cast<__half*>(y), mul,
+        launch_overlapped(ctx, channel_affine_kernel<__half>, grid, kThreads, st, static_cast<const __half*>(x), static_cast<__half*>(y), mul,
                                                                  add, count, C, cs, inner, channel_last, act, slope, n_slope);
     else
-        channel_affine_kernel<float><<<grid, kThreads, 0, st>>>(static_cast<const float*>(x), static_cast<float*>(y), mul,
+        launch_overlapped(ctx, channel_affine_kernel<float>, grid, kThreads, st, static_cast<const float*>(x), static_cast<float*>(y), mul,
                                                                 add, count, C, cs, inner, channel_last, act, slope, n_slope);
     return after_launch(what);
 }
@@ -601,16 +616,16 @@ extern "C" int exb_prelu_fwd(exb_ctx* ctx, const void* x, void* y, const float* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == EXB_F16 && channel_last && cs % 8 == 0 && aligned16(x) && aligned16(y)) {
         const int64_t nvec = count / 8;
-        channel_affine_nhwc_f16x8_kernel<<<slice_grid(ctx, nvec, cs / 8), kThreads, 0, st>>>(
+        launch_overlapped(ctx, channel_affine_nhwc_f16x8_kernel, slice_grid(ctx, nvec, cs / 8), kThreads, st, 
             static_cast<const uint4*>(x), static_cast<uint4*>(y), nullptr, nullptr, slope, n_slope, EXB_ACT_NONE, nvec, C, cs / 8);
         return after_launch("exb_prelu_fwd");
     }
     int grid = stream_grid(ctx, count, kThreads);
     if (dtype == EXB_F16)
-        prelu_kernel<__half><<<grid, kThreads, 0, st>>>(static_cast<const __half*>(x), static_cast<__half*>(y), slope, n_slope,
+        launch_overlapped(ctx, prelu_kernel<__half>, grid, kThreads, st, static_cast<const __half*>(x), static_cast<__half*>(y), slope, n_slope,
                                                         count, C, cs, inner, channel_last);
     else
-        prelu_kernel<float><<<grid, kThreads, 0, st>>>(static_cast<const float*>(x), static_cast<float*>(y), slope, n_slope,
+        launch_overlapped(ctx, prelu_kernel<float>, grid, kThreads, st, static_cast<const float*>(x), static_cast<float*>(y), slope, n_slope,
                                                        count, C, cs, inner, channel_last);
     return after_launch("exb_prelu_fwd");
 }
@@ -631,19 +646,19 @@ extern "C" int exb_depth_to_space_fwd(exb_ctx* ctx, const void* x, void* y, int 
         const bool whole = C % 8 == 0 && xs % 8 == 0 && aligned16(x);
         const int g8 = stream_grid(ctx, work / 8, kThreads);
         if (whole)
-            depth_to_space_f16x8_kernel<false><<<g8, kThreads, 0, st>>>(static_cast<const __half*>(x), static_cast<uint4*>(y), N, H,
+            launch_overlapped(ctx, depth_to_space_f16x8_kernel<false>, g8, kThreads, st, static_cast<const __half*>(x), static_cast<uint4*>(y), N, H,
                                                                         W, rh, rw, C, xs, ys / 8);
         else
-            depth_to_space_f16x8_kernel<true><<<g8, kThreads, 0, st>>>(static_cast<const __half*>(x), static_cast<uint4*>(y), N, H,
+            launch_overlapped(ctx, depth_to_space_f16x8_kernel<true>, g8, kThreads, st, static_cast<const __half*>(x), static_cast<uint4*>(y), N, H,
                                                                        W, rh, rw, C, xs, ys / 8);
         return after_launch("exb_depth_to_space_fwd");
     }
     int grid = stream_grid(ctx, work, kThreads);
     if (es == 2)
-        depth_to_space_kernel<uint16_t><<<grid, kThreads, 0, st>>>(static_cast<const uint16_t*>(x), static_cast<uint16_t*>(y),
+        launch_overlapped(ctx, depth_to_space_kernel<uint16_t>, grid, kThreads, st, static_cast<const uint16_t*>(x), static_cast<uint16_t*>(y),
                                                                    N, H, W, rh, rw, C, xs, ys);
     else
-        depth_to_space_kernel<uint32_t><<<grid, kThreads, 0, st>>>(static_cast<const uint32_t*>(x), static_cast<uint32_t*>(y),
+        launch_overlapped(ctx, depth_to_space_kernel<uint32_t>, grid, kThreads, st, static_cast<const uint32_t*>(x), static_cast<uint32_t*>(y),
                                                                    N, H, W, rh, rw, C, xs, ys);
     return after_launch("exb_depth_to_space_fwd");
 }
@@ -658,7 +673,7 @@ extern "C" int exb_transpose_hw_f32(exb_ctx* ctx, const float* x, float* y, int6
     for (int64_t p0 = 0; p0 < planes; p0 += 65535) {
         const int64_t np = planes - p0 < 65535 ? planes - p0 : 65535;
         dim3 grid((W + 31) / 32, (H + 31) / 32, (unsigned)np);
-        transpose_planes_f32_kernel<<<grid, 256, 0, st>>>(x + p0 * (int64_t)H * W, y + p0 * (int64_t)H * W, H, W);
+        launch_overlapped(ctx, transpose_planes_f32_kernel, grid, 256, st, x + p0 * (int64_t)H * W, y + p0 * (int64_t)H * W, H, W);
     }
     return after_launch("exb_transpose_hw_f32");
 }
@@ -680,18 +695,18 @@ extern "C" int exb_binaryop_channel_bcast_fwd(exb_ctx* ctx, int op, const void* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == EXB_F16 && channel_last && cs % 8 == 0 && aligned16(a) && aligned16(b) && aligned16(y)) {
         const int64_t nvec = count / 8;
-        binary_bcast_nhwc_f16x8_kernel<<<stream_grid(ctx, nvec, kThreads), kThreads, 0, st>>>(
+        launch_overlapped(ctx, binary_bcast_nhwc_f16x8_kernel, stream_grid(ctx, nvec, kThreads), kThreads, st, 
             static_cast<const uint4*>(a), static_cast<const uint4*>(b), static_cast<uint4*>(y), nvec, C, cs / 8, inner * (cs / 8), op,
             b_batch, b_first);
         return after_launch("exb_binaryop_channel_bcast_fwd");
     }
     const int grid = stream_grid(ctx, count, kThreads);
     if (dtype == EXB_F16)
-        binary_bcast_kernel<__half><<<grid, kThreads, 0, st>>>(static_cast<const __half*>(a), static_cast<const __half*>(b),
+        launch_overlapped(ctx, binary_bcast_kernel<__half>, grid, kThreads, st, static_cast<const __half*>(a), static_cast<const __half*>(b),
                                                                static_cast<__half*>(y), count, C, cs, inner, channel_last, op, b_batch,
                                                                b_first);
     else
-        binary_bcast_kernel<float><<<grid, kThreads, 0, st>>>(static_cast<const float*>(a), static_cast<const float*>(b),
+        launch_overlapped(ctx, binary_bcast_kernel<float>, grid, kThreads, st, static_cast<const float*>(a), static_cast<const float*>(b),
                                                               static_cast<float*>(y), count, C, cs, inner, channel_last, op, b_batch,
                                                               b_first);
     return after_launch("exb_binaryop_channel_bcast_fwd");
@@ -705,7 +720,7 @@ extern "C" int exb_softmax_channels_f32(exb_ctx* ctx, const float* x, float* y, 
     EXB_REQUIRE(x_image_stride >= (int64_t)C * inner, "exb_softmax_channels_f32: image stride smaller than an image");
     if (N == 0) return EXB_OK;
     EXB_REQUIRE(x && y && x != y, "exb_softmax_channels_f32: null or aliased buffer");
-    softmax_channels_kernel<<<stream_grid(ctx, (int64_t)N * inner, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_overlapped(ctx, softmax_channels_kernel, stream_grid(ctx, (int64_t)N * inner, kThreads), kThreads, static_cast<cudaStream_t>(stream), 
         x, y, N, C, inner, x_image_stride);
     return after_launch("exb_softmax_channels_f32");
 }
@@ -719,7 +734,7 @@ extern "C" int exb_nhwc_f16_split_heads_f32(exb_ctx* ctx, const void* x, float* 
     EXB_REQUIRE(x && y, "exb_nhwc_f16_split_heads_f32: null buffer");
     EXB_REQUIRE(A * K <= 65536, "exb_nhwc_f16_split_heads_f32: %d channels", A * K);
     const int64_t rows = (int64_t)N * P;
-    split_heads_kernel<<<stream_grid(ctx, rows * 32, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_overlapped(ctx, split_heads_kernel, stream_grid(ctx, rows * 32, kThreads), kThreads, static_cast<cudaStream_t>(stream), 
         static_cast<const __half*>(x), y, rows, P, c_stride, A, K);
     return after_launch("exb_nhwc_f16_split_heads_f32");
 }
@@ -733,7 +748,7 @@ extern "C" int exb_depth_to_space_nchw_f32(exb_ctx* ctx, const void* x, float* y
     const int64_t work = (int64_t)N * C * H * rh * W * rw;
     if (work == 0) return EXB_OK;
     EXB_REQUIRE(x && y, "exb_depth_to_space_nchw_f32: null buffer");
-    depth_to_space_nchw_f32_kernel<<<stream_grid(ctx, work, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_overlapped(ctx, depth_to_space_nchw_f32_kernel, stream_grid(ctx, work, kThreads), kThreads, static_cast<cudaStream_t>(stream), 
         static_cast<const __half*>(x), y, N, H, W, rh, rw, C, xs);
     return after_launch("exb_depth_to_space_nchw_f32");
 }

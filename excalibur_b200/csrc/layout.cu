@@ -21,6 +21,7 @@ template <> __device__ __forceinline__ float cvt_out<float>(float v, float, int)
 template <typename Out>
 __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const float* __restrict__ x, Out* __restrict__ y,
                                                            int C, int HW, int c_stride, float scale, int rounding) {
+    pdl_enter();
     __shared__ float tile[kTile][kTile + 1];
     const int n = blockIdx.z;
     const int hw0 = blockIdx.x * kTile, c0 = blockIdx.y * kTile;
@@ -46,6 +47,7 @@ template <> __device__ __forceinline__ float cvt_in<float>(float v, float) { ret
 template <typename In>
 __global__ void __launch_bounds__(256) nhwc_to_nchw_kernel(const In* __restrict__ x, float* __restrict__ y,
                                                            int C, int HW, int c_stride, float scale) {
+    pdl_enter();
     __shared__ float tile[kTile][kTile + 1];
     const int n = blockIdx.z;
     const int hw0 = blockIdx.x * kTile, c0 = blockIdx.y * kTile;
@@ -66,6 +68,7 @@ __global__ void __launch_bounds__(256) nhwc_to_nchw_kernel(const In* __restrict_
 template <typename In>
 __global__ void __launch_bounds__(256) nhwc_to_nchw_fewc_kernel(const In* __restrict__ x, float* __restrict__ y, int N,
                                                                 int C, int HW, int c_stride, float scale) {
+    pdl_enter();
     const int64_t total = (int64_t)N * HW;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t n = i / HW, hw = i - n * HW;
@@ -81,6 +84,7 @@ template <typename Out, int CS>
 __global__ void __launch_bounds__(256) nchw_to_nhwc_padded_kernel(const float* __restrict__ x, Out* __restrict__ y,
                                                                   int N, int C, int H, int W, int w_pad, int w_pitch,
                                                                   float scale, int rounding) {
+    pdl_enter();
     const int64_t total = (int64_t)N * H * w_pitch;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int wp = (int)(i % w_pitch);
@@ -113,6 +117,7 @@ template <typename Out, int CS>
 __global__ void __launch_bounds__(256) image_to_nhwc_kernel(const float* __restrict__ x, Out* __restrict__ y, int N, int C,
                                                             int64_t HW, const float* __restrict__ mul,
                                                             const float* __restrict__ add, float scale, int rounding) {
+    pdl_enter();
     const int64_t total = (int64_t)N * HW;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t n = i / HW, hw = i - n * HW;
@@ -142,6 +147,7 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc4_f16_quad_kernel(const float
                                                                      int C, int H, int W, int w_pad, int w_pitch,
                                                                      int64_t rows, const float* __restrict__ mul,
                                                                      const float* __restrict__ add) {
+    pdl_enter();
     const int quads = w_pitch >> 2;
     const int64_t plane = (int64_t)H * W;
     for (int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; row < rows; row += (int64_t)gridDim.x * blockDim.y) {
@@ -183,6 +189,7 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc4_f16_quad_kernel(const float
 __global__ void __launch_bounds__(256) nchw_f16_to_nhwc4_f16_quad_kernel(const __half* __restrict__ x, __half* __restrict__ y,
                                                                          int C, int H, int W, int w_pad, int w_pitch,
                                                                          int64_t rows) {
+    pdl_enter();
     const int quads = w_pitch >> 2;
     const int64_t plane = (int64_t)H * W;
     for (int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; row < rows; row += (int64_t)gridDim.x * blockDim.y) {
@@ -233,9 +240,9 @@ extern "C" int exb_nchw_f32_to_nhwc(exb_ctx* ctx, const float* x, void* y, int d
     dim3 grid((HW + kTile - 1) / kTile, (c_stride + kTile - 1) / kTile, N), block(kTile, 8);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     switch (dtype) {
-    case EXB_F16: nchw_to_nhwc_kernel<__half><<<grid, block, 0, st>>>(x, static_cast<__half*>(y), C, HW, c_stride, scale, rounding); break;
-    case EXB_I8: nchw_to_nhwc_kernel<int8_t><<<grid, block, 0, st>>>(x, static_cast<int8_t*>(y), C, HW, c_stride, scale, rounding); break;
-    case EXB_F32: nchw_to_nhwc_kernel<float><<<grid, block, 0, st>>>(x, static_cast<float*>(y), C, HW, c_stride, scale, rounding); break;
+    case EXB_F16: launch_overlapped(ctx, nchw_to_nhwc_kernel<__half>, grid, block, st, x, static_cast<__half*>(y), C, HW, c_stride, scale, rounding); break;
+    case EXB_I8: launch_overlapped(ctx, nchw_to_nhwc_kernel<int8_t>, grid, block, st, x, static_cast<int8_t*>(y), C, HW, c_stride, scale, rounding); break;
+    case EXB_F32: launch_overlapped(ctx, nchw_to_nhwc_kernel<float>, grid, block, st, x, static_cast<float*>(y), C, HW, c_stride, scale, rounding); break;
     default: return fail(EXB_ERR_UNSUPPORTED, "exb_nchw_f32_to_nhwc: dtype %d", dtype);
     }
     return after_launch("nchw_to_nhwc_kernel");
@@ -252,17 +259,17 @@ extern "C" int exb_nhwc_to_nchw_f32(exb_ctx* ctx, const void* x, int dtype, floa
     if (C <= 8) {
         const int g = stream_grid(ctx, (int64_t)N * HW, 256);
         switch (dtype) {
-        case EXB_F16: nhwc_to_nchw_fewc_kernel<__half><<<g, 256, 0, st>>>(static_cast<const __half*>(x), y, N, C, HW, c_stride, scale); break;
-        case EXB_I8: nhwc_to_nchw_fewc_kernel<int8_t><<<g, 256, 0, st>>>(static_cast<const int8_t*>(x), y, N, C, HW, c_stride, scale); break;
-        case EXB_F32: nhwc_to_nchw_fewc_kernel<float><<<g, 256, 0, st>>>(static_cast<const float*>(x), y, N, C, HW, c_stride, scale); break;
+        case EXB_F16: launch_overlapped(ctx, nhwc_to_nchw_fewc_kernel<__half>, g, 256, st, static_cast<const __half*>(x), y, N, C, HW, c_stride, scale); break;
+        case EXB_I8: launch_overlapped(ctx, nhwc_to_nchw_fewc_kernel<int8_t>, g, 256, st, static_cast<const int8_t*>(x), y, N, C, HW, c_stride, scale); break;
+        case EXB_F32: launch_overlapped(ctx, nhwc_to_nchw_fewc_kernel<float>, g, 256, st, static_cast<const float*>(x), y, N, C, HW, c_stride, scale); break;
         default: return fail(EXB_ERR_UNSUPPORTED, "exb_nhwc_to_nchw_f32: dtype %d", dtype);
         }
         return after_launch("nhwc_to_nchw_fewc_kernel");
     }
     switch (dtype) {
-    case EXB_F16: nhwc_to_nchw_kernel<__half><<<grid, block, 0, st>>>(static_cast<const __half*>(x), y, C, HW, c_stride, scale); break;
-    case EXB_I8: nhwc_to_nchw_kernel<int8_t><<<grid, block, 0, st>>>(static_cast<const int8_t*>(x), y, C, HW, c_stride, scale); break;
-    case EXB_F32: nhwc_to_nchw_kernel<float><<<grid, block, 0, st>>>(static_cast<const float*>(x), y, C, HW, c_stride, scale); break;
+    case EXB_F16: launch_overlapped(ctx, nhwc_to_nchw_kernel<__half>, grid, block, st, static_cast<const __half*>(x), y, C, HW, c_stride, scale); break;
+    case EXB_I8: launch_overlapped(ctx, nhwc_to_nchw_kernel<int8_t>, grid, block, st, static_cast<const int8_t*>(x), y, C, HW, c_stride, scale); break;
+    case EXB_F32: launch_overlapped(ctx, nhwc_to_nchw_kernel<float>, grid, block, st, static_cast<const float*>(x), y, C, HW, c_stride, scale); break;
     default: return fail(EXB_ERR_UNSUPPORTED, "exb_nhwc_to_nchw_f32: dtype %d", dtype);
     }
     return after_launch("nhwc_to_nchw_kernel");
@@ -283,12 +290,12 @@ extern "C" int exb_nchw_f32_to_nhwc_padded(exb_ctx* ctx, const float* x, void* y
         const int64_t rows = (int64_t)N * H;
         const dim3 block(64, 4);
         const int grid = (int)std::min<int64_t>((rows + 3) / 4, (int64_t)ctx->sm_count * 32);
-        nchw_to_nhwc4_f16_quad_kernel<false><<<grid, block, 0, st>>>(x, static_cast<__half*>(y), C, H, W, w_pad, w_pitch, rows,
+        launch_overlapped(ctx, nchw_to_nhwc4_f16_quad_kernel<false>, grid, block, st, x, static_cast<__half*>(y), C, H, W, w_pad, w_pitch, rows,
                                                                      nullptr, nullptr);
         return after_launch("nchw_to_nhwc4_f16_quad_kernel");
     }
     const int grid = stream_grid(ctx, (int64_t)N * H * w_pitch, 256, 16);
-#define EXB_LAUNCH(T, CS) nchw_to_nhwc_padded_kernel<T, CS><<<grid, 256, 0, st>>>(x, static_cast<T*>(y), N, C, H, W, w_pad, w_pitch, scale, rounding)
+#define EXB_LAUNCH(T, CS) launch_overlapped(ctx, nchw_to_nhwc_padded_kernel<T, CS>, grid, 256, st, x, static_cast<T*>(y), N, C, H, W, w_pad, w_pitch, scale, rounding)
     if (dtype == EXB_F16) { if (c_stride == 4) EXB_LAUNCH(__half, 4); else EXB_LAUNCH(__half, 8); }
     else if (dtype == EXB_I8) { if (c_stride == 4) EXB_LAUNCH(int8_t, 4); else EXB_LAUNCH(int8_t, 8); }
     else return fail(EXB_ERR_UNSUPPORTED, "padded ingest supports EXB_F16 and EXB_I8 output");
@@ -309,13 +316,13 @@ extern "C" int exb_image_f32_to_nhwc_norm(exb_ctx* ctx, const float* x, void* y,
     const int64_t HW = (int64_t)H * W;
     const int grid = stream_grid(ctx, (int64_t)N * HW, 256, 16);
     if (dtype == EXB_F16 && c_stride == 16)
-        image_to_nhwc_kernel<__half, 16><<<grid, 256, 0, st>>>(x, static_cast<__half*>(y), N, C, HW, mul, add, scale, rounding);
+        launch_overlapped(ctx, image_to_nhwc_kernel<__half, 16>, grid, 256, st, x, static_cast<__half*>(y), N, C, HW, mul, add, scale, rounding);
     else if (dtype == EXB_F16 && c_stride == 8)
-        image_to_nhwc_kernel<__half, 8><<<grid, 256, 0, st>>>(x, static_cast<__half*>(y), N, C, HW, mul, add, scale, rounding);
+        launch_overlapped(ctx, image_to_nhwc_kernel<__half, 8>, grid, 256, st, x, static_cast<__half*>(y), N, C, HW, mul, add, scale, rounding);
     else if (dtype == EXB_I8 && c_stride == 32)
-        image_to_nhwc_kernel<int8_t, 32><<<grid, 256, 0, st>>>(x, static_cast<int8_t*>(y), N, C, HW, mul, add, scale, rounding);
+        launch_overlapped(ctx, image_to_nhwc_kernel<int8_t, 32>, grid, 256, st, x, static_cast<int8_t*>(y), N, C, HW, mul, add, scale, rounding);
     else if (dtype == EXB_I8 && c_stride == 16)
-        image_to_nhwc_kernel<int8_t, 16><<<grid, 256, 0, st>>>(x, static_cast<int8_t*>(y), N, C, HW, mul, add, scale, rounding);
+        launch_overlapped(ctx, image_to_nhwc_kernel<int8_t, 16>, grid, 256, st, x, static_cast<int8_t*>(y), N, C, HW, mul, add, scale, rounding);
     else
         return fail(EXB_ERR_UNSUPPORTED, "exb_image_f32_to_nhwc_norm: dtype %d with channel stride %d", dtype, c_stride);
     return after_launch("image_to_nhwc_kernel");
@@ -333,7 +340,7 @@ extern "C" int exb_nchw_f32_to_nhwc4_padded_norm(exb_ctx* ctx, const float* x, v
     const int64_t rows = (int64_t)N * H;
     const dim3 block(64, 4);
     const int grid = (int)std::min<int64_t>((rows + 3) / 4, (int64_t)ctx->sm_count * 32);
-    nchw_to_nhwc4_f16_quad_kernel<true><<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(x, static_cast<__half*>(y), C, H, W,
+    launch_overlapped(ctx, nchw_to_nhwc4_f16_quad_kernel<true>, grid, block, static_cast<cudaStream_t>(stream), x, static_cast<__half*>(y), C, H, W,
                                                                                                 w_pad, w_pitch, rows, mul, add);
     return after_launch("nchw_to_nhwc4_f16_quad_kernel");
 }
@@ -349,7 +356,7 @@ extern "C" int exb_nchw_f16_to_nhwc4_padded(exb_ctx* ctx, const void* x, void* y
     const int64_t rows = (int64_t)N * H;
     const dim3 block(64, 4);
     const int grid = (int)std::min<int64_t>((rows + 3) / 4, (int64_t)ctx->sm_count * 32);
-    nchw_f16_to_nhwc4_f16_quad_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_overlapped(ctx, nchw_f16_to_nhwc4_f16_quad_kernel, grid, block, static_cast<cudaStream_t>(stream), 
         static_cast<const __half*>(x), static_cast<__half*>(y), C, H, W, w_pad, w_pitch, rows);
     return after_launch("nchw_f16_to_nhwc4_f16_quad_kernel");
 }
@@ -364,6 +371,7 @@ template <int CS, int C>
 __global__ void __launch_bounds__(256) focus_ingest_kernel(const float* __restrict__ x, __half* __restrict__ y, int N,
                                                            int H, int W, const float* __restrict__ mul,
                                                            const float* __restrict__ add) {
+    pdl_enter();
     const int OH = H / 2, OW = W / 2;
     const int64_t total = (int64_t)N * OH * OW;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -408,7 +416,7 @@ extern "C" int exb_nchw_f32_focus_to_nhwc_f16(exb_ctx* ctx, const float* x, void
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int grid = exb::stream_grid(ctx, (int64_t)N * (H / 2) * (W / 2), 256);
     __half* yh = static_cast<__half*>(y);
-#define EXB_FOCUS(CS, CC) exb::focus_ingest_kernel<CS, CC><<<grid, 256, 0, st>>>(x, yh, N, H, W, mul, add)
+#define EXB_FOCUS(CS, CC) launch_overlapped(ctx, exb::focus_ingest_kernel<CS, CC>, grid, 256, st, x, yh, N, H, W, mul, add)
     if (c_stride == 16) {
         if (C == 1) EXB_FOCUS(16, 1); else if (C == 2) EXB_FOCUS(16, 2); else if (C == 3) EXB_FOCUS(16, 3); else EXB_FOCUS(16, 4);
     } else {

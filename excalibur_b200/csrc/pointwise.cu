@@ -48,6 +48,7 @@ __device__ __forceinline__ void stf(float* p, float v) { *p = v; }
 // ---- generic unary / binary map ---------------------------------------------------------
 template <typename T, typename F>
 __global__ void __launch_bounds__(kThreads) map1_kernel(const T* x, T* y, int64_t count, F f) {
+    pdl_enter();
     constexpr int V = Vec<T>::N;
     const int64_t nvec = count / V;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(kThreads) map1_kernel(const T* x, T* y, int64_
 template <typename T, typename F>
 __global__ void __launch_bounds__(kThreads) map2_kernel(const T* a, const T* b, T* y,
                                                         int64_t count, F f) {
+    pdl_enter();
     constexpr int V = Vec<T>::N;
     const int64_t nvec = count / V;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -109,6 +111,7 @@ __device__ __forceinline__ float eltwise_combine(int type, float acc, float v, f
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) eltwise_kernel(EltwiseArgs args, T* y, int64_t count) {
+    pdl_enter();
     constexpr int V = Vec<T>::N;
     const int64_t nvec = count / V;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -162,6 +165,7 @@ __global__ void __launch_bounds__(kThreads) eltwise_kernel(EltwiseArgs args, T* 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_kernel(const T* x, int8_t* q, int64_t count,
                                                             float scale, int rounding) {
+    pdl_enter();
     // 16 outputs (16 bytes) per thread step.
     const int64_t nvec = count / 16;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -187,6 +191,7 @@ __global__ void __launch_bounds__(kThreads) quantize_kernel(const T* x, int8_t* 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) dequantize_kernel(const int8_t* q, T* y, int64_t count,
                                                               float scale) {
+    pdl_enter();
     const int64_t nvec = count / 16;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     constexpr int V = Vec<T>::N;
@@ -252,10 +257,10 @@ int launch_map1(exb_ctx* ctx, const void* x, void* y, int64_t count, int dtype, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == EXB_F16) {
         int grid = stream_grid(ctx, count / 8 + 1, kThreads);
-        map1_kernel<__half, F><<<grid, kThreads, 0, st>>>(static_cast<const __half*>(x), static_cast<__half*>(y), count, f);
+        launch_overlapped(ctx, map1_kernel<__half, F>, grid, kThreads, st, static_cast<const __half*>(x), static_cast<__half*>(y), count, f);
     } else {
         int grid = stream_grid(ctx, count / 4 + 1, kThreads);
-        map1_kernel<float, F><<<grid, kThreads, 0, st>>>(static_cast<const float*>(x), static_cast<float*>(y), count, f);
+        launch_overlapped(ctx, map1_kernel<float, F>, grid, kThreads, st, static_cast<const float*>(x), static_cast<float*>(y), count, f);
     }
     return after_launch(name);
 }
@@ -301,11 +306,11 @@ extern "C" int exb_binaryop_fwd(exb_ctx* ctx, int op, const void* a, const void*
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == EXB_F16) {
         int grid = stream_grid(ctx, count / 8 + 1, kThreads);
-        map2_kernel<__half, BinFn><<<grid, kThreads, 0, st>>>(static_cast<const __half*>(a), static_cast<const __half*>(b),
+        launch_overlapped(ctx, map2_kernel<__half, BinFn>, grid, kThreads, st, static_cast<const __half*>(a), static_cast<const __half*>(b),
                                                               static_cast<__half*>(y), count, BinFn{op});
     } else {
         int grid = stream_grid(ctx, count / 4 + 1, kThreads);
-        map2_kernel<float, BinFn><<<grid, kThreads, 0, st>>>(static_cast<const float*>(a), static_cast<const float*>(b),
+        launch_overlapped(ctx, map2_kernel<float, BinFn>, grid, kThreads, st, static_cast<const float*>(a), static_cast<const float*>(b),
                                                              static_cast<float*>(y), count, BinFn{op});
     }
     return after_launch("exb_binaryop_fwd");
@@ -332,10 +337,10 @@ extern "C" int exb_eltwise_fwd(exb_ctx* ctx, int type, int n_in, const void* con
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == EXB_F16) {
         int grid = stream_grid(ctx, count / 8 + 1, kThreads);
-        eltwise_kernel<__half><<<grid, kThreads, 0, st>>>(args, static_cast<__half*>(y), count);
+        launch_overlapped(ctx, eltwise_kernel<__half>, grid, kThreads, st, args, static_cast<__half*>(y), count);
     } else {
         int grid = stream_grid(ctx, count / 4 + 1, kThreads);
-        eltwise_kernel<float><<<grid, kThreads, 0, st>>>(args, static_cast<float*>(y), count);
+        launch_overlapped(ctx, eltwise_kernel<float>, grid, kThreads, st, args, static_cast<float*>(y), count);
     }
     return after_launch("exb_eltwise_fwd");
 }
@@ -349,9 +354,9 @@ extern "C" int exb_quantize_fwd(exb_ctx* ctx, const void* x, int in_dtype, int8_
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int grid = stream_grid(ctx, count / 16 + 1, kThreads);
     if (in_dtype == EXB_F16)
-        quantize_kernel<__half><<<grid, kThreads, 0, st>>>(static_cast<const __half*>(x), q, count, scale, rounding);
+        launch_overlapped(ctx, quantize_kernel<__half>, grid, kThreads, st, static_cast<const __half*>(x), q, count, scale, rounding);
     else
-        quantize_kernel<float><<<grid, kThreads, 0, st>>>(static_cast<const float*>(x), q, count, scale, rounding);
+        launch_overlapped(ctx, quantize_kernel<float>, grid, kThreads, st, static_cast<const float*>(x), q, count, scale, rounding);
     return after_launch("exb_quantize_fwd");
 }
 
@@ -364,8 +369,8 @@ extern "C" int exb_dequantize_fwd(exb_ctx* ctx, const int8_t* q, void* y, int ou
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int grid = stream_grid(ctx, count / 16 + 1, kThreads);
     if (out_dtype == EXB_F16)
-        dequantize_kernel<__half><<<grid, kThreads, 0, st>>>(q, static_cast<__half*>(y), count, scale);
+        launch_overlapped(ctx, dequantize_kernel<__half>, grid, kThreads, st, q, static_cast<__half*>(y), count, scale);
     else
-        dequantize_kernel<float><<<grid, kThreads, 0, st>>>(q, static_cast<float*>(y), count, scale);
+        launch_overlapped(ctx, dequantize_kernel<float>, grid, kThreads, st, q, static_cast<float*>(y), count, scale);
     return after_launch("exb_dequantize_fwd");
 }
