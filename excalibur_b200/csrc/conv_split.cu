@@ -2,7 +2,7 @@
 // cluster of CTAs that share its reduction dimension.
 //
 // The persistent kernel of conv_tc.cu gives a tile to one CTA (or pair): with one image a 3x3 layer of 512 channels @7x7
-// is two tiles, and one thread issues the whole reduction - 144 dependent MMAs and the loads that feed them, 19 us
+// is two tiles, and one warp issues the whole reduction - 144 dependent MMAs and the loads that feed them, 19 us
 // (int8), on two of 148 SMs.  Here N tiles are at most 64 channels and the K blocks of a tile are divided over a cluster
 // of 1, 2, 4 or 8 CTAs.  Each accumulates its part in TMEM and spills it to its shared memory; after a cluster barrier
 // every CTA sums one slice of the tile's pixels over all parts through distributed shared memory and runs the epilogue
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
     __shared__ int abort_flag;
     // operand ring (1024-byte aligned: the widest swizzle atom); the partial tile takes its place when the MMAs are done
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::uniform_warp(), lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x % p.splits;
     int t = (int)blockIdx.x / p.splits;
     const int ntile = t % p.n_tiles;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
     ptx::tc_fence_before_sync();
     __syncthreads();
     ptx::tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_smem;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
     const uint32_t ring0 = ptx::smem_u32(ring), slot = (uint32_t)(p.a_bytes + p.b_bytes);
     const uint32_t full0 = ptx::smem_u32(&full_bar[0]), empty0 = ptx::smem_u32(&empty_bar[0]);
 
@@ -185,7 +185,8 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
         __syncwarp();
     } else if (warp == 1) {
         pdl_wait();
-        if (lane == 0) {
+        {       // the whole warp, uniformly; one elected lane issues (see uniform_warp)
+            const uint32_t leader = ptx::elect_one() ? 1u : 0u;
             const uint64_t d0 = ptx::make_smem_desc(ring0, (uint32_t)p.kb_bytes);
             const uint32_t desc_hi = (uint32_t)(d0 >> 32);
             const int ksteps = p.kb_bytes / 32;
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
             int s = 0;
             uint32_t phase = 0;
             for (int i = 0; i < units; ++i) {
-                if (!ptx::mbar_wait_bounded_u32(full0 + s * 8, phase, &abort_flag, kSplitMaxSpins)) {
+                if (!ptx::mbar_wait_bounded_uniform(full0 + s * 8, phase, &abort_flag, kSplitMaxSpins)) {
                     ok = false;
                     break;
                 }
@@ -201,19 +202,19 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
                 if (ksteps == 4) {
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks)
-                        ptx::tc_mma_lohi<kInt8>(tmem_base, a_lo + 2 * ks, b_lo + 2 * ks, desc_hi, idesc, ks ? 1u : (uint32_t)(i > 0));
+                        ptx::tc_mma_lohi<kInt8>(tmem_base, a_lo + 2 * ks, b_lo + 2 * ks, desc_hi, idesc, ks ? 1u : (uint32_t)(i > 0), leader);
                 } else {
                     for (int ks = 0; ks < ksteps; ++ks)
-                        ptx::tc_mma_lohi<kInt8>(tmem_base, a_lo + 2 * ks, b_lo + 2 * ks, desc_hi, idesc, (i | ks) ? 1u : 0u);
+                        ptx::tc_mma_lohi<kInt8>(tmem_base, a_lo + 2 * ks, b_lo + 2 * ks, desc_hi, idesc, (i | ks) ? 1u : 0u, leader);
                 }
-                if (i + p.stages < units) ptx::tc_commit_u32(empty0 + s * 8);
+                if (i + p.stages < units) ptx::tc_commit_u32(empty0 + s * 8, leader);
                 if (++s == p.stages) {
                     s = 0;
                     phase ^= 1u;
                 }
             }
-            ptx::tc_commit_u32(ptx::smem_u32(&done_bar));
-            if (!ok) atomicExch(p.error, 2);
+            ptx::tc_commit_u32(ptx::smem_u32(&done_bar), leader);
+            if (!ok && leader) atomicExch(p.error, 2);
         }
         __syncwarp();
     }

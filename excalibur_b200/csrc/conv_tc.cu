@@ -11,17 +11,18 @@
 // Persistent CTAs: two per SM with 10 warps each for N tiles of up to 128 channels, one per SM with
 // 18 warps for wider ones.
 //   warp 0   TMA producer (lane g issues K block g of a stage) - fills a ring of shared-memory stages
-//   warp 1   MMA issuer (one lane) + TMEM owner                 - tcgen05.mma, fp32 / int32 accumulators
+//   warp 1   MMA issuer (uniform, one lane elected) + TMEM owner - tcgen05.mma, fp32 / int32 accumulators
 //                                                                 in as many TMEM buffers as fit (2-4)
 //   warps 2+ epilogue, in groups of four warps (one per TMEM     - tile i uses buffer i % buffers and
 //            lane quarter)                                        group i % groups
 //
 // Main loops: the tap loop above; the row-box loop for stride-1 layers (one box of TW + kw - 1 pixels per kernel
 // row, the kw taps read through descriptors that start 0, 1, .. pixels into the swizzled box); CTA pairs for wide
-// tiles (two CTAs of a cluster share every MMA, tcgen05 cta_group::2, and each loads half of the weight rows).
-// What bounds this kernel are its serial roles - one producing and one issuing thread per CTA, epilogue warps
+// tiles and long reductions (two CTAs of a cluster share every MMA, tcgen05 cta_group::2, and each loads half of the
+// weight rows).
+// What bounds this kernel are its serial roles - one producing and one issuing warp per CTA, epilogue warps
 // whose own instruction streams stall - and, for narrow N tiles, the shared-memory reads of the tensor pipe; every
-// loop of a single-thread role is therefore table-driven, unrolled and free of divisions.  Two epilogues exist:
+// loop of these two is therefore table-driven, unrolled and free of divisions.  Two epilogues exist:
 //   quad  (N tile a multiple of 32 channels): accumulators leave TMEM in the 16x256b shape, in which four
 //         neighbouring lanes hold one pixel; the B operand is loaded through a tensor map that permutes the
 //         output channels inside each 32-channel block so that those four lanes hold channels 0-7, 8-15,
@@ -100,7 +101,8 @@ struct ConvTcParams {
     const void* w_global;   // packed weights (patch mode copies them into core-matrix layout)
     // Tile origins: first output column / row of tile index i is i * step + org (step = TW / TH and
     // org = 0 unless tiles overlap).
-    int step_w, step_h, org;
+    int step_w, step_h, step_n, org;
+    int pair_h, pair_n;     // CTA pairs: how far rank 1's tile lies from rank 0's, rows / images (one of them is 0)
     // Fused 3x3/2 pad-1 max pooling (patch mode, BN = 64): an 8 x 16 tile of the convolution output
     // starts at (6*tx - 1, 14*ty - 1), so it holds every input of the 3 x 7 pooled outputs that
     // start at (3*tx, 7*ty); neighbouring tiles overlap by two rows / columns, which are recomputed.
@@ -156,7 +158,7 @@ struct TileCursor {
         c.ntile = nt;
         c.ow0 = w * p.step_w + p.org;
         c.oh0 = h * p.step_h + p.org;
-        c.n0 = n * p.TN;
+        c.n0 = n * p.step_n;
         return c;
     }
 };
@@ -256,21 +258,21 @@ __device__ __forceinline__ void epi_quad_rows(const EpiParams& e, const float* q
 }
 
 // The MMAs of one row-box unit, fully unrolled: tap s reads the box s pixels further in (kSteps 32-byte K steps per
-// pixel) against the weight block of that tap.  The issuing thread retires one instruction every few cycles, so
+// pixel) against the weight block of that tap.  The issuing warp retires one instruction every few cycles, so
 // every address computed at run time shows in the MMA rate of narrow tiles.
 template <bool kInt8, int kTaps, int kSteps, bool kPair>
 __device__ __forceinline__ void rowbox_unit(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
-                                            uint32_t idesc, uint32_t b_tap, uint32_t accumulate) {
+                                            uint32_t idesc, uint32_t b_tap, uint32_t accumulate, uint32_t leader) {
 #pragma unroll
     for (int sx = 0; sx < kTaps; ++sx) {
 #pragma unroll
         for (int ks = 0; ks < kSteps; ++ks) {
             if (kPair)
                 ptx::tc_mma_ab_pair<kInt8>(d_tmem, a_lo + (uint32_t)(sx * 2 * kSteps + 2 * ks), a_hi, b_lo + (uint32_t)(2 * ks), b_hi,
-                                           idesc, (sx | ks) ? 1u : accumulate);
+                                           idesc, (sx | ks) ? 1u : accumulate, leader);
             else
                 ptx::tc_mma_ab<kInt8>(d_tmem, a_lo + (uint32_t)(sx * 2 * kSteps + 2 * ks), a_hi, b_lo + (uint32_t)(2 * ks), b_hi, idesc,
-                                      (sx | ks) ? 1u : accumulate);
+                                      (sx | ks) ? 1u : accumulate, leader);
         }
         b_lo += b_tap;
     }
@@ -282,7 +284,7 @@ __device__ __forceinline__ void rowbox_unit(uint32_t d_tmem, uint32_t a_lo, uint
 // kEpi: which epilogue (see the head of the file); each is its own instantiation so that the others keep
 // their register allocation.  kPrelu: the activation is the per-channel PReLU.
 // kPair: the CTA is one of a cluster of two that share every MMA (tcgen05 cta_group::2, M = 256): each CTA loads
-//        the A box of its own M tile and HALF of the N tile's weight rows, the rank-0 CTA's thread issues the MMAs
+//        the A box of its own M tile and HALF of the N tile's weight rows, the rank-0 CTA's warp issues the MMAs
 //        for both, each CTA drains its own 128 accumulator rows.  Halves the weight stream per SM (wide layers).
 template <bool kInt8, int kEpiWarps, int kEpi, bool kPrelu = false, bool kPair = false>
 __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps == 8 ? 2 : 1)
@@ -310,17 +312,20 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
     // Pool mode: one 128-pixel x 64-channel fp16 staging tile per epilogue group.
     uint8_t* pool_stage = reinterpret_cast<uint8_t*>(k_tab + p.k_iters);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = ptx::uniform_warp();
     const int lane = threadIdx.x & 31;
-    // Units of work: tiles, or (pair mode) pairs of tiles that are neighbours along the image-group dimension; unit u
-    // of a pair is tile (.., 2 * q + rank).  first_unit / unit_step: this CTA's (cluster's) share of the sequence.
-    const uint32_t cta_rank = kPair ? ptx::cluster_ctarank() : 0u;
-    const int total_tiles = p.tiles_w * p.tiles_h * (kPair ? (p.tiles_nb + 1) / 2 : p.tiles_nb) * p.n_tiles;
+    // Units of work: tiles, or (pair mode) pairs of tiles that are neighbours along the image groups or, with one image
+    // group, along the rows: the steps of that dimension are doubled and rank 1 is pair_n images or pair_h rows on.  first_unit / unit_step: this CTA's (cluster's) share of the sequence.
+    const uint32_t cta_rank = kPair ? __shfl_sync(0xffffffffu, ptx::cluster_ctarank(), 0) : 0u;
+    const int total_tiles = p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;      // (pair mode: of pairs)
     const int first_unit = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const int unit_step = kPair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     auto tile_of = [&](const TileCursor& c) -> TileCoord {
         TileCoord tc = c.coord(p);
-        if (kPair) tc.n0 = (2 * c.n + (int)cta_rank) * p.TN;
+        if (kPair) {
+            tc.oh0 += (int)cta_rank * p.pair_h;
+            tc.n0 += (int)cta_rank * p.pair_n;
+        }
         return tc;
     };
     const int k_iters = p.k_iters;
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
     __syncthreads();
     if (kPair) ptx::cluster_sync();      // the peer's barriers are initialised before anything signals them
     ptx::tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_smem;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
 
     if (warp == 0) {
         // ------------------------------- TMA producer --------------------------------------
@@ -460,7 +465,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                     // Fused pooling: patch ring and accumulator ring have the same length and tile i uses slot i % length
                     // of both, so the patch of a slot is free when the MMAs of the tile that used it have retired, which is
                     // what the slot's "accumulator full" barrier says - one commit per tile serves producer and epilogue
-                    // (the issuing thread is what bounds that kernel).  The plain stem keeps its longer ring of patches.
+                    // (issuing is what bounds that kernel).  The plain stem keeps its longer ring of patches.
                     if (!ptx::mbar_wait_bounded_u32((p.pool ? ptx::smem_u32(&tfull_bar[0]) : empty0) + stage * 8, phase ^ 1u, &abort_flag,
                                                     kMaxSpins)) {
                         ok = 0;
@@ -547,7 +552,9 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
         }
     } else if (warp == 1) {
         // ------------------------------- MMA issuer ----------------------------------------
-        if (lane == 0 && cta_rank == 0) {      // pair mode: the rank-0 CTA issues for both
+        // The whole warp walks the loops (see uniform_warp); one elected lane issues.
+        if (cta_rank == 0) {      // pair mode: the rank-0 CTA issues for both
+            const uint32_t leader = ptx::elect_one() ? 1u : 0u;
             const int G = p.kgroup;
             int stage = 0;
             uint32_t phase = 0;
@@ -572,9 +579,9 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
             const uint32_t b_tap = bres ? b_blk * p.cblks : b_blk;
             const uint32_t rb_row = (uint32_t)((p.kw - 1) * p.cblks) * b_blk;   // after a row's last channel block: skip its other taps
             const uint32_t idesc = p.idesc;
-            if (bres && !ptx::mbar_wait_bounded(&bres_bar, 0, &abort_flag, kMaxSpins)) ok = false;
+            if (bres && !ptx::mbar_wait_bounded_uniform(ptx::smem_u32(&bres_bar), 0, &abort_flag, kMaxSpins)) ok = false;
             for (int t = first_unit; t < total_tiles && ok; t += unit_step) {
-                if (!ptx::mbar_wait_bounded_u32(tempty0 + acc * 8, acc_phase ^ 1u, &abort_flag, kMaxSpins)) {
+                if (!ptx::mbar_wait_bounded_uniform(tempty0 + acc * 8, acc_phase ^ 1u, &abort_flag, kMaxSpins)) {
                     ok = false;
                     break;
                 }
@@ -584,7 +591,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                 uint32_t rb_b = b_lo0;
                 int rb_cb = 0;
                 if (p.patch) {
-                    if (!ptx::mbar_wait_bounded_u32(full0 + stage * 8, phase, &abort_flag, kMaxSpins)) {
+                    if (!ptx::mbar_wait_bounded_uniform(full0 + stage * 8, phase, &abort_flag, kMaxSpins)) {
                         ok = false;
                         break;
                     }
@@ -600,18 +607,19 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
 #pragma unroll
                         for (int ks = 0; ks < 2; ++ks) {
                             asm volatile(
-                                "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+                                "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
                                 "mov.b64 da, {%1, %2};\n\t"
                                 "mov.b64 db, {%3, %4};\n\t"
                                 "setp.ne.b32 p, %6, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
+                                "setp.ne.b32 q, %7, 0;\n\t"
+                                "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
                                 "r"(ar + ks * 2), "r"(a_hi), "r"(br + (uint32_t)(ks * 2 * (p.BN * 16 >> 4))), "r"(b_hi),
-                                "r"(idesc), "r"(accumulate)
+                                "r"(idesc), "r"(accumulate), "r"(leader)
                                 : "memory");
                             accumulate = 1;
                         }
                     }
-                    if (!p.pool) ptx::tc_commit_u32(empty0 + stage * 8);
+                    if (!p.pool) ptx::tc_commit_u32(empty0 + stage * 8, leader);
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1u;
@@ -619,7 +627,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                 } else
                 for (int it0 = 0; it0 < k_iters; it0 += G) {
                     const int nb = min(G, k_iters - it0);
-                    if (!ptx::mbar_wait_bounded_u32(full0 + stage * 8, phase, &abort_flag, kMaxSpins)) {
+                    if (!ptx::mbar_wait_bounded_uniform(full0 + stage * 8, phase, &abort_flag, kMaxSpins)) {
                         ok = false;
                         break;
                     }
@@ -629,17 +637,17 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                         for (int g = 0; g < nb; ++g) {
                             // resident weights: the unit's first block (tap-major order); streamed: the stage's
                             const uint32_t bu = bres ? rb_b : b_lo0 + stage * b_stage + (uint32_t)g * b_tap * p.taps;
-                            if (p.taps == 3 && ksteps == 4) rowbox_unit<kInt8, 3, 4, kPair>(d_tmem, a_lo, a_hi, bu, desc_hi, idesc, b_tap, accumulate);
-                            else if (p.taps == 3 && ksteps == 2) rowbox_unit<kInt8, 3, 2, kPair>(d_tmem, a_lo, a_hi, bu, desc_hi, idesc, b_tap, accumulate);
+                            if (p.taps == 3 && ksteps == 4) rowbox_unit<kInt8, 3, 4, kPair>(d_tmem, a_lo, a_hi, bu, desc_hi, idesc, b_tap, accumulate, leader);
+                            else if (p.taps == 3 && ksteps == 2) rowbox_unit<kInt8, 3, 2, kPair>(d_tmem, a_lo, a_hi, bu, desc_hi, idesc, b_tap, accumulate, leader);
                             else
                                 for (int sx = 0; sx < p.taps; ++sx)
                                     for (int ks = 0; ks < ksteps; ++ks)
                                         if (kPair)
                                             ptx::tc_mma_ab_pair<kInt8>(d_tmem, a_lo + sx * a_tap + 2 * ks, a_hi, bu + sx * b_tap + 2 * ks,
-                                                                       desc_hi, idesc, (sx | ks) ? 1u : accumulate);
+                                                                       desc_hi, idesc, (sx | ks) ? 1u : accumulate, leader);
                                         else
                                         ptx::tc_mma_ab<kInt8>(d_tmem, a_lo + sx * a_tap + 2 * ks, a_hi, bu + sx * b_tap + 2 * ks, desc_hi,
-                                                              idesc, (sx | ks) ? 1u : accumulate);
+                                                              idesc, (sx | ks) ? 1u : accumulate, leader);
                             accumulate = 1;
                             a_lo += a_blk;
                             rb_b += b_blk;
@@ -652,32 +660,32 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                     for (int g = 0; g < nb; ++g) {
                         if (kPair) {
                             if (ksteps == 4) {
-                                ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate);
-                                ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1);
-                                ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1);
-                                ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1);
+                                ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate, leader);
+                                ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1, leader);
+                                ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1, leader);
+                                ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1, leader);
                             } else {
                                 for (int ks = 0; ks < ksteps; ++ks)
-                                    ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo + 2 * ks, b_lo + 2 * ks, desc_hi, idesc, ks ? 1u : accumulate);
+                                    ptx::tc_mma_lohi_pair<kInt8>(d_tmem, a_lo + 2 * ks, b_lo + 2 * ks, desc_hi, idesc, ks ? 1u : accumulate, leader);
                             }
                         } else if (ksteps == 4) {
-                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate);
-                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1);
-                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1);
-                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1);
+                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate, leader);
+                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1, leader);
+                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1, leader);
+                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1, leader);
                         } else if (ksteps == 2) {
-                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate);
-                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1);
+                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate, leader);
+                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1, leader);
                         } else {
-                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate);
+                            ptx::tc_mma_lohi<kInt8>(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate, leader);
                         }
                         accumulate = 1;
                         a_lo += a_blk;
                         b_lo += b_blk;
                     }
                     // stage is free once these MMAs retire (pair mode: in both CTAs)
-                    if (kPair) ptx::tc_commit_pair_u32(empty0 + stage * 8);
-                    else ptx::tc_commit_u32(empty0 + stage * 8);
+                    if (kPair) ptx::tc_commit_pair_u32(empty0 + stage * 8, leader);
+                    else ptx::tc_commit_u32(empty0 + stage * 8, leader);
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1u;
@@ -685,14 +693,14 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                 }
                 if (!ok) break;
                 // accumulator complete (pair mode: each CTA's epilogue drains its own 128 rows)
-                if (kPair) ptx::tc_commit_pair_u32(tfull0 + acc * 8);
-                else ptx::tc_commit_u32(tfull0 + acc * 8);
+                if (kPair) ptx::tc_commit_pair_u32(tfull0 + acc * 8, leader);
+                else ptx::tc_commit_u32(tfull0 + acc * 8, leader);
                 if (++acc == p.acc_bufs) {
                     acc = 0;
                     acc_phase ^= 1u;
                 }
             }
-            if (!ok) atomicExch(p.error, 2);
+            if (!ok && leader) atomicExch(p.error, 2);
         }
     } else if (warp >= kFirstEpiWarp) {
         // ------------------------------- epilogue ------------------------------------------
@@ -1111,7 +1119,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     p.tiles_w = (g.OW + p.TW - 1) / p.TW;
     p.tiles_h = (g.OH + p.TH - 1) / p.TH;
     p.tiles_nb = (g.N + p.TN - 1) / p.TN;
-    p.step_w = p.TW; p.step_h = p.TH; p.org = 0;
+    p.step_w = p.TW; p.step_h = p.TH; p.step_n = p.TN; p.org = 0;
     p.n_tiles = (w->cout_pad + 255) / 256;
     p.BN = round_up((w->cout_pad + p.n_tiles - 1) / p.n_tiles, 16);
     // Two CTAs per SM when the N tile is narrow (see the kernel's comment).
@@ -1145,7 +1153,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
         p.patch_pitch = (2 * p.TW + 8) * 8;   // 2*TW + 6 pixels needed, rounded to 24
         p.a_bytes = round_up(p.patch_rows * p.patch_pitch, 128);
         p.w_global = w->d_w;
-        p.step_w = p.TW; p.step_h = p.TH;
+        p.step_w = p.TW; p.step_h = p.TH; p.step_n = 1;
         if (g.pool) {
             p.pool = 1;
             p.PH = g.PH; p.PW = g.PW;
@@ -1189,9 +1197,10 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
         // weights stay resident with two CTAs per SM (as before) or, in row-box mode, with one CTA per SM as well
         const bool res_two = p.n_tiles == 1 && two && b_tile <= 48 * 1024;
         const bool res_one = p.n_tiles == 1 && b_tile <= 150 * 1024;
-        // One CTA per SM (to keep the weights resident) only for N tiles of 128 and more: a single issuing thread
-        // cannot keep the tensor pipe busy with N = 64 instructions.
-        const bool one_cta = res_one && !res_two && two && p.BN >= 128;
+        // One CTA per SM (to keep the weights resident) for N tiles of 128 and more, and for 64 where tiles can be
+        // paired and there are enough of them: one CTA's own N = 64 instructions do not fill the tensor pipe.
+        const bool one_cta = res_one && !res_two && two &&
+                             (p.BN >= 128 || (p.BN == 64 && tiles_rb > 2 * ctx->sm_count && g.act != EXB_ACT_PRELU));
         const bool res_rb = (two && !one_cta) ? res_two : res_one;
         const double cost_tap = (double)tiles_tap * (a_tap + (res_two ? 0 : b_tile));
         const double cost_rb = (double)tiles_rb * (a_rb + (res_rb ? 0 : b_tile));
@@ -1214,20 +1223,59 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
         p.tiles_w = (g.OW + 7) / 8;
         p.tiles_h = (g.OH + p.TH - 1) / p.TH;
         p.tiles_nb = (g.N + p.TN - 1) / p.TN;
-        p.step_w = p.TW; p.step_h = p.TH; p.org = 0;
+        p.step_w = p.TW; p.step_h = p.TH; p.step_n = p.TN; p.org = 0;
         p.a_sbo = (8 + g.kw - 1) * p.kb_bytes;
         p.a_bytes = (8 + g.kw - 1) * 16 * p.kb_bytes;      // one box: a multiple of 1024 bytes for every kb_bytes >= 64
         p.a_bytes = round_up(p.a_bytes, 1024);
         p.a_tx_bytes = (8 + g.kw - 1) * 16 * p.kb_bytes;
         if (rb.one_cta) two = false;
     }
-    const int ctas_per_sm = two ? 2 : 1;
-    // CTA pairs (see the kernel's kPair): N tiles of 256 on one CTA per SM in the plain tap loop, and N tiles of 128
-    // in the row-box loop with resident weights (each CTA then keeps half of them and a stage can hold a whole tile);
-    // at least two image groups to pair up.  Each CTA holds half of the tile's weight rows.
-    const bool pair = !two && !patch && !fold.on && !g.pool && p.tiles_nb >= 2 && ctx->sm_count >= 2 && g.act != EXB_ACT_PRELU &&
-                      (p.rowbox ? (p.BN == 128 && p.n_tiles == 1 && rb.one_cta) : p.BN == 256);
-    if (pair) p.b_bytes = (p.BN / 2) * p.kb_bytes;
+    // Quad epilogue: N tiles of whole 32-channel blocks, every channel group of 8 either fully inside the output or
+    // fully outside, weights stored in whole 32-row blocks (the permuting map walks rows 32 at a time).  Taken when
+    // the epilogue moves fp16 / fp32 data (an fp16 output or residual): there its whole-sector accesses are worth
+    // 15-20 % of the layer; a lone int8 output is as fast from the thread-per-pixel epilogue (measured on the
+    // ResNet-18-style layers at batch 256), which needs fewer TMEM loads.
+    const bool quad = !patch && !p.pool && p.BN % 32 == 0 && w->cout_pad % 32 == 0 && (g.cout_stride & 7) == 0 &&
+                      g.out_dtype != EXB_I32 && !(g.out_dtype == EXB_I8 && g.out2_dtype < 0) &&
+                      p.TW <= 255 && p.TH <= 255 && p.TN <= 32767;
+    // CTA pairs (see the kernel's kPair): two tiles that are neighbours along the image groups, or along the rows when
+    // there is one image group, share every MMA and each CTA holds half of the weight rows.  Taken for
+    //  - row-box tiles of 64 or 128 channels whose weights stay resident on one CTA per SM: a stage then holds a whole
+    //    tile, and a pair's MMA reads half as many weight bytes per SM as two CTAs' own instructions;
+    //  - tap-loop tiles of more than 128 channels (an SM to themselves anyway) with at least 512 bytes of K: the
+    //    epilogue bounds shorter ones, and units of two tiles only coarsen its work (32 -> 192 channels 1x1, 48 images
+    //    of 28 x 28: 9.3 us in pairs, 8.3 single; 960 -> 160 int8, 256 images of 7 x 7: 11.4 in pairs, 13.5 single);
+    //  - tap-loop tiles of 64 to 128 channels with at least 1152 bytes of K (64 fp16 channels 3x3), where streaming the
+    //    weights sets the pace, and more than two tiles per SM, so that the coarser units do not leave the last wave
+    //    half empty: 256 -> 64 at 4 x 120 x 184 48.4 -> 42.7 us, but 18.2 -> 19.4 at 4 x 60 x 92 (173 tiles);
+    //    32 -> 64 stride 2 at 32 x 320 x 320 (576 bytes of K) 77 -> 117.
+    // 3x3 of 64 fp16 channels (row-box): 28.6 -> 22.3 us at 64 x 56 x 56; of 128 channels 24.7 -> 20.9 at 64 x 28 x 28.
+    // Resident weights beside a tap-loop ring were tried in pairs as well: 1.3 to 1.5 times slower (the ring is too short).
+    // The channel-permuting map of the quad epilogue moves 32-channel blocks, so a half must be made of whole ones.
+    const int64_t k_bytes = (int64_t)g.kh * g.kw * row_bytes;      // one pixel's reduction
+    const int64_t all_tiles = (int64_t)p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;
+    const bool pairable = !patch && !fold.on && !g.pool && ctx->sm_count >= 2 && g.act != EXB_ACT_PRELU &&
+                          p.BN % (quad ? 64 : 32) == 0 && (p.tiles_nb >= 2 || p.tiles_h >= 2);
+    bool pair = false;
+    if (p.rowbox)
+        pair = pairable && rb.one_cta && (p.BN == 64 || p.BN == 128);
+    else if (p.BN > 128)
+        pair = pairable && k_bytes >= 512;
+    else if (p.BN >= 64)
+        pair = pairable && k_bytes >= 1152 && all_tiles > 2 * ctx->sm_count;
+    if (pair) {
+        two = false;
+        p.b_bytes = (p.BN / 2) * p.kb_bytes;
+        if (p.tiles_nb >= 2) {
+            p.pair_n = p.step_n;
+            p.step_n *= 2;
+            p.tiles_nb = (p.tiles_nb + 1) / 2;
+        } else {
+            p.pair_h = p.step_h;
+            p.step_h *= 2;
+            p.tiles_h = (p.tiles_h + 1) / 2;
+        }
+    }
     const int k_iters = fold.on ? g.kh : (p.rowbox ? g.kh * p.cblks : g.kh * g.kw * p.cblks);
     p.k_iters = k_iters;
     if ((int64_t)g.N * g.OH * g.OW >= (int64_t)1 << 31) return fail(EXB_ERR_UNSUPPORTED, "more than 2^31 output pixels");
@@ -1258,7 +1306,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
         }
     while (G > 1 && budget / (G * blk_bytes) < 3) --G;
     if (pair) {
-        // One thread issues for two SMs: every commit and barrier wait it spends idles both tensor pipes, so a stage
+        // One warp issues for two SMs: every commit and barrier wait it spends idles both tensor pipes, so a stage
         // carries as many K blocks as two stages allow (three 32 KB blocks of A + half-B).  Measured on the 256 / 512-
         // channel layers: pairs with one block per stage 0.038 ms, with three 0.031 ms, single CTAs 0.035 ms.
         G = 1;
@@ -1267,7 +1315,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     }
     if (p.rowbox) {
         // A row-box unit already carries kw taps.  One stage per tile (all its units behind one barrier and one
-        // commit) when two such stages fit - every hand-over costs the single issuing thread a few hundred
+        // commit) when two such stages fit - every hand-over costs the issuing warp a few hundred
         // cycles - else one unit per stage and as many stages as fit.
         G = (k_iters * blk_bytes <= (pair ? 96 : 48) * 1024 && budget / (k_iters * blk_bytes) >= 2) ? k_iters : 1;
     }
@@ -1328,14 +1376,6 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     }
     if (!patch)
         if (int rc = encode_input_views(g, fold, x, p.kb_elems, sw, p.rowbox ? p.TW + g.kw - 1 : p.TW, p.TH, p.TN, p.tmA)) return rc;
-    // Quad epilogue: N tiles of whole 32-channel blocks, every channel group of 8 either fully inside the output or
-    // fully outside, weights stored in whole 32-row blocks (the permuting map walks rows 32 at a time).  Taken when
-    // the epilogue moves fp16 / fp32 data (an fp16 output or residual): there its whole-sector accesses are worth
-    // 15-20 % of the layer; a lone int8 output is as fast from the thread-per-pixel epilogue (measured on the
-    // ResNet-18-style layers at batch 256), which needs fewer TMEM loads.
-    const bool quad = !patch && !p.pool && p.BN % 32 == 0 && w->cout_pad % 32 == 0 && (g.cout_stride & 7) == 0 &&
-                      g.out_dtype != EXB_I32 && !(g.out_dtype == EXB_I8 && g.out2_dtype < 0) &&
-                      p.TW <= 255 && p.TH <= 255 && p.TN <= 32767;
     p.b_perm = quad ? 1 : 0;
     {
         const int K = g.kh * w->kw_pack * w->cin_pad;
@@ -1362,14 +1402,9 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
         if (r != CUDA_SUCCESS) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled(B) failed with %d", (int)r);
     }
 
-    const int total_tiles = p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;
-    const int max_ctas = ctx->sm_count * ctas_per_sm;
-    int grid = total_tiles < max_ctas ? total_tiles : max_ctas;
-    if (pair) {      // clusters of two CTAs, one per pair of tiles
-        const int pairs = p.tiles_w * p.tiles_h * ((p.tiles_nb + 1) / 2) * p.n_tiles;
-        const int clusters = pairs < ctx->sm_count / 2 ? pairs : ctx->sm_count / 2;
-        grid = 2 * clusters;
-    }
+    const int units = p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;      // tiles, or pairs of them (clusters of two CTAs)
+    const int max_units = pair ? ctx->sm_count / 2 : ctx->sm_count * (two ? 2 : 1);
+    const int grid = (units < max_units ? units : max_units) * (pair ? 2 : 1);
     const size_t smem = (size_t)p.stages * p.kgroup * p.a_bytes + p.b_region + 1024 + epi_bytes;
     const bool prelu = p.e.act == EXB_ACT_PRELU;
     void (*kern)(const ConvTcParams);

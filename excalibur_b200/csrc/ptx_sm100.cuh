@@ -124,6 +124,25 @@ __device__ __forceinline__ bool mbar_wait_bounded_warp(uint64_t* bar, uint32_t p
     return ok != 0;
 }
 
+// The warp's index, known to the compiler as uniform.  A role whose whole warp runs one uniform instruction stream, with
+// only the tensor-core and commit instructions predicated on one elected lane, keeps descriptors and addresses in uniform
+// registers; a lone thread in a divergent branch moves each of them there for every instruction.  Measured on MMAs of
+// 128 x 64 x 32 bytes, one CTA per SM: 53 cycles each against 80, and 79 against 128 in a run-time loop of two.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
+// Bounded wait by a whole warp that runs uniformly; the same answer for all lanes, and known to be.
+__device__ __forceinline__ bool mbar_wait_bounded_uniform(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t max_spins) {
+    for (uint32_t i = 0; i < max_spins; ++i) {
+        if (__all_sync(0xffffffffu, mbar_try_wait_u32(bar, parity))) return true;
+        if ((i & 63u) == 63u) {
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+            __nanosleep(64);
+        }
+    }
+    *abort_flag = 1;
+    return false;
+}
+
 // Variants taking 32-bit shared-memory addresses, for loops that keep addresses in registers.
 __device__ __forceinline__ bool mbar_test_wait_u32(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -227,10 +246,10 @@ __device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, uint64_t map, uin
         : "memory");
 }
 // Commit of the pair's MMAs: one arrival on the barrier at this shared-memory offset in BOTH CTAs.
-__device__ __forceinline__ void tc_commit_pair_u32(uint32_t bar) {
+__device__ __forceinline__ void tc_commit_pair_u32(uint32_t bar, uint32_t leader = 1u) {
     asm volatile(
-        "{\n\t.reg .b16 m;\n\tmov.b16 m, 3;\n\t"
-        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(bar)
+        "{\n\t.reg .b16 m;\n\t.reg .pred q;\n\tmov.b16 m, 3;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(bar), "r"(leader)
         : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
@@ -248,77 +267,86 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 // The same with separate high halves for A and B (row-box operands: A's stride differs from B's).
 template <bool kInt8>
 __device__ __forceinline__ void tc_mma_ab_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
-                                               uint32_t idesc, uint32_t accumulate) {
+                                               uint32_t idesc, uint32_t accumulate, uint32_t leader = 1u) {
     if (kInt8) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
             "mov.b64 da, {%1, %2};\n\t"
             "mov.b64 db, {%3, %4};\n\t"
             "setp.ne.b32 p, %6, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+            "setp.ne.b32 q, %7, 0;\n\t"
+            "@q tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
     } else {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
             "mov.b64 da, {%1, %2};\n\t"
             "mov.b64 db, {%3, %4};\n\t"
             "setp.ne.b32 p, %6, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+            "setp.ne.b32 q, %7, 0;\n\t"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
     }
 }
 template <bool kInt8>
 __device__ __forceinline__ void tc_mma_lohi_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
-                                                 uint32_t idesc, uint32_t accumulate) {
+                                                 uint32_t idesc, uint32_t accumulate, uint32_t leader = 1u) {
     if (kInt8) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
             "mov.b64 da, {%1, %3};\n\t"
             "mov.b64 db, {%2, %3};\n\t"
             "setp.ne.b32 p, %5, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+            "setp.ne.b32 q, %6, 0;\n\t"
+            "@q tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
     } else {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
             "mov.b64 da, {%1, %3};\n\t"
             "mov.b64 db, {%2, %3};\n\t"
             "setp.ne.b32 p, %5, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+            "setp.ne.b32 q, %6, 0;\n\t"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
     }
 }
 
-__device__ __forceinline__ void tc_commit_u32(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void tc_commit_u32(uint32_t bar, uint32_t leader = 1u) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(leader)
+        : "memory");
 }
 // MMA with the two shared-memory descriptors given as (low, high) 32-bit halves: the high half
 // (stride, version, swizzle) is loop-invariant and the low half (address >> 4 | LBO) advances by
 // plain 32-bit adds.
 template <bool kInt8>
 __device__ __forceinline__ void tc_mma_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
-                                            uint32_t idesc, uint32_t accumulate) {
+                                            uint32_t idesc, uint32_t accumulate, uint32_t leader = 1u) {
     if (kInt8) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
             "mov.b64 da, {%1, %3};\n\t"
             "mov.b64 db, {%2, %3};\n\t"
             "setp.ne.b32 p, %5, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+            "setp.ne.b32 q, %6, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
     } else {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
             "mov.b64 da, {%1, %3};\n\t"
             "mov.b64 db, {%2, %3};\n\t"
             "setp.ne.b32 p, %5, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+            "setp.ne.b32 q, %6, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
     }
 }
@@ -326,24 +354,26 @@ __device__ __forceinline__ void tc_mma_lohi(uint32_t d_tmem, uint32_t a_lo, uint
 // The same with separate high halves for the two descriptors (A and B tiles with different strides).
 template <bool kInt8>
 __device__ __forceinline__ void tc_mma_ab(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
-                                          uint32_t idesc, uint32_t accumulate) {
+                                          uint32_t idesc, uint32_t accumulate, uint32_t leader = 1u) {
     if (kInt8) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
             "mov.b64 da, {%1, %2};\n\t"
             "mov.b64 db, {%3, %4};\n\t"
             "setp.ne.b32 p, %6, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+            "setp.ne.b32 q, %7, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
     } else {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
             "mov.b64 da, {%1, %2};\n\t"
             "mov.b64 db, {%3, %4};\n\t"
             "setp.ne.b32 p, %6, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+            "setp.ne.b32 q, %7, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
     }
 }

@@ -2,7 +2,7 @@
 //
 // Every CTA fills a few K blocks of A (128 rows) and B (n rows) in shared memory with seeded values
 // in the 128-byte-swizzled K-major layout the convolution kernel uses, allocates n TMEM columns and lets
-// one thread issue tcgen05.mma (kind::i8 or kind::f16, M = 128, N = n, K = 32 bytes) back to back:
+// one warp issue tcgen05.mma (kind::i8 or kind::f16, M = 128, N = n, K = 32 bytes) back to back:
 // no TMA, no epilogue, no global memory traffic.  What comes out is the denominator of the
 // convolution kernel's tensor roofline: the rate the tensor pipe sustains when nothing else is in
 // its way (for one and for two CTAs per SM, and per N - narrow N tiles run below the peak because
@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(128, 1) tensor_peak_kernel(int m, int n, int k
     const int a_bytes = (m / 8) * a_sbo + 1024, b_bytes = n * kb_bytes;
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem + (size_t)kblk * a_bytes;
-    const int warp = threadIdx.x >> 5;
+    const int warp = ptx::uniform_warp();
     if (threadIdx.x == 0) {
         abort_flag = 0;
         ptx::mbar_init(&done_bar, 1);
@@ -60,7 +60,8 @@ __global__ void __launch_bounds__(128, 1) tensor_peak_kernel(int m, int n, int k
     __syncthreads();
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_smem;
-    if (threadIdx.x == 0) {
+    if (warp == 0) {       // the whole warp, uniformly; one elected lane issues
+        const uint32_t leader = ptx::elect_one() ? 1u : 0u;
         const uint64_t d0 = ptx::make_smem_desc(ptx::smem_u32(smem_a) + (uint32_t)a_shift, (uint32_t)kb_bytes);
         const uint32_t desc_hi = (uint32_t)(d0 >> 32);
         const uint32_t a_hi = (desc_hi & ~0x3FFFu) | (((uint32_t)a_sbo >> 4) & 0x3FFFu);
@@ -73,23 +74,23 @@ __global__ void __launch_bounds__(128, 1) tensor_peak_kernel(int m, int n, int k
         for (int it = 0; it < iters; ++it) {
             uint32_t a_lo = a_lo0, b_lo = b_lo0;
             for (int kb = 0; kb < kblk; ++kb) {
-                if (ksteps == 4) {      // unrolled: the issuing thread's own loop overhead must not be what is measured
-                    ptx::tc_mma_ab<kInt8>(tmem_base, a_lo, a_hi, b_lo, desc_hi, idesc, accumulate);
-                    ptx::tc_mma_ab<kInt8>(tmem_base, a_lo + 2, a_hi, b_lo + 2, desc_hi, idesc, 1);
-                    ptx::tc_mma_ab<kInt8>(tmem_base, a_lo + 4, a_hi, b_lo + 4, desc_hi, idesc, 1);
-                    ptx::tc_mma_ab<kInt8>(tmem_base, a_lo + 6, a_hi, b_lo + 6, desc_hi, idesc, 1);
+                if (ksteps == 4) {      // unrolled: the issuing warp's own loop overhead must not be what is measured
+                    ptx::tc_mma_ab<kInt8>(tmem_base, a_lo, a_hi, b_lo, desc_hi, idesc, accumulate, leader);
+                    ptx::tc_mma_ab<kInt8>(tmem_base, a_lo + 2, a_hi, b_lo + 2, desc_hi, idesc, 1, leader);
+                    ptx::tc_mma_ab<kInt8>(tmem_base, a_lo + 4, a_hi, b_lo + 4, desc_hi, idesc, 1, leader);
+                    ptx::tc_mma_ab<kInt8>(tmem_base, a_lo + 6, a_hi, b_lo + 6, desc_hi, idesc, 1, leader);
                 } else {
                     for (int ks = 0; ks < ksteps; ++ks)
-                        ptx::tc_mma_ab<kInt8>(tmem_base, a_lo + 2 * ks, a_hi, b_lo + 2 * ks, desc_hi, idesc, ks ? 1u : accumulate);
+                        ptx::tc_mma_ab<kInt8>(tmem_base, a_lo + 2 * ks, a_hi, b_lo + 2 * ks, desc_hi, idesc, ks ? 1u : accumulate, leader);
                 }
                 accumulate = 1;
                 a_lo += a_blk;
                 b_lo += b_blk;
             }
         }
-        ptx::tc_commit(&done_bar);
-        if (!ptx::mbar_wait_bounded(&done_bar, 0, &abort_flag, kProbeMaxSpins)) atomicExch(error, 8);
-        if (cycles && blockIdx.x == 0) *cycles = clock64() - t0;
+        ptx::tc_commit_u32(ptx::smem_u32(&done_bar), leader);
+        if (!ptx::mbar_wait_bounded_uniform(ptx::smem_u32(&done_bar), 0, &abort_flag, kProbeMaxSpins) && leader) atomicExch(error, 8);
+        if (cycles && blockIdx.x == 0 && leader) *cycles = clock64() - t0;
     }
     ptx::tc_fence_before_sync();
     __syncthreads();

@@ -442,3 +442,30 @@ def test_conv_persistent_kernel_small(ctx, case):
     np.testing.assert_array_equal(y, np.maximum(acc, 0))
     q, _, _ = run_conv_i8(ctx, xq, wq, None, np.ones(Cout, np.float32), 1.0, stride, pad, capi.EXB_I8, act=1, out_scale=np.float32(1e-3), impl=2)
     np.testing.assert_array_equal(q, O.requantize_rne(np.maximum(acc, 0), np.float32(1e-3)))
+
+
+# CTA pairs of the persistent kernel: along the images (odd group counts) and, with one image, along the rows (odd tile
+# rows); row-box and tap loops, both epilogues, two N tiles.  Integer values, so that every path is exact.
+@pytest.mark.parametrize("case", [(3, 64, 115, 113, 64, 3, 1, "f16"), (1, 64, 200, 210, 64, 3, 1, "f16"),
+                                  (1, 64, 401, 400, 64, 3, 2, "f16"), (3, 64, 230, 226, 128, 3, 2, "f16"),
+                                  (1, 128, 401, 400, 96, 3, 2, "i8"), (2, 128, 300, 270, 64, 3, 2, "i8"),
+                                  (5, 512, 9, 7, 160, 1, 1, "i8"), (5, 256, 9, 7, 192, 1, 1, "f16"),
+                                  (3, 64, 9, 9, 320, 3, 1, "i8"), (1, 64, 37, 9, 320, 3, 1, "f16")])
+def test_conv_pairs(ctx, case):
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s, dtype = case
+    r = rng(sum(case[:7]) + 22)
+    xq = r.integers(-8, 9, (N, Cin, H, W)).astype(np.int8)
+    wq = r.integers(-8, 9, (Cout, Cin, k, k)).astype(np.int8)
+    ref = O.conv2d_i8_acc(xq, wq, s, k // 2)
+    if dtype == "i8":
+        q, _, _ = run_conv_i8(ctx, xq, wq, None, np.ones(Cout, np.float32), 1.0, s, k // 2, capi.EXB_I8, out_scale=np.float32(0.03), impl=2)
+        np.testing.assert_array_equal(q, O.requantize_rne(ref.astype(np.float32), np.float32(0.03)))
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8 if dtype == "i8" else capi.EXB_F16, capi.EXB_F32, impl=2)
+    if dtype == "i8":
+        p = capi.ConvWeights(ctx, d, wq, None, np.ones(Cout, np.float32), 1.0)
+    else:
+        p = capi.ConvWeights(ctx, d, wq.astype(np.float32), np.zeros(Cout, np.float32))
+    y, _ = capi.conv2d(ctx, d, dev(to_nhwc(xq).astype(np.int8 if dtype == "i8" else np.float16)), p)
+    ctx.sync_check()
+    np.testing.assert_array_equal(to_nchw(host(y)), ref.astype(np.float32))
