@@ -404,10 +404,10 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
         s_scale[at] = in ? p.e.scale[c] : 0.f;
         s_bias[at] = in ? p.e.bias[c] : 0.f;
     }
-    // Programmatic dependent launch: everything above touches only this launch's own parameters,
-    // constant weights and on-chip state, so it may run while the previous kernel of the stream is
-    // still draining; nothing below may start before that kernel's memory is complete and visible.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // Programmatic dependent launch: everything up to a role's own griddepcontrol.wait touches only this launch's
+    // parameters, constant weights and on-chip state, so it may run while the previous kernel of the stream is still
+    // draining.  The producer waits before its first activation load, the epilogue before it reads or writes global
+    // memory; the weights of the first stages (or all of them, resident) are on their way by then.
     ptx::tc_fence_before_sync();
     __syncthreads();
     if (kPair) ptx::cluster_sync();      // the peer's barriers are initialised before anything signals them
@@ -456,6 +456,35 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                 }
             }
         }
+        auto load_b = [&](uint32_t fb, int stage_, int w, int ncoord) {
+            for (int sx = 0; sx < p.taps; ++sx) {
+                const uint32_t dst = b_base + stage_ * b_stage + (uint32_t)(sx * p.b_bytes);
+                const int kc = (w & 0x0fffffff) + sx * p.cin_pad;
+                if (kPair) {
+                    if (bperm) ptx::tma_load_5d_pair(dst, mapB, fb, kc, 0, 0, 0, ncoord >> 5);
+                    else ptx::tma_load_2d_pair(dst, mapB, fb, kc, ncoord);
+                } else {
+                    if (bperm) ptx::tma_load_5d_u32(dst, mapB, fb, kc, 0, 0, 0, ncoord >> 5);
+                    else ptx::tma_load_2d_u32(dst, mapB, fb, kc, ncoord);
+                }
+            }
+        };
+        // a stage's barrier (pair mode: both CTAs' boxes complete on the rank-0 CTA's, which expects the bytes of both)
+        auto stage_bar = [&](int stage_) { return kPair ? ptx::map_to_cta(full0 + stage_ * 8, 0) : full0 + stage_ * 8; };
+        auto expect = [&](int stage_, int nb) {
+            if (lane == 0 && cta_rank == 0) ptx::mbar_arrive_expect_tx_u32(full0 + stage_ * 8, (kPair ? 2u : 1u) * tx * (uint32_t)nb);
+        };
+        // streamed weights: the first tile's, as far as the ring reaches
+        int early = 0;
+        if (!p.patch && !bres && lane < G && first_unit < total_tiles) {
+            const int ncoord = tile_of(TileCursor(p, first_unit, unit_step)).ntile * p.BN + (kPair ? (int)cta_rank * (p.BN >> 1) : 0);
+            for (int it0 = 0; it0 < k_iters && early < p.stages; it0 += G, ++early) {
+                const int nb = min(G, k_iters - it0);
+                expect(early, nb);
+                if (lane < nb) load_b(stage_bar(early), early, k_tab[it0 + lane].w, ncoord);
+            }
+        }
+        pdl_wait();
         if (p.patch) {
             if (lane == 0) {
                 const uint32_t bytes = (uint32_t)(p.patch_rows * p.patch_pitch);
@@ -505,38 +534,16 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                         ok = 0;
                         break;
                     }
-                    if (kPair) {
-                        // both CTAs' boxes complete on the rank-0 CTA's barrier, which expects the bytes of both
-                        const uint32_t fb = ptx::map_to_cta(full0 + stage * 8, 0);
-                        if (lane == 0 && cta_rank == 0) ptx::mbar_arrive_expect_tx_u32(full0 + stage * 8, 2u * tx * (uint32_t)nb);
-                        if (mine) {
-                            ptx::tma_load_4d_pair(a_base + stage * a_stage, mapA0 + ((uint32_t)e.w >> 28) * sizeof(CUtensorMap), fb,
-                                                  e.x, tc.ow0 + e.y, tc.oh0 + e.z, tc.n0);
-                            if (!bres) {
-                                for (int sx = 0; sx < p.taps; ++sx) {
-                                    const uint32_t dst = b_base + stage * b_stage + (uint32_t)(sx * p.b_bytes);
-                                    const int kc = (e.w & 0x0fffffff) + sx * p.cin_pad;
-                                    if (bperm) ptx::tma_load_5d_pair(dst, mapB, fb, kc, 0, 0, 0, ncoord >> 5);
-                                    else ptx::tma_load_2d_pair(dst, mapB, fb, kc, ncoord);
-                                }
-                            }
-                        }
-                    } else {
-                    const uint32_t fb = full0 + stage * 8;
-                    if (lane == 0) ptx::mbar_arrive_expect_tx_u32(fb, tx * (uint32_t)nb);
+                    const uint32_t fb = stage_bar(stage);
+                    if (early == 0) expect(stage, nb);
                     if (mine) {
-                        ptx::tma_load_4d_u32(a_base + stage * a_stage, mapA0 + ((uint32_t)e.w >> 28) * sizeof(CUtensorMap), fb,
-                                             e.x, tc.ow0 + e.y, tc.oh0 + e.z, tc.n0);
-                        if (!bres) {
-                            for (int sx = 0; sx < p.taps; ++sx) {
-                                const uint32_t dst = b_base + stage * b_stage + (uint32_t)(sx * p.b_bytes);
-                                const int kc = (e.w & 0x0fffffff) + sx * p.cin_pad;
-                                if (bperm) ptx::tma_load_5d_u32(dst, mapB, fb, kc, 0, 0, 0, ncoord >> 5);
-                                else ptx::tma_load_2d_u32(dst, mapB, fb, kc, ncoord);
-                            }
-                        }
+                        const uint64_t mapA = mapA0 + ((uint32_t)e.w >> 28) * sizeof(CUtensorMap);
+                        const uint32_t dst = a_base + stage * a_stage;
+                        if (kPair) ptx::tma_load_4d_pair(dst, mapA, fb, e.x, tc.ow0 + e.y, tc.oh0 + e.z, tc.n0);
+                        else ptx::tma_load_4d_u32(dst, mapA, fb, e.x, tc.ow0 + e.y, tc.oh0 + e.z, tc.n0);
+                        if (!bres && early == 0) load_b(fb, stage, e.w, ncoord);
                     }
-                    }
+                    if (early > 0) --early;
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1u;
@@ -707,6 +714,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
         // Tile i of this CTA's sequence is accumulated in buffer i % acc_bufs (use number i / acc_bufs of that
         // buffer gives the barrier parity) and drained by group i % epi_groups.  A group has kEpiWarps /
         // epi_groups warps: one or two per TMEM lane quarter; two share the quarter's work.
+        pdl_wait();
         const int e = warp - kFirstEpiWarp;
         const int q = warp & 3;                 // TMEM lane quarter: a warp can only reach lanes 32*(warp%4)..+31
         const int nsub = kEpiWarps / 4 / p.epi_groups;
