@@ -310,12 +310,11 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
 
 }  // namespace
 
-// Which kernel, and how a tile is divided: modelled time in us of both kernels, fitted to 170 layers (batch 1 to 64,
-// 1x1 and 3x3, 16 to 512 channels, 1 to 96 x 128-pixel tiles of one image group; every split of 32 and 64 channels).
+// Which kernel, and how a tile is divided: modelled time in us of both kernels, fitted to 330 layers (batch 1 to 64,
+// 1x1 and 3x3, 32 to 1280 channels, maps of 7 x 7 to 80 x 80; every split of 32 and 64 channels).
 // Split kernel: a constant, the cluster's exchange, then K blocks and epilogue of a tile one after the other, stretched by
-// the tiles per SM once there are more than SMs.  Persistent kernel: a constant and rounds of tiles.  The pick is within
-// 1 % of the faster kernel's best split on average and never slower than the persistent kernel on these layers; the line
-// lies near one tile of 64 channels per SM and a half, later for deep reductions.
+// the tiles per SM once there are more than SMs.  Persistent kernel: a constant and rounds of tiles.  On these layers the
+// pick is on average 1 to 2 % slower than the fastest of all; the line lies near two tiles of 64 channels per SM.
 ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
     const ConvSplit none = {0, 0};
     if (g.pool || g.out_dtype == EXB_I32 || (g.cout_stride & 7) || (g.y_pitch & 7) || conv_fold_plan(g).on) return none;
@@ -327,26 +326,38 @@ ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
     if (m_tiles > 8.0 * ctx->sm_count) return none;
     ConvSplit best = none;
     double best_t = 1e30;
-    static const double kSync[4] = {0.0, 0.56, 1.33, 2.33};
+    static const double kSync[4] = {0.0, 0.43, 1.23, 2.02};
     for (int bn = 32; bn <= 64; bn *= 2)
         for (int sp = 1, i = 0; sp <= 8 && sp <= k_iters; sp *= 2, ++i) {
             const double ctas = m_tiles * ((w->cout_pad + bn - 1) / bn) * sp;
-            const double stretch = ctas > 1.035 * ctx->sm_count ? ctas / (1.035 * ctx->sm_count) : 1.0;
+            const double stretch = ctas > 1.05 * ctx->sm_count ? ctas / (1.05 * ctx->sm_count) : 1.0;
             const double units = (k_iters + sp - 1) / sp;
-            const double t = 1.9 + kSync[i] + stretch * (units * (kb == 32 ? 0.24 : 0.31) + (bn == 32 ? 1.05 : 2.35) + 0.52 * kSync[i]);
+            const double step = kb == 32 ? 0.203 : kb == 64 ? 0.239 : 0.246;
+            const double t = 1.93 + kSync[i] + stretch * (units * step + (bn == 32 ? 1.09 : 2.23) + 0.36 * kSync[i]);
             if (t < best_t) {
                 best_t = t;
                 best.BN = bn;
                 best.splits = sp;
             }
         }
-    const int n_tiles = (w->cout_pad + 255) / 256, bn = round_up((w->cout_pad + n_tiles - 1) / n_tiles, 16);
-    const double tiles = m_tiles * n_tiles, slots = (double)ctx->sm_count * (bn <= 128 ? 2 : 1);
+    const ConvNTile nt = conv_n_tile(ctx, g, w->cout_pad, (int64_t)m_tiles);
+    const int bn = nt.BN;
+    const bool two = bn <= 128 && !nt.paired;
+    const double tiles = m_tiles * nt.n_tiles, slots = (double)ctx->sm_count * (two ? 2 : 1);
     const double rounds = tiles <= slots ? 1.0 : ceil(tiles / slots);
     double share = 1.0;      // two CTAs of an SM share its tensor pipe
-    if (bn <= 128 && tiles > ctx->sm_count) share += 0.29 * (tiles < 2 * ctx->sm_count ? tiles / ctx->sm_count - 1 : 1.0);
-    const double step = (bn <= 64 ? 0.30 : bn <= 128 ? 0.28 : 0.35) * (kb == 128 ? 1.0 : kb == 64 ? 0.68 : 0.61);
-    const double persistent = 4.6 + rounds * (k_iters * step + (bn <= 64 ? 0.54 : bn <= 128 ? 2.9 : 1.84) + (g.has_res ? 0.5 : 0.0)) * share;
+    if (two && tiles > ctx->sm_count) share += 0.20 * (tiles < 2 * ctx->sm_count ? tiles / ctx->sm_count - 1 : 1.0);
+    double step = 0.305, rest = 5.14;       // one CTA (or pair) per SM, more than 128 channels
+    if (two) {
+        step = bn <= 64 ? 0.246 : 0.19;
+        rest = bn <= 64 ? 0.93 : 2.94;
+    } else if (nt.paired) {
+        step = 0.208;
+        rest = 2.24;
+    }
+    if (bn > 128 && k_iters * kb < 512) rest = 1.6;      // single CTAs of short reductions
+    step *= kb == 128 ? 1.0 : kb == 64 ? 0.21 : 0.39;
+    const double persistent = 4.58 + rounds * (k_iters * step + rest + (g.has_res ? 0.45 : 0.0)) * share;
     return best_t < 0.98 * persistent ? best : none;
 }
 

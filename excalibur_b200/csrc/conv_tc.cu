@@ -1111,6 +1111,33 @@ bool conv_tc_eligible(const ConvGeom& g) {
     return true;
 }
 
+// The N tile: 256 channels, or 128 where that is the faster one.
+//  - Below 512 bytes of K, and up to 1152 in the first two rounds of tiles, the epilogue sets the pace, and two CTAs of
+//    128 channels per SM drain more than one of 256: 96 -> 576 int8 1x1 at 256 x 14 x 14 23.8 -> 21.4 us, 320 -> 1280 at
+//    256 x 7 x 7 18.4 -> 16.1, 128 -> 256 int8 3x3 stride 2 at 50 x 28 x 28 11.2 -> 9.3 (but 19.8 -> 21.4 at 256 images).
+//    Not for fewer than 256 channels and a shorter K, which two smaller tiles only read twice (32 -> 192 at
+//    256 x 28 x 28: 23.6 us in one tile, 28.4 in two).
+//  - Beyond that tiles run as pairs, sm_count / 2 at a time, and a pair of 128-channel tiles takes about 0.63 of the time
+//    of one of 256 (half the MMA time, but the same activations): 128 where its rounds of pairs come to less.
+//    512 -> 512 3x3 fp16 at 64 x 7 x 7: 26 pairs of 256 on 74 places 30.9 us, 52 of 128 24.0; 256 -> 256 int8 at
+//    100 x 14 x 14: two rounds 21.8, three of 128 19.4; 256 -> 256 fp16 at 64 x 14 x 14: one round 22.3, two of 128 23.5.
+ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64_t m_tiles) {
+    auto tile = [&](int most) {
+        const int n = (cout_pad + most - 1) / most;
+        return ConvNTile{n, round_up((cout_pad + n - 1) / n, 16), false};
+    };
+    const ConvNTile wide = tile(256), narrow = tile(128);
+    const int64_t k_bytes = (int64_t)g.kh * g.kw * g.cin_stride * (g.in_dtype == EXB_I8 ? 1 : 2);
+    if (cout_pad <= 128 || (cout_pad < 256 && k_bytes < 512) || conv_fold_plan(g).on) return wide;
+    if (k_bytes < 512 || (k_bytes <= 1152 && m_tiles * narrow.n_tiles <= 4 * ctx->sm_count)) return narrow;
+    const int64_t places = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
+    auto rounds = [&](const ConvNTile& t) { return (double)(((m_tiles + 1) / 2 * t.n_tiles + places - 1) / places); };
+    if (narrow.BN % 64 != 0 || 0.63 * rounds(narrow) >= rounds(wide)) return wide;      // (a pair splits whole 32-channel blocks)
+    ConvNTile t = narrow;
+    t.paired = true;
+    return t;
+}
+
 int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_conv_weights* w,
                    const void* residual, void* y, void* y2, cudaStream_t st) {
     auto encode = tensor_map_encoder();
@@ -1128,8 +1155,9 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     p.tiles_h = (g.OH + p.TH - 1) / p.TH;
     p.tiles_nb = (g.N + p.TN - 1) / p.TN;
     p.step_w = p.TW; p.step_h = p.TH; p.step_n = p.TN; p.org = 0;
-    p.n_tiles = (w->cout_pad + 255) / 256;
-    p.BN = round_up((w->cout_pad + p.n_tiles - 1) / p.n_tiles, 16);
+    const ConvNTile nt = conv_n_tile(ctx, g, w->cout_pad, (int64_t)p.tiles_w * p.tiles_h * p.tiles_nb);
+    p.n_tiles = nt.n_tiles;
+    p.BN = nt.BN;
     // Two CTAs per SM when the N tile is narrow (see the kernel's comment).
     bool two = p.BN <= 128;
     p.kh = g.kh; p.kw = g.kw; p.stride = g.sh; p.pad_t = g.pt; p.pad_l = g.pl;
@@ -1270,7 +1298,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     else if (p.BN > 128)
         pair = pairable && k_bytes >= 512;
     else if (p.BN >= 64)
-        pair = pairable && k_bytes >= 1152 && all_tiles > 2 * ctx->sm_count;
+        pair = pairable && k_bytes >= 1152 && (nt.paired || all_tiles > 2 * ctx->sm_count);
     if (pair) {
         two = false;
         p.b_bytes = (p.BN / 2) * p.kb_bytes;

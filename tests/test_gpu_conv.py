@@ -450,7 +450,10 @@ def test_conv_persistent_kernel_small(ctx, case):
                                   (1, 64, 401, 400, 64, 3, 2, "f16"), (3, 64, 230, 226, 128, 3, 2, "f16"),
                                   (1, 128, 401, 400, 96, 3, 2, "i8"), (2, 128, 300, 270, 64, 3, 2, "i8"),
                                   (5, 512, 9, 7, 160, 1, 1, "i8"), (5, 256, 9, 7, 192, 1, 1, "f16"),
-                                  (3, 64, 9, 9, 320, 3, 1, "i8"), (1, 64, 37, 9, 320, 3, 1, "f16")])
+                                  (3, 64, 9, 9, 320, 3, 1, "i8"), (1, 64, 37, 9, 320, 3, 1, "f16"),
+                                  # more than 256 channels: N tiles of 128 or fewer, single and as pairs
+                                  (2, 128, 9, 9, 272, 1, 1, "i8"), (3, 64, 17, 9, 408, 3, 1, "f16"), (2, 128, 9, 9, 384, 3, 1, "f16"),
+                                  (3, 256, 7, 7, 512, 3, 1, "i8")])
 def test_conv_pairs(ctx, case):
     capi = _capi()
     N, Cin, H, W, Cout, k, s, dtype = case
