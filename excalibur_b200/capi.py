@@ -22,8 +22,8 @@ EXPORTED_SYMBOLS = [
     "exb_conv2d_fwd", "exb_conv2d_uses_tensor_cores", "exb_conv2d_pool_fusable", "exb_dw_weights_pack", "exb_dw_weights_destroy",
     "exb_dwconv2d_fwd", "exb_pool_out_dims", "exb_pool2d_fwd", "exb_pool2d_nchw_f32_static", "exb_eltwise_fwd", "exb_binaryop_fwd",
     "exb_binaryop_scalar_fwd", "exb_relu_fwd", "exb_activation_fwd", "exb_quantize_fwd",
-    "exb_dequantize_fwd", "exb_concat_fwd", "exb_interp_nearest_fwd", "exb_channel_affine_fwd",
-    "exb_conv_weights_set_slopes", "exb_dw_weights_set_slopes", "exb_depth_to_space_nchw_f32", "exb_image_f32_to_nhwc_norm", "exb_nchw_f32_to_nhwc4_padded_norm", "exb_nhwc_f16_split_heads_f32", "exb_hardsigmoid_fwd", "exb_softmax_channels_f32", "exb_binaryop_channel_bcast_fwd", "exb_nchw_f16_to_nhwc4_padded", "exb_nchw_f32_focus_to_nhwc_f16", "exb_channel_affine_prelu_fwd", "exb_hardswish_fwd", "exb_focus_fwd", "exb_prelu_fwd", "exb_depth_to_space_fwd", "exb_transpose_hw_f32",
+    "exb_dequantize_fwd", "exb_concat_fwd", "exb_concat_nearest_fwd", "exb_interp_nearest_fwd", "exb_channel_affine_fwd",
+    "exb_conv_weights_set_slopes", "exb_dw_weights_set_slopes", "exb_depth_to_space_nchw_f32", "exb_deconv_few_f32", "exb_image_f32_to_nhwc_norm", "exb_nchw_f32_to_nhwc4_padded_norm", "exb_nhwc_f16_split_heads_f32", "exb_hardsigmoid_fwd", "exb_softmax_channels_f32", "exb_binaryop_channel_bcast_fwd", "exb_nchw_f16_to_nhwc4_padded", "exb_nchw_f32_focus_to_nhwc_f16", "exb_channel_affine_prelu_fwd", "exb_hardswish_fwd", "exb_focus_fwd", "exb_prelu_fwd", "exb_depth_to_space_fwd", "exb_transpose_hw_f32",
 ]
 
 
@@ -99,6 +99,9 @@ def lib():
         L.exb_quantize_fwd.argtypes = [vp, vp, i32, vp, i64, f32, i32, vp]
         L.exb_dequantize_fwd.argtypes = [vp, vp, vp, i32, i64, f32, vp]
         L.exb_concat_fwd.argtypes = [vp, i32, C.POINTER(vp), C.POINTER(i64), C.POINTER(i64), vp, i64, i64, i32, vp]
+        pi32 = C.POINTER(C.c_int32)
+        L.exb_deconv_few_f32.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp]
+        L.exb_concat_nearest_fwd.argtypes = [vp, i32, C.POINTER(vp), pi32, pi32, pi32, pi32, vp, i32, i32, i32, i32, vp]
         L.exb_interp_nearest_fwd.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp]
         L.exb_channel_affine_fwd.argtypes = [vp, vp, vp, vp, vp, i64, i32, i32, i64, i32, i32, i32, vp]
         L.exb_hardswish_fwd.argtypes = [vp, vp, vp, i64, i32, f32, f32, vp]

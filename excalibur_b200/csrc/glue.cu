@@ -3,6 +3,8 @@
 // are single-pass, bandwidth-bound copies; 16-byte vectors where strides allow, scalars otherwise.
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace exb {
 namespace {
 
@@ -32,6 +34,38 @@ __global__ void __launch_bounds__(kThreads) concat_rows_kernel(ConcatArgs a, U* 
         for (int j = 1; j < kMaxConcatInputs; ++j)
             if (j < a.n_in && c >= a.offset[j]) k = j;
         y[r * y_stride + c] = static_cast<const U*>(a.x[k])[r * a.stride[k] + (c - a.offset[k])];
+    }
+}
+
+// Channel concatenation of fp16 maps, each read through its own nearest resize: a block writes a stretch of one output
+// row.  Bound by its writes.  One pass instead of a resize pass per input (each writing what the concatenation then
+// reads) and the copy: four inputs of 64 channels, three of them 2, 4 and 8 times smaller, onto 4 x 120 x 184:
+// about 45 us in five launches, 14 in one.  A thread per vector that looked its input up for each took 28.
+struct ConcatNearestArgs {
+    const uint4* x[kMaxConcatInputs];      // inputs that are copied here
+    int first[kMaxConcatInputs + 1];       // their first vector, counted over the copied ones
+    int to[kMaxConcatInputs];              // and in the output pixel
+    int stride[kMaxConcatInputs], H[kMaxConcatInputs], W[kMaxConcatInputs];
+    float hs[kMaxConcatInputs], ws[kMaxConcatInputs];
+    int n_in, OH, OW, y_stride;
+};
+__global__ void __launch_bounds__(kThreads) concat_nearest_kernel(const __grid_constant__ ConcatNearestArgs a, uint4* __restrict__ y) {
+    pdl_enter();
+    const int row = blockIdx.x, n = row / a.OH, oy = row - n * a.OH;
+    const int chunk = (a.OW + gridDim.y - 1) / gridDim.y, x0 = blockIdx.y * chunk, x1 = min(x0 + chunk, a.OW);
+    // a thread keeps its vector of the pixel, and with it the input and the input's row
+    const int total = a.first[a.n_in], per = min(total, kThreads), step = kThreads / per;
+    const int dx = threadIdx.x / per;
+    if (dx >= step) return;
+    for (int v = threadIdx.x - dx * per; v < total; v += per) {
+        int p = 0;
+        while (v >= a.first[p + 1]) ++p;
+        const int iy = min((int)(oy * a.hs[p]), a.H[p] - 1), k = v - a.first[p], last = a.W[p] - 1, xs = a.stride[p];
+        const float ws = a.ws[p];
+        const uint4* src = a.x[p] + ((int64_t)n * a.H[p] + iy) * a.W[p] * xs + k;
+        uint4* out = y + (int64_t)row * a.OW * a.y_stride + a.to[p] + k;
+#pragma unroll 4
+        for (int ox = x0 + dx; ox < x1; ox += step) out[(int64_t)ox * a.y_stride] = __ldg(src + min((int)(ox * ws), last) * xs);
     }
 }
 
@@ -477,6 +511,48 @@ extern "C" int exb_concat_fwd(exb_ctx* ctx, int n_in, const void* const* xs, con
         else launch_overlapped(ctx, concat_rows_kernel<uint32_t>, grid, kThreads, st, a, static_cast<uint32_t*>(y), y_stride, rows);
     }
     return after_launch("exb_concat_fwd");
+}
+
+extern "C" int exb_concat_nearest_fwd(exb_ctx* ctx, int n_in, const void* const* xs, const int32_t* channels,
+                                      const int32_t* x_strides, const int32_t* heights, const int32_t* widths, void* y,
+                                      int y_stride, int N, int OH, int OW, void* stream) {
+    EXB_REQUIRE(ctx != nullptr, "null context");
+    EXB_REQUIRE(n_in >= 1 && xs && channels && x_strides && heights && widths && y, "exb_concat_nearest_fwd: null argument or no inputs");
+    if (n_in > kMaxConcatInputs)
+        return fail(EXB_ERR_UNSUPPORTED, "concat supports at most %d inputs, got %d", kMaxConcatInputs, n_in);
+    EXB_REQUIRE(N >= 0 && OH > 0 && OW > 0 && y_stride % 8 == 0 && aligned16(y), "exb_concat_nearest_fwd: bad output shape or alignment");
+    ConcatNearestArgs a;
+    memset(&a, 0, sizeof(a));
+    int off = 0, copied = 0;
+    for (int i = 0; i < n_in; ++i) {
+        EXB_REQUIRE(channels[i] > 0 && channels[i] % 8 == 0 && x_strides[i] % 8 == 0 && x_strides[i] >= channels[i] && heights[i] > 0 &&
+                        widths[i] > 0 && aligned16(xs[i]), "exb_concat_nearest_fwd: input %d: channels and strides need to be multiples of 8", i);
+        if (xs[i]) {
+            const int k = a.n_in++;
+            a.x[k] = static_cast<const uint4*>(xs[i]);
+            a.first[k] = copied;
+            a.to[k] = off / 8;
+            a.stride[k] = x_strides[i] / 8;
+            a.H[k] = heights[i]; a.W[k] = widths[i];
+            a.hs[k] = heights[i] / (float)OH; a.ws[k] = widths[i] / (float)OW;
+            copied += channels[i] / 8;
+            a.first[k + 1] = copied;
+        }
+        off += channels[i];
+    }
+    EXB_REQUIRE(y_stride >= off, "exb_concat_nearest_fwd: output stride %d smaller than the summed width %d", y_stride, off);
+    if (N == 0 || copied == 0) return EXB_OK;
+    a.OH = OH; a.OW = OW; a.y_stride = y_stride / 8;
+    const int64_t rows = (int64_t)N * OH;
+    EXB_REQUIRE(rows < (1ll << 31) && (int64_t)OW * copied < (1ll << 31), "exb_concat_nearest_fwd: map too large");
+    // pieces of a row: up to the eight blocks an SM holds, but no block gets less than one vector per thread
+    int64_t pieces = std::max<int64_t>(1, 8ll * ctx->sm_count / rows);
+    const int64_t most = ((int64_t)OW * copied + kThreads - 1) / kThreads;
+    if (pieces > most) pieces = most;
+    if (pieces > OW) pieces = OW;
+    launch_overlapped(ctx, concat_nearest_kernel, dim3((unsigned)rows, (unsigned)pieces), kThreads, static_cast<cudaStream_t>(stream), a,
+                      static_cast<uint4*>(y));
+    return after_launch("exb_concat_nearest_fwd");
 }
 
 extern "C" int exb_interp_nearest_fwd(exb_ctx* ctx, const void* x, void* y, int N, int H, int W, int C, int c_stride,

@@ -9,6 +9,7 @@
 #include <cmath>
 #include <fstream>
 #include <functional>
+#include <map>
 #include <set>
 
 #include "host_convert.hpp"
@@ -580,30 +581,92 @@ void fused_plan::layout(slice& sl, bool f16_src) {
     // no fused pooling) that nothing else reads and whose channel count is a multiple of 16.  A BatchNorm (+
     // activation) behind such a Concat of activation-free convolutions is folded slice by slice into them
     // (the BottleneckCSP tail: conv, conv -> Concat -> BatchNorm -> LeakyRelu).
+    // A Concat with other inputs too is one copy kernel of those: it leaves out what such groups store themselves and
+    // reads a nearest Interp that only feeds the Concat at the Interp's own input.
     std::vector<int> cat_left(n_ops, 0);      // producers of a direct Concat still to be emitted
+    std::map<int, int> cat_source;            // output of an Interp that a Concat's copy stands in for -> the Interp
+    std::set<int> cat_stored;                 // inputs of a Concat that their groups store
+    std::vector<std::vector<int>> cat_copy(n_ops);      // channels of the inputs of such a Concat
+    // channels of a map, -1 where its producer does not tell before shapes are known
+    std::function<int(int)> channels_of = [&](int f) -> int {
+        for (size_t i = 0; i < n_ops; ++i) {
+            if (groups[i].conv >= 0 && groups[i].out == f && groups[i].cat < 0) {
+                if (lower_type(params_[i]) != "convolution") return -1;
+                auto* c = dynamic_cast<operation_convolution<float>*>(ops_[groups[i].conv].get());
+                return c ? c->output_channel_ : -1;
+            }
+            if (absorbed[i] || alias_op[i] || groups[i].conv >= 0 || out_ids[i].size() != 1 || root(out_ids[i][0]) != f) continue;
+            const std::string t = lower_type(params_[i]);
+            if (t == "interp" || t == "pooling" || act_of_op((int)i) >= 0 || (t == "binaryop" && is_plain_add((int)i)))
+                return channels_of(root(in_ids[i][0]));
+            return -1;
+        }
+        return -1;
+    };
     for (size_t k = 0; k < n_ops; ++k) {
         if (absorbed[k] || lower_type(params_[k]) != "concat") continue;
         auto* cc = dynamic_cast<operation_concat<float>*>(ops_[k].get());
         if (!cc || !cc->is_channel_concat() || in_ids[k].size() < 2) continue;
         std::vector<int> prod;
-        bool ok = true, plain = true;
+        bool plain = true;
         int total = 0;
-        for (int f : in_ids[k]) {
-            const int rf = root(f);
+        // the group that can store input rf itself, or -1
+        auto storing_group = [&](int rf) -> int {
             int gi = -1;
             for (size_t i = 0; i < k; ++i)
                 if (groups[i].conv >= 0 && groups[i].out == rf) gi = (int)i;
-            if (gi < 0 || sole_consumer(rf) != (int)k || std::find(prod.begin(), prod.end(), gi) != prod.end()) { ok = false; break; }
+            if (gi < 0 || sole_consumer(rf) != (int)k) return -1;
             const group& g = groups[gi];
             auto* conv = dynamic_cast<operation_convolution<float>*>(ops_[g.conv].get());
             if (lower_type(params_[g.conv]) != "convolution" || !conv || conv->group_ != 1 || g.residual >= 0 || g.pool >= 0 ||
                 g.cat >= 0 || conv->output_channel_ % 16 != 0 || conv->stride_h_ != conv->stride_w_ ||
-                (conv->stride_h_ != 1 && conv->stride_h_ != 2)) { ok = false; break; }
-            plain = plain && g.act == EXB_ACT_NONE && g.bn < 0;
+                (conv->stride_h_ != 1 && conv->stride_h_ != 2)) return -1;
+            return gi;
+        };
+        for (int f : in_ids[k]) {
+            const int gi = storing_group(root(f));
+            if (gi < 0 || std::find(prod.begin(), prod.end(), gi) != prod.end()) break;
+            plain = plain && groups[gi].act == EXB_ACT_NONE && groups[gi].bn < 0;
             prod.push_back(gi);
-            total += conv->output_channel_;
+            total += dynamic_cast<operation_convolution<float>*>(ops_[groups[gi].conv].get())->output_channel_;
         }
-        if (!ok) continue;
+        if (prod.size() != in_ids[k].size()) {
+            std::vector<int> width;
+            bool whole16 = in_ids[k].size() <= 8;
+            total = 0;
+            for (int f : in_ids[k]) {
+                width.push_back(channels_of(root(f)));
+                whole16 = whole16 && width.back() > 0 && width.back() % 16 == 0;
+                total += width.back();
+            }
+            if (!whole16) continue;
+            int off = 0;
+            bool fused = false;
+            for (size_t q = 0; q < in_ids[k].size(); off += width[q++]) {
+                const int rf = root(in_ids[k][q]), gi = storing_group(rf);
+                if (gi >= 0) {
+                    groups[gi].cat = (int)k;
+                    groups[gi].cat_off = off;
+                    groups[gi].cat_total = total;
+                    groups[gi].out = root(out_ids[k][0]);
+                    cat_stored.insert(rf);
+                    fused = true;
+                    continue;
+                }
+                if (sole_consumer(rf) != (int)k) continue;
+                for (size_t j = 0; j < k; ++j) {
+                    if (absorbed[j] || lower_type(params_[j]) != "interp" || in_ids[j].size() != 1 || root(out_ids[j][0]) != rf) continue;
+                    auto* ip = dynamic_cast<operation_interp<float>*>(ops_[j].get());
+                    if (!ip || ip->resize_type_ != 1 || ip->align_corner_ != 0) continue;
+                    cat_source[rf] = (int)j;
+                    absorbed[j] = 1;
+                    fused = true;
+                    break;
+                }
+            }
+            if (fused) cat_copy[k] = width;
+            continue;
+        }
         int out = root(out_ids[k][0]), bn_op = -1, act = EXB_ACT_NONE, slope_op = -1;
         if (plain) {
             const int j = sole_consumer(out);
@@ -666,7 +729,10 @@ void fused_plan::layout(slice& sl, bool f16_src) {
             else fmaps_[f].need_f16 = true;
             if (groups[i].residual >= 0) fmaps_[groups[i].residual].need_f16 = true;
         } else {
-            for (int f : in_ids[i]) fmaps_[root(f)].need_f16 = true;
+            for (int f : in_ids[i]) {
+                const auto src = cat_source.find(root(f));
+                fmaps_[src == cat_source.end() ? root(f) : root(in_ids[src->second][0])].need_f16 = true;
+            }
         }
     }
     for (int f : output_roots) {
@@ -844,7 +910,6 @@ void fused_plan::layout(slice& sl, bool f16_src) {
             d.cout_stride = round_up(d.Cout, d.Cout > 16 ? 32 : 16);
             const void* xin = form_f16(x);
             auto mid = std::make_shared<dev_buf>();
-            void* tmp = mid->ensure((size_t)x.N * x.H * x.W * d.cout_stride * 2, device_);
             // a few-channel result that only leaves the network: scattered straight into the fp32 NCHW output
             // instead of a 16-channel-padded fp16 map that an export kernel would read back
             const bool to_output = Cout <= 8 && output_roots.count(g.out) && consumers[g.out].empty() && !y.need_i8;
@@ -862,13 +927,21 @@ void fused_plan::layout(slice& sl, bool f16_src) {
                 y.N = x.N; y.C = Cout; y.H = x.H * rh; y.W = x.W * rw; y.cs = Cout;
                 float* dst = static_cast<float*>(form_f32(y));
                 const int n = x.N, h = x.H, wd = x.W, xs = d.cout_stride;
+                y.produced = true;
+                if (rh * rw * Cout <= 4 && x.cs <= 64 && x.cs % 8 == 0) {
+                    const int act = g.act;
+                    add_step(params_[i].name_, [=](cudaStream_t st) {
+                        exb_check(exb_deconv_few_f32(ctx, xin, ow, dst, n, h, wd, rh, rw, Cout, act, st), "exb_deconv_few_f32");
+                    });
+                    return;
+                }
+                void* tmp = mid->ensure((size_t)x.N * x.H * x.W * d.cout_stride * 2, device_);
                 add_step(params_[i].name_, [=](cudaStream_t st) {
                     (void)mid;
                     exb_check(exb_conv2d_fwd(ctx, &d, xin, ow, nullptr, tmp, nullptr, st), "exb_conv2d_fwd");
                     exb_check(exb_depth_to_space_nchw_f32(ctx, tmp, dst, n, h, wd, rh, rw, Cout, xs, st),
                               "exb_depth_to_space_nchw_f32");
                 }, 2);
-                y.produced = true;
                 return;
             }
             y.need_f16 = true;
@@ -884,6 +957,7 @@ void fused_plan::layout(slice& sl, bool f16_src) {
                 exb_check(exb_conv_weights_set_slopes(ctx, w, rep.data(), (int)rep.size()), "exb_conv_weights_set_slopes");
             }
             const int n = x.N, h = x.H, wd = x.W, xs = d.cout_stride, ys = y.cs;
+            void* tmp = mid->ensure((size_t)x.N * x.H * x.W * d.cout_stride * 2, device_);
             add_step(params_[i].name_, [=](cudaStream_t st) {
                 (void)mid;       // keeps the intermediate tensor alive as long as the step
                 exb_check(exb_conv2d_fwd(ctx, &d, xin, w, nullptr, tmp, nullptr, st), "exb_conv2d_fwd");
@@ -941,7 +1015,7 @@ void fused_plan::layout(slice& sl, bool f16_src) {
             add_step(params_[i].name_, [=](cudaStream_t st) {
                 exb_check(exb_conv2d_fwd(ctx, &d, xin, w, nullptr, y1, nullptr, st), "exb_conv2d_fwd");
             });
-            if (--cat_left[g.cat] == 0) finish_forms(y, false);
+            if (cat_copy[g.cat].empty() && --cat_left[g.cat] == 0) finish_forms(y, false);
             return;
         }
         set_shape(y, x.N, conv->output_channel_, OH, OW);
@@ -998,7 +1072,7 @@ void fused_plan::layout(slice& sl, bool f16_src) {
         if (absorbed[i] || alias_op[i] || t == "convolution" || t == "convolutiondepthwise" || t == "deconvolution") continue;
         fmap_info& x = fmaps_[root(in_ids[i][0])];
         fmap_info& y = fmaps_[root(out_ids[i][0])];
-        CHECK(x.produced) << "feature map " << x.name << " is consumed before it is produced";
+        CHECK(x.produced || !cat_copy[i].empty()) << "feature map " << x.name << " is consumed before it is produced";
         bool plain_copy = false;
         if (t == "reshape" && !x.f32_only && !x.need_f32)
             plain_copy = dynamic_cast<operation_reshape<float>*>(ops_[i].get())->out_shape({x.N, x.C, x.H, x.W}) ==
@@ -1171,6 +1245,47 @@ void fused_plan::layout(slice& sl, bool f16_src) {
         } else if (t == "concat") {
             auto* cc = dynamic_cast<operation_concat<float>*>(ops_[i].get());
             if (!cc->is_channel_concat()) PLAN_REFUSE << "(Concat is implemented along the channel axis, key 0=-1)";
+            if (!cat_copy[i].empty()) {
+                struct inputs {
+                    std::vector<const void*> x;
+                    std::vector<int32_t> channels, strides, heights, widths;
+                };
+                auto in = std::make_shared<inputs>();
+                int OH = 0, OW = 0, total = 0;
+                for (size_t q = 0; q < in_ids[i].size(); ++q) {
+                    const int f = in_ids[i][q];
+                    const auto src = cat_source.find(root(f));
+                    fmap_info& xi = fmaps_[src == cat_source.end() ? root(f) : root(in_ids[src->second][0])];
+                    const bool stored = cat_stored.count(root(f)) != 0;
+                    int h = stored ? y.H : xi.H, w = stored ? y.W : xi.W;
+                    if (src != cat_source.end())
+                        dynamic_cast<operation_interp<float>*>(ops_[src->second].get())->out_dims(xi.H, xi.W, &h, &w);
+                    CHECK((stored || (xi.produced && xi.C == cat_copy[i][q])) && (OH == 0 || (OH == h && OW == w))) << "Concat operands differ in shape";
+                    OH = h;
+                    OW = w;
+                    in->x.push_back(stored ? nullptr : form_f16(xi));
+                    in->channels.push_back(cat_copy[i][q]);
+                    in->strides.push_back(stored ? in->channels.back() : xi.cs);
+                    in->heights.push_back(stored ? h : xi.H);
+                    in->widths.push_back(stored ? w : xi.W);
+                    total += in->channels.back();
+                }
+                const int n = emit_n_;
+                if (y.N == 0) {
+                    y.need_f16 = true;
+                    set_shape(y, n, total, OH, OW);
+                    if (y.cs > total) CUDA_CHECK(cudaMemset(form_f16(y), 0, (size_t)y.N * y.H * y.W * y.cs * 2));
+                }
+                CHECK(y.C == total && y.H == OH && y.W == OW) << "Concat operands differ in shape";
+                void* yo = form_f16(y);
+                const int ys = y.cs;
+                add_step(params_[i].name_, [=](cudaStream_t st) {
+                    exb_check(exb_concat_nearest_fwd(ctx, (int)in->x.size(), in->x.data(), in->channels.data(), in->strides.data(),
+                                                     in->heights.data(), in->widths.data(), yo, ys, n, OH, OW, st), "exb_concat_nearest_fwd");
+                });
+                finish_forms(y, false);
+                continue;
+            }
             auto xs = std::make_shared<std::vector<const void*>>();
             auto widths = std::make_shared<std::vector<int64_t>>();
             auto strides = std::make_shared<std::vector<int64_t>>();

@@ -428,6 +428,11 @@ EXB_API int exb_nhwc_f16_split_heads_f32(exb_ctx* ctx, const void* x, float* y, 
  * is a network output): y[n][c][h*rh + a][w*rw + b] = x[n][h][w][(a*rw + b)*C + c]. */
 EXB_API int exb_depth_to_space_nchw_f32(exb_ctx* ctx, const void* x, float* y, int N, int H, int W, int rh, int rw,
                                         int C, int x_stride, void* stream);
+/* The whole of such a transposed convolution where it has few outputs per pixel: act(1x1 convolution with w) of a
+ * channel-last fp16 x, scattered as above.  rh * rw * C <= 4; x's channel stride is that of the packed weights, a multiple
+ * of 8 up to 64. */
+EXB_API int exb_deconv_few_f32(exb_ctx* ctx, const void* x, const exb_conv_weights* w, float* y, int N, int H, int W,
+                               int rh, int rw, int C, int act, void* stream);
 /* y[p][w][h] = x[p][h][w] for `planes` fp32 planes: operation_transpose with permutation 1,0,2
  * (src/Excalibur/operation_transpose.cpp:47-66). */
 EXB_API int exb_transpose_hw_f32(exb_ctx* ctx, const float* x, float* y, int64_t planes, int H, int W,
@@ -435,6 +440,12 @@ EXB_API int exb_transpose_hw_f32(exb_ctx* ctx, const float* x, float* y, int64_t
 EXB_API int exb_concat_fwd(exb_ctx* ctx, int n_in, const void* const* xs, const int64_t* widths,
                            const int64_t* x_strides, void* y, int64_t y_stride, int64_t rows,
                            int dtype, void* stream);
+/* Channel concat of EXB_F16 NHWC tensors of N images, input i read through a nearest resize (as
+ * exb_interp_nearest_fwd) from heights[i] x widths[i] to OH x OW.  channels and strides are multiples of 8; an input
+ * whose pointer is NULL is left out: its channels of y are written by somebody else. */
+EXB_API int exb_concat_nearest_fwd(exb_ctx* ctx, int n_in, const void* const* xs, const int32_t* channels,
+                                   const int32_t* x_strides, const int32_t* heights, const int32_t* widths,
+                                   void* y, int y_stride, int N, int OH, int OW, void* stream);
 EXB_API int exb_interp_nearest_fwd(exb_ctx* ctx, const void* x, void* y, int N, int H, int W, int C,
                                    int c_stride, int OH, int OW, int dtype, int channel_last,
                                    void* stream);

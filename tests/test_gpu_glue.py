@@ -130,3 +130,57 @@ def test_focus(ctx, shape):
     np.testing.assert_array_equal(y[..., :4 * shape[1]].astype(np.float32), O.nchw_to_nhwc(O.focus(f16_round(x))))
     assert not y[..., 4 * shape[1]:].any()
     ctx.sync_check()
+
+
+@pytest.mark.parametrize("parts,out_hw,n", [
+    ([(64, 64, 30, 1), (64, 96, 15, 1), (32, 32, 8, 1)], (30, 17), 2),      # (channels, stride, height, copied): three sizes
+    ([(16, 16, 4, 1), (48, 48, 8, 0), (8, 16, 8, 1)], (8, 300), 1),         # one input left out, rows in pieces
+    ([(8, 8, 1, 1)], (5, 1), 3),
+])
+def test_concat_nearest(ctx, parts, out_hw, n):
+    import ctypes as C
+    capi = _capi()
+    OH, OW = out_hw
+    r = rng(sum(p[0] for p in parts) + OW)
+    total = sum(p[0] for p in parts)
+    ys = total + 16
+    xs = [r.standard_normal((n, h, max(1, OW * h // OH), cs)).astype(np.float16) for _, cs, h, _ in parts]
+    ref = np.full((n, OH, OW, ys), 7, np.float16)
+    off = 0
+    for (c, cs, h, copied), x in zip(parts, xs):
+        if copied:
+            up = O.interp_nearest(np.transpose(x[..., :c], (0, 3, 1, 2)).astype(np.float32), OH, OW)
+            ref[..., off:off + c] = np.transpose(up, (0, 2, 3, 1))
+        off += c
+    xd = [dev(x) for x in xs]
+    y = dev(np.full((n, OH, OW, ys), 7, np.float16))
+    k = len(parts)
+    i32 = lambda v: (C.c_int32 * k)(*v)
+    capi.check(capi.lib().exb_concat_nearest_fwd(
+        ctx.handle, k, (C.c_void_p * k)(*[t.data_ptr() if p[3] else None for t, p in zip(xd, parts)]), i32([p[0] for p in parts]),
+        i32([p[1] for p in parts]), i32([p[2] for p in parts]), i32([x.shape[2] for x in xs]), capi.ptr(y), ys, n, OH, OW, capi.cur_stream()))
+    ctx.sync_check()
+    np.testing.assert_array_equal(host(y), ref)
+
+
+@pytest.mark.parametrize("case", [(2, 64, 33, 21, 1, 2, 2, 4), (1, 24, 5, 7, 1, 1, 3, 106), (3, 8, 1, 1, 2, 2, 1, 0), (1, 64, 200, 191, 1, 2, 2, 1)])
+def test_deconv_few_outputs(ctx, case):
+    capi = _capi()
+    n, cin, h, w, c, rh, rw, act = case
+    r = rng(sum(case))
+    x = f16_round(r.standard_normal((n, cin, h, w)))
+    wt = f16_round(r.standard_normal((rh * rw * c, cin, 1, 1)) * 0.2)
+    b = r.standard_normal(rh * rw * c).astype(np.float32)
+    d = capi.make_conv_desc(n, h, w, cin, rh * rw * c, 1, 1, 0, capi.EXB_F16, capi.EXB_F16, act=act)
+    p = capi.ConvWeights(ctx, d, wt, b)
+    slopes = np.full(rh * rw * c, 0.1, np.float32)
+    if act == 106:
+        p.set_slopes(ctx, slopes)
+    xd = dev(np.ascontiguousarray(np.transpose(x, (0, 2, 3, 1))).astype(np.float16))
+    y = dev(np.zeros((n, c, h * rh, w * rw), np.float32))
+    capi.check(capi.lib().exb_deconv_few_f32(ctx.handle, capi.ptr(xd), p.handle, capi.ptr(y), n, h, w, rh, rw, c, act, capi.cur_stream()))
+    ctx.sync_check()
+    v = np.einsum("nihw,qi->nqhw", x.astype(np.float64), wt[:, :, 0, 0].astype(np.float64)) + b[None, :, None, None]
+    v = {0: v, 1: np.maximum(v, 0), 4: 1 / (1 + np.exp(-v)), 106: np.where(v >= 0, v, 0.1 * v)}[act]
+    ref = v.reshape(n, rh, rw, c, h, w).transpose(0, 3, 4, 1, 5, 2).reshape(n, c, h * rh, w * rw)
+    np.testing.assert_allclose(host(y), ref, rtol=1e-4, atol=1e-4)
