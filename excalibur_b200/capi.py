@@ -19,7 +19,7 @@ EXPORTED_SYMBOLS = [
     "exb_ctx_create", "exb_ctx_destroy", "exb_last_error_string", "exb_version", "exb_ctx_sm_count",
     "exb_ctx_sync_check", "exb_selftest_bounded_wait", "exb_tensor_peak_probe", "exb_tensor_peak_probe_layout", "exb_nchw_f32_to_nhwc", "exb_nchw_f32_to_nhwc_padded", "exb_nhwc_to_nchw_f32", "exb_conv_out_dims",
     "exb_conv_weights_pack_f16", "exb_conv_weights_pack_i8", "exb_conv_weights_destroy",
-    "exb_conv2d_fwd", "exb_conv2d_uses_tensor_cores", "exb_conv2d_pool_fusable", "exb_dw_weights_pack", "exb_dw_weights_destroy",
+    "exb_conv2d_fwd", "exb_conv2d_uses_tensor_cores", "exb_conv2d_pool_fusable", "exb_conv2d_d2s_fusable", "exb_dw_weights_pack", "exb_dw_weights_destroy",
     "exb_dwconv2d_fwd", "exb_pool_out_dims", "exb_pool2d_fwd", "exb_pool2d_nchw_f32_static", "exb_eltwise_fwd", "exb_binaryop_fwd",
     "exb_binaryop_scalar_fwd", "exb_relu_fwd", "exb_activation_fwd", "exb_quantize_fwd",
     "exb_dequantize_fwd", "exb_concat_fwd", "exb_concat_nearest_fwd", "exb_interp_nearest_fwd", "exb_channel_affine_fwd",
@@ -33,7 +33,7 @@ class ConvDesc(C.Structure):
         "pad_t", "pad_b", "pad_l", "pad_r", "dilation", "group", "in_dtype", "out_dtype", "out2_dtype",
         "res_dtype", "act")] + [("out_scale", C.c_float), ("out2_scale", C.c_float), ("impl", C.c_int32),
                                       ("x_w_pitch", C.c_int32), ("x_w_pad", C.c_int32), ("fuse_pool", C.c_int32),
-                                      ("y_pitch", C.c_int32)]
+                                      ("y_pitch", C.c_int32), ("d2s_h", C.c_int32), ("d2s_w", C.c_int32), ("res_half", C.c_int32)]
 
 
 class DwConvDesc(C.Structure):
@@ -80,6 +80,7 @@ def lib():
         L.exb_nhwc_to_nchw_f32.argtypes = [vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, vp]
         L.exb_conv_out_dims.argtypes = [C.POINTER(ConvDesc), C.POINTER(i32), C.POINTER(i32)]
         L.exb_conv2d_uses_tensor_cores.argtypes = [C.POINTER(ConvDesc)]
+        L.exb_conv2d_d2s_fusable.argtypes = [C.POINTER(ConvDesc)]
         L.exb_conv2d_pool_fusable.argtypes = [C.POINTER(ConvDesc)]
         L.exb_conv_weights_pack_f16.argtypes = [vp, C.POINTER(ConvDesc), vp, vp, C.POINTER(vp)]
         L.exb_conv_weights_pack_i8.argtypes = [vp, C.POINTER(ConvDesc), vp, vp, vp, i32, f32, C.POINTER(vp)]

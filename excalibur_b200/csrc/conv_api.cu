@@ -61,6 +61,17 @@ int resolve(const exb_conv_desc* d, ConvGeom& g) {
         if (g.out_dtype != EXB_F16 || g.out2_dtype != -1 || g.has_res || g.pool)
             return fail(EXB_ERR_UNSUPPORTED, "y_pitch is implemented for one fp16 output without residual or pooling");
     }
+    EXB_REQUIRE(d->d2s_h >= 0 && d->d2s_w >= 0 && (d->d2s_h > 0) == (d->d2s_w > 0), "bad depth-to-space factors %d x %d", d->d2s_h, d->d2s_w);
+    g.rh = d->d2s_h > 0 ? d->d2s_h : 1;
+    g.rw = d->d2s_w > 0 ? d->d2s_w : 1;
+    if (g.rh * g.rw > 1) {
+        EXB_REQUIRE(g.y_pitch == g.cout_stride && g.Cout == g.cout_stride && g.Cout % (g.rh * g.rw) == 0,
+                    "depth-to-space needs an unpadded channel count divisible by %d", g.rh * g.rw);
+        g.y_pitch = g.cout_stride / (g.rh * g.rw);
+    }
+    g.res_half = d->res_half;
+    EXB_REQUIRE(g.res_half == 0 || (g.res_half == 1 && g.has_res && g.OH % 2 == 0 && g.OW % 2 == 0 && !g.pool),
+                "res_half needs a residual and an even output size");
     return EXB_OK;
 }
 
@@ -124,6 +135,12 @@ extern "C" int exb_conv2d_pool_fusable(const exb_conv_desc* d) {
     ConvGeom g;
     if (int rc = resolve(d, g)) return rc;
     return (d->impl != 1 && conv_tc_eligible(g) && conv_tc_pool_fusable(g)) ? 1 : 0;
+}
+
+extern "C" int exb_conv2d_d2s_fusable(const exb_conv_desc* d) {
+    ConvGeom g;
+    if (int rc = resolve(d, g)) return rc;
+    return (d->impl != 1 && conv_tc_eligible(g) && conv_tc_mappable(g)) ? 1 : 0;
 }
 
 extern "C" int exb_conv2d_uses_tensor_cores(const exb_conv_desc* d) {
@@ -219,6 +236,13 @@ extern "C" int exb_conv2d_fwd(exb_ctx* ctx, const exb_conv_desc* d, const void* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (g.pool && !(d->impl != 1 && conv_tc_eligible(g) && conv_tc_pool_fusable(g)))
         return fail(EXB_ERR_UNSUPPORTED, "fuse_pool is not available for this convolution (see exb_conv2d_pool_fusable)");
+    if (g.rh * g.rw > 1) {
+        if (d->impl == 1 || !conv_tc_eligible(g) || !conv_tc_mappable(g))
+            return fail(EXB_ERR_UNSUPPORTED, "depth-to-space is not available for this convolution (see exb_conv2d_d2s_fusable)");
+        return conv_tc_launch(ctx, g, x, w, residual, y, y2, st);
+    }
+    if (g.res_half && !(d->impl != 1 && conv_tc_eligible(g) && conv_tc_mappable(g)))
+        return fail(EXB_ERR_UNSUPPORTED, "res_half is not available for this convolution");
     if (g.y_pitch != g.cout_stride && !(d->impl != 1 && conv_tc_eligible(g)))
         return fail(EXB_ERR_UNSUPPORTED, "y_pitch needs the tensor-core kernel");
     if (d->impl != 1 && conv_tc_eligible(g)) {

@@ -35,6 +35,8 @@ struct ConvGeom {
     int pool;             // 1: 3x3/2 pad-1 max pooling fused into the epilogue; y is [N][PH][PW][cout_stride]
     int PH, PW;
     int y_pitch;                    // elements between output pixels of y (== cout_stride unless y is a slice of a wider tensor)
+    int rh, rw;                     // depth-to-space factors of the stored result (1, 1: none); y_pitch is then C
+    int res_half;                   // residual at half the resolution
 };
 
 // "Folded" K layout for convolutions with very few input channels (a stem): one K row of an
@@ -215,6 +217,8 @@ int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, cons
                       void* y, void* y2, cudaStream_t st);
 // True when the tcgen05 kernel can run this geometry.
 bool conv_tc_eligible(const ConvGeom& g);
+// True when the tensor-core kernels can store the result depth-to-space / read the residual at half the resolution.
+bool conv_tc_mappable(const ConvGeom& g);
 // True when the tcgen05 kernel can also apply the 3x3/2 max pooling in its epilogue.
 bool conv_tc_pool_fusable(const ConvGeom& g);
 

@@ -35,6 +35,7 @@ struct ConvSplitParams {
     int k_iters;                        // (tap, channel block) pairs; CTA r of a cluster takes [r*k/splits, (r+1)*k/splits)
     int stages, a_bytes, b_bytes, a_tx_bytes;
     int tmem_cols, cout_pad, has_res;
+    int res_half;           // the residual is read through a nearest resize by 2
     uint32_t idesc;
     EpiParams e;
     int* error;
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
     __shared__ __align__(8) uint64_t done_bar;
     __shared__ __align__(16) float s_scale[64];
     __shared__ __align__(16) float s_bias[64];
-    __shared__ int s_pixel[kTileM];
+    __shared__ int s_pixel[kTileM], s_res_pixel[kTileM];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
     // operand ring (1024-byte aligned: the widest swizzle atom); the partial tile takes its place when the MMAs are done
@@ -108,6 +109,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
         const int tw = row % p.TW, q = row / p.TW, th = q % p.TH, tn = q / p.TH;
         const int ow = ow0 + tw, oh = oh0 + th, n = n0 + tn;
         s_pixel[row] = tn < p.TN && ow < p.OW && oh < p.OH && n < p.N ? (n * p.OH + oh) * p.OW + ow : -1;
+        s_res_pixel[row] = p.res_half ? (n * (p.OH >> 1) + (oh >> 1)) * (p.OW >> 1) + (ow >> 1) : s_pixel[row];
     }
     ptx::tc_fence_before_sync();
     __syncthreads();
@@ -226,8 +228,9 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
 #pragma unroll
             for (int j = 0; j < kSplitMaxItems; ++j) {
                 const int item = et + j * kSplitEpiThreads;
-                const int px = item < n_items ? s_pixel[row0 + (item >> vshift)] : -1, cl = c0 + (item & ((1 << vshift) - 1)) * 8;
-                if (px >= 0 && cl < p.e.cout_stride) res[j] = *reinterpret_cast<const uint4*>(p.e.residual + (int64_t)px * p.e.cout_stride + cl);
+                const int row = row0 + (item >> vshift), cl = c0 + (item & ((1 << vshift) - 1)) * 8;
+                if (item < n_items && s_pixel[row] >= 0 && cl < p.e.cout_stride)
+                    res[j] = *reinterpret_cast<const uint4*>(p.e.residual + (int64_t)s_res_pixel[row] * p.e.cout_stride + cl);
             }
         }
         // accumulator -> shared memory, rows padded by 16 bytes: eight lanes' 16-byte stores cover all banks
@@ -395,6 +398,7 @@ int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, cons
     p.tmem_cols = p.BN <= 32 ? 32 : 64;
     p.cout_pad = w->cout_pad;
     p.has_res = g.has_res;
+    p.res_half = g.res_half;
     p.idesc = ptx::make_idesc(int8, kTileM, (uint32_t)p.BN);
     p.e.scale = w->d_scale; p.e.bias = w->d_bias; p.e.slope = w->d_slope; p.e.residual = static_cast<const __half*>(residual);
     p.e.y = y; p.e.y2 = y2; p.e.out_dtype = g.out_dtype; p.e.out2_dtype = g.out2_dtype; p.e.act = g.act;

@@ -42,12 +42,15 @@ namespace exb {
 namespace {
 
 constexpr int kMaxStages = 8;
+constexpr int kMaxD2sBlocks = 16;     // 32-channel blocks of a result stored depth-to-space
 constexpr int kFirstEpiWarp = 2;   // warp 0 producer, warp 1 MMA issuer, epilogue warps from here on
 constexpr int kMaxAccBufs = 4;
 constexpr int kConstCh = 64;      // output channels of the pool epilogue (scale / bias travel as launch parameters)
 constexpr uint32_t kMaxSpins = 1u << 21;  // tens of milliseconds at least; a legitimate wait is microseconds
 
-enum EpiKind { kEpiRow = 0, kEpiQuad = 1, kEpiPool = 2 };
+// kEpiMapped: the quad epilogue with a result stored depth-to-space or a residual at half the resolution (a kernel of its
+// own: the few instructions that the mapping takes cost the plain epilogue 2 %)
+enum EpiKind { kEpiRow = 0, kEpiQuad = 1, kEpiPool = 2, kEpiMapped = 3 };
 
 struct ConvTcParams {
     CUtensorMap tmA[4];
@@ -102,6 +105,11 @@ struct ConvTcParams {
     // Tile origins: first output column / row of tile index i is i * step + org (step = TW / TH and
     // org = 0 unless tiles overlap).
     int step_w, step_h, step_n, org;
+    // Depth-to-space factors of the stored result (quad epilogue; 1, 1: none).  Channels of tap t = (a, b) go to pixel
+    // (oh * d2s_h + a, ow * d2s_w + b); with y_pitch channels per pixel that is the pixel index of (a, b) = (0, 0) plus
+    // d2s_shift of the 32-channel block, if the channel offset is left counted over all taps.
+    int d2s_h, d2s_w, d2s_shift[kMaxD2sBlocks];
+    int res_half;           // the residual is read through a nearest resize by 2
     int pair_h, pair_n;     // CTA pairs: how far rank 1's tile lies from rank 0's, rows / images (one of them is 0)
     // Fused 3x3/2 pad-1 max pooling (patch mode, BN = 64): an 8 x 16 tile of the convolution output
     // starts at (6*tx - 1, 14*ty - 1), so it holds every input of the 3 x 7 pooled outputs that
@@ -400,7 +408,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
     for (int c = threadIdx.x; c < p.n_tiles * p.BN; c += kThreads) {
         const bool in = c < p.cout_pad;
         // quad epilogue: channel 32*b + 8*j + 4*i + k is kept at 32*b + 16*i + 4*j + k (see epi_quad_rows)
-        const int at = kEpi == kEpiQuad ? ((c & ~31) | ((c & 4) << 2) | ((c & 24) >> 1) | (c & 3)) : c;
+        const int at = kEpi == kEpiQuad || kEpi == kEpiMapped ? ((c & ~31) | ((c & 4) << 2) | ((c & 24) >> 1) | (c & 3)) : c;
         s_scale[at] = in ? p.e.scale[c] : 0.f;
         s_bias[at] = in ? p.e.bias[c] : 0.f;
     }
@@ -818,7 +826,8 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                 if (grp == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
                 else asm volatile("bar.sync 2, 128;" ::: "memory");
             }
-        } else if constexpr (kEpi == kEpiQuad) {
+        } else if constexpr (kEpi == kEpiQuad || kEpi == kEpiMapped) {
+            constexpr bool kMapped = kEpi == kEpiMapped;
             // Four neighbouring lanes hold one pixel: lane l of a 16-lane half covers tile rows r = l / 4 and
             // r + 8 and, of every 32-channel block, channels 8 * (l % 4) .. + 7 (the B tensor map stores
             // channel 8*j + 2*g + e of a block in accumulator column 8*g + 2*j + e, which is where the 16x256b
@@ -843,7 +852,15 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                 const int ow = c.ow0 + (int)(rp & 0xff), oh = c.oh0 + (int)((rp >> 8) & 0xff);
                 const int n = c.n0 + (int)((rp >> 16) & 0x7fff);
                 if ((rp >> 31) || ow >= p.OW || oh >= p.OH || n >= p.N) return -1;
+                if (kMapped) return ((n * p.OH + oh) * p.d2s_h * p.OW + ow) * p.d2s_w;
                 return (n * p.OH + oh) * p.OW + ow;
+            };
+            // and of its residual
+            auto res_pixel_of = [&](const TileCoord& c, uint32_t rp, int px) -> int {
+                if (!kMapped || !p.res_half || px < 0) return px;
+                const int ow = c.ow0 + (int)(rp & 0xff), oh = c.oh0 + (int)((rp >> 8) & 0xff);
+                const int n = c.n0 + (int)((rp >> 16) & 0x7fff);
+                return (n * (p.OH >> 1) + (oh >> 1)) * (p.OW >> 1) + (ow >> 1);
             };
             const bool want_res = p.has_res != 0;
             TileCursor cur(p, first_unit + grp * unit_step, p.epi_groups * unit_step);
@@ -862,7 +879,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                         if (h < h_begin || h >= h_end) continue;
 #pragma unroll
                         for (int k = 0; k < 2; ++k) {
-                            const int px = pixel_of(c2, rowpack[h][k]);
+                            const int px = res_pixel_of(c2, rowpack[h][k], pixel_of(c2, rowpack[h][k]));
                             if (px < 0) continue;
                             const __half* r2 = p.e.residual + (int64_t)px * p.e.cout_stride + c2.ntile * p.BN;
                             for (int l = cq; l * 64 < p.BN; l += 4)      // one 128-byte line per pixel and 64 channels
@@ -883,7 +900,9 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                     const bool second = f >= nblk;
                     const int cl = c0 + (second ? f - nblk : f) * 32;
                     if (want_res && f < nfrag && cl < p.e.cout_stride) {
-                        const int pa = second ? pa1 : pa0, pb = second ? pb1 : pb0;
+                        int pa = second ? pa1 : pa0, pb = second ? pb1 : pb0;
+                        pa = res_pixel_of(tc, second || h_begin ? rowpack[1][0] : rowpack[0][0], pa);
+                        pb = res_pixel_of(tc, second || h_begin ? rowpack[1][1] : rowpack[0][1], pb);
                         if (pa >= 0) a = __ldg(reinterpret_cast<const uint4*>(p.e.residual + (int64_t)pa * p.e.cout_stride + cl));
                         if (pb >= 0) b = __ldg(reinterpret_cast<const uint4*>(p.e.residual + (int64_t)pb * p.e.cout_stride + cl));
                     }
@@ -906,9 +925,14 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                     uint32_t raw[16];
                     ptx::tmem_ld_16x256b_x4(taddr0 + ((uint32_t)(h * 16) << 16) + (uint32_t)(buf * p.BN + b * 32), raw);
                     ptx::tmem_ld_wait();
+                    int pa = second ? pa1 : pa0, pb = second ? pb1 : pb0;
+                    if (kMapped && p.d2s_h * p.d2s_w > 1) {
+                        const int shift = p.d2s_shift[(tc.ntile * p.BN >> 5) + b < kMaxD2sBlocks ? (tc.ntile * p.BN >> 5) + b : 0];
+                        if (pa >= 0) pa += shift;
+                        if (pb >= 0) pb += shift;
+                    }
                     if (cl < p.e.cout_stride)
-                        epi_quad_rows<kInt8, kPrelu>(p.e, s_scale, s_bias, cl, cq, second ? pa1 : pa0, second ? pb1 : pb0, want_res, ra,
-                                                     rb, raw);
+                        epi_quad_rows<kInt8, kPrelu>(p.e, s_scale, s_bias, cl, cq, pa, pb, want_res, ra, rb, raw);
                     ra = na;
                     rb = nb;
                 }
@@ -1101,6 +1125,15 @@ bool conv_tc_pool_fusable(const ConvGeom& g) {
            !g.has_res && (g.act == EXB_ACT_RELU || g.act == EXB_ACT_RELU6) && g.group == 1;
 }
 
+// Every N tile and the weights in whole 32-channel blocks, and an output of the kind the quad epilogue takes.
+bool conv_tc_mappable(const ConvGeom& g) {
+    if (g.cout_stride % 32 || (g.cout_stride > 128 && g.cout_stride % 128) || (g.out_dtype != EXB_F16 && g.out_dtype != EXB_F32) ||
+        g.act == EXB_ACT_PRELU || g.pool || g.group != 1 || conv_fold_plan(g).on) return false;
+    if (g.rh * g.rw == 1) return true;
+    return g.y_pitch % 32 == 0 && g.cout_stride / 32 <= kMaxD2sBlocks && g.out_dtype == EXB_F16 && g.out2_dtype < 0 && !g.has_res &&
+           (int64_t)g.N * g.OH * g.rh * g.OW * g.rw < (int64_t)1 << 31;
+}
+
 bool conv_tc_eligible(const ConvGeom& g) {
     const int es = g.in_dtype == EXB_I8 ? 1 : 2;
     if (g.group != 1) return false;
@@ -1274,6 +1307,17 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     const bool quad = !patch && !p.pool && p.BN % 32 == 0 && w->cout_pad % 32 == 0 && (g.cout_stride & 7) == 0 &&
                       g.out_dtype != EXB_I32 && !(g.out_dtype == EXB_I8 && g.out2_dtype < 0) &&
                       p.TW <= 255 && p.TH <= 255 && p.TN <= 32767;
+    p.res_half = g.res_half;
+    p.d2s_h = g.rh;
+    p.d2s_w = g.rw;
+    const bool mapped = g.rh * g.rw > 1 || g.res_half;
+    if (mapped) {
+        if (!quad) return fail(EXB_ERR_UNSUPPORTED, "a mapped result or residual needs the quad epilogue");
+        for (int b = 0; g.rh * g.rw > 1 && b < g.cout_stride / 32; ++b) {
+            const int t = b * 32 / g.y_pitch;
+            p.d2s_shift[b] = t / g.rw * (g.OW * g.rw) + t % g.rw - t;
+        }
+    }
     // CTA pairs (see the kernel's kPair): two tiles that are neighbours along the image groups, or along the rows when
     // there is one image group, share every MMA and each CTA holds half of the weight rows.  Taken for
     //  - row-box tiles of 64 or 128 channels whose weights stay resident on one CTA per SM: a stage then holds a whole
@@ -1290,7 +1334,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     // The channel-permuting map of the quad epilogue moves 32-channel blocks, so a half must be made of whole ones.
     const int64_t k_bytes = (int64_t)g.kh * g.kw * row_bytes;      // one pixel's reduction
     const int64_t all_tiles = (int64_t)p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;
-    const bool pairable = !patch && !fold.on && !g.pool && ctx->sm_count >= 2 && g.act != EXB_ACT_PRELU &&
+    const bool pairable = !mapped && !patch && !fold.on && !g.pool && ctx->sm_count >= 2 && g.act != EXB_ACT_PRELU &&
                           p.BN % (quad ? 64 : 32) == 0 && (p.tiles_nb >= 2 || p.tiles_h >= 2);
     bool pair = false;
     if (p.rowbox)
@@ -1445,6 +1489,9 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     const bool prelu = p.e.act == EXB_ACT_PRELU;
     void (*kern)(const ConvTcParams);
     if (p.pool) kern = conv_tc_kernel<false, 8, kEpiPool>;
+    else if (mapped)
+        kern = int8 ? (two ? conv_tc_kernel<true, 8, kEpiMapped> : conv_tc_kernel<true, 16, kEpiMapped>)
+                    : (two ? conv_tc_kernel<false, 8, kEpiMapped> : conv_tc_kernel<false, 16, kEpiMapped>);
     else if (pair && !prelu)
         kern = int8 ? (quad ? conv_tc_kernel<true, 16, kEpiQuad, false, true> : conv_tc_kernel<true, 16, kEpiRow, false, true>)
                     : (quad ? conv_tc_kernel<false, 16, kEpiQuad, false, true> : conv_tc_kernel<false, 16, kEpiRow, false, true>);

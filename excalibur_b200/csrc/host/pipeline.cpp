@@ -419,6 +419,7 @@ void fused_plan::layout(slice& sl, bool f16_src) {
     struct group {
         int conv = -1;          // leading op
         int residual = -1;      // root featmap added in the epilogue
+        bool res_half = false;  // .. through a nearest resize by 2, whose Interp is absorbed
         int act = EXB_ACT_NONE;
         int pool = -1;          // 3x3/2 max pooling op applied in the conv epilogue
         int bn = -1;            // BatchNorm op folded into the conv's weights and bias
@@ -538,10 +539,25 @@ void fused_plan::layout(slice& sl, bool f16_src) {
             const int a = root(in_ids[j][0]), b = root(in_ids[j][1]);
             g.residual = a == g.out ? b : a;
             absorbed[j] = 1;
+            // a feature pyramid's top-down path: the residual is a map of half the size behind a nearest Interp
+            for (size_t q = 0; q < n_ops && sole_consumer(g.residual) == j; ++q) {
+                if (absorbed[q] || lower_type(params_[q]) != "interp" || in_ids[q].size() != 1 || root(out_ids[q][0]) != g.residual) continue;
+                auto* ip = dynamic_cast<operation_interp<float>*>(ops_[q].get());
+                if (!ip || ip->resize_type_ != 1 || ip->align_corner_ != 0 || conv->group_ != 1 || conv->in_channels() % 32 ||
+                    conv->output_channel_ % 32 || (conv->output_channel_ > 128 && conv->output_channel_ % 128) || conv->stride_h_ != conv->stride_w_ || conv->stride_h_ > 2) break;
+                int h = 0, w = 0, h2 = 0, w2 = 0;
+                ip->out_dims(5, 8, &h, &w);
+                ip->out_dims(64, 7, &h2, &w2);
+                if (h != 10 || w != 16 || h2 != 128 || w2 != 14) break;      // not a resize by 2 whatever the size
+                absorbed[q] = 1;
+                g.residual = root(in_ids[q][0]);
+                g.res_half = true;
+                break;
+            }
             g.out = root(out_ids[j][0]);
             g.exec_at = j;
             int k;
-            if ((k = sole_consumer(g.out)) >= 0 && !absorbed[k] && act_of_op(k) > 0) {
+            if ((k = sole_consumer(g.out)) >= 0 && !absorbed[k] && act_of_op(k) > 0 && !(g.res_half && act_of_op(k) == EXB_ACT_PRELU)) {
                 g.act = act_of_op(k);
                 if (g.act == EXB_ACT_PRELU) g.slope_op = k;
                 absorbed[k] = 1;
@@ -956,6 +972,16 @@ void fused_plan::layout(slice& sl, bool f16_src) {
                 for (int c = 0; c < d.Cout; ++c) rep[c] = sl[c % Cout];
                 exb_check(exb_conv_weights_set_slopes(ctx, w, rep.data(), (int)rep.size()), "exb_conv_weights_set_slopes");
             }
+            exb_conv_desc scattered = d;
+            scattered.d2s_h = rh;
+            scattered.d2s_w = rw;
+            if (rh * rw > 1 && d.cout_stride == d.Cout && y.cs == Cout && exb_conv2d_d2s_fusable(&scattered) == 1) {
+                add_step(params_[i].name_, [=](cudaStream_t st) {
+                    exb_check(exb_conv2d_fwd(ctx, &scattered, xin, w, nullptr, yo, nullptr, st), "exb_conv2d_fwd");
+                });
+                finish_forms(y, false);
+                return;
+            }
             const int n = x.N, h = x.H, wd = x.W, xs = d.cout_stride, ys = y.cs;
             void* tmp = mid->ensure((size_t)x.N * x.H * x.W * d.cout_stride * 2, device_);
             add_step(params_[i].name_, [=](cudaStream_t st) {
@@ -1026,14 +1052,16 @@ void fused_plan::layout(slice& sl, bool f16_src) {
         if (g.residual >= 0) {
             fmap_info& r = fmaps_[g.residual];
             CHECK(r.produced) << "residual " << r.name << " is not available when " << params_[i].name_ << " runs";
-            CHECK(r.N == y.N && r.C == y.C && r.H == y.H && r.W == y.W && r.cs == y.cs) << "residual shape mismatch";
+            const int half = g.res_half ? 2 : 1;
+            CHECK(r.N == y.N && r.C == y.C && r.H * half == y.H && r.W * half == y.W && r.cs == y.cs) << "residual shape mismatch";
+            d.res_half = g.res_half ? 1 : 0;
             res = form_f16(r);
             d.res_dtype = EXB_F16;
         }
         void* y1 = nullptr;
         void* y2 = nullptr;
         bool wrote_i8 = false;
-        if (y.need_f16 || !y.need_i8) {
+        if (y.need_f16 || !y.need_i8 || g.res_half) {
             y.need_f16 = true;
             d.out_dtype = EXB_F16;
             y1 = form_f16(y);

@@ -193,6 +193,15 @@ typedef struct exb_conv_desc {
      * (operation_concat, src/Excalibur/operation_concat.cpp:30-80).  Needs the tensor-core kernel, one fp16
      * output, no residual, cout_stride % 16 == 0 and y_pitch % 16 == 0. */
     int32_t y_pitch;
+    /* d2s_h * d2s_w > 1: the result is scattered as exb_depth_to_space_fwd would (a transposed convolution with kernel =
+     * stride): output channel t * C + c, C = cout_stride / (d2s_h * d2s_w), goes to channel c of pixel
+     * (oh * d2s_h + t / d2s_w, ow * d2s_w + t % d2s_w) of an [N][OH * d2s_h][OW * d2s_w][C] tensor.  Only for descriptors
+     * for which exb_conv2d_d2s_fusable() returns 1; 0 / 0 = plain convolution. */
+    int32_t d2s_h;
+    int32_t d2s_w;
+    /* 1: the residual is [N][OH / 2][OW / 2][cout_stride], read through a nearest resize by 2 (OH, OW even).  Needs the
+     * tensor-core kernel, an fp16 or fp32 first output, cout_stride a multiple of 32 and, above 128, of 128. */
+    int32_t res_half;
 } exb_conv_desc;
 
 /* Output spatial size: (in + pad_a + pad_b - k) / stride + 1
@@ -230,6 +239,7 @@ EXB_API int exb_conv2d_uses_tensor_cores(const exb_conv_desc* d);
 /* 1 when exb_conv2d_fwd can run this descriptor with fuse_pool = 1 (a few-channel stride-2 fp16
  * stem on padded NHWC4 rows with 64 output channels, ReLU or ReLU6, fp16 output and an optional
  * int8 copy, no residual), else 0; negative = error.  The descriptor's own fuse_pool is ignored. */
+EXB_API int exb_conv2d_d2s_fusable(const exb_conv_desc* desc);
 EXB_API int exb_conv2d_pool_fusable(const exb_conv_desc* d);
 
 /* ---------------------------------------------------------------------------------------

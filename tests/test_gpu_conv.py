@@ -472,3 +472,46 @@ def test_conv_pairs(ctx, case):
     y, _ = capi.conv2d(ctx, d, dev(to_nhwc(xq).astype(np.int8 if dtype == "i8" else np.float16)), p)
     ctx.sync_check()
     np.testing.assert_array_equal(to_nchw(host(y)), ref.astype(np.float32))
+
+
+# Residual read through a nearest resize by 2: one and several N tiles of the persistent kernel, the split kernel.
+@pytest.mark.parametrize("case", [(2, 64, 30, 46, 256, "f16", 2), (1, 64, 16, 10, 32, "f16", 2), (2, 64, 14, 12, 384, "i8", 2), (4, 512, 16, 8, 512, "f16", 2),
+                                  (3, 128, 8, 6, 64, "i8", 0), (1, 256, 14, 14, 96, "f16", 0), (300, 64, 14, 14, 128, "i8", 2)])
+def test_conv_half_resolution_residual(ctx, case):
+    capi = _capi()
+    N, Cin, H, W, Cout, dtype, impl = case
+    r = rng(sum(case[:5]) + 23)
+    xq = r.integers(-4, 5, (N, Cin, H, W)).astype(np.int8)
+    wq = r.integers(-3, 4, (Cout, Cin, 1, 1)).astype(np.int8)
+    res = r.integers(-64, 65, (N, Cout, H // 2, W // 2)).astype(np.float32)
+    ref = O.conv2d_i8_acc(xq, wq, 1, 0).astype(np.float32) + np.repeat(np.repeat(res, 2, 2), 2, 3)
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, 1, 1, 0, capi.EXB_I8 if dtype == "i8" else capi.EXB_F16, capi.EXB_F32, res=True, impl=impl)
+    d.res_half = 1
+    p = (capi.ConvWeights(ctx, d, wq, None, np.ones(Cout, np.float32), 1.0) if dtype == "i8"
+         else capi.ConvWeights(ctx, d, wq.astype(np.float32), np.zeros(Cout, np.float32)))
+    y, _ = capi.conv2d(ctx, d, dev(to_nhwc(xq).astype(np.int8 if dtype == "i8" else np.float16)), p, dev(to_nhwc(res).astype(np.float16)))
+    ctx.sync_check()
+    np.testing.assert_array_equal(to_nchw(host(y)), ref)
+
+
+# Depth-to-space in the epilogue: one and several N tiles, factors that differ.
+@pytest.mark.parametrize("case", [(2, 64, 9, 7, 64, 2, 2), (1, 32, 20, 33, 32, 1, 3), (3, 128, 12, 11, 32, 2, 4), (2, 256, 60, 92, 128, 2, 2)])
+def test_conv_depth_to_space(ctx, case):
+    import torch
+    capi = _capi()
+    N, Cin, H, W, C, rh, rw = case
+    r = rng(sum(case) + 24)
+    Cout = rh * rw * C
+    x = r.integers(-4, 5, (N, Cin, H, W)).astype(np.int8)
+    wq = r.integers(-2, 3, (Cout, Cin, 1, 1)).astype(np.int8)
+    b = r.integers(-9, 10, Cout).astype(np.float32)
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, 1, 1, 0, capi.EXB_F16, capi.EXB_F16, act=1)
+    p = capi.ConvWeights(ctx, d, wq.astype(np.float32), b)
+    d.d2s_h, d.d2s_w = rh, rw
+    assert capi.lib().exb_conv2d_d2s_fusable(d) == 1
+    y = torch.full((N, H * rh, W * rw, C), -1.0, device="cuda", dtype=torch.float16)
+    capi.conv2d(ctx, d, dev(to_nhwc(x).astype(np.float16)), p, y=y)
+    ctx.sync_check()
+    acc = np.maximum(O.conv2d_i8_acc(x, wq, 1, 0) + b[None, :, None, None], 0)
+    ref = acc.reshape(N, rh, rw, C, H, W).transpose(0, 4, 1, 5, 2, 3).reshape(N, H * rh, W * rw, C)
+    np.testing.assert_array_equal(host(y).astype(np.float32), ref.astype(np.float16).astype(np.float32))
