@@ -88,6 +88,8 @@ struct fmap_info {
     // the device buffers of a feature map stay when its steps are laid out again for another division of the batch
     void keep(const fmap_info& o) { f16 = o.f16; i8 = o.i8; f32 = o.f32; extra_i8 = o.extra_i8; }
     bool produced = false;
+    // not materialised, but read from another map on request: its nearest resize, or channels within_at .. of it
+    int resized_from = -1, within = -1, within_at = 0;
     bool f32_only = false;         // result of a Reshape / Transpose at the tail of the graph: fp32 NCHW only
 };
 
@@ -419,7 +421,8 @@ void fused_plan::layout(slice& sl, bool f16_src) {
     struct group {
         int conv = -1;          // leading op
         int residual = -1;      // root featmap added in the epilogue
-        bool res_half = false;  // .. through a nearest resize by 2, whose Interp is absorbed
+        bool res_half = false;  // .. through a nearest resize by 2, whose Interp (with the result `resized`) is absorbed
+        int resized = -1;
         int act = EXB_ACT_NONE;
         int pool = -1;          // 3x3/2 max pooling op applied in the conv epilogue
         int bn = -1;            // BatchNorm op folded into the conv's weights and bias
@@ -550,6 +553,7 @@ void fused_plan::layout(slice& sl, bool f16_src) {
                 ip->out_dims(64, 7, &h2, &w2);
                 if (h != 10 || w != 16 || h2 != 128 || w2 != 14) break;      // not a resize by 2 whatever the size
                 absorbed[q] = 1;
+                g.resized = g.residual;
                 g.residual = root(in_ids[q][0]);
                 g.res_half = true;
                 break;
@@ -1055,6 +1059,11 @@ void fused_plan::layout(slice& sl, bool f16_src) {
             const int half = g.res_half ? 2 : 1;
             CHECK(r.N == y.N && r.C == y.C && r.H * half == y.H && r.W * half == y.W && r.cs == y.cs) << "residual shape mismatch";
             d.res_half = g.res_half ? 1 : 0;
+            if (g.res_half) {
+                fmap_info& up = fmaps_[g.resized];
+                up.resized_from = g.residual;
+                up.N = y.N; up.C = y.C; up.H = y.H; up.W = y.W;
+            }
             res = form_f16(r);
             d.res_dtype = EXB_F16;
         }
@@ -1305,6 +1314,14 @@ void fused_plan::layout(slice& sl, bool f16_src) {
                     if (y.cs > total) CUDA_CHECK(cudaMemset(form_f16(y), 0, (size_t)y.N * y.H * y.W * y.cs * 2));
                 }
                 CHECK(y.C == total && y.H == OH && y.W == OW) << "Concat operands differ in shape";
+                for (size_t q = 0, at = 0; q < in_ids[i].size(); at += cat_copy[i][q++]) {
+                    const int rf = root(in_ids[i][q]);
+                    const auto src = cat_source.find(rf);
+                    if (src != cat_source.end()) fmaps_[rf].resized_from = root(in_ids[src->second][0]);
+                    else if (cat_stored.count(rf)) { fmaps_[rf].within = root(out_ids[i][0]); fmaps_[rf].within_at = (int)at; }
+                    else continue;
+                    fmaps_[rf].N = n; fmaps_[rf].C = cat_copy[i][q]; fmaps_[rf].H = OH; fmaps_[rf].W = OW;
+                }
                 void* yo = form_f16(y);
                 const int ys = y.cs;
                 add_step(params_[i].name_, [=](cudaStream_t st) {
@@ -1814,6 +1831,26 @@ std::shared_ptr<memory::tensor<float>> fused_plan::fetch(const std::string& name
     if (f.w_pitch) {
         LOG(WARNING) << "feature map " << name << " is kept in a padded row layout and is not exported";
         return nullptr;
+    }
+    if (!f.produced && (f.resized_from >= 0 || f.within >= 0)) {
+        const fmap_info& src = fmaps_[f.within >= 0 ? f.within : f.resized_from];
+        auto t = std::shared_ptr<memory::tensor<float>>(
+            new memory::tensor<float>(std::vector<int>{f.N, f.C, f.H, f.W}, device_, memory::NCHW, nullptr));
+        CUDA_CHECK(cudaStreamSynchronize(stream_));
+        dev_buf resized;
+        const void* from = src.f16->p;
+        if (f.within >= 0) {
+            from = static_cast<const char*>(from) + (size_t)f.within_at * 2;
+        } else {
+            from = resized.ensure((size_t)f.N * f.H * f.W * src.cs * 2, device_);
+            exb_check(exb_interp_nearest_fwd(ctx_, src.f16->p, resized.p, f.N, src.H, src.W, src.C, src.cs, f.H, f.W, EXB_F16, 1, nullptr),
+                      "exb_interp_nearest_fwd");
+        }
+        exb_check(exb_nhwc_to_nchw_f32(ctx_, from, EXB_F16, t->mutable_gpu_data(), f.N, f.C, f.H, f.W, src.cs, 1.f, nullptr),
+                  "exb_nhwc_to_nchw_f32");
+        CUDA_CHECK(cudaDeviceSynchronize());
+        t->cpu_data();
+        return t;
     }
     if (!f.produced) {
         LOG(WARNING) << "feature map " << name << " was fused into its consumer and is not materialised; "

@@ -441,3 +441,29 @@ def test_divided_forward_and_pageable_input():
     small = np.ascontiguousarray(x[:3])      # one sub-batch from pageable memory, another shape
     np.testing.assert_allclose(p.forward(small)["logits"], whole[:3], rtol=2e-5, atol=2e-5)
     p.close()
+
+
+def test_maps_inside_a_concat_and_a_resized_residual_are_read_on_request():
+    """What a Concat's producers store in place, and nearest resizes that only a Concat or an addition reads, are not
+    kept; get() derives them, whatever the division of the batch, and they equal those of the plan without fusion."""
+    import numpy as np
+    from excalibur_b200 import model_zoo, models
+    for g, maps in ((models.yolov5s(5)[0], ("neck_up1_out", "c3_1_cv2_act", "neck_down1_act", "neck_cat1_out")),
+                    (model_zoo.det_db_resnet18(seed=3, size=64)[0], ("up4_out", "p3_up_out", "p2_out", "fuse_out", "add3_out"))):
+        x = np.random.default_rng(2).uniform(0, 1, (4, 3, 64, 96)).astype(np.float32)
+        p, q = host_pipeline(g, True), host_pipeline(g, False)
+        p.set_option("h2d_chunks", 2)
+        for _ in range(2):
+            p.forward(x)
+        q.forward(x)
+        for n in maps:
+            a, b = p.get(n), q.get(n)
+            assert a.shape == b.shape, n
+            np.testing.assert_allclose(a, b, rtol=2e-2, atol=2e-2 * np.abs(b).max(), err_msg=n)
+        p.close()
+        q.close()
+
+
+def host_pipeline(g, fusion):
+    from excalibur_b200 import host
+    return host.Pipeline(g.phai_text(), g.racy_bytes(), 0, fusion=fusion)
