@@ -1,6 +1,7 @@
 // C-ABI front of the dense convolution: descriptor validation, weight packing and the choice
 // between the tcgen05 implicit-GEMM kernel and the direct kernel.
 #include "conv_common.cuh"
+#include "host/host_convert.hpp"
 
 #include <math.h>
 #include <string.h>
@@ -75,10 +76,6 @@ int resolve(const exb_conv_desc* d, ConvGeom& g) {
     return EXB_OK;
 }
 
-uint16_t f32_to_f16_bits(float f) {
-    return __half_as_ushort(__float2half_rn(f));  // round to nearest even
-}
-
 int pack_common(exb_ctx* ctx, const ConvGeom& g, int dtype, const void* hw, size_t wbytes,
                 const std::vector<float>& scale, const std::vector<float>& bias, int cout_pad, int cin_pad,
                 int kw_pack, int s_shift, exb_conv_weights** out) {
@@ -105,16 +102,18 @@ int pack_common(exb_ctx* ctx, const ConvGeom& g, int dtype, const void* hw, size
     return EXB_OK;
 }
 
-// OIHW [Cout][cin_g][kh][kw] -> [cout_pad][kh][kw_pack][cin_pad] (zero filled), tap s at column s + s_shift
-template <typename TSrc, typename TDst, typename F>
-void repack(const TSrc* src, std::vector<TDst>& dst, const ConvGeom& g, int cin_g, int cin_pad, int kw_pack,
-            int s_shift, F cvt) {
+// OIHW [Cout][cin_g][kh][kw] -> [cout_pad][kh][kw_pack][cin_pad] (zero filled), tap s at column s + s_shift.  Runs in a
+// network's first forward, on the host; writes are contiguous and the reads of an output channel stay in the L1 cache.
+template <typename T>
+void repack(const T* src, std::vector<T>& dst, const ConvGeom& g, int cin_g, int cin_pad, int kw_pack, int s_shift) {
+    const size_t taps = (size_t)g.kh * g.kw;
     for (int o = 0; o < g.Cout; ++o)
-        for (int c = 0; c < cin_g; ++c)
-            for (int r = 0; r < g.kh; ++r)
-                for (int s = 0; s < g.kw; ++s)
-                    dst[(((size_t)o * g.kh + r) * kw_pack + s + s_shift) * cin_pad + c] =
-                        cvt(src[(((size_t)o * cin_g + c) * g.kh + r) * g.kw + s]);
+        for (int r = 0; r < g.kh; ++r)
+            for (int s = 0; s < g.kw; ++s) {
+                T* to = &dst[(((size_t)o * g.kh + r) * kw_pack + s + s_shift) * cin_pad];
+                const T* from = src + (size_t)o * cin_g * taps + (size_t)r * g.kw + s;
+                for (int c = 0; c < cin_g; ++c) to[c] = from[c * taps];
+            }
 }
 
 }  // namespace
@@ -162,7 +161,9 @@ extern "C" int exb_conv_weights_pack_f16(exb_ctx* ctx, const exb_conv_desc* d, c
     const FoldPlan fold = conv_fold_plan(g);
     const int kw_pack = fold.on ? fold.F : g.kw, s_shift = fold.on ? fold.shift : 0;
     std::vector<uint16_t> packed((size_t)cout_pad * g.kh * kw_pack * cin_pad, 0);
-    repack(w_oihw, packed, g, cin_g, cin_pad, kw_pack, s_shift, f32_to_f16_bits);
+    std::vector<uint16_t> half((size_t)g.Cout * cin_g * g.kh * g.kw);
+    glasssix::excalibur::convert_f32_to_f16(w_oihw, half.data(), half.size());      // round to nearest even
+    repack(half.data(), packed, g, cin_g, cin_pad, kw_pack, s_shift);
     std::vector<float> scale(cout_pad, 0.f), b(cout_pad, 0.f);
     for (int o = 0; o < g.Cout; ++o) {
         scale[o] = 1.0f;
@@ -186,7 +187,7 @@ extern "C" int exb_conv_weights_pack_i8(exb_ctx* ctx, const exb_conv_desc* d, co
     const FoldPlan fold = conv_fold_plan(g);
     const int kw_pack = fold.on ? fold.F : g.kw, s_shift = fold.on ? fold.shift : 0;
     std::vector<int8_t> packed((size_t)cout_pad * g.kh * kw_pack * cin_pad, 0);
-    repack(w_oihw, packed, g, cin_g, cin_pad, kw_pack, s_shift, [](int8_t v) { return v; });
+    repack(w_oihw, packed, g, cin_g, cin_pad, kw_pack, s_shift);
     std::vector<float> scale(cout_pad, 0.f), b(cout_pad, 0.f);
     for (int o = 0; o < g.Cout; ++o) {
         const float ws = n_wscale == 1 ? wscale[0] : wscale[o];
