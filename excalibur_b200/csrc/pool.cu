@@ -288,15 +288,11 @@ __global__ void __launch_bounds__(kRowThreads, 2)
                 for (int k = 0; k < kRowCols; ++k) {
                     const int ws = (t.ow0 + k) * S - p.pl, we = min(ws + K, p.W + p.pr);
                     const float d = (float)(hc * (p.count_include_pad ? we - ws : min(we, p.W) - max(ws, 0)));
-                    const float r = __frcp_rn(d);
                     float f[4];
                     unpack2(a[k][0], f[0], f[1]);
                     unpack2(a[k][1], f[2], f[3]);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {       // f / d: quotient by the reciprocal and one correction by its remainder
-                        const float q = f[i] * r;
-                        f[i] = fmaf(fmaf(-q, d, f[i]), r, q);
-                    }
+                    for (int i = 0; i < 4; ++i) f[i] /= d;
                     const __half2 h0 = __floats2half2_rn(f[0], f[1]), h1 = __floats2half2_rn(f[2], f[3]);
                     v[k] = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
                 }

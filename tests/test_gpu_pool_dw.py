@@ -201,3 +201,32 @@ def test_pool_stream_edges(ctx, case):
 @pytest.mark.parametrize("shape", [(1, 8, 112, 111), (3, 264, 33, 29), (1, 64, 40, 40), (70, 272, 9, 9)])
 def test_global_pool_split(ctx, type_, shape):
     test_global_pool(ctx, type_, shape)
+
+
+def _averages(ctx, capi, x, k, s, pad, pad_mode, cip, dtype, out2_scale=None):
+    N, Cc, H, W = x.shape
+    d = capi.make_pool_desc(N, H, W, Cc, 1, k, s, pad, False, pad_mode, cip, capi.EXB_F16 if dtype == np.float16 else capi.EXB_F32,
+                            *(() if out2_scale is None else (capi.EXB_I8, out2_scale)))
+    y, y2 = capi.pool2d(ctx, d, dev(to_nhwc(x).astype(dtype)))
+    ctx.sync_check()
+    return host(y), None if y2 is None else host(y2)
+
+
+# Averages of small windows (row stream) against the kernel with a thread per output vector, which an fp32 map takes: small
+# integers, so that the sums are exact in any order and only the division is left, with every divisor that the window
+# can have at the borders, and infinities, NaN and zeros among the values.
+@pytest.mark.parametrize("cip", [0, 1])
+@pytest.mark.parametrize("window", [(5, 1, 2, 1), (5, 1, 0, 1), (3, 1, 1, 1), (3, 2, 1, 0), (3, 2, 0, 0), (2, 2, 0, 0), (2, 2, 1, 1)])
+def test_pool_stream_average_is_a_division(ctx, window, cip):
+    capi = _capi()
+    k, s, pad, pad_mode = window
+    r = rng(sum(window) + cip)
+    x = r.integers(-1000, 1001, (3, 40, 14, 17)).astype(np.float32)
+    x[0, :8] = 0
+    for v, at in ((np.inf, 8), (-np.inf, 16), (np.nan, 24)):
+        x[:, at:at + 8][r.random((3, 8, 14, 17)) < 0.02] = v
+    x[1, 8, 3, 3], x[1, 8, 3, 4] = np.inf, -np.inf
+    y, _ = _averages(ctx, capi, x, k, s, pad, pad_mode, cip, np.float16)
+    ref, _ = _averages(ctx, capi, x, k, s, pad, pad_mode, cip, np.float32)
+    assert np.isinf(ref).any() and np.isnan(ref).any()
+    np.testing.assert_array_equal(y, ref.astype(np.float16))
