@@ -232,6 +232,7 @@ __device__ __forceinline__ uint32_t hmax2_u32(uint32_t a, uint32_t b) {
 // thread per output vector read each input vector K * K times and divided 64-bit indices for each of them.
 // 5x5/1, 24 maps of 256 channels @45x39: 62 -> 12 us; 3x3/2, 256 maps of 64 channels @112: 127 -> 84 us = 94 % of the HBM
 // copy rate (a former kernel of its own, 2x2 outputs per thread).
+constexpr uint32_t kNegInf2 = 0xFC00FC00u;       // (-inf, -inf) in fp16
 struct PoolStreamParams : RowStreamParams {
     int H, W, pt, pb, pl, pr, count_include_pad;
     float out2_scale;
@@ -279,8 +280,9 @@ __global__ void __launch_bounds__(kRowThreads, 2)
         if (o >= 0 && o < t.rows) {
             uint2 v[kRowCols];
             if constexpr (kMax) {
+                // a window of nothing but padding or NaN has the maximum of no values
 #pragma unroll
-                for (int k = 0; k < kRowCols; ++k) v[k] = make_uint2(a[k][0], a[k][1]);
+                for (int k = 0; k < kRowCols; ++k) v[k] = make_uint2(hmax2_u32(a[k][0], kNegInf2), hmax2_u32(a[k][1], kNegInf2));
             } else {
                 const int hs = (t.oh0 + o) * S - p.pt, he = min(hs + K, p.H + p.pb);
                 const int hc = p.count_include_pad ? he - hs : min(he, p.H) - max(hs, 0);
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(kRowThreads, 2)
 #pragma unroll
             for (int a = 0; a < A; ++a)
 #pragma unroll
-                for (int k = 0; k < kRowCols; ++k) acc[a][k][0] = acc[a][k][1] = kMax ? (Acc)0xFC00FC00u : (Acc)0;     // (-inf, -inf)
+                for (int k = 0; k < kRowCols; ++k) acc[a][k][0] = acc[a][k][1] = kMax ? (Acc)kNegInf2 : (Acc)0;
         },
         [&](const int rr, const uint2 (&rv)[IN]) {
             Acc h[kRowCols][2];

@@ -230,3 +230,28 @@ def test_pool_stream_average_is_a_division(ctx, window, cip):
     ref, _ = _averages(ctx, capi, x, k, s, pad, pad_mode, cip, np.float32)
     assert np.isinf(ref).any() and np.isnan(ref).any()
     np.testing.assert_array_equal(y, ref.astype(np.float16))
+
+
+# Windows that lie wholly in the padding (ceil mode on odd sides, padding as wide as the window) or hold nothing but NaN:
+# the row stream gives what the kernel with a thread per output vector gives, whatever kernel the channel count selects.
+@pytest.mark.parametrize("type_", [0, 1])
+@pytest.mark.parametrize("case", [(1, 32, 3, 5, 2, 2, 1, 0), (2, 40, 3, 3, 2, 2, 1, 0), (1, 32, 4, 6, 2, 2, 2, 1), (2, 64, 7, 5, 3, 2, 3, 1), (1, 24, 5, 9, 3, 1, 4, 1),
+                                  (1, 8, 6, 4, 5, 1, 6, 1), (1, 264, 2, 2, 5, 1, 5, 0)])
+def test_pool_stream_windows_without_values(ctx, case, type_):
+    import torch
+    capi = _capi()
+    N, Cc, H, W, k, s, pad, pad_mode = case
+    x = rng(sum(case)).integers(-30, -2, (N, Cc, H, W)).astype(np.float32)
+    x[:, 1] = np.nan
+    x[:, 2, :2] = np.nan
+    got = []
+    for dt in (np.float16, np.float32):
+        d = capi.make_pool_desc(N, H, W, Cc, type_, k, s, pad, False, pad_mode, 0, capi.EXB_F16 if dt == np.float16 else capi.EXB_F32,
+                                *((capi.EXB_I8, np.float32(2.5)) if type_ == 0 else ()))
+        y, y2 = capi.pool2d(ctx, d, dev(to_nhwc(x).astype(dt)))
+        ctx.sync_check()
+        got.append((y.to(torch.float16), y2))
+    assert not torch.isfinite(got[1][0][..., 0]).all(), "no window without values"
+    np.testing.assert_array_equal(host(got[0][0]), host(got[1][0]))
+    if type_ == 0:
+        np.testing.assert_array_equal(host(got[0][1]), host(got[1][1]))
