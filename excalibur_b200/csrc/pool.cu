@@ -242,15 +242,13 @@ template <int K, int S> constexpr RowStreamKind kPoolKind = {
 
 // One output row of a thread to memory.
 template <bool kOut2>
-__device__ __forceinline__ void pool_store_row(const uint2 (&v)[kRowCols], __half* y, int8_t* y2, int64_t off, int cs, int cols, float q) {
+__device__ __forceinline__ void pool_store_row(const uint2 (&v)[kRowCols], const uint32_t (&q)[kRowCols], __half* y, int8_t* y2, int64_t off, int cs,
+                                               int cols) {
 #pragma unroll
     for (int t = 0; t < kRowCols; ++t) {
         if (t >= cols) continue;
         *reinterpret_cast<uint2*>(y + off + t * cs) = v[t];
-        if (kOut2) {
-            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v[t].x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v[t].y));
-            *reinterpret_cast<uint32_t*>(y2 + off + t * cs) = quant_pack4(a.x, a.y, b.x, b.y, q);
-        }
+        if (kOut2) *reinterpret_cast<uint32_t*>(y2 + off + t * cs) = q[t];
     }
 }
 
@@ -279,10 +277,17 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     auto finish = [&](const Acc (&a)[kRowCols][2]) {
         if (o >= 0 && o < t.rows) {
             uint2 v[kRowCols];
+            uint32_t q[kRowCols];
             if constexpr (kMax) {
                 // a window of nothing but padding or NaN has the maximum of no values
 #pragma unroll
-                for (int k = 0; k < kRowCols; ++k) v[k] = make_uint2(hmax2_u32(a[k][0], kNegInf2), hmax2_u32(a[k][1], kNegInf2));
+                for (int k = 0; k < kRowCols; ++k) {
+                    v[k] = make_uint2(hmax2_u32(a[k][0], kNegInf2), hmax2_u32(a[k][1], kNegInf2));
+                    if (kOut2) {
+                        const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&v[k].x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&v[k].y));
+                        q[k] = quant_pack4(lo.x, lo.y, hi.x, hi.y, p.out2_scale);
+                    }
+                }
             } else {
                 const int hs = (t.oh0 + o) * S - p.pt, he = min(hs + K, p.H + p.pb);
                 const int hc = p.count_include_pad ? he - hs : min(he, p.H) - max(hs, 0);
@@ -297,9 +302,14 @@ __global__ void __launch_bounds__(kRowThreads, 2)
                     for (int i = 0; i < 4; ++i) f[i] /= d;
                     const __half2 h0 = __floats2half2_rn(f[0], f[1]), h1 = __floats2half2_rn(f[2], f[3]);
                     v[k] = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+                    if (kOut2) {       // of the fp32 average, by quant_rne as in the other kernel: NaN is the lowest value
+                        q[k] = 0;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) q[k] |= (uint32_t)(uint8_t)quant_rne(f[i] * p.out2_scale) << (8 * i);
+                    }
                 }
             }
-            pool_store_row<kOut2>(v, y, y2, off, p.cs, t.cols, p.out2_scale);
+            pool_store_row<kOut2>(v, q, y, y2, off, p.cs, t.cols);
         }
         ++o;
         off += ypitch;

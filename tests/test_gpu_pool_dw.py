@@ -255,3 +255,17 @@ def test_pool_stream_windows_without_values(ctx, case, type_):
     np.testing.assert_array_equal(host(got[0][0]), host(got[1][0]))
     if type_ == 0:
         np.testing.assert_array_equal(host(got[0][1]), host(got[1][1]))
+
+
+# The int8 second output of an average is the rounded fp32 average (a value rounded to fp16 first lands on the other side of
+# a half in a few per mille): integers whose sums are exact, against the kernel that an fp32 map takes.
+@pytest.mark.parametrize("window", [(5, 1, 2, 1), (3, 1, 1, 1), (3, 2, 1, 0), (2, 2, 0, 0)])
+def test_pool_stream_average_quantised_from_fp32(ctx, window):
+    capi = _capi()
+    k, s, pad, pad_mode = window
+    x = rng(sum(window)).integers(-1000, 1001, (8, 64, 28, 31)).astype(np.float32)
+    x[:, 3][rng(1).random((8, 28, 31)) < 0.05] = np.nan
+    scale = np.float32(0.28)
+    _, q = _averages(ctx, capi, x, k, s, pad, pad_mode, 0, np.float16, scale)
+    _, ref = _averages(ctx, capi, x, k, s, pad, pad_mode, 0, np.float32, scale)
+    np.testing.assert_array_equal(q, ref)
