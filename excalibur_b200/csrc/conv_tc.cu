@@ -46,7 +46,7 @@ constexpr int kMaxD2sBlocks = 16;     // 32-channel blocks of a result stored de
 constexpr int kFirstEpiWarp = 2;   // warp 0 producer, warp 1 MMA issuer, epilogue warps from here on
 constexpr int kMaxAccBufs = 4;
 constexpr int kConstCh = 64;      // output channels of the pool epilogue (scale / bias travel as launch parameters)
-constexpr uint32_t kMaxSpins = 1u << 21;  // tens of milliseconds at least; a legitimate wait is microseconds
+constexpr uint32_t kMaxSpins = 1u << 21;  // polls of 4 us, 8 s; a legitimate wait is microseconds
 
 // kEpiMapped: the quad epilogue with a result stored depth-to-space or a residual at half the resolution (a kernel of its
 // own: the few instructions that the mapping takes cost the plain epilogue 2 %)
@@ -595,6 +595,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
             const uint32_t rb_row = (uint32_t)((p.kw - 1) * p.cblks) * b_blk;   // after a row's last channel block: skip its other taps
             const uint32_t idesc = p.idesc;
             if (bres && !ptx::mbar_wait_bounded_uniform(ptx::smem_u32(&bres_bar), 0, &abort_flag, kMaxSpins)) ok = false;
+            pdl_wait();      // the bounded waits below are for this kernel's own loads, not for what is left of the previous kernel
             for (int t = first_unit; t < total_tiles && ok; t += unit_step) {
                 if (!ptx::mbar_wait_bounded_uniform(tempty0 + acc * 8, acc_phase ^ 1u, &abort_flag, kMaxSpins)) {
                     ok = false;
