@@ -179,10 +179,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
                     phase ^= 1u;
                 }
             }
-            if (!ok) {
-                atomicExch(p.error, 1);
-                for (int i = 0; i < 2000; ++i) __nanosleep(100);      // copies in flight land before the block ends
-            }
+            if (!ok) ptx::give_up(p.error, 1);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -215,8 +212,9 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
                     phase ^= 1u;
                 }
             }
+            // the producer may have left already, with its loads still in flight; the abort flag is set
+            if (!ok) ptx::give_up(p.error, 2);
             ptx::tc_commit_u32(ptx::smem_u32(&done_bar), leader);
-            if (!ok && leader) atomicExch(p.error, 2);
         }
         __syncwarp();
     }
@@ -234,7 +232,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
             }
         }
         // accumulator -> shared memory, rows padded by 16 bytes: eight lanes' 16-byte stores cover all banks
-        ok = ptx::mbar_wait_bounded_warp(&done_bar, 0, &abort_flag, kSplitMaxSpins);
+        ok = ptx::mbar_wait_bounded_warp(&done_bar, 0, &abort_flag, kSplitMaxSpins) && !__any_sync(0xffffffffu, *(volatile int*)&abort_flag);
         if (ok) {
             ptx::tc_fence_after_sync();
             const int q = warp & 3;

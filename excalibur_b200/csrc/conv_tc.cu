@@ -522,10 +522,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                         phase ^= 1u;
                     }
                 }
-                if (!ok) {
-                    atomicExch(p.error, 1);
-                    for (int i = 0; i < 2000; ++i) __nanosleep(100);
-                }
+                if (!ok) ptx::give_up(p.error, 1);
             }
         } else if (lane < G) {
             TileCursor cur(p, first_unit, unit_step);
@@ -558,12 +555,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                     }
                 }
             }
-            if (!ok) {
-                if (lane == 0) atomicExch(p.error, 1);
-                // Give copies already in flight time to land before this CTA's shared memory
-                // can be handed to another CTA.
-                for (int i = 0; i < 2000; ++i) __nanosleep(100);
-            }
+            if (!ok) ptx::give_up(p.error, 1);
         }
     } else if (warp == 1) {
         // ------------------------------- MMA issuer ----------------------------------------
@@ -716,7 +708,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                     acc_phase ^= 1u;
                 }
             }
-            if (!ok && leader) atomicExch(p.error, 2);
+            if (!ok) ptx::give_up(p.error, 2);      // the producer may have left already, with its loads still in flight
         }
     } else if (warp >= kFirstEpiWarp) {
         // ------------------------------- epilogue ------------------------------------------

@@ -124,6 +124,13 @@ __device__ __forceinline__ bool mbar_wait_bounded_warp(uint64_t* bar, uint32_t p
     return ok != 0;
 }
 
+// What a role does whose bounded wait ran out: the error word, and a pause in which the CTA's copies in flight land, so that
+// its shared memory can be used for something else or handed on.
+__device__ __forceinline__ void give_up(int* error, int code) {
+    atomicExch(error, code);
+    for (int i = 0; i < 2000; ++i) __nanosleep(100);
+}
+
 // The warp's index, known to the compiler as uniform.  A role whose whole warp runs one uniform instruction stream, with
 // only the tensor-core and commit instructions predicated on one elected lane, keeps descriptors and addresses in uniform
 // registers; a lone thread in a divergent branch moves each of them there for every instruction.  Measured on MMAs of

@@ -134,10 +134,7 @@ __device__ __forceinline__ void row_stream_run(const CUtensorMap& map, const Row
             // everybody has read the slot (it is requested again at the top of the next stage); a wait that ran out
             // takes all threads out together
             if (!__syncthreads_and(got)) {
-                if (tid == 0) {
-                    atomicExch(p.error, 4);
-                    for (int i = 0; i < 2000; ++i) __nanosleep(100);      // copies in flight land before the shared memory is handed on
-                }
+                if (tid == 0) ptx::give_up(p.error, 4);
                 return;
             }
             if (++slot == NS) {

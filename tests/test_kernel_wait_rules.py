@@ -29,3 +29,20 @@ def test_mma_role_waits_for_the_previous_kernel_before_it_polls_for_loads(name):
     role = _part(name, *MMA_ROLES[name])
     assert "pdl_wait();" in role
     assert role.index("pdl_wait();") < role.index("full0 +")
+
+
+@pytest.mark.parametrize("name", sorted(MMA_ROLES))
+def test_mma_role_that_gives_up_pauses_for_the_loads_in_flight(name):
+    """With a reduction that fits the ring the producer has left by then: nobody else would wait before the shared memory
+    becomes the partial tile or another block's."""
+    role = _part(name, *MMA_ROLES[name])
+    assert "if (!ok) ptx::give_up(" in role
+    if name == "conv_split.cu":      # before the commit that lets the epilogue write over the ring, which then does not
+        assert role.index("give_up(") < role.index("&done_bar")
+        spill = _part(name, "uint4 res[kSplitMaxItems];", "ptx::tc_fence_after_sync();")
+        assert "abort_flag" in spill[spill.index("&done_bar") + len("&done_bar, 0, &abort_flag"):]
+
+
+def test_giving_up_sets_the_error_word_and_pauses():
+    body = _part("ptx_sm100.cuh", "void give_up(", "}\n\n")
+    assert re.search(r"atomicExch\(error, code\);\s*for \(int i = 0; i < 2000; \+\+i\) __nanosleep\(100\);", body)
