@@ -1155,6 +1155,8 @@ ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64
     const ConvNTile wide = tile(256), narrow = tile(128);
     const int64_t k_bytes = (int64_t)g.kh * g.kw * g.cin_stride * (g.in_dtype == EXB_I8 ? 1 : 2);
     if (cout_pad <= 128 || (cout_pad < 256 && k_bytes < 512) || conv_fold_plan(g).on) return wide;
+    // The mapped epilogue takes whole 32-channel blocks, which 1152, 1408, 1664 and 1920 channels in tiles of 240 are not.
+    if ((g.res_half || g.rh * g.rw > 1) && wide.BN % 32) return narrow;
     if (k_bytes < 512 || (k_bytes <= 1152 && m_tiles * narrow.n_tiles <= 4 * ctx->sm_count)) return narrow;
     const int64_t places = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
     auto rounds = [&](const ConvNTile& t) { return (double)(((m_tiles + 1) / 2 * t.n_tiles + places - 1) / places); };

@@ -494,6 +494,12 @@ def test_conv_half_resolution_residual(ctx, case):
     np.testing.assert_array_equal(to_nchw(host(y)), ref)
 
 
+# Channel counts whose 256-channel tiles are not whole 32-channel blocks.
+@pytest.mark.parametrize("case", [(1, 640, 50, 50, 1152, "f16", 2), (1, 640, 46, 48, 1920, "f16", 2)])
+def test_conv_half_resolution_residual_of_many_channels(ctx, case):
+    test_conv_half_resolution_residual(ctx, case)
+
+
 # Depth-to-space in the epilogue: one and several N tiles, factors that differ.
 @pytest.mark.parametrize("case", [(2, 64, 9, 7, 64, 2, 2), (1, 32, 20, 33, 32, 1, 3), (3, 128, 12, 11, 32, 2, 4), (2, 256, 60, 92, 128, 2, 2)])
 def test_conv_depth_to_space(ctx, case):
