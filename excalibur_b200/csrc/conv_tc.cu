@@ -1137,6 +1137,12 @@ bool conv_tc_eligible(const ConvGeom& g) {
     return true;
 }
 
+// Whether tiles of this layer can run as CTA pairs at all (see conv_tc_launch): there is no pair kernel with PReLU, a mapped
+// result or residual, folded rows or pooling.
+static bool conv_pairable(const exb_ctx* ctx, const ConvGeom& g) {
+    return ctx->sm_count >= 2 && g.act != EXB_ACT_PRELU && !g.res_half && g.rh * g.rw == 1 && !g.pool && !conv_fold_plan(g).on;
+}
+
 // The N tile: 256 channels, or 128 where that is the faster one.
 //  - Below 512 bytes of K, and up to 1152 in the first two rounds of tiles, the epilogue sets the pace, and two CTAs of
 //    128 channels per SM drain more than one of 256: 96 -> 576 int8 1x1 at 256 x 14 x 14 23.8 -> 21.4 us, 320 -> 1280 at
@@ -1158,7 +1164,8 @@ ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64
     // The mapped epilogue takes whole 32-channel blocks, which 1152, 1408, 1664 and 1920 channels in tiles of 240 are not.
     if ((g.res_half || g.rh * g.rw > 1) && wide.BN % 32) return narrow;
     if (k_bytes < 512 || (k_bytes <= 1152 && m_tiles * narrow.n_tiles <= 4 * ctx->sm_count)) return narrow;
-    const int64_t places = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
+    if (!conv_pairable(ctx, g)) return wide;
+    const int64_t places = ctx->sm_count / 2;
     auto rounds = [&](const ConvNTile& t) { return (double)(((m_tiles + 1) / 2 * t.n_tiles + places - 1) / places); };
     if (narrow.BN % 64 != 0 || 0.63 * rounds(narrow) >= rounds(wide)) return wide;      // (a pair splits whole 32-channel blocks)
     ConvNTile t = narrow;
@@ -1329,8 +1336,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     // The channel-permuting map of the quad epilogue moves 32-channel blocks, so a half must be made of whole ones.
     const int64_t k_bytes = (int64_t)g.kh * g.kw * row_bytes;      // one pixel's reduction
     const int64_t all_tiles = (int64_t)p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;
-    const bool pairable = !mapped && !patch && !fold.on && !g.pool && ctx->sm_count >= 2 && g.act != EXB_ACT_PRELU &&
-                          p.BN % (quad ? 64 : 32) == 0 && (p.tiles_nb >= 2 || p.tiles_h >= 2);
+    const bool pairable = conv_pairable(ctx, g) && !patch && p.BN % (quad ? 64 : 32) == 0 && (p.tiles_nb >= 2 || p.tiles_h >= 2);
     bool pair = false;
     if (p.rowbox)
         pair = pairable && rb.one_cta && (p.BN == 64 || p.BN == 128);

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from oracle import exb_oracle as O
-from tests.util import dev, host, rng, f16_round, to_nhwc, to_nchw, assert_close_f16, quant_weights
+from tests.util import kernels_of, dev, host, rng, f16_round, to_nhwc, to_nchw, assert_close_f16, quant_weights
 
 pytestmark = pytest.mark.gpu
 
@@ -521,3 +521,23 @@ def test_conv_depth_to_space(ctx, case):
     acc = np.maximum(O.conv2d_i8_acc(x, wq, 1, 0) + b[None, :, None, None], 0)
     ref = acc.reshape(N, rh, rw, C, H, W).transpose(0, 4, 1, 5, 2, 3).reshape(N, H * rh, W * rw, C)
     np.testing.assert_array_equal(host(y).astype(np.float32), ref.astype(np.float16).astype(np.float32))
+
+
+# There is no pair kernel with PReLU or a mapped residual: N tiles of such layers are not chosen as if they ran in pairs.
+# 128-channel tiles, two CTAs of 320 threads per SM, took 65 us for the first one where 256-channel tiles take 60.
+@pytest.mark.parametrize("case", [(256, 7, 7, 512, 512, "prelu"), (256, 8, 6, 512, 512, "half")])
+def test_layers_without_a_pair_kernel_keep_wide_tiles(ctx, case):
+    import torch
+    capi = _capi()
+    N, H, W, Cin, Cout, kind = case
+    half = kind == "half"
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, 3, 1, 1, capi.EXB_F16, capi.EXB_F16, act=1 if half else 106, res=half, impl=2)
+    d.res_half = int(half)
+    p = capi.ConvWeights(ctx, d, (rng(3).standard_normal((Cout, Cin, 3, 3)) * 0.02).astype(np.float32), None)
+    p.set_slopes(ctx, np.full(Cout, 0.1, np.float32))
+    x = torch.zeros((N, H, W, Cin), device="cuda", dtype=torch.float16)
+    res = torch.zeros((N, H // 2, W // 2, Cout), device="cuda", dtype=torch.float16) if half else None
+    launches = kernels_of(lambda: capi.conv2d(ctx, d, x, p, res))
+    ctx.sync_check()
+    conv = [k for k in launches if "conv_tc_kernel" in k[0]]
+    assert len(conv) == 1 and conv[0][2][0] == 576, launches

@@ -86,3 +86,19 @@ def sample(a, limit=8192):
     flat = np.ascontiguousarray(a, np.float32).reshape(-1)
     step = max(1, -(-flat.size // limit))
     return flat[::step].copy()
+
+
+def kernels_of(fn):
+    """The kernels that fn() launches, as (name, grid, block), from the CUDA activity trace."""
+    import json
+    import tempfile
+    import torch
+    fn()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    with tempfile.NamedTemporaryFile(suffix=".json") as f:
+        prof.export_chrome_trace(f.name)
+        events = json.load(open(f.name))["traceEvents"]
+    return [(e["name"], tuple(e["args"]["grid"]), tuple(e["args"]["block"])) for e in events if e.get("cat") == "kernel"]
