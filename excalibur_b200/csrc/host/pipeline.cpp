@@ -1675,9 +1675,11 @@ void fused_plan::run(const float* host_input, int chunks, bool use_graph, int ho
     const bool ahead = many && !pageable && !convert;
     if (ahead)
         for (auto& s : prog.slices) send(*s);
-    CUDA_CHECK(cudaEventRecord(ev0_, stream_));
+    // device_ms(): of a divided batch the kernels and the copies they wait for, else the kernels alone
+    if (many) CUDA_CHECK(cudaEventRecord(ev0_, stream_));
     for (auto& s : prog.slices) {
         if (!ahead) send(*s);
+        if (!many) CUDA_CHECK(cudaEventRecord(ev0_, stream_));
         if (many) CUDA_CHECK(cudaStreamWaitEvent(stream_, s->copied, 0));
         launch(*s, use_graph);
         if (many) {

@@ -65,7 +65,8 @@ public:
     int trace_size() const;
     bool trace_entry(int i, std::string& name, double& begin_ms, double& end_ms) const;
     int launches_last_forward() const;   // kernels launched by the last forward
-    double device_ms_last_forward() const;   // device time of the last forward's kernels (events)
+    // Device time of the last forward's kernels (events); of a divided batch with the copies they wait for.
+    double device_ms_last_forward() const;
     std::vector<std::string> input_names() const;
     std::vector<std::string> output_names() const;
 

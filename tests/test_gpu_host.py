@@ -443,6 +443,22 @@ def test_divided_forward_and_pageable_input():
     p.close()
 
 
+def test_device_time_of_an_undivided_forward_is_its_kernels():
+    """stats() reports the device time of the last forward's kernels: the copy of the input is not part of it."""
+    h = _host()
+    scales = {str(n): np.float32(s) for n, s in zip(G["resnet_scale_names"], G["resnet_scales"])}
+    g, _ = models.resnet18(2, act_scales=scales)
+    x = np.random.default_rng(12).uniform(0, 1, (200, 3, 160, 128)).astype(np.float32)       # 49 MB: 0.9 ms of copy and more
+    p = h.Pipeline(g.phai_text(), g.racy_bytes(), 0, fusion=True)
+    p.set_option("h2d_chunks", 1)
+    for _ in range(3):
+        p.forward_ptr(x.ctypes.data, *x.shape)
+    device_ms = p.stats()[1]
+    resident = p.run_resident(10) / 10
+    assert 0.5 * resident < device_ms < 1.3 * resident + 0.1, (device_ms, resident)
+    p.close()
+
+
 def test_maps_inside_a_concat_and_a_resized_residual_are_read_on_request():
     """What a Concat's producers store in place, and nearest resizes that only a Concat or an addition reads, are not
     kept; get() derives them, whatever the division of the batch, and they equal those of the plan without fusion."""
