@@ -186,9 +186,8 @@ private:
     // that of its first image.
     void* form(std::shared_ptr<dev_buf>& b, const fmap_info& f, size_t per_image) {
         if (!b) b = std::make_shared<dev_buf>();
-        if (f.N != emit_n_) uneven_ = true;      // a map whose first dimension is not the batch cannot be divided
-        const size_t images = f.N == emit_n_ ? (size_t)N_ : (size_t)f.N;
-        return static_cast<char*>(b->ensure(images * per_image, device_)) + (f.N == emit_n_ ? (size_t)emit_n0_ * per_image : 0);
+        CHECK_EQ(f.N, emit_n_) << f.name << ": every operation keeps the batch as the first dimension";
+        return static_cast<char*>(b->ensure((size_t)N_ * per_image, device_)) + (size_t)emit_n0_ * per_image;
     }
     void* form_f16(fmap_info& f) { return form(f.f16, f, (size_t)f.H * (f.w_pitch ? f.w_pitch : f.W) * f.cs * 2); }
     void* form_i8(fmap_info& f) { return form(f.i8, f, (size_t)f.H * f.W * f.cs); }
@@ -241,7 +240,7 @@ private:
     // A way to run the batch: its division, and whether the input arrives as fp16 planes.
     struct program {
         std::vector<int> sizes;
-        bool f16_src = false, uneven = false;
+        bool f16_src = false;
         double flops_i8 = 0, flops_f16 = 0;      // dense convolutions
         std::vector<std::unique_ptr<slice>> slices;
         int launches() const {
@@ -256,7 +255,6 @@ private:
     std::vector<int> choose_slices(bool f16_src);
     void layout(slice& s, bool f16_src);   // the steps of images [s.n0, s.n0 + s.n)
     int emit_n0_ = 0, emit_n_ = 0;
-    bool uneven_ = false;
     std::vector<plan_step>* emit_steps_ = nullptr;
     double body_flops_i8_ = 0, body_flops_f16_ = 0;
     std::vector<int> auto_sizes_[2];       // choose_slices' answers
@@ -345,8 +343,7 @@ void fused_plan::build(int N, int C, int H, int W) {
     built_ = true;
 }
 
-// The program for a division of the batch, laid out when it is first asked for.  A graph with a map whose first dimension
-// is not the batch runs undivided.
+// The program for a division of the batch, laid out when it is first asked for.
 fused_plan::program& fused_plan::program_for(const std::vector<int>& sizes, bool f16_src) {
     for (auto& p : programs_)
         if (p->sizes == sizes && p->f16_src == f16_src) return *p;
@@ -361,15 +358,12 @@ fused_plan::program& fused_plan::program_for(const std::vector<int>& sizes, bool
         n0 += n;
         layout(*s, f16_src);
         CUDA_CHECK(cudaStreamSynchronize(nullptr));      // clears of padding channels, on the default stream
-        p->uneven = uneven_;
         p->flops_i8 += body_flops_i8_;
         p->flops_f16 += body_flops_f16_;
-        if (uneven_ && sizes.size() > 1) break;
         CUDA_CHECK(cudaEventCreateWithFlags(&s->copied, cudaEventDisableTiming));
         CUDA_CHECK(cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming));
         p->slices.push_back(std::move(s));
     }
-    if (uneven_ && sizes.size() > 1) return program_for({N_}, f16_src);
     programs_.push_back(std::move(p));
     return *programs_.back();
 }
@@ -379,7 +373,6 @@ void fused_plan::layout(slice& sl, bool f16_src) {
     emit_n0_ = sl.n0;
     emit_n_ = sl.n;
     emit_steps_ = &sl.steps;
-    uneven_ = false;
     body_flops_i8_ = body_flops_f16_ = 0;
     for (auto& f : fmaps_) kept_[f.name].keep(f);
     fmaps_.clear();
@@ -1564,7 +1557,7 @@ void fused_plan::layout(slice& sl, bool f16_src) {
         });
     }
     for (auto& f : fmaps_)
-        if (f.N == sl.n) f.N = N_;       // what fetch() and the results see is the whole batch
+        if (f.N) f.N = N_;       // what fetch() and the results see is the whole batch
 }
 
 // The kernels of a sub-batch: eagerly the first time, as one CUDA graph afterwards.
@@ -1588,8 +1581,7 @@ void fused_plan::launch(slice& s, bool use_graph) {
 void fused_plan::copy_results(const slice& s, cudaStream_t st) {
     for (auto& kv : host_out_) {
         fmap_info& f = fmaps_[root(index_[kv.first])];
-        const bool whole = f.N != N_;        // not divisible: the only sub-batch is the batch
-        const size_t first = whole ? 0 : s.n0, images = whole ? f.N : s.n, per = (size_t)f.C * f.H * f.W;
+        const size_t first = s.n0, images = s.n, per = (size_t)f.C * f.H * f.W;
         float* dst = kv.second->mutable_cpu_data() + first * per;
         const float* src = static_cast<const float*>(f.f32->p) + first * (f.f32_pitch ? (size_t)f.f32_pitch : per);
         if (f.f32_pitch)
@@ -1758,7 +1750,7 @@ double fused_plan::run_resident(int iters, bool use_graph) {
 std::vector<int> fused_plan::choose_slices(bool f16_src) {
     const program& prog = program_for({N_}, f16_src);
     const std::vector<int> undivided{N_};
-    if (prog.uneven || N_ < 2) return undivided;
+    if (N_ < 2) return undivided;
     double bytes = 0, out_bytes = 0;
     for (auto& f : fmaps_) {
         const double px = (double)f.N * f.H * f.W;

@@ -49,3 +49,26 @@ def test_shipped_architecture(arch, fusion):
         print("%s: %d launches" % (name, launches))
         assert (launches > 0) == (name not in ("pfld11_landmark65_simp", "singel_char_classfi_simp")), launches
     p.close()
+
+
+@pytest.mark.parametrize("arch", ARCHS, ids=[a["name"][:28] for a in ARCHS])
+def test_shipped_architecture_divided(arch):
+    """A batch run as sub-batches gives what the whole batch at once gives, whatever operations the graph ends in (Reshape,
+    Transpose, Flatten, Softmax, InnerProduct): they all keep the batch as the first dimension."""
+    from excalibur_b200 import host
+    g, outs = model_zoo.graph_from_structure(arch["structure"], arch["seed"], gain=arch["gain"])
+    p = host.Pipeline(g.phai_text(), g.racy_bytes(), 0, fusion=True)
+    x = model_zoo.architecture_input(arch, 6)
+    p.set_option("h2d_chunks", 1)
+    whole = {n: a.copy() for n, a in p.forward(x).items()}
+    launches = p.stats()[0]
+    for chunks in (3, 2, 6):
+        p.set_option("h2d_chunks", chunks)
+        for _ in range(2):
+            res = p.forward(x)
+        assert p.stats()[0] > launches or launches < 0      # (< 0: the two that run op by op)
+        for n in outs:
+            assert res[n].shape == whole[n].shape
+            # fp16 maps: another order of the fp32 sums moves a rounding here and there
+            assert _rel(res[n], whole[n]) < 5e-3, (n, chunks)
+    p.close()
