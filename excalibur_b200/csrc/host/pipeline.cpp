@@ -12,6 +12,7 @@
 #include <map>
 #include <set>
 
+#include "batch_division.hpp"
 #include "host_convert.hpp"
 #include "ops.hpp"
 
@@ -1741,16 +1742,12 @@ double fused_plan::run_resident(int iters, bool use_graph) {
     return ms;
 }
 
-// How a forward is divided when the caller leaves it open: the division whose modelled time is shortest.  Copies to the
-// device, kernels and copies back are three lanes that run side by side; a sub-batch passes through them one after the
-// other.  The kernels of n of N images are taken as launches * 4.6 us + body * (n / N)^0.8 (small sub-batches fill the
-// chip less), with the body from the plan's own traffic and arithmetic: within 15 % of the measured time of the
-// benchmark networks from 4 images on.  Copies move 53 GB/s.  Divisions are looked for among all ways to put 16 units
-// together in at most eight parts; one has to promise 3 % and 20 us to be taken.
+// How a forward is divided when the caller leaves it open (see divide_batch): kernels are taken as 4.6 us a launch and a
+// body from the plan's own traffic and arithmetic, within 15 % of the measured time of the benchmark networks from 4 images
+// on.  Copies move 53 GB/s.
 std::vector<int> fused_plan::choose_slices(bool f16_src) {
     const program& prog = program_for({N_}, f16_src);
-    const std::vector<int> undivided{N_};
-    if (N_ < 2) return undivided;
+    if (N_ < 2) return {N_};
     double bytes = 0, out_bytes = 0;
     for (auto& f : fmaps_) {
         const double px = (double)f.N * f.H * f.W;
@@ -1764,41 +1761,7 @@ std::vector<int> fused_plan::choose_slices(bool f16_src) {
     const double in_us = (double)N_ * C_ * H_ * W_ * (f16_src ? 2 : 4) / 53e3, out_us = out_bytes / 53e3;
     const double fixed = 4.6 * prog.launches();
     const double body = 2 * bytes / 4.5e6 + prog.flops_i8 / 1.2e9 + prog.flops_f16 / 0.6e9;
-    constexpr int kUnits = 16, kParts = 8;
-    double kernels[kUnits + 1];
-    for (int u = 0; u <= kUnits; ++u) kernels[u] = fixed + body * std::pow(u / (double)kUnits, 0.8);
-    const double whole = in_us + kernels[kUnits] + out_us;
-    double best = std::min(0.97 * whole, whole - 20.0);
-    std::vector<int> parts, best_parts;
-    const int step = N_ >= kUnits ? 1 : (kUnits + N_ - 1) / N_;      // a unit is at least one image
-    std::function<void(int, double, double, double)> walk = [&](int left, double in, double run, double out) {
-        if (out >= best) return;
-        if (left == 0) {
-            best = out;
-            best_parts = parts;
-            return;
-        }
-        if ((int)parts.size() == kParts) return;
-        for (int u = step; u <= left; u += step) {
-            if (left - u > 0 && left - u < step) continue;
-            const double in2 = in + in_us * u / kUnits + 6.0, run2 = std::max(run, in2) + kernels[u] + 4.0;
-            const double out2 = std::max(out, run2) + out_us * u / kUnits + 6.0;
-            parts.push_back(u);
-            walk(left - u, in2, run2, out2);
-            parts.pop_back();
-        }
-    };
-    walk(kUnits, 0, 0, 0);
-    if (best_parts.empty()) return undivided;
-    std::vector<int> sizes;
-    int units = 0, done = 0;
-    for (int u : best_parts) {
-        units += u;
-        const int upto = (int)((int64_t)N_ * units / kUnits);
-        if (upto > done) sizes.push_back(upto - done);
-        done = upto;
-    }
-    return sizes;
+    return divide_batch(N_, in_us, out_us, fixed, body);
 }
 
 std::shared_ptr<memory::tensor<float>> fused_plan::fetch(const std::string& name_in) {

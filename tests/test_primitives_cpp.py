@@ -31,3 +31,8 @@ def _build_and_run(name, tmp_path):
 def test_pool_allocator_reuse_rule_and_two_thread_stress(tmp_path):
     out = _build_and_run("pool_allocator_test", tmp_path)
     assert out.strip().endswith("ok"), out
+
+
+def test_every_batch_size_can_be_divided(tmp_path):
+    out = _build_and_run("batch_division_test", tmp_path)
+    assert out.strip().endswith("ok"), out
