@@ -3,6 +3,7 @@
 // pixel (8 fp16, 16 int8 or 4 fp32 channels).  Global pooling splits the map across the threads of a CTA, and across a
 // cluster where that leaves SMs idle.
 #include "common.cuh"
+#include "host/known_divisor.hpp"
 #include "row_stream.cuh"
 
 #include <cooperative_groups.h>
@@ -236,6 +237,7 @@ constexpr uint32_t kNegInf2 = 0xFC00FC00u;       // (-inf, -inf) in fp16
 struct PoolStreamParams : RowStreamParams {
     int H, W, pt, pb, pl, pr, count_include_pad;
     float out2_scale;
+    KnownDivisor count[kMaxKnownDivisor];       // of averages: windows of 1 to 25 values
 };
 template <int K, int S> constexpr RowStreamKind kPoolKind = {
     100 + 10 * K + S, S, K, S == 1 ? K : 2, K == 5 ? 2 : 3, K == 3 && S == 2 ? 1 : 0, 15.0 + 8.0 * K / S};
@@ -294,12 +296,19 @@ __global__ void __launch_bounds__(kRowThreads, 2)
 #pragma unroll
                 for (int k = 0; k < kRowCols; ++k) {
                     const int ws = (t.ow0 + k) * S - p.pl, we = min(ws + K, p.W + p.pr);
-                    const float d = (float)(hc * (p.count_include_pad ? we - ws : min(we, p.W) - max(ws, 0)));
+                    const int d = hc * (p.count_include_pad ? we - ws : min(we, p.W) - max(ws, 0));
                     float f[4];
                     unpack2(a[k][0], f[0], f[1]);
                     unpack2(a[k][1], f[2], f[3]);
+                    // 16 quotients a thread and row: a division each took 2x2/2 at 4 x 60 x 92 x 128 from 9.0 to 14.3 us
+                    if ((unsigned)(d - 1) < (unsigned)kMaxKnownDivisor) {
+                        const KnownDivisor kd = p.count[d - 1];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) f[i] /= d;
+                        for (int i = 0; i < 4; ++i) f[i] = divide_by(f[i], kd);
+                    } else {        // a window without values
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) f[i] /= (float)d;
+                    }
                     const __half2 h0 = __floats2half2_rn(f[0], f[1]), h1 = __floats2half2_rn(f[2], f[3]);
                     v[k] = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
                     if (kOut2) {       // of the fp32 average, by quant_rne as in the other kernel: NaN is the lowest value
@@ -386,6 +395,7 @@ int launch_pool_stream(exb_ctx* ctx, const PoolParams& d, const __half* x, __hal
     if (grid < 0) return grid;
     p.H = d.H; p.W = d.W; p.pt = d.pt; p.pb = d.pb; p.pl = d.pl; p.pr = d.pr;
     p.count_include_pad = d.count_include_pad; p.out2_scale = d.out2_scale;
+    for (int i = 0; i < kMaxKnownDivisor; ++i) p.count[i] = known_divisor(i + 1);
     auto kern = pool_stream_kernel<K, S, kMax, kOut2>;
     if (int rc = raise_smem_limit(ctx, kern)) return rc;
     return launch_pdl(ctx, "pool_stream_kernel", kern, dim3((unsigned)grid), dim3((unsigned)pl.threads), smem, st, map, y, y2, p);

@@ -36,3 +36,8 @@ def test_pool_allocator_reuse_rule_and_two_thread_stress(tmp_path):
 def test_every_batch_size_can_be_divided(tmp_path):
     out = _build_and_run("batch_division_test", tmp_path)
     assert out.strip().endswith("ok"), out
+
+
+def test_division_by_a_known_divisor_is_correctly_rounded(tmp_path):
+    out = _build_and_run("known_divisor_test", tmp_path)
+    assert out.strip().endswith("ok"), out
