@@ -212,9 +212,10 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
                     phase ^= 1u;
                 }
             }
-            // the producer may have left already, with its loads still in flight; the abort flag is set
-            if (!ok) ptx::give_up(p.error, 2);
-            ptx::tc_commit_u32(ptx::smem_u32(&done_bar), leader);
+            // without the commit the epilogue sees the abort flag and leaves the ring alone; the producer may be gone already,
+            // with its loads still in flight
+            if (ok) ptx::tc_commit_u32(ptx::smem_u32(&done_bar), leader);
+            else ptx::give_up(p.error, 2);
         }
         __syncwarp();
     }
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
             }
         }
         // accumulator -> shared memory, rows padded by 16 bytes: eight lanes' 16-byte stores cover all banks
-        ok = ptx::mbar_wait_bounded_warp(&done_bar, 0, &abort_flag, kSplitMaxSpins) && !__any_sync(0xffffffffu, *(volatile int*)&abort_flag);
+        ok = ptx::mbar_wait_bounded_warp(&done_bar, 0, &abort_flag, kSplitMaxSpins);
         if (ok) {
             ptx::tc_fence_after_sync();
             const int q = warp & 3;
