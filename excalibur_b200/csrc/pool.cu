@@ -237,7 +237,8 @@ constexpr uint32_t kNegInf2 = 0xFC00FC00u;       // (-inf, -inf) in fp16
 struct PoolStreamParams : RowStreamParams {
     int H, W, pt, pb, pl, pr, count_include_pad;
     float out2_scale;
-    KnownDivisor count[kMaxKnownDivisor];       // of averages: windows of 1 to 25 values
+    // Averages: the divisors 1 to 25.  A window outside the map has a sum of 0 and any other: NaN for 0, else 0.
+    KnownDivisor count[kMaxKnownDivisor + 2];
 };
 template <int K, int S> constexpr RowStreamKind kPoolKind = {
     100 + 10 * K + S, S, K, S == 1 ? K : 2, K == 5 ? 2 : 3, K == 3 && S == 2 ? 1 : 0, 15.0 + 8.0 * K / S};
@@ -300,15 +301,10 @@ __global__ void __launch_bounds__(kRowThreads, 2)
                     float f[4];
                     unpack2(a[k][0], f[0], f[1]);
                     unpack2(a[k][1], f[2], f[3]);
-                    // 16 quotients a thread and row: a division each took 2x2/2 at 4 x 60 x 92 x 128 from 9.0 to 14.3 us
-                    if ((unsigned)(d - 1) < (unsigned)kMaxKnownDivisor) {
-                        const KnownDivisor kd = p.count[d - 1];
+                    // 16 quotients a thread and row: as divisions they took 2x2/2 at 4 x 60 x 92 x 128 from 9.0 to 14.3 us
+                    const KnownDivisor kd = p.count[min((unsigned)d, (unsigned)kMaxKnownDivisor + 1)];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) f[i] = divide_by(f[i], kd);
-                    } else {        // a window without values
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) f[i] /= (float)d;
-                    }
+                    for (int i = 0; i < 4; ++i) f[i] = divide_by(f[i], kd);
                     const __half2 h0 = __floats2half2_rn(f[0], f[1]), h1 = __floats2half2_rn(f[2], f[3]);
                     v[k] = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
                     if (kOut2) {       // of the fp32 average, by quant_rne as in the other kernel: NaN is the lowest value
@@ -395,7 +391,9 @@ int launch_pool_stream(exb_ctx* ctx, const PoolParams& d, const __half* x, __hal
     if (grid < 0) return grid;
     p.H = d.H; p.W = d.W; p.pt = d.pt; p.pb = d.pb; p.pl = d.pl; p.pr = d.pr;
     p.count_include_pad = d.count_include_pad; p.out2_scale = d.out2_scale;
-    for (int i = 0; i < kMaxKnownDivisor; ++i) p.count[i] = known_divisor(i + 1);
+    p.count[0] = {NAN, NAN};
+    for (int i = 1; i <= kMaxKnownDivisor; ++i) p.count[i] = known_divisor(i);
+    p.count[kMaxKnownDivisor + 1] = {0.f, 0.f};
     auto kern = pool_stream_kernel<K, S, kMax, kOut2>;
     if (int rc = raise_smem_limit(ctx, kern)) return rc;
     return launch_pdl(ctx, "pool_stream_kernel", kern, dim3((unsigned)grid), dim3((unsigned)pl.threads), smem, st, map, y, y2, p);
