@@ -174,9 +174,13 @@ def _address(t):
 
 
 def _stream():
-    """Handle of the current stream of the current device as an integer (the Stream object costs 2 us)."""
-    c = _torch()._C
-    return c._cuda_getCurrentRawStream(c._cuda_getDevice())
+    """Handle of the current stream of the current device as an integer (the public Stream object costs 2 us; it is used
+    where this torch does not have the private functions)."""
+    t = _torch()
+    try:
+        return t._C._cuda_getCurrentRawStream(t._C._cuda_getDevice())
+    except AttributeError:
+        return t.cuda.current_stream().cuda_stream
 
 
 def _np_ptr(a):
