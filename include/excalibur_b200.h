@@ -239,8 +239,11 @@ EXB_API int exb_conv2d_uses_tensor_cores(const exb_conv_desc* d);
 /* 1 when exb_conv2d_fwd can run this descriptor with fuse_pool = 1 (a few-channel stride-2 fp16
  * stem on padded NHWC4 rows with 64 output channels, ReLU or ReLU6, fp16 output and an optional
  * int8 copy, no residual), else 0; negative = error.  The descriptor's own fuse_pool is ignored. */
-EXB_API int exb_conv2d_d2s_fusable(const exb_conv_desc* desc);
 EXB_API int exb_conv2d_pool_fusable(const exb_conv_desc* d);
+/* 1 when exb_conv2d_fwd can run this descriptor with its d2s_h, d2s_w (a dense tensor-core convolution to one fp16 output
+ * without residual, whose channels per tap are a multiple of 32; cout_stride up to 512 and, above 128, a multiple of 128),
+ * else 0; negative = error. */
+EXB_API int exb_conv2d_d2s_fusable(const exb_conv_desc* d);
 
 /* ---------------------------------------------------------------------------------------
  * Depthwise convolution forward.  Stands in for operation_convolutiondepthwise::forward_*
