@@ -24,7 +24,7 @@ using namespace exb;
 
 extern "C" const char* exb_last_error_string(void) { return g_last_error; }
 
-extern "C" const char* exb_version(void) { return "0.1.0"; }
+extern "C" const char* exb_version(void) { return "0.2.0"; }
 
 extern "C" int exb_ctx_create(int device, exb_ctx** out) {
     EXB_REQUIRE(out != nullptr, "exb_ctx_create: null output pointer");

@@ -70,7 +70,9 @@ EXB_API int exb_ctx_create(int device, exb_ctx** out);
 EXB_API int exb_ctx_destroy(exb_ctx* ctx);
 /* Message of the last failing call on this thread (never NULL). */
 EXB_API const char* exb_last_error_string(void);
-/* Library version string, e.g. "0.1.0". (pipeline<Dtype>::version, include/Excalibur/pipeline.hpp:41) */
+/* Library version string, e.g. "0.2.0". (pipeline<Dtype>::version, include/Excalibur/pipeline.hpp:41)
+ * The second number changes when a structure below does: the library reads descriptors by pointer, so a program compiled
+ * against another one has to be compiled again.  0.2: exb_conv_desc gained d2s_h, d2s_w and res_half. */
 EXB_API const char* exb_version(void);
 /* Number of SMs of the context's device (grid sizing of persistent kernels). */
 EXB_API int exb_ctx_sm_count(const exb_ctx* ctx, int* out);

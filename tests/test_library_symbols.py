@@ -3,6 +3,7 @@ entry point the public headers declare.  No compute call is made here."""
 import ctypes
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -79,3 +80,25 @@ def test_no_cpu_fallback_in_the_product(so_path):
     from excalibur_b200 import capi
     with pytest.raises(capi.ExbError):
         capi.Context(0)
+
+
+# Sizes of the structures that the library reads by pointer, by version: a program compiled against other sizes hands over
+# something else, so a size changes only together with the version's second number.
+ABI_SIZES = {
+    "0.1": {"exb_conv_desc": 116, "exb_dwconv_desc": 68, "exb_pool_desc": 80},
+    "0.2": {"exb_conv_desc": 128, "exb_dwconv_desc": 68, "exb_pool_desc": 80},
+}
+
+
+def test_structure_sizes_belong_to_the_version(so_path, tmp_path):
+    from excalibur_b200 import capi
+    names = sorted(ABI_SIZES["0.1"])
+    src = tmp_path / "sizes.c"
+    src.write_text('#include <stdio.h>\n#include "excalibur_b200.h"\nint main(void) {%s return 0; }\n' % "".join(
+        'printf("%%zu\\n", sizeof(%s));' % n for n in names))
+    exe = str(tmp_path / "sizes")
+    subprocess.check_call(["gcc", "-I", os.path.join(ROOT, "include"), str(src), "-o", exe])
+    sizes = dict(zip(names, map(int, subprocess.check_output([exe], text=True).split())))
+    assert sizes == ABI_SIZES[".".join(capi.lib().exb_version().decode().split(".")[:2])]
+    assert sizes == {"exb_conv_desc": ctypes.sizeof(capi.ConvDesc), "exb_dwconv_desc": ctypes.sizeof(capi.DwConvDesc),
+                     "exb_pool_desc": ctypes.sizeof(capi.PoolDesc)}
