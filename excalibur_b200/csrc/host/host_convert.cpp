@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstring>
 #include <memory>
+#include <system_error>
 
 #if defined(__x86_64__) || defined(__i386__)
 #include <immintrin.h>
@@ -160,7 +161,11 @@ void copy_streaming(char* dst, const char* src, size_t n) {
 class copy_pool {
 public:
     explicit copy_pool(int threads) : pid_(getpid()) {
-        for (int t = 1; t < threads; ++t) workers_.emplace_back([this] { work(); });
+        workers_.reserve(threads);
+        try {
+            for (int t = 1; t < threads; ++t) workers_.emplace_back([this] { work(); });
+        } catch (const std::system_error&) {      // the process may not have more: those there are do the work
+        }
     }
     ~copy_pool() {
         if (getpid() != pid_) {      // a forked child has no workers to join

@@ -41,3 +41,8 @@ def test_every_batch_size_can_be_divided(tmp_path):
 def test_division_by_a_known_divisor_is_correctly_rounded(tmp_path):
     out = _build_and_run("known_divisor_test", tmp_path)
     assert out.strip().endswith("ok"), out
+
+
+def test_host_copy_with_fewer_threads_than_it_asks_for(tmp_path):
+    out = _build_and_run("host_copy_test", tmp_path)
+    assert out.strip().endswith("ok"), out
