@@ -352,7 +352,8 @@ int launch(exb_ctx* ctx, const DwParams& p, const void* x, const exb_dw_weights*
     const int cvecs = p.cs / V;
     if (p.kh == 3 && p.kw == 3 && p.sh == p.sw && (p.sh == 1 || p.sh == 2)) {
         if constexpr (std::is_same<TIn, __half>::value) {
-            return p.sh == 1 ? launch_stream<TOut, 1>(ctx, p, xi, w, yo, st) : launch_stream<TOut, 2>(ctx, p, xi, w, yo, st);
+            const int rc = p.sh == 1 ? launch_stream<TOut, 1>(ctx, p, xi, w, yo, st) : launch_stream<TOut, 2>(ctx, p, xi, w, yo, st);
+            if (rc != EXB_ERR_UNSUPPORTED) return rc;      // (more tiles than it counts: 2^30 and more tiny maps)
         } else {
             constexpr int TW = 4;
             const int64_t total = (int64_t)p.N * p.OH * ((p.OW + TW - 1) / TW) * cvecs;

@@ -435,10 +435,12 @@ int launch(exb_ctx* ctx, const exb_pool_desc* d, const PoolParams& p, const void
     // below 32 channels the kernel with a thread per output vector is 1.2-1.4 times as fast (64 maps @50x51, 16 and 24
     // channels: 4.8-5.4 against 6.2-7.1 us); with stride 1 the stream wins at every width.
     if (std::is_same<T, __half>::value && p.kh == p.kw && p.sh == p.sw) {
-        if (p.kh == 5 && p.sh == 1) return launch_pool_stream<5, 1>(ctx, p, x, y, y2, out2, st);
-        if (p.kh == 3 && p.sh == 1) return launch_pool_stream<3, 1>(ctx, p, x, y, y2, out2, st);
-        if (p.kh == 3 && p.sh == 2 && p.cs >= 32) return launch_pool_stream<3, 2>(ctx, p, x, y, y2, out2, st);
-        if (p.kh == 2 && p.sh == 2 && p.cs >= 32) return launch_pool_stream<2, 2>(ctx, p, x, y, y2, out2, st);
+        int rc = EXB_ERR_UNSUPPORTED;       // also the answer to more tiles than the stream counts: 2^30 and more tiny maps
+        if (p.kh == 5 && p.sh == 1) rc = launch_pool_stream<5, 1>(ctx, p, x, y, y2, out2, st);
+        else if (p.kh == 3 && p.sh == 1) rc = launch_pool_stream<3, 1>(ctx, p, x, y, y2, out2, st);
+        else if (p.kh == 3 && p.sh == 2 && p.cs >= 32) rc = launch_pool_stream<3, 2>(ctx, p, x, y, y2, out2, st);
+        else if (p.kh == 2 && p.sh == 2 && p.cs >= 32) rc = launch_pool_stream<2, 2>(ctx, p, x, y, y2, out2, st);
+        if (rc != EXB_ERR_UNSUPPORTED) return rc;
     }
     const int64_t total = (int64_t)p.N * p.PH * p.PW * (p.cs / V);
     const dim3 grid((unsigned)stream_grid(ctx, total, 256));

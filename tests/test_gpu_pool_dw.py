@@ -269,3 +269,29 @@ def test_pool_stream_average_quantised_from_fp32(ctx, window):
     _, q = _averages(ctx, capi, x, k, s, pad, pad_mode, 0, np.float16, scale)
     _, ref = _averages(ctx, capi, x, k, s, pad, pad_mode, 0, np.float32, scale)
     np.testing.assert_array_equal(q, ref)
+
+
+# More tiles than the row stream counts (2^30 images of one pixel, 17 GB each way): the kernels for other windows take them.
+@pytest.mark.parametrize("op", ["dwconv", "pool"])
+def test_row_stream_tile_limit(ctx, op):
+    import torch
+    capi = _capi()
+    N, Cc = (1 << 30) + 5, 8
+    if torch.cuda.mem_get_info()[0] < 48 << 30:
+        pytest.skip("needs 48 GB of device memory")
+    x = torch.empty((N, 1, 1, Cc), device="cuda", dtype=torch.float16).fill_(2)
+    x[7], x[-1] = 3, -5
+    if op == "dwconv":
+        w = np.zeros((Cc, 1, 3, 3), np.float32)
+        w[:, 0, 1, 1] = 1.5
+        d = capi.make_dw_desc(N, 1, 1, Cc, 3, 1, 1, capi.EXB_F16, capi.EXB_F16, 0)
+        y = capi.dwconv2d(ctx, d, x, capi.DwWeights(ctx, d, w, np.zeros(Cc, np.float32)))
+        k = 1.5
+    else:
+        y, _ = capi.pool2d(ctx, capi.make_pool_desc(N, 1, 1, Cc, 0, 5, 1, 2, False, 1, 0, capi.EXB_F16), x)
+        k = 1.0
+    ctx.sync_check()
+    for i, v in ((0, 2), (7, 3), (8, 2), (1 << 29, 2), (N - 2, 2), (N - 1, -5)):
+        assert (y[i].float() == v * k).all(), i
+    del x, y
+    torch.cuda.empty_cache()
