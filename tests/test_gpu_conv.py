@@ -2,6 +2,8 @@
 oracle: int32 accumulators bit-exact, dequantised fp32 bit-exact, requantised int8 bit-exact
 against the oracle's half-even rule and within 1 LSB of the reference's half-away rule, fp16
 within 1e-2 relative of the fp32 result."""
+import re
+
 import numpy as np
 import pytest
 
@@ -446,14 +448,19 @@ def test_conv_persistent_kernel_small(ctx, case):
 
 # CTA pairs of the persistent kernel: along the images (odd group counts) and, with one image, along the rows (odd tile
 # rows); row-box and tap loops, both epilogues, two N tiles.  Integer values, so that every path is exact.
-@pytest.mark.parametrize("case", [(3, 64, 115, 113, 64, 3, 1, "f16"), (1, 64, 200, 210, 64, 3, 1, "f16"),
-                                  (1, 64, 401, 400, 64, 3, 2, "f16"), (3, 64, 230, 226, 128, 3, 2, "f16"),
-                                  (1, 128, 401, 400, 96, 3, 2, "i8"), (2, 128, 300, 270, 64, 3, 2, "i8"),
-                                  (5, 512, 9, 7, 160, 1, 1, "i8"), (5, 256, 9, 7, 192, 1, 1, "f16"),
-                                  (3, 64, 9, 9, 320, 3, 1, "i8"), (1, 64, 37, 9, 320, 3, 1, "f16"),
-                                  # more than 256 channels: N tiles of 128 or fewer, single and as pairs
-                                  (2, 128, 9, 9, 272, 1, 1, "i8"), (3, 64, 17, 9, 408, 3, 1, "f16"), (2, 128, 9, 9, 384, 3, 1, "f16"),
-                                  (3, 256, 7, 7, 512, 3, 1, "i8")])
+PAIR_CASES = [(3, 64, 115, 113, 64, 3, 1, "f16"), (1, 64, 200, 210, 64, 3, 1, "f16"),
+              (1, 64, 401, 400, 64, 3, 2, "f16"), (3, 64, 230, 226, 128, 3, 2, "f16"),
+              (1, 128, 401, 400, 96, 3, 2, "i8"), (2, 128, 300, 270, 64, 3, 2, "i8"),
+              # more than 128 channels
+              (5, 1184, 9, 7, 160, 1, 1, "i8"), (1, 160, 37, 9, 192, 3, 1, "i8"), (5, 608, 9, 7, 192, 1, 1, "f16"),
+              (3, 160, 9, 9, 320, 3, 1, "i8"), (1, 96, 37, 9, 304, 3, 1, "f16"), (3, 96, 9, 9, 304, 3, 1, "f16"),
+              (2, 128, 9, 9, 384, 3, 1, "f16"), (3, 256, 7, 7, 512, 3, 1, "i8")]
+# N tiles of 128 channels or fewer, single
+SINGLE_CASES = [(5, 512, 9, 7, 160, 1, 1, "i8"), (5, 256, 9, 7, 192, 1, 1, "f16"), (3, 64, 9, 9, 320, 3, 1, "i8"), (1, 64, 37, 9, 320, 3, 1, "f16"),
+                (2, 128, 9, 9, 272, 1, 1, "i8"), (3, 64, 17, 9, 408, 3, 1, "f16")]
+
+
+@pytest.mark.parametrize("case", PAIR_CASES + SINGLE_CASES)
 def test_conv_pairs(ctx, case):
     capi = _capi()
     N, Cin, H, W, Cout, k, s, dtype = case
@@ -541,3 +548,35 @@ def test_layers_without_a_pair_kernel_keep_wide_tiles(ctx, case):
     ctx.sync_check()
     conv = [k for k in launches if "conv_tc_kernel" in k[0]]
     assert len(conv) == 1 and conv[0][2][0] == 576, launches
+
+
+def _route(ctx, case, i8, out, impl):
+    """The convolution kernels that a case launches, by their demangled names."""
+    import torch
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s = case
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8 if i8 else capi.EXB_F16, out, impl=impl)
+    w = np.zeros((Cout, Cin, k, k), np.int8 if i8 else np.float32)
+    p = capi.ConvWeights(ctx, d, w, None, np.ones(Cout, np.float32), 1.0) if i8 else capi.ConvWeights(ctx, d, w)
+    x = torch.zeros((N, H, W, Cin), device="cuda", dtype=torch.int8 if i8 else torch.float16)
+    names = [n for n, _, _ in kernels_of(lambda: capi.conv2d(ctx, d, x, p))]
+    ctx.sync_check()
+    return [n for n in names if "conv_" in n]
+
+
+# The shapes above run in the kernels they are there for.
+@pytest.mark.parametrize("case", SPLIT_CASES)
+def test_split_cases_take_the_split_kernel(ctx, case):
+    capi = _capi()
+    for i8 in (True, False):
+        names = _route(ctx, case, i8, capi.EXB_I8 if i8 else capi.EXB_F32, 0)
+        assert len(names) == 1 and "conv_split_kernel" in names[0], names
+
+
+@pytest.mark.parametrize("case", PAIR_CASES + SINGLE_CASES)
+def test_pair_cases_take_the_pair_kernel(ctx, case):
+    capi = _capi()
+    i8 = case[7] == "i8"
+    names = _route(ctx, case[:7], i8, capi.EXB_I8 if i8 else capi.EXB_F32, 2)
+    paired = re.search(r"conv_tc_kernel<(true|false), \w+, \w+, false, true>", names[0]) is not None
+    assert len(names) == 1 and paired == (case in PAIR_CASES), names

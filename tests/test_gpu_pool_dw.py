@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from oracle import exb_oracle as O
-from tests.util import dev, host, rng, f16_round, to_nhwc, to_nchw
+from tests.util import kernels_of, dev, host, rng, f16_round, to_nhwc, to_nchw
 
 pytestmark = pytest.mark.gpu
 
@@ -141,13 +141,16 @@ def test_dwconv_int8_in_out(ctx):
 # Edges of the streaming 3x3 kernel: maps smaller than a thread's four columns, one row, ragged column groups, channel
 # counts that do not fill (8, 24) or do not fit (264, 1240) one CTA, rows that end inside a stage, no padding; fp16 and
 # int8 results.
-@pytest.mark.parametrize("out_i8", [False, True])
-@pytest.mark.parametrize("case", [
+DW_STREAM_CASES = [
     # N, C, H, W, stride, pad, act
     (1, 8, 1, 1, 1, 1, 103), (2, 8, 3, 3, 1, 0, 0), (3, 24, 5, 2, 1, 1, 1), (1, 264, 9, 33, 1, 1, 103), (2, 1240, 7, 6, 1, 1, 104),
     (1, 8, 2, 2, 2, 1, 103), (1, 16, 3, 4, 2, 1, 1), (2, 264, 13, 12, 2, 1, 103), (1, 40, 31, 257, 2, 1, 0), (5, 96, 40, 11, 2, 0, 103),
     (37, 32, 30, 31, 1, 1, 1), (64, 144, 14, 14, 1, 1, 103),
-])
+]
+
+
+@pytest.mark.parametrize("out_i8", [False, True])
+@pytest.mark.parametrize("case", DW_STREAM_CASES)
 def test_dwconv_stream_edges(ctx, case, out_i8):
     capi = _capi()
     N, Cc, H, W, s, pad, act = case
@@ -172,12 +175,15 @@ def test_dwconv_stream_edges(ctx, case, out_i8):
 # Edges of the streaming pooling kernel: windows hanging over every border of maps smaller than a thread's four columns,
 # negative values next to padding (a maximum must not see the fill), channel counts around one CTA's, ceil mode, the
 # int8 second output; below 32 channels stride 2 takes the other kernel.
-@pytest.mark.parametrize("case", [
+POOL_STREAM_CASES = [
     # N, C, H, W, type, k, s, pad, pad_mode, cip
     (1, 8, 1, 1, 0, 5, 1, 2, 1, 0), (2, 264, 6, 3, 0, 5, 1, 2, 1, 0), (3, 40, 27, 33, 1, 5, 1, 2, 1, 1), (1, 520, 9, 5, 1, 3, 1, 1, 1, 0),
     (2, 24, 5, 7, 0, 3, 1, 1, 1, 0), (2, 32, 2, 2, 0, 3, 2, 1, 1, 0), (1, 72, 37, 41, 0, 3, 2, 1, 0, 0), (2, 64, 30, 9, 1, 3, 2, 1, 0, 1),
     (1, 32, 3, 5, 0, 2, 2, 0, 0, 0), (2, 136, 29, 31, 1, 2, 2, 0, 1, 0), (40, 64, 20, 20, 0, 5, 1, 2, 1, 0), (1, 16, 9, 9, 0, 3, 2, 1, 1, 0),
-])
+]
+
+
+@pytest.mark.parametrize("case", POOL_STREAM_CASES)
 def test_pool_stream_edges(ctx, case):
     capi = _capi()
     N, Cc, H, W, type_, k, s, pad, pad_mode, cip = case
@@ -295,3 +301,21 @@ def test_row_stream_tile_limit(ctx, op):
         assert (y[i].float() == v * k).all(), i
     del x, y
     torch.cuda.empty_cache()
+
+
+# The shapes of the edge tests run in the kernels they are there for (below 32 channels stride 2 takes the other one).
+def test_stream_cases_take_the_stream_kernels(ctx):
+    import torch
+    capi = _capi()
+    for N, Cc, H, W, s, pad, act in DW_STREAM_CASES:
+        d = capi.make_dw_desc(N, H, W, Cc, 3, s, pad, capi.EXB_F16, capi.EXB_F16, act)
+        w = capi.DwWeights(ctx, d, np.zeros((Cc, 1, 3, 3), np.float32), np.zeros(Cc, np.float32))
+        x = torch.zeros((N, H, W, Cc), device="cuda", dtype=torch.float16)
+        names = [n for n, _, _ in kernels_of(lambda: capi.dwconv2d(ctx, d, x, w))]
+        assert any("dw3x3_stream_kernel" in n for n in names), ((N, Cc, H, W, s), names)
+    for N, Cc, H, W, type_, k, s, pad, pad_mode, cip in POOL_STREAM_CASES:
+        d = capi.make_pool_desc(N, H, W, Cc, type_, k, s, pad, False, pad_mode, cip, capi.EXB_F16)
+        x = torch.zeros((N, H, W, Cc), device="cuda", dtype=torch.float16)
+        names = [n for n, _, _ in kernels_of(lambda: capi.pool2d(ctx, d, x))]
+        assert any("pool_stream_kernel" in n for n in names) == (s == 1 or Cc >= 32), ((N, Cc, H, W, k, s), names)
+    ctx.sync_check()
