@@ -102,8 +102,8 @@ def measure(seconds=2.0, device=0, shapes=((64, 1), (64, 2), (128, 1), (128, 2),
             res[name].append(probe(ctx, dt, n, ctas, 0.0, ClockSampler, device, m=64))
     ctx.close()
     out = {
-        "how": "tcgen05.mma cta_group::1 M=128 K=32B back to back from one thread per CTA, operands resident in shared "
-               "memory, no TMA / epilogue; burst = best ~0.3 ms launch, sustained = launches back to back for %.1f s" % seconds,
+        "how": "tcgen05.mma cta_group::1 M=128 K=32B back to back from one warp per CTA (uniform, one elected lane issues), "
+               "operands resident in shared memory, no TMA / epilogue; burst = best ~0.3 ms launch, sustained = launches back to back for %.1f s" % seconds,
         "int8_peak_tops": max([r["burst"] for r in res["int8"] if r["m"] == 128] or [0.0]),
         "f16_peak_tflops": max([r["burst"] for r in res["f16"] if r["m"] == 128] or [0.0]),
         "int8_peak_tops_sustained": max([r.get("sustained", 0.0) for r in res["int8"]] or [0.0]),

@@ -1,8 +1,8 @@
-// Depthwise convolution on NHWC tensors, fp32 math on fp16 or int8 activations.
-// A thread owns 8 consecutive channels of a strip of TW output pixels along W: every input
-// vector of the strip is loaded once per kernel row and reused by all taps that touch it, and
-// each weight vector is loaded once per strip.  Weights are kept tap-major [kh*kw][C] in fp32
-// so consecutive threads read consecutive channels.
+// Depthwise convolution on NHWC tensors, fp32 math on fp16 or int8 activations.  Weights are kept tap-major [kh*kw][C] in
+// fp32 so consecutive threads read consecutive channels.  Three kernels: 3x3 windows of fp16 maps run on the row stream
+// (dw3x3_stream_kernel); 3x3 windows of int8 maps with a thread per 8 channels of a strip of TW output pixels, in which every
+// input vector is loaded once per kernel row and reused by all taps that touch it (dw_strip_kernel); any other window with
+// a thread per output vector (dw_generic_kernel).
 #include <math.h>
 
 #include <type_traits>
@@ -136,8 +136,9 @@ __global__ void __launch_bounds__(128) dw_strip_kernel(const TIn* __restrict__ x
 
 // 3x3, stride 1 or 2, fp16 input, on the row stream of row_stream.cuh.  A thread keeps its 9 x 4 weights in registers for
 // the whole launch; an input row adds to the three output rows it belongs to (stride 2: one or two).  Products are packed
-// fma.rn.f32x2, each lane the same fma, in the same order, as a scalar loop's.  144 channels @56, batch 256: 81 us = 88 %
-// of the HBM copy rate (140 us with the window of rows in registers); 960 channels @7x6, batch 9: 3.7 us (22.6).
+// fma.rn.f32x2, each lane the same fma, in the same order, as a scalar loop's.  144 channels @56, batch 256: 85 to 92 us
+// from card to card, 77 to 83 % of the HBM copy rate (143 us with the window of rows in registers); 960 channels @7x6,
+// batch 9: 3.7 us (22.6).
 struct DwStreamParams : RowStreamParams {
     int act;
     float out_scale, clamp_hi;      // clamp_hi: upper bound of a ReLU / ReLU6 result (int8: of its multiple of out_scale)

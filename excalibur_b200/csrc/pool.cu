@@ -9,6 +9,7 @@
 #include <cooperative_groups.h>
 #include <float.h>
 
+#include <array>
 #include <type_traits>
 
 namespace exb {
@@ -383,7 +384,7 @@ template <int K, int S, bool kMax, bool kOut2>
 int launch_pool_stream(exb_ctx* ctx, const PoolParams& d, const __half* x, __half* y, int8_t* y2, cudaStream_t st) {
     static constexpr RowStreamKind kind = kPoolKind<K, S>;
     const RowStreamPlan pl = row_stream_plan(kind, ctx->sm_count, d.N, d.PH, d.PW, d.cs);
-    PoolStreamParams p;
+    PoolStreamParams p{};
     CUtensorMap map;
     size_t smem;
     const int grid = row_stream_setup(ctx, kind, pl, x, d.N, d.H, d.W, d.pt, d.pl,
@@ -391,9 +392,16 @@ int launch_pool_stream(exb_ctx* ctx, const PoolParams& d, const __half* x, __hal
     if (grid < 0) return grid;
     p.H = d.H; p.W = d.W; p.pt = d.pt; p.pb = d.pb; p.pl = d.pl; p.pr = d.pr;
     p.count_include_pad = d.count_include_pad; p.out2_scale = d.out2_scale;
-    p.count[0] = {NAN, NAN};
-    for (int i = 1; i <= kMaxKnownDivisor; ++i) p.count[i] = known_divisor(i);
-    p.count[kMaxKnownDivisor + 1] = {0.f, 0.f};
+    if (!kMax) {
+        static const std::array<KnownDivisor, kMaxKnownDivisor + 2> table = [] {
+            std::array<KnownDivisor, kMaxKnownDivisor + 2> t;
+            t.front() = {NAN, NAN};
+            for (int i = 1; i <= kMaxKnownDivisor; ++i) t[i] = known_divisor(i);
+            t.back() = {0.f, 0.f};
+            return t;
+        }();
+        memcpy(p.count, table.data(), sizeof(p.count));
+    }
     auto kern = pool_stream_kernel<K, S, kMax, kOut2>;
     if (int rc = raise_smem_limit(ctx, kern)) return rc;
     return launch_pdl(ctx, "pool_stream_kernel", kern, dim3((unsigned)grid), dim3((unsigned)pl.threads), smem, st, map, y, y2, p);
