@@ -1144,11 +1144,14 @@ static bool conv_pairable(const exb_ctx* ctx, const ConvGeom& g) {
 }
 
 // The N tile: 256 channels, or 128 where that is the faster one.
-//  - Below 512 bytes of K, and up to 1152 in the first two rounds of tiles, the epilogue sets the pace, and two CTAs of
-//    128 channels per SM drain more than one of 256: 96 -> 576 int8 1x1 at 256 x 14 x 14 23.8 -> 21.4 us, 320 -> 1280 at
-//    256 x 7 x 7 18.4 -> 16.1, 128 -> 256 int8 3x3 stride 2 at 50 x 28 x 28 11.2 -> 9.3 (but 19.8 -> 21.4 at 256 images).
-//    Not for fewer than 256 channels and a shorter K, which two smaller tiles only read twice (32 -> 192 at
-//    256 x 28 x 28: 23.6 us in one tile, 28.4 in two).
+//  - Below 512 bytes of K, and up to 1152 in the first round of tiles (two of them for two N tiles), the epilogue sets the
+//    pace, and two CTAs of 128 channels per SM drain more than one of 256: 96 -> 576 int8 1x1 at 256 x 14 x 14 23.8 ->
+//    21.4 us, 320 -> 1280 at 256 x 7 x 7 18.4 -> 16.1, 128 -> 256 int8 3x3 stride 2 at 50 x 28 x 28 11.2 -> 9.3 (but 19.8 ->
+//    21.4 at 256 images; 48 -> 1280 fp16 3x3 at 80 x 80, 500 tiles, 20.7 -> 23.4; 128 -> 1280 int8 3x3 at 32 x 14 x 14, 490
+//    tiles, 15.9 -> 17.4).  Of 98 such int8 layers none is slower; on average they are 15 % faster.
+//    Not for fp16 layers below 256 bytes, whose shorter reads of the activations each tile repeats (112 -> 320 at
+//    256 x 28 x 28 54 us in tiles of 256, 67 in tiles of 128; 37 layers 2 % slower on average), and not for fewer than 256
+//    channels, which two smaller tiles only read twice (32 -> 192 at 256 x 28 x 28: 23.6 us in one tile, 28.4 in two).
 //  - Beyond that tiles run as pairs, sm_count / 2 at a time, and a pair of 128-channel tiles takes about 0.63 of the time
 //    of one of 256 (half the MMA time, but the same activations): 128 where its rounds of pairs come to less.
 //    512 -> 512 3x3 fp16 at 64 x 7 x 7: 26 pairs of 256 on 74 places 30.9 us, 52 of 128 24.0; 256 -> 256 int8 at
@@ -1163,11 +1166,15 @@ ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64
     if (cout_pad <= 128 || (cout_pad < 256 && k_bytes < 512) || conv_fold_plan(g).on) return wide;
     // The mapped epilogue takes whole 32-channel blocks, which 1152, 1408, 1664 and 1920 channels in tiles of 240 are not.
     if ((g.res_half || g.rh * g.rw > 1) && wide.BN % 32) return narrow;
-    if (k_bytes < 512 || (k_bytes <= 1152 && m_tiles * narrow.n_tiles <= 4 * ctx->sm_count)) return narrow;
+    if (k_bytes < 512) return g.in_dtype == EXB_I8 || k_bytes >= 256 ? narrow : wide;
+    if (k_bytes <= 1152 && m_tiles * narrow.n_tiles <= (narrow.n_tiles > 2 ? 2 : 4) * ctx->sm_count) return narrow;
     if (!conv_pairable(ctx, g)) return wide;
     const int64_t places = ctx->sm_count / 2;
     auto rounds = [&](const ConvNTile& t) { return (double)(((m_tiles + 1) / 2 * t.n_tiles + places - 1) / places); };
-    if (narrow.BN % 64 != 0 || 0.63 * rounds(narrow) >= rounds(wide)) return wide;      // (a pair splits whole 32-channel blocks)
+    // (a pair splits whole 32-channel blocks; 160 -> 256 int8 3x3 stride 2 at 32 x 56 x 56 in K blocks of 32 bytes: two rounds of
+    // 256 21.8 us, three of 128 29.1)
+    const bool k32 = g.cin_stride * (g.in_dtype == EXB_I8 ? 1 : 2) % 64 != 0;
+    if (narrow.BN % 64 != 0 || k32 || 0.63 * rounds(narrow) >= rounds(wide)) return wide;
     ConvNTile t = narrow;
     t.paired = true;
     return t;

@@ -580,3 +580,27 @@ def test_pair_cases_take_the_pair_kernel(ctx, case):
     names = _route(ctx, case[:7], i8, capi.EXB_I8 if i8 else capi.EXB_F32, 2)
     paired = re.search(r"conv_tc_kernel<(true|false), \w+, \w+, false, true>", names[0]) is not None
     assert len(names) == 1 and paired == (case in PAIR_CASES), names
+
+
+# N tiles of short reductions: 128 channels where the epilogue sets the pace (CTAs of 320 threads, two per SM), 256 where the
+# activations that every tile reads again do (CTAs of 576): fp16 below 256 bytes of K, more than two tiles per SM.
+@pytest.mark.parametrize("case,wide", [((64, 112, 28, 28, 320, 1, 1, "f16"), True), ((16, 48, 28, 28, 408, 3, 1, "f16"), True),
+                                       ((32, 128, 14, 14, 1280, 3, 1, "i8"), True), ((100, 384, 10, 10, 256, 1, 1, "i8"), False),
+                                       ((25, 96, 56, 56, 192, 3, 2, "i8"), False), ((32, 160, 28, 28, 320, 1, 1, "f16"), False)])
+def test_n_tile_of_short_reductions(ctx, case, wide):
+    import torch
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s, dtype = case
+    i8 = dtype == "i8"
+    r = rng(sum(case[:7]))
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8 if i8 else capi.EXB_F16, capi.EXB_F32, impl=2)
+    wq = r.integers(-8, 9, (Cout, Cin, k, k)).astype(np.int8)
+    p = capi.ConvWeights(ctx, d, wq, None, np.ones(Cout, np.float32), 1.0) if i8 else capi.ConvWeights(ctx, d, wq.astype(np.float32))
+    x = r.integers(-8, 9, (N, H, W, Cin)).astype(np.int8)
+    xd = dev(x if i8 else x.astype(np.float16))
+    launches = [l for l in kernels_of(lambda: capi.conv2d(ctx, d, xd, p)) if "conv_tc_kernel" in l[0]]
+    assert len(launches) == 1 and launches[0][2][0] == (576 if wide else 320), launches
+    y, _ = capi.conv2d(ctx, d, xd, p)
+    ctx.sync_check()
+    for n in (0, N - 1):
+        np.testing.assert_array_equal(host(y[n]).transpose(2, 0, 1), O.conv2d_i8_acc(x[n:n + 1].transpose(0, 3, 1, 2), wq, s, k // 2)[0].astype(np.float32))
