@@ -1276,9 +1276,10 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
         const bool res_two = p.n_tiles == 1 && two && b_tile <= 48 * 1024;
         const bool res_one = p.n_tiles == 1 && b_tile <= 150 * 1024;
         // One CTA per SM (to keep the weights resident) for N tiles of 128 and more, and for 64 where tiles can be
-        // paired and there are enough of them: one CTA's own N = 64 instructions do not fill the tensor pipe.
+        // paired and there are enough of them: one CTA's own N = 64 instructions do not fill the tensor pipe.  In whole K blocks
+        // only: 96 -> 64 fp16 at 100 x 44 x 44 takes 50.5 us that way (blocks of 64 bytes), 35.4 in the tap loop.
         const bool one_cta = res_one && !res_two && two &&
-                             (p.BN >= 128 || (p.BN == 64 && tiles_rb > 2 * ctx->sm_count && g.act != EXB_ACT_PRELU));
+                             (p.BN >= 128 || (p.BN == 64 && p.kb_bytes == 128 && tiles_rb > 2 * ctx->sm_count && g.act != EXB_ACT_PRELU));
         const bool res_rb = (two && !one_cta) ? res_two : res_one;
         const double cost_tap = (double)tiles_tap * (a_tap + (res_two ? 0 : b_tile));
         const double cost_rb = (double)tiles_rb * (a_rb + (res_rb ? 0 : b_tile));

@@ -604,3 +604,22 @@ def test_n_tile_of_short_reductions(ctx, case, wide):
     ctx.sync_check()
     for n in (0, N - 1):
         np.testing.assert_array_equal(host(y[n]).transpose(2, 0, 1), O.conv2d_i8_acc(x[n:n + 1].transpose(0, 3, 1, 2), wq, s, k // 2)[0].astype(np.float32))
+
+
+# 64-channel tiles keep their weights resident on one CTA per SM (576 threads, pairs) for K blocks of 128 bytes only: 96 fp16
+# channels took 50.5 us that way at 100 x 44 x 44, 35.4 with two CTAs of 320 threads per SM.
+@pytest.mark.parametrize("cin,threads", [(96, 320), (64, 576), (128, 576)])
+def test_resident_weights_of_64_channel_tiles(ctx, cin, threads):
+    import torch
+    capi = _capi()
+    d = capi.make_conv_desc(50, 44, 44, cin, 64, 3, 1, 1, capi.EXB_F16, capi.EXB_F32, impl=2)
+    r = rng(cin)
+    wq = r.integers(-8, 9, (64, cin, 3, 3)).astype(np.int8)
+    x = r.integers(-8, 9, (50, 44, 44, cin)).astype(np.int8)
+    p, xd = capi.ConvWeights(ctx, d, wq.astype(np.float32)), dev(x.astype(np.float16))
+    launches = [l for l in kernels_of(lambda: capi.conv2d(ctx, d, xd, p)) if "conv_tc_kernel" in l[0]]
+    assert len(launches) == 1 and launches[0][2][0] == threads, launches
+    y, _ = capi.conv2d(ctx, d, xd, p)
+    ctx.sync_check()
+    for n in (0, 49):
+        np.testing.assert_array_equal(host(y[n]).transpose(2, 0, 1), O.conv2d_i8_acc(x[n:n + 1].transpose(0, 3, 1, 2), wq, 1, 1)[0].astype(np.float32))
