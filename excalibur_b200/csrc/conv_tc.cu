@@ -1334,7 +1334,9 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     //    tile, and a pair's MMA reads half as many weight bytes per SM as two CTAs' own instructions;
     //  - tap-loop tiles of more than 128 channels (an SM to themselves anyway) with at least 512 bytes of K: the
     //    epilogue bounds shorter ones, and units of two tiles only coarsen its work (32 -> 192 channels 1x1, 48 images
-    //    of 28 x 28: 9.3 us in pairs, 8.3 single; 960 -> 160 int8, 256 images of 7 x 7: 11.4 in pairs, 13.5 single);
+    //    of 28 x 28: 9.3 us in pairs, 8.3 single; 960 -> 160 int8, 256 images of 7 x 7: 11.4 in pairs, 13.5 single), unless an
+    //    odd number of tiles to pair up takes a round more than single ones do (512 -> 1280 fp16 3x3 at 2 x 40 x 40: 125
+    //    tiles are one round, their 75 pairs two: 52.3 us, 37.6 single);
     //  - tap-loop tiles of 64 to 128 channels with at least 1152 bytes of K (64 fp16 channels 3x3), where streaming the
     //    weights sets the pace, and more than two tiles per SM, so that the coarser units do not leave the last wave
     //    half empty: 256 -> 64 at 4 x 120 x 184 48.4 -> 42.7 us, but 18.2 -> 19.4 at 4 x 60 x 92 (173 tiles);
@@ -1344,12 +1346,14 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     // The channel-permuting map of the quad epilogue moves 32-channel blocks, so a half must be made of whole ones.
     const int64_t k_bytes = (int64_t)g.kh * g.kw * row_bytes;      // one pixel's reduction
     const int64_t all_tiles = (int64_t)p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;
+    const int64_t pair_units = (p.tiles_nb >= 2 ? (int64_t)p.tiles_h * ((p.tiles_nb + 1) / 2) : (p.tiles_h + 1) / 2) * p.tiles_w * p.n_tiles;
+    const int64_t places = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1, pair_rounds = (pair_units + places - 1) / places;
     const bool pairable = conv_pairable(ctx, g) && !patch && p.BN % (quad ? 64 : 32) == 0 && (p.tiles_nb >= 2 || p.tiles_h >= 2);
     bool pair = false;
     if (p.rowbox)
         pair = pairable && rb.one_cta && (p.BN == 64 || p.BN == 128);
     else if (p.BN > 128)
-        pair = pairable && k_bytes >= 512;
+        pair = pairable && k_bytes >= 512 && pair_rounds <= (all_tiles + ctx->sm_count - 1) / ctx->sm_count;
     else if (p.BN >= 64)
         pair = pairable && k_bytes >= 1152 && (nt.paired || all_tiles > 2 * ctx->sm_count);
     if (pair) {

@@ -623,3 +623,12 @@ def test_resident_weights_of_64_channel_tiles(ctx, cin, threads):
     ctx.sync_check()
     for n in (0, 49):
         np.testing.assert_array_equal(host(y[n]).transpose(2, 0, 1), O.conv2d_i8_acc(x[n:n + 1].transpose(0, 3, 1, 2), wq, 1, 1)[0].astype(np.float32))
+
+
+# Tiles of more than 128 channels do not run as pairs where that takes a round more: 125 tiles on 148 SMs, 75 pairs on 74.
+@pytest.mark.parametrize("case,paired", [((2, 128, 40, 40, 1280, "f16"), False), ((2, 256, 40, 40, 1280, "i8"), False), ((2, 128, 40, 40, 1024, "f16"), True)])
+def test_pairs_take_no_extra_round(ctx, case, paired):
+    capi = _capi()
+    N, Cin, H, W, Cout, dtype = case
+    names = _route(ctx, (N, Cin, H, W, Cout, 3, 1), dtype == "i8", capi.EXB_I8 if dtype == "i8" else capi.EXB_F16, 2)
+    assert len(names) == 1 and (re.search(r"conv_tc_kernel<(true|false), \w+, \w+, false, true>", names[0]) is not None) == paired, names
