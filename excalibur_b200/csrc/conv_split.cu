@@ -315,8 +315,12 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
 // Which kernel, and how a tile is divided: modelled time in us of both kernels, fitted to 330 layers (batch 1 to 64,
 // 1x1 and 3x3, 32 to 1280 channels, maps of 7 x 7 to 80 x 80; every split of 32 and 64 channels).
 // Split kernel: a constant, the cluster's exchange, then K blocks and epilogue of a tile one after the other, stretched by
-// the tiles per SM once there are more than SMs.  Persistent kernel: a constant and rounds of tiles.  On these layers the
-// pick is on average 1 to 2 % slower than the fastest of all; the line lies near two tiles of 64 channels per SM.
+// the tiles per SM once there are more than SMs.  Persistent kernel: a constant and rounds of tiles.  The constants are
+// regression weights, not times of parts: those of 32- and 64-byte K blocks make up for terms the form does not have.  On 330
+// other layers (batch 1 to 256, 7 x 7 to 80 x 80, 16 to 960 -> 64 to 1280 channels) the pick is 2 % slower than the fastest
+// of both kernels on average, and 5 % or more slower in one of nine, at worst 33 to 39 % where the persistent kernel's N
+// tile does not suit either (256 -> 1000 int8 1x1 at 32 x 10 x 10: 10.3 us, divided 7.4).  The line lies near two tiles of 64
+// channels per SM.
 ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
     const ConvSplit none = {0, 0};
     if (g.pool || g.out_dtype == EXB_I32 || (g.cout_stride & 7) || (g.y_pitch & 7) || conv_fold_plan(g).on) return none;
@@ -359,7 +363,10 @@ ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
     }
     if (bn > 128 && k_iters * kb < 512) rest = 1.6;      // single CTAs of short reductions
     step *= kb == 128 ? 1.0 : kb == 64 ? 0.21 : 0.39;
-    const double persistent = 4.58 + rounds * (k_iters * step + rest + (g.has_res ? 0.45 : 0.0)) * share;
+    double body = rounds * (k_iters * step + rest + (g.has_res ? 0.45 : 0.0)) * share;
+    // int8 tiles of a short K, more of them than fit the SMs as clusters: 96 -> 320 1x1 at 8 x 40 x 40 8.1 us, divided 11.4
+    if (two && g.in_dtype == EXB_I8 && k_iters * kb <= 256 && m_tiles * ((w->cout_pad + 63) / 64) > ctx->sm_count) body *= 0.75;
+    const double persistent = 4.58 + body;
     return best_t < 0.98 * persistent ? best : none;
 }
 

@@ -632,3 +632,12 @@ def test_pairs_take_no_extra_round(ctx, case, paired):
     N, Cin, H, W, Cout, dtype = case
     names = _route(ctx, (N, Cin, H, W, Cout, 3, 1), dtype == "i8", capi.EXB_I8 if dtype == "i8" else capi.EXB_F16, 2)
     assert len(names) == 1 and (re.search(r"conv_tc_kernel<(true|false), \w+, \w+, false, true>", names[0]) is not None) == paired, names
+
+
+# The choice between the kernels: divided tiles where they do not fill the SMs, the persistent kernel for short int8 reductions
+# of more tiles (96 -> 320 1x1 at 8 x 40 x 40 took 11.4 us divided, 8.1 not).
+@pytest.mark.parametrize("case,split", [((8, 96, 40, 40, 320, 1, 1), False), ((8, 128, 56, 56, 96, 1, 1), False), ((8, 256, 7, 7, 960, 1, 1), True)])
+def test_short_int8_reductions_are_divided_only_when_few(ctx, case, split):
+    capi = _capi()
+    names = _route(ctx, case, True, capi.EXB_I8, 0)
+    assert len(names) == 1 and ("conv_split_kernel" in names[0]) == split, names
