@@ -88,17 +88,43 @@ def sample(a, limit=8192):
     return flat[::step].copy()
 
 
+def _demangle(name):
+    import ctypes
+    f = ctypes.CDLL("libstdc++.so.6").__cxa_demangle
+    f.restype = ctypes.c_void_p
+    f.argtypes = [ctypes.c_char_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    p = f(name, None, None, None)
+    if not p:
+        return name.decode()
+    out = ctypes.string_at(p).decode()
+    free = ctypes.CDLL(None).free
+    free.argtypes = [ctypes.c_void_p]
+    free(p)
+    return out
+
+
 def kernels_of(fn):
-    """The kernels that fn() launches, as (name, grid, block), from the CUDA activity trace."""
-    import json
-    import tempfile
+    """The kernels that fn() launches, as (name, grid, block), from the nodes of a stream capture (an activity trace of one
+    launch comes back empty late in a long process)."""
     import torch
+    from cuda.bindings import driver as cu
+
+    def ok(r):
+        assert int(r[0]) == 0, r[0]
+        return r[1:] if len(r) > 2 else r[1]
     fn()
     torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        fn()
-        torch.cuda.synchronize()
-    with tempfile.NamedTemporaryFile(suffix=".json") as f:
-        prof.export_chrome_trace(f.name)
-        events = json.load(open(f.name))["traceEvents"]
-    return [(e["name"], tuple(e["args"]["grid"]), tuple(e["args"]["block"])) for e in events if e.get("cat") == "kernel"]
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        keep = fn()
+    graph = cu.CUgraph(g.raw_cuda_graph())
+    n = ok(cu.cuGraphGetNodes(graph))[1]
+    out = []
+    for node in ok(cu.cuGraphGetNodes(graph, n))[0][:n]:
+        if ok(cu.cuGraphNodeGetType(node)) != cu.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        k = ok(cu.cuGraphKernelNodeGetParams(node))
+        name = ok(cu.cuFuncGetName(k.func)) if int(k.func) else ok(cu.cuKernelGetName(k.kern))
+        out.append((_demangle(name), (k.gridDimX, k.gridDimY, k.gridDimZ), (k.blockDimX, k.blockDimY, k.blockDimZ)))
+    del keep
+    return out
