@@ -164,10 +164,36 @@ __device__ __forceinline__ int quant_rne(float v) {
     return (int)t;
 }
 
-// Four floats -> four int8 (round half to even, saturate), packed little-endian in 32 bits.
-__device__ __forceinline__ uint32_t quant_pack4(float a, float b, float c, float d, float qscale) {
-    const int q0 = __float2int_rn(a * qscale), q1 = __float2int_rn(b * qscale);
-    const int q2 = __float2int_rn(c * qscale), q3 = __float2int_rn(d * qscale);
+// Two floats in a 64-bit register pair: one instruction for two IEEE operations.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, const f32x2& c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 cvt2(uint32_t h) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    return pack2(f.x, f.y);
+}
+
+// Four integers -> four int8 (saturated), packed little-endian in 32 bits.
+__device__ __forceinline__ uint32_t sat_pack4(int q0, int q1, int q2, int q3) {
     uint32_t r;
     // cvt.pack.sat.s8.s32.b32 d, a, b, c:  d = (c << 16) | (sat8(a) << 8) | sat8(b)
     asm("{\n\t.reg .b32 t;\n\t"
@@ -176,6 +202,10 @@ __device__ __forceinline__ uint32_t quant_pack4(float a, float b, float c, float
         : "=r"(r)
         : "r"(q0), "r"(q1), "r"(q2), "r"(q3));
     return r;
+}
+// Four floats -> four int8 (round half to even, saturate).
+__device__ __forceinline__ uint32_t quant_pack4(float a, float b, float c, float d, float qscale) {
+    return sat_pack4(__float2int_rn(a * qscale), __float2int_rn(b * qscale), __float2int_rn(c * qscale), __float2int_rn(d * qscale));
 }
 
 // 1 / (1 + e^-v) for the sigmoid-type activations: hardware reciprocal plus one Newton step (within 1 ulp of the

@@ -33,28 +33,6 @@ struct RowStreamParams {
     int* error;
 };
 
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, const f32x2& c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 cvt2(uint32_t h) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-    return pack2(f.x, f.y);
-}
-
 // Start of a kernel on the stream: barriers initialised (a __syncthreads and pdl_wait() must follow), ring address.
 template <int NS>
 __device__ __forceinline__ uint8_t* row_stream_init(const CUtensorMap& map, uint8_t* smem_raw, uint64_t* full, int* abort_flag) {

@@ -641,3 +641,56 @@ def test_short_int8_reductions_are_divided_only_when_few(ctx, case, split):
     capi = _capi()
     names = _route(ctx, case, True, capi.EXB_I8, 0)
     assert len(names) == 1 and ("conv_split_kernel" in names[0]) == split, names
+
+
+# The lean quad epilogue (fp16 result, alone or with an int8 copy) against the same kernel's fp32 result, which is read from the
+# general form: whole-number operands, so the sums are exact whatever their order, and scale, bias, residual, activation and
+# rounding are repeated here in the same fp32 steps.  N tiles of one, two, three and five blocks, a tile that ends inside its
+# last block, one CTA per SM and two, pairs, three and eight accumulators in flight; infinities and NaN.
+LEAN_CASES = [(5, 32, 17, 13, 32, 1, 1), (3, 64, 9, 7, 72, 1, 1), (2, 32, 11, 13, 160, 1, 1), (40, 64, 28, 28, 96, 1, 1), (3, 96, 8, 8, 64, 3, 2),
+              (50, 64, 24, 24, 64, 3, 1), (9, 32, 30, 30, 320, 1, 1)]
+
+
+@pytest.mark.parametrize("i8", [True, False])
+@pytest.mark.parametrize("case", LEAN_CASES)
+def test_lean_quad_epilogue(ctx, case, i8):
+    import torch
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s = case
+    r = rng(sum(case) + i8)
+    wq = r.integers(-3, 4, (Cout, Cin, k, k)).astype(np.int8)
+    bias = r.integers(-40, 40, Cout).astype(np.float32) / 8
+    ws = np.exp2(r.integers(2, 6, Cout)).astype(np.float32)
+
+    def desc(out, out2, act, res):
+        return capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8 if i8 else capi.EXB_F16, out, out2, res=res, act=act,
+                                   out_scale=0.7, out2_scale=0.7, impl=2)
+    d0 = desc(capi.EXB_F32, -1, 0, False)
+    p = capi.ConvWeights(ctx, d0, wq, bias, ws, 0.25) if i8 else capi.ConvWeights(ctx, d0, wq.astype(np.float32), bias)
+    x = r.integers(-4, 5, (N, H, W, Cin)).astype(np.int8 if i8 else np.float16)
+    if not i8:
+        x[0, 0, 0, 0], x[-1, -1, -1, 1] = np.inf, np.nan
+    xd = dev(x)
+    v = capi.conv2d(ctx, d0, xd, p)[0]
+    oh, ow = capi.conv_out_dims(d0)
+    skip = dev(r.standard_normal((N, oh, ow, Cout)).astype(np.float16))
+    for act in (0, 1, 103, 104):
+        for res in (False, True):
+            for out2 in (-1, capi.EXB_I8):
+                y, y2 = capi.conv2d(ctx, desc(capi.EXB_F16, out2, act, res), xd, p, residual=skip if res else None)
+                u = v + skip.float() if res else v
+                if act == 104:
+                    want = u * torch.sigmoid(u)
+                    ok = torch.isfinite(want)
+                    # the sigmoid is within 2 ulp of fp32: at most one fp16 rounding apart
+                    assert ((y.float() - want.half().float()).abs()[ok] <= (want.abs() * 2.0 ** -10 + 2.0 ** -24)[ok]).all(), (act, res, out2)
+                else:
+                    # fmaxf / fminf: a NaN gives the bound
+                    want = u if act == 0 else torch.where(u > 0, u, torch.zeros_like(u))
+                    if act == 103:
+                        want = torch.where(want < 6, want, torch.full_like(u, 6.0))
+                    assert torch.equal(torch.nan_to_num(y, nan=12345.0), torch.nan_to_num(want.half(), nan=12345.0)), (act, res, out2)
+                    if y2 is not None:
+                        ok = ~torch.isnan(want)
+                        assert torch.equal(y2[ok], (want * 0.7).round().clamp(-128, 127).to(torch.int8)[ok]), (act, res, out2)
+    ctx.sync_check()
