@@ -64,14 +64,17 @@ template <typename K>
 inline int raise_smem_limit(const exb_ctx* ctx, K kern) {
     static std::mutex attr_mutex;
     static std::set<std::pair<const void*, int>> raised;
-    std::lock_guard<std::mutex> lock(attr_mutex);
+    static thread_local std::pair<const void*, int> last;      // what this thread launched before, without the lock
     const auto key = std::make_pair(reinterpret_cast<const void*>(kern), ctx->device);
+    if (last == key) return EXB_OK;
+    std::lock_guard<std::mutex> lock(attr_mutex);
     if (!raised.count(key)) {
         cudaFuncAttributes fa;
         EXB_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));      // static + dynamic shared memory share the device limit
         EXB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_optin - (int)fa.sharedSizeBytes));
         raised.insert(key);
     }
+    last = key;
     return EXB_OK;
 }
 

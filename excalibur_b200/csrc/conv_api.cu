@@ -160,7 +160,7 @@ extern "C" int exb_conv_weights_pack_f16(exb_ctx* ctx, const exb_conv_desc* d, c
     const int cout_pad = (g.cout_stride + 15) / 16 * 16;  // covers the padding channels of y too
     const FoldPlan fold = conv_fold_plan(g);
     const int kw_pack = fold.on ? fold.F : g.kw, s_shift = fold.on ? fold.shift : 0;
-    std::vector<uint16_t> packed((size_t)cout_pad * g.kh * kw_pack * cin_pad, 0);
+    std::vector<uint16_t> packed((size_t)weight_rows(cout_pad) * g.kh * kw_pack * cin_pad, 0);
     std::vector<uint16_t> half((size_t)g.Cout * cin_g * g.kh * g.kw);
     glasssix::excalibur::convert_f32_to_f16(w_oihw, half.data(), half.size());      // round to nearest even
     repack(half.data(), packed, g, cin_g, cin_pad, kw_pack, s_shift);
@@ -186,7 +186,7 @@ extern "C" int exb_conv_weights_pack_i8(exb_ctx* ctx, const exb_conv_desc* d, co
     const int cout_pad = (g.cout_stride + 15) / 16 * 16;  // covers the padding channels of y too
     const FoldPlan fold = conv_fold_plan(g);
     const int kw_pack = fold.on ? fold.F : g.kw, s_shift = fold.on ? fold.shift : 0;
-    std::vector<int8_t> packed((size_t)cout_pad * g.kh * kw_pack * cin_pad, 0);
+    std::vector<int8_t> packed((size_t)weight_rows(cout_pad) * g.kh * kw_pack * cin_pad, 0);
     repack(w_oihw, packed, g, cin_g, cin_pad, kw_pack, s_shift);
     std::vector<float> scale(cout_pad, 0.f), b(cout_pad, 0.f);
     for (int o = 0; o < g.Cout; ++o) {

@@ -11,7 +11,7 @@ struct exb_conv_weights {
     int cin_pad;      // channels per tap in the packed matrix (== x's physical channel count / group)
     int kw_pack;      // taps per kernel row in the packed matrix: kw, or the fold width F (>= kw)
     int s_shift;      // column of tap s = 0 inside a packed kernel row (0 unless folded)
-    void* d_w;        // [cout_pad][kh][kw_pack][cin_pad], K-major rows
+    void* d_w;        // [weight_rows(cout_pad)][kh][kw_pack][cin_pad], K-major rows
     float* d_scale;   // [cout_pad] epilogue multiplier (fp16: 1; int8: 1/(wscale*act_scale))
     float* d_bias;    // [cout_pad] zeros when the layer has no bias
     float* d_slope;   // [cout_pad + kSlopeSlack] PReLU slopes (zero beyond Cout), or null
@@ -21,6 +21,9 @@ struct exb_conv_weights {
 };
 
 namespace exb {
+
+// Rows of the packed matrix in memory: whole blocks of 32, which the quad epilogue's tensor map walks (zero beyond cout_pad).
+inline int weight_rows(int cout_pad) { return (cout_pad + 31) / 32 * 32; }
 
 // The epilogue reads 16 slopes at any channel offset below the output's channel stride.
 constexpr int kSlopeSlack = 1024;
@@ -202,9 +205,10 @@ int conv_direct_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb
                        const void* residual, void* y, void* y2, cudaStream_t st);
 int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_conv_weights* w,
                    const void* residual, void* y, void* y2, cudaStream_t st);
-// The split kernel (conv_split.cu): N tile and CTAs per tile of a launch, splits = 0 where the persistent kernel is used.
+// The split kernel (conv_split.cu): N tile, CTAs per tile and pixel box of a launch, splits = 0 where the persistent kernel is used.
 struct ConvSplit {
     int BN, splits;
+    int TW, TH, TN;
 };
 ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w);
 // N tiles of the persistent kernel: how many, of how many channels, and whether they were chosen to run as CTA pairs.

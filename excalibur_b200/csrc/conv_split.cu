@@ -4,11 +4,21 @@
 // The persistent kernel of conv_tc.cu gives a tile to one CTA (or pair): with one image a 3x3 layer of 512 channels @7x7
 // is two tiles, and one warp issues the whole reduction - 144 dependent MMAs and the loads that feed them, 19 us
 // (int8), on two of 148 SMs.  Here N tiles are at most 64 channels and the K blocks of a tile are divided over a cluster
-// of 1, 2, 4 or 8 CTAs.  Each accumulates its part in TMEM and spills it to its shared memory; after a cluster barrier
-// every CTA sums one slice of the tile's pixels over all parts through distributed shared memory and runs the epilogue
-// for that slice.  Weights never change on the stream, so their first loads are issued before the programmatic wait for
-// the previous kernel; what remains after that wait is one activation load, the MMAs of a few K blocks, the exchange and
-// the store.  int8 sums are exact whatever the split; fp16 ones are fp32 sums of at most eight partial sums.
+// of 1, 2, 4 or 8 CTAs.  Each accumulates its part in TMEM, moves it to its shared memory and sends every other CTA of the
+// cluster that one's slice of the tile's pixels in one bulk copy, which counts its bytes on the receiver's mbarrier; each CTA
+// sums the parts of its own slice out of its own shared memory and runs the epilogue for it.  Weights never change on the stream, so their first loads
+// are issued before the programmatic wait for the previous kernel; what remains after that wait is one activation load, the
+// MMAs of a few K blocks, the exchange and the store.  int8 sums are exact whatever the split; fp16 ones are fp32 sums of at
+// most eight partial sums.  An undivided tile goes from TMEM to the result directly, in the column order of the quad epilogue.
+//
+// Such launches are chains of latencies.  Time stamps of the roles showed 2.2 to 3 us behind the last MMA: 0.6 until the parts
+// lay in shared memory behind a cluster barrier, 1.2 to sum them out of the other CTAs' shared memory item after item and to
+// store, 0.3-0.7 for the barrier that kept every CTA until its neighbours had read; undivided tiles took the same way through
+// shared memory.  Per layer of a captured chain, before and after: undivided 64 -> 384 fp16 1x1 at 9 x 13 x 12 3.46 -> 2.26 us,
+// 256 -> 256 int8 3x3 at 32 x 14 x 14 9.6 -> 8.3; divided 512 -> 512 int8 3x3 at 7 x 7 5.6 -> 4.6, 256 -> 256 at 14 x 14 5.4 -> 4.6.
+// Copies between CTAs move some 14 bytes per cycle and SM, so only the box's rows are sent.  Tried: st.async of 16 bytes
+// per lane straight from registers (1 us to issue, 1 more to arrive: every packet is counted by itself).
+#include "conv_quad.cuh"
 #include "conv_tc_host.cuh"
 #include "ptx_sm100.cuh"
 
@@ -20,7 +30,8 @@ namespace {
 constexpr int kSplitStages = 16;     // at most
 constexpr int kSplitEpiThreads = 256;
 constexpr int kSplitThreads = 64 + kSplitEpiThreads;      // warp 0 loads, warp 1 issues MMAs, warps 2-9 drain and store
-constexpr int kSplitMaxItems = kTileM * 8 / kSplitEpiThreads;      // of 8 channels, with 64 channels per tile
+constexpr int kSplitMaxItems = kTileM * 8 / kSplitEpiThreads;      // of 8 channels of a pixel, with 64 channels per tile
+constexpr int kSplitMaxParts = 8;
 constexpr uint32_t kSplitMaxSpins = 1u << 21;
 
 struct ConvSplitParams {
@@ -34,18 +45,14 @@ struct ConvSplitParams {
     int cin_pad, cblks, kb_elems, kb_bytes;
     int k_iters;                        // (tap, channel block) pairs; CTA r of a cluster takes [r*k/splits, (r+1)*k/splits)
     int stages, a_bytes, b_bytes, a_tx_bytes;
+    int rows, slice;        // pixels of a tile's box, and of a CTA's share of it: CTA r finishes [r*slice, (r+1)*slice)
+    int recv;               // where the parts of this CTA's slice arrive, in bytes behind the ring's start
     int tmem_cols, cout_pad, has_res;
     int res_half;           // the residual is read through a nearest resize by 2
     uint32_t idesc;
     EpiParams e;
     int* error;
 };
-
-__device__ __forceinline__ uint4 ld_cluster_16(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
-}
 
 template <bool kInt8>
 __device__ __forceinline__ void acc_add(uint4& a, const uint4& b) {
@@ -59,18 +66,54 @@ __device__ __forceinline__ void acc_add(uint4& a, const uint4& b) {
     }
 }
 
+// Four channels of a pixel: v = act(acc * scale + bias + residual) -> first / second output.
 template <bool kInt8, bool kPrelu>
+__device__ __forceinline__ void split_store4(const EpiParams& e, const uint4& acc, const float4& sc, const float4& bi, bool has_res,
+                                             uint32_t r01, uint32_t r23, int64_t off, int cl) {
+    float f[4] = {epi_value<kInt8>(acc.x, sc.x, bi.x), epi_value<kInt8>(acc.y, sc.y, bi.y), epi_value<kInt8>(acc.z, sc.z, bi.z),
+                  epi_value<kInt8>(acc.w, sc.w, bi.w)};
+    if (has_res) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r01)), b = __half22float2(*reinterpret_cast<const __half2*>(&r23));
+        f[0] += a.x;
+        f[1] += a.y;
+        f[2] += b.x;
+        f[3] += b.y;
+    }
+    if constexpr (kPrelu) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[i] = f[i] >= 0.f ? f[i] : f[i] * __ldg(e.slope + cl + i);
+    } else {
+        apply_act_vec(f, e.act);
+    }
+    auto store = [&](void* y, int dtype, float q) {
+        if (dtype == EXB_I8) {
+            *reinterpret_cast<uint32_t*>(static_cast<int8_t*>(y) + off) = quant_pack4(f[0], f[1], f[2], f[3], q);
+        } else if (dtype == EXB_F16) {
+            const __half2 a = __floats2half2_rn(f[0], f[1]), b = __floats2half2_rn(f[2], f[3]);
+            *reinterpret_cast<uint2*>(static_cast<__half*>(y) + off) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        } else {
+            *reinterpret_cast<float4*>(static_cast<float*>(y) + off) = make_float4(f[0], f[1], f[2], f[3]);
+        }
+    };
+    store(e.y, e.out_dtype, e.out_scale);
+    if (e.out2_dtype >= 0) store(e.y2, e.out2_dtype, e.out2_scale);
+}
+
+// kDirect: an undivided tile in the quad epilogue's column order.  Otherwise the parts of the cluster's CTAs (two at least) go
+// through shared memory.
+template <bool kInt8, bool kPrelu, bool kDirect>
 __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_constant__ ConvSplitParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[kSplitStages];
     __shared__ __align__(8) uint64_t empty_bar[kSplitStages];
     __shared__ __align__(8) uint64_t done_bar;
+    __shared__ __align__(8) uint64_t recv_bar;
     __shared__ __align__(16) float s_scale[64];
     __shared__ __align__(16) float s_bias[64];
     __shared__ int s_pixel[kTileM], s_res_pixel[kTileM];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
-    // operand ring (1024-byte aligned: the widest swizzle atom); the partial tile takes its place when the MMAs are done
+    // operand ring (1024-byte aligned: the widest swizzle atom)
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int warp = ptx::uniform_warp(), lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x % p.splits;
@@ -91,6 +134,7 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
             ptx::mbar_init(&empty_bar[s], 1);
         }
         ptx::mbar_init(&done_bar, 1);
+        ptx::mbar_init(&recv_bar, 1);
         ptx::fence_mbar_init();
         ptx::tma_prefetch_desc(&p.tmB);
         ptx::tma_prefetch_desc(&p.tmA[0]);
@@ -101,8 +145,9 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
     }
     if (threadIdx.x >= 64 && threadIdx.x < 64 + p.BN) {
         const int c = (int)threadIdx.x - 64, ch = c0 + c;
-        s_scale[c] = ch < p.cout_pad ? p.e.scale[ch] : 0.f;
-        s_bias[c] = ch < p.cout_pad ? p.e.bias[ch] : 0.f;
+        const int at = kDirect ? quad_order(c) : c;
+        s_scale[at] = ch < p.cout_pad ? p.e.scale[ch] : 0.f;
+        s_bias[at] = ch < p.cout_pad ? p.e.bias[ch] : 0.f;
     }
     if (warp >= 2 && warp < 6) {       // accumulator row -> pixel of the output, or -1
         const int row = (int)threadIdx.x - 64;
@@ -113,15 +158,21 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
     }
     ptx::tc_fence_before_sync();
     __syncthreads();
+    // first round of the cluster's barrier: every CTA runs, its mbarriers are initialised (waited for before the first part is
+    // sent; bytes that arrive ahead of the expectation are counted all the same)
+    if (!kDirect) {
+        ptx::cluster_arrive();
+        if (threadIdx.x == 64) ptx::mbar_arrive_expect_tx(&recv_bar, (uint32_t)(max(min(p.slice, p.rows - rank * p.slice), 0) * (p.splits - 1) * (p.BN * 4 + 16)));
+    }
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
     const uint32_t ring0 = ptx::smem_u32(ring), slot = (uint32_t)(p.a_bytes + p.b_bytes);
     const uint32_t full0 = ptx::smem_u32(&full_bar[0]), empty0 = ptx::smem_u32(&empty_bar[0]);
 
-    // This thread's share of the epilogue: items of 8 channels of a pixel in this CTA's slice of the tile.
+    // This thread's share of the epilogue: items of 4 channels of a pixel in this CTA's slice of the tile.
     const int et = (int)threadIdx.x - 64;               // 0..255 in warps 2-9
-    const int vshift = p.BN == 64 ? 3 : 2, n_items = (kTileM / p.splits) << vshift;
-    const int row0 = rank * (kTileM / p.splits);
+    const int vshift = p.BN == 64 ? 4 : 3, row0 = rank * p.slice;
+    const int n_items = max(min(p.slice, p.rows - row0), 0) << vshift;
     bool ok = true;
 
     if (warp == 0) {
@@ -136,7 +187,9 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
         };
         auto load_b = [&](int s) {
             ptx::mbar_arrive_expect_tx_u32(full0 + s * 8, (uint32_t)(p.a_tx_bytes + p.b_bytes));
-            ptx::tma_load_2d_u32(ring0 + s * slot + p.a_bytes, mapB, full0 + s * 8, (r * p.kw + sx) * p.cin_pad + cb * p.kb_elems, c0);
+            const int kc = (r * p.kw + sx) * p.cin_pad + cb * p.kb_elems;
+            if (kDirect) ptx::tma_load_5d_u32(ring0 + s * slot + p.a_bytes, mapB, full0 + s * 8, kc, 0, 0, 0, c0 >> 5);
+            else ptx::tma_load_2d_u32(ring0 + s * slot + p.a_bytes, mapB, full0 + s * 8, kc, c0);
         };
         auto load_a = [&](int s) {
             int view = 0, dw = sx - p.pad_l, dh = r - p.pad_t;
@@ -191,12 +244,22 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
             const int ksteps = p.kb_bytes / 32;
             const uint32_t idesc = p.idesc;
             int s = 0;
-            uint32_t phase = 0;
+            uint32_t phase = 0, ready = 0;
+            const uint32_t stage_mask = (1u << p.stages) - 1u;
             for (int i = 0; i < units; ++i) {
-                if (!ptx::mbar_wait_bounded_uniform(full0 + s * 8, phase, &abort_flag, kSplitMaxSpins)) {
+                // Lane l looks at stage l, and one look serves all the units that have landed: a wait for each of them kept the
+                // tensor pipe idle for a third of the loop.  All lanes look, without a branch: the code after it takes the
+                // warp's uniform registers for its own, which lanes that run apart would overwrite for each other.
+                if (!((ready >> s) & 1u)) {
+                    const bool landed = ptx::mbar_test_wait_u32(full0 + min(lane, p.stages - 1) * 8, lane < s ? phase ^ 1u : phase);
+                    ready = __ballot_sync(0xffffffffu, landed) & stage_mask;
+                    __syncwarp();
+                }
+                if (!((ready >> s) & 1u) && !ptx::mbar_wait_bounded_uniform(full0 + s * 8, phase, &abort_flag, kSplitMaxSpins)) {
                     ok = false;
                     break;
                 }
+                ready &= ~(1u << s);
                 const uint32_t a_lo = (uint32_t)d0 + ((s * slot) >> 4), b_lo = a_lo + ((uint32_t)p.a_bytes >> 4);
                 if (ksteps == 4) {
 #pragma unroll
@@ -221,89 +284,161 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
     }
     // The residual of this thread's items is asked for while the MMAs run.
     uint4 res[kSplitMaxItems];
-    if (warp >= 2) {
-        pdl_wait();
-        if (p.has_res) {
-#pragma unroll
-            for (int j = 0; j < kSplitMaxItems; ++j) {
-                const int item = et + j * kSplitEpiThreads;
-                const int row = row0 + (item >> vshift), cl = c0 + (item & ((1 << vshift) - 1)) * 8;
-                if (item < n_items && s_pixel[row] >= 0 && cl < p.e.cout_stride)
-                    res[j] = *reinterpret_cast<const uint4*>(p.e.residual + (int64_t)s_res_pixel[row] * p.e.cout_stride + cl);
-            }
-        }
-        // accumulator -> shared memory, rows padded by 16 bytes: eight lanes' 16-byte stores cover all banks
-        ok = ptx::mbar_wait_bounded_warp(&done_bar, 0, &abort_flag, kSplitMaxSpins);
-        if (ok) {
-            ptx::tc_fence_after_sync();
-            const int q = warp & 3;
-            uint8_t* row = ring + (size_t)(q * 32 + lane) * (p.BN * 4 + 16);
-            // two warps per lane quarter, half of the columns each
-            for (int b = warp < 6 ? 0 : p.BN / 2, e = b + p.BN / 2; b < e; b += 16) {
-                uint32_t raw[16];
-                ptx::tmem_ld_32x32b_x16(tmem_base + ((uint32_t)(q * 32) << 16) + b, raw);
-                ptx::tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    *reinterpret_cast<uint4*>(row + b * 4 + i * 16) = make_uint4(raw[4 * i], raw[4 * i + 1], raw[4 * i + 2], raw[4 * i + 3]);
-            }
-            ptx::tc_fence_before_sync();
-        } else if (lane == 0) {
-            atomicExch(p.error, 3);
-        }
-    }
-    __syncwarp();
-    if (p.splits > 1) ptx::cluster_sync();
-    else __syncthreads();
-    if (warp >= 2 && ok) {
-#pragma unroll
-        for (int j = 0; j < kSplitMaxItems; ++j) {
-            const int item = et + j * kSplitEpiThreads;
-            const int row = row0 + (item >> vshift), px = item < n_items ? s_pixel[row] : -1;
-            const int v = (item & ((1 << vshift) - 1)) * 8, cl = c0 + v;
-            if (px < 0 || cl >= p.e.cout_stride) continue;
-            const uint32_t at = ring0 + (uint32_t)row * (uint32_t)(p.BN * 4 + 16) + (uint32_t)v * 4;
-            uint4 lo, hi;
-            if (p.splits == 1) {
-                lo = *reinterpret_cast<const uint4*>(ring + (at - ring0));
-                hi = *reinterpret_cast<const uint4*>(ring + (at - ring0) + 16);
-            } else {
-                lo = hi = make_uint4(0, 0, 0, 0);
-#pragma unroll 4
-                for (int s = 0; s < p.splits; ++s) {
-                    const uint32_t a = ptx::map_to_cta(at, (uint32_t)s);
-                    acc_add<kInt8>(lo, ld_cluster_16(a));
-                    acc_add<kInt8>(hi, ld_cluster_16(a + 16));
-                }
-            }
-            const uint32_t raw[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = epi_value<kInt8>(raw[i], s_scale[v + i], s_bias[v + i]);
+    if constexpr (kDirect) {
+        if (warp >= 2) {
+            pdl_wait();
+            // two warps per lane quarter, 16 accumulator rows each; lane quads as in the persistent kernel's quad epilogue
+            const int q = warp & 3, cq = lane & 3, h = warp < 6 ? 0 : 1, row = q * 32 + h * 16 + (lane >> 2);
+            const int pa = s_pixel[row], pb = s_pixel[row + 8], nblk = p.BN >> 5, c = c0 + cq * 8;
             if (p.has_res) {
-                const __half2* h = reinterpret_cast<const __half2*>(&res[j]);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 r = __half22float2(h[i]);
-                    f[2 * i] += r.x;
-                    f[2 * i + 1] += r.y;
+                for (int b = 0; b < 2; ++b) {
+                    const bool in = b < nblk && c + b * 32 < p.e.cout_stride;
+                    res[2 * b] = in && pa >= 0 ? __ldg(reinterpret_cast<const uint4*>(p.e.residual + (int64_t)s_res_pixel[row] * p.e.cout_stride + c + b * 32)) : make_uint4(0, 0, 0, 0);
+                    res[2 * b + 1] = in && pb >= 0 ? __ldg(reinterpret_cast<const uint4*>(p.e.residual + (int64_t)s_res_pixel[row + 8] * p.e.cout_stride + c + b * 32)) : make_uint4(0, 0, 0, 0);
                 }
             }
-            if constexpr (kPrelu) {
+            ok = ptx::mbar_wait_bounded_warp(&done_bar, 0, &abort_flag, kSplitMaxSpins);
+            if (ok) {
+                ptx::tc_fence_after_sync();
+                uint32_t raw[2][16];
+                const uint32_t taddr = tmem_base + ((uint32_t)(q * 32 + h * 16) << 16);
+                ptx::tmem_ld_16x256b_x4(taddr, raw[0]);
+                if (nblk == 2) ptx::tmem_ld_16x256b_x4(taddr + 32, raw[1]);
+                ptx::tmem_ld_wait(raw[0]);
+                ptx::tmem_ld_wait(raw[1]);
+                ptx::tc_fence_before_sync();
+                auto drain = [&](auto act, auto with_res, auto outputs) __attribute__((always_inline)) {
+                    constexpr int kAct = decltype(act)::value;
+                    constexpr bool kRes = decltype(with_res)::value;
+                    constexpr int kOut = decltype(outputs)::value;
+                    const float qs = kOut == kQuadI8 ? p.e.out_scale : p.e.out2_scale;
+                    const f32x2 out2_scale = pack2(qs, qs);
+                    __half* const y = static_cast<__half*>(p.e.y);
+                    int8_t* const y2 = static_cast<int8_t*>(kOut == kQuadI8 ? p.e.y : p.e.y2);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) f[i] = f[i] >= 0.f ? f[i] : f[i] * __ldg(p.e.slope + cl + i);
-            } else {
-                apply_act_vec(f, p.e.act);
+                    for (int b = 0; b < 2; ++b) {
+                        if (b >= nblk) break;
+                        f32x2 sc[4], bi[4];
+                        quad_scales(s_scale, s_bias, b * 32, cq, sc, bi);
+                        const bool in = c + b * 32 < p.e.cout_stride;
+                        const int64_t oa = (int64_t)pa * p.e.y_pitch + c + b * 32, ob = (int64_t)pb * p.e.y_pitch + c + b * 32;
+                        quad_pixel<kInt8, kAct, kRes, kOut, 0>(raw[b], sc, bi, res[2 * b], in && pa >= 0, y + oa, y2 + oa, out2_scale);
+                        quad_pixel<kInt8, kAct, kRes, kOut, 2>(raw[b], sc, bi, res[2 * b + 1], in && pb >= 0, y + ob, y2 + ob, out2_scale);
+                    }
+                };
+                if (!quad_dispatch<true>(kPrelu ? -1 : quad_variant(p.e, p.has_res != 0), drain)) {
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)      // (scales are kept from this tile's first channel on)
+                        if (b < nblk && c + b * 32 < p.e.cout_stride)
+                            epi_quad_rows<kInt8, kPrelu>(p.e, s_scale - c0, s_bias - c0, c + b * 32, cq, pa, pb, p.has_res != 0, res[2 * b], res[2 * b + 1],
+                                                         raw[b]);
+                }
+            } else if (lane == 0) {
+                atomicExch(p.error, 3);
             }
-            const int64_t off = (int64_t)px * p.e.y_pitch + cl;
-            epi_store_vec8(p.e.y, p.e.out_dtype, off, f, p.e.out_scale);
-            if (p.e.out2_dtype >= 0) epi_store_vec8(p.e.y2, p.e.out2_dtype, off, f, p.e.out2_scale);
         }
+    } else {
+        const int pitch = p.BN * 4 + 16;      // a part's row: eight lanes' 16-byte accesses cover all banks
+        uint8_t* recv = ring + p.recv;
+        if (warp >= 2) {
+            pdl_wait();
+            if (p.has_res) {
+#pragma unroll
+                for (int j = 0; j < 2 * kSplitMaxItems; ++j) {
+                    const int item = et + j * kSplitEpiThreads;
+                    const int row = row0 + (item >> vshift), cl = c0 + (item & ((1 << vshift) - 1)) * 4;
+                    if (item < n_items && s_pixel[row] >= 0 && cl < p.e.cout_stride) {
+                        const uint2 v = *reinterpret_cast<const uint2*>(p.e.residual + (int64_t)s_res_pixel[row] * p.e.cout_stride + cl);
+                        if (j & 1) {
+                            res[j >> 1].z = v.x;
+                            res[j >> 1].w = v.y;
+                        } else {
+                            res[j >> 1].x = v.x;
+                            res[j >> 1].y = v.y;
+                        }
+                    }
+                }
+            }
+            ok = ptx::mbar_wait_bounded_warp(&done_bar, 0, &abort_flag, kSplitMaxSpins);
+        }
+        __syncwarp();
+        ptx::cluster_wait();
+        if (warp >= 2) {
+            const int q = warp & 3, row = q * 32 + lane;
+            if (ok && q * 32 < p.rows) {
+                ptx::tc_fence_after_sync();
+                // the box's rows take the ring's place; two warps per lane quarter, half of the columns each
+                const int b0 = warp < 6 ? 0 : p.BN / 2;
+                const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + b0;
+                uint32_t raw[2][16];
+                ptx::tmem_ld_32x32b_x16(taddr, raw[0]);
+                if (p.BN == 64) ptx::tmem_ld_32x32b_x16(taddr + 16, raw[1]);
+                ptx::tmem_ld_wait(raw[0]);
+                ptx::tmem_ld_wait(raw[1]);
+                if (row < p.rows) {      // there is room for no more
+                    uint4* dst = reinterpret_cast<uint4*>(ring + row * pitch + b0 * 4);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) dst[i] = make_uint4(raw[0][4 * i], raw[0][4 * i + 1], raw[0][4 * i + 2], raw[0][4 * i + 3]);
+                    if (p.BN == 64)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) dst[4 + i] = make_uint4(raw[1][4 * i], raw[1][4 * i + 1], raw[1][4 * i + 2], raw[1][4 * i + 3]);
+                }
+                __syncwarp();
+                ptx::tc_fence_before_sync();
+                ptx::fence_proxy_async();
+            }
+            __syncwarp();
+            asm volatile("bar.sync 1, 256;" ::: "memory");      // warps 2-9 (all of them, whatever their waits gave)
+            ok = ok && *static_cast<volatile int*>(&abort_flag) == 0;
+            // lane r of the first of them sends CTA r the rows of its slice, part `rank` of what that one sums
+            const int theirs = min(p.slice, p.rows - lane * p.slice);
+            if (ok && warp == 2 && lane < p.splits && lane != rank && theirs > 0)
+                ptx::copy_to_cta(ptx::map_to_cta(ptx::smem_u32(recv) + (uint32_t)(rank * p.slice * pitch), (uint32_t)lane), ring0 + (uint32_t)(lane * p.slice * pitch),
+                                 (uint32_t)(theirs * pitch), ptx::map_to_cta(ptx::smem_u32(&recv_bar), (uint32_t)lane));
+            __syncwarp();
+            if (ok) ok = ptx::mbar_wait_bounded_warp(&recv_bar, 0, &abort_flag, kSplitMaxSpins);
+            if (!ok && lane == 0) atomicExch(p.error, 3);
+        }
+        // second round: no CTA leaves while parts may still be on their way to it (waited for at the end)
+        __syncwarp();
+        ptx::cluster_arrive();
+        if (warp >= 2 && ok) {
+            auto finish = [&](auto parts) __attribute__((always_inline)) {
+                constexpr int S = decltype(parts)::value, kItems = kSplitMaxParts / S;
+                uint4 part[kItems][S];
+#pragma unroll
+                for (int j = 0; j < kItems; ++j) {
+                    const int item = et + j * kSplitEpiThreads;
+                    const int at = (item >> vshift) * pitch + (item & ((1 << vshift) - 1)) * 16;
+                    if (item < n_items)
+#pragma unroll
+                        for (int s = 0; s < S; ++s)
+                            part[j][s] = *reinterpret_cast<const uint4*>((s == rank ? ring + row0 * pitch : recv + s * p.slice * pitch) + at);
+                }
+#pragma unroll
+                for (int j = 0; j < kItems; ++j) {
+                    const int item = et + j * kSplitEpiThreads;
+                    const int v = (item & ((1 << vshift) - 1)) * 4, cl = c0 + v;
+                    const int px = item < n_items ? s_pixel[row0 + (item >> vshift)] : -1;
+                    if (px < 0 || cl >= p.e.cout_stride) continue;
+                    uint4 a = part[j][0];
+#pragma unroll
+                    for (int s = 1; s < S; ++s) acc_add<kInt8>(a, part[j][s]);
+                    const float4 sc = *reinterpret_cast<const float4*>(s_scale + v), bi = *reinterpret_cast<const float4*>(s_bias + v);
+                    split_store4<kInt8, kPrelu>(p.e, a, sc, bi, p.has_res != 0, j & 1 ? res[j >> 1].z : res[j >> 1].x, j & 1 ? res[j >> 1].w : res[j >> 1].y,
+                                                (int64_t)px * p.e.y_pitch + cl, cl);
+                }
+            };
+            if (p.splits == 8) finish(std::integral_constant<int, 8>());
+            else if (p.splits == 4) finish(std::integral_constant<int, 4>());
+            else finish(std::integral_constant<int, 2>());
+        }
+        __syncwarp();
+        ptx::cluster_wait();
     }
-    // no CTA leaves while another one may read its shared memory
     __syncwarp();
-    if (p.splits > 1) ptx::cluster_sync();
-    else __syncthreads();
+    __syncthreads();
     if (warp == 1) {
         ptx::tc_fence_after_sync();
         ptx::tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
@@ -312,17 +447,16 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
 
 }  // namespace
 
-// Which kernel, and how a tile is divided: modelled time in us of both kernels, fitted to 330 layers (batch 1 to 64,
-// 1x1 and 3x3, 32 to 1280 channels, maps of 7 x 7 to 80 x 80; every split of 32 and 64 channels).
-// Split kernel: a constant, the cluster's exchange, then K blocks and epilogue of a tile one after the other, stretched by
-// the tiles per SM once there are more than SMs.  Persistent kernel: a constant and rounds of tiles.  The constants are
-// regression weights, not times of parts: those of 32- and 64-byte K blocks make up for terms the form does not have.  On 330
-// other layers (batch 1 to 256, 7 x 7 to 80 x 80, 16 to 960 -> 64 to 1280 channels) the pick is 2 % slower than the fastest
-// of both kernels on average, and 5 % or more slower in one of nine, at worst 33 to 39 % where the persistent kernel's N
-// tile does not suit either (256 -> 1000 int8 1x1 at 32 x 10 x 10: 10.3 us, divided 7.4).  The line lies near two tiles of 64
-// channels per SM.
+// Which kernel, and how a tile is divided: modelled time in us of both kernels in a captured chain, fitted to 590 layers (batch
+// 1 to 256, 1x1 and 3x3, 16 to 1024 -> 16 to 1280 channels, maps of 4 x 4 to 80 x 80; every split of 32 and 64 channels).
+// Split kernel: a constant, what the exchange costs by the number of parts and by the bytes a CTA receives, then K blocks and
+// epilogue of a tile one after the other, stretched by the tiles per SM once there are more than SMs.  Persistent kernel: a
+// constant and rounds of tiles.  The constants are regression weights, not times of parts.  On those layers the pick is 2 %
+// slower than the fastest of all of them on average and 5 % or more slower in one of eight (at worst 68 %: 304 -> 288 fp16 3x3
+// stride 2 at 31 x 13 x 14).  Against the kernels with parts summed out of the other CTAs' shared memory, and their constants, 220
+// of the layers took 0.83 of the time on average.
 ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
-    const ConvSplit none = {0, 0};
+    const ConvSplit none = {0, 0, 0, 0, 0};
     if (g.pool || g.out_dtype == EXB_I32 || (g.cout_stride & 7) || (g.y_pitch & 7) || conv_fold_plan(g).on) return none;
     const int row_bytes = g.cin_stride * (g.in_dtype == EXB_I8 ? 1 : 2);
     const int kb = row_bytes % 128 == 0 ? 128 : (row_bytes % 64 == 0 ? 64 : 32);
@@ -330,16 +464,18 @@ ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
     const PixelBox box = choose_pixel_box(g.N, g.OH, g.OW);
     const double m_tiles = (double)((g.OW + box.TW - 1) / box.TW) * ((g.OH + box.TH - 1) / box.TH) * ((g.N + box.TN - 1) / box.TN);
     if (m_tiles > 8.0 * ctx->sm_count) return none;
-    ConvSplit best = none;
+    ConvSplit best = {0, 0, box.TW, box.TH, box.TN};
     double best_t = 1e30;
-    static const double kSync[4] = {0.0, 0.43, 1.23, 2.02};
+    static const double kParts[4] = {0.0, 1.0, 0.53, 0.46};      // an exchange of 1, 2, 4, 8 parts beside its volume
+    const double unit = kb == 128 ? 0.218 : kb == 64 ? 0.209 : 0.192;
     for (int bn = 32; bn <= 64; bn *= 2)
-        for (int sp = 1, i = 0; sp <= 8 && sp <= k_iters; sp *= 2, ++i) {
+        for (int sp = 1, i = 0; sp <= kSplitMaxParts && (sp == 1 || 2 * sp <= k_iters); sp *= 2, ++i) {      // two K blocks a part
             const double ctas = m_tiles * ((w->cout_pad + bn - 1) / bn) * sp;
-            const double stretch = ctas > 1.05 * ctx->sm_count ? ctas / (1.05 * ctx->sm_count) : 1.0;
+            const double stretch = ctas > 1.02 * ctx->sm_count ? ctas / (1.02 * ctx->sm_count) : 1.0;
             const double units = (k_iters + sp - 1) / sp;
-            const double step = kb == 32 ? 0.203 : kb == 64 ? 0.239 : 0.246;
-            const double t = 1.93 + kSync[i] + stretch * (units * step + (bn == 32 ? 1.09 : 2.23) + 0.36 * kSync[i]);
+            const double volume = box.TW * box.TH * box.TN * bn * (sp - 1) / (sp * 8192.0);
+            const double t = 0.8 + kParts[i] + 1.29 * volume +
+                             stretch * (units * unit * (bn == 32 ? 0.962 : 1.0) + (bn == 32 ? 1.40 : 1.52) + 1.31 * volume - (sp > 1 ? 0.36 : 0.0));
             if (t < best_t) {
                 best_t = t;
                 best.BN = bn;
@@ -352,22 +488,22 @@ ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
     const double tiles = m_tiles * nt.n_tiles, slots = (double)ctx->sm_count * (two ? 2 : 1);
     const double rounds = tiles <= slots ? 1.0 : ceil(tiles / slots);
     double share = 1.0;      // two CTAs of an SM share its tensor pipe
-    if (two && tiles > ctx->sm_count) share += 0.20 * (tiles < 2 * ctx->sm_count ? tiles / ctx->sm_count - 1 : 1.0);
-    double step = 0.305, rest = 5.14;       // one CTA (or pair) per SM, more than 128 channels
+    if (two && tiles > ctx->sm_count) share += 0.35 * (tiles < 2 * ctx->sm_count ? tiles / ctx->sm_count - 1 : 1.0);
+    double step = 0.292, rest = 1.45;       // one CTA (or pair) per SM, more than 128 channels
     if (two) {
-        step = bn <= 64 ? 0.246 : 0.19;
-        rest = bn <= 64 ? 0.93 : 2.94;
+        step = bn <= 64 ? 0.216 : 0.304;
+        rest = bn <= 64 ? 0.0 : 1.09;
     } else if (nt.paired) {
-        step = 0.208;
-        rest = 2.24;
+        step = 0.207;
+        rest = 1.71;
     }
-    if (bn > 128 && k_iters * kb < 512) rest = 1.6;      // single CTAs of short reductions
-    step *= kb == 128 ? 1.0 : kb == 64 ? 0.21 : 0.39;
-    double body = rounds * (k_iters * step + rest + (g.has_res ? 0.45 : 0.0)) * share;
-    // int8 tiles of a short K, more of them than fit the SMs as clusters: 96 -> 320 1x1 at 8 x 40 x 40 8.1 us, divided 11.4
-    if (two && g.in_dtype == EXB_I8 && k_iters * kb <= 256 && m_tiles * ((w->cout_pad + 63) / 64) > ctx->sm_count) body *= 0.75;
-    const double persistent = 4.58 + body;
-    return best_t < 0.98 * persistent ? best : none;
+    step *= kb == 128 ? 1.0 : kb == 64 ? 0.65 : 0.56;
+    double body = rounds * (k_iters * step + rest + (g.has_res ? 1.5 : 0.0)) * share;
+    // int8 tiles of a short K, more of them than fit the SMs as clusters; an int8 result alone has a loop of its own in the row
+    // epilogue (96 -> 320 1x1 at 8 x 40 x 40: int8 7.8 us, undivided tiles of this kernel 7.6; fp16 8.3 and 7.6)
+    if (two && g.in_dtype == EXB_I8 && k_iters * kb <= 256 && m_tiles * ((w->cout_pad + 63) / 64) > ctx->sm_count)
+        body *= g.out_dtype == EXB_I8 && g.out2_dtype < 0 ? 0.8 : 1.28;
+    return best_t < 3.92 + body ? best : none;
 }
 
 int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, const void* x, const exb_conv_weights* w, const void* residual,
@@ -379,8 +515,7 @@ int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, cons
     ConvSplitParams p;
     memset(&p, 0, sizeof(p));
     p.N = g.N; p.OH = g.OH; p.OW = g.OW;
-    const PixelBox box = choose_pixel_box(g.N, g.OH, g.OW);
-    p.TW = box.TW; p.TH = box.TH; p.TN = box.TN;
+    p.TW = sp.TW; p.TH = sp.TH; p.TN = sp.TN;
     p.tiles_w = (g.OW + p.TW - 1) / p.TW;
     p.tiles_h = (g.OH + p.TH - 1) / p.TH;
     const int tiles_nb = (g.N + p.TN - 1) / p.TN;
@@ -392,13 +527,20 @@ int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, cons
     p.kb_elems = p.kb_bytes / es;
     p.cblks = row_bytes / p.kb_bytes;
     p.k_iters = g.kh * g.kw * p.cblks;
+    p.rows = p.TW * p.TH * p.TN;
+    p.slice = (p.rows + p.splits - 1) / p.splits;
     p.a_tx_bytes = p.TW * p.TH * p.TN * p.kb_bytes;
     p.a_bytes = round_up(p.a_tx_bytes, 1024);      // the MMA reads 128 rows whatever the box holds: unused ones from what follows
     p.b_bytes = p.BN * p.kb_bytes;
     const int overread = kTileM * p.kb_bytes - p.a_bytes;
     const int units = (p.k_iters + p.splits - 1) / p.splits;
-    // two CTAs of neighbouring launches fit an SM side by side (programmatic launch): half of the shared memory each
-    p.stages = (96 * 1024 - overread) / (p.a_bytes + p.b_bytes);
+    const bool direct = p.splits == 1;
+    const int grid = p.tiles_w * p.tiles_h * tiles_nb * p.n_tiles * p.splits;
+    const int part = p.slice * p.splits * (p.BN * 4 + 16);      // of all CTAs of a cluster for one's slice
+    // two CTAs of neighbouring launches fit an SM side by side (programmatic launch): half of the shared memory each, and all
+    // of it where the neighbours find SMs of their own
+    const int room = 2 * grid <= ctx->sm_count ? ctx->smem_optin - 6 * 1024 : 109 * 1024;
+    p.stages = (room - overread - (direct ? 0 : part)) / (p.a_bytes + p.b_bytes);
     if (p.stages > kSplitStages) p.stages = kSplitStages;
     if (p.stages > units) p.stages = units;
     p.tmem_cols = p.BN <= 32 ? 32 : 64;
@@ -413,23 +555,20 @@ int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, cons
     const FoldPlan no_fold = {false, 0, 0, 0, 0};
     const CUtensorMapSwizzle sw = swizzle_for(p.kb_bytes);
     if (int rc = encode_input_views(g, no_fold, x, p.kb_elems, sw, p.TW, p.TH, p.TN, p.tmA)) return rc;
-    {
-        const int K = g.kh * w->kw_pack * w->cin_pad;
-        cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)w->cout_pad};
-        cuuint64_t strides[1] = {(cuuint64_t)K * es};
-        cuuint32_t bx[2] = {(cuuint32_t)p.kb_elems, (cuuint32_t)p.BN};
-        cuuint32_t estr[2] = {1, 1};
-        const CUresult r = encode(&p.tmB, int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, w->d_w, dims, strides, bx, estr,
-                                  CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled(B) failed with %d", (int)r);
-    }
-    const int grid = p.tiles_w * p.tiles_h * tiles_nb * p.n_tiles * p.splits;
+    if (int rc = encode_weights(g, w, p.kb_elems, sw, p.BN, direct, &p.tmB)) return rc;
     size_t smem = (size_t)p.stages * (p.a_bytes + p.b_bytes) + (overread > p.b_bytes ? overread - p.b_bytes : 0);
-    const size_t part = (size_t)kTileM * (p.BN * 4 + 16);
-    smem = (smem > part ? smem : part) + 1024;
+    if (!direct) {
+        if (smem < (size_t)part) smem = part;      // the box's rows take the ring's place
+        p.recv = (int)((smem + 15) / 16 * 16);
+        smem = (size_t)p.recv + part;
+    }
+    smem += 1024;
     const bool prelu = g.act == EXB_ACT_PRELU;
-    auto kern = int8 ? (prelu ? conv_split_kernel<true, true> : conv_split_kernel<true, false>)
-                     : (prelu ? conv_split_kernel<false, true> : conv_split_kernel<false, false>);
+    auto kern = int8 ? (prelu ? conv_split_kernel<true, true, false> : conv_split_kernel<true, false, false>)
+                     : (prelu ? conv_split_kernel<false, true, false> : conv_split_kernel<false, false, false>);
+    if (direct)
+        kern = int8 ? (prelu ? conv_split_kernel<true, true, true> : conv_split_kernel<true, false, true>)
+                    : (prelu ? conv_split_kernel<false, true, true> : conv_split_kernel<false, false, true>);
     if (int rc = raise_smem_limit(ctx, kern)) return rc;
     return launch_pdl_cluster(ctx, "conv_split_kernel", kern, dim3((unsigned)grid), dim3(kSplitThreads), dim3((unsigned)p.splits), smem, st, p);
 }

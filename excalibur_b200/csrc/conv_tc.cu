@@ -36,9 +36,8 @@
 // All mbarrier waits are bounded; when one runs out the kernel raises the context's error
 // word, every role leaves its loop, TMEM is freed and the launch returns normally.
 #include "conv_tc_host.cuh"
+#include "conv_quad.cuh"
 #include "ptx_sm100.cuh"
-
-#include <type_traits>
 
 namespace exb {
 namespace {
@@ -208,129 +207,6 @@ __device__ __forceinline__ void epi_row16(const EpiParams& e, const float4 (&sc)
     if (e.out2_dtype >= 0) epi_store_vec16(e.y2, e.out2_dtype, off, v, e.out2_scale, acc);
 }
 
-// Two pixels' 8 consecutive channels from one 16x256b.x4 fragment (raw[4g + e] first pixel, raw[4g + 2 + e] second
-// pixel, channels cl + 2g + e).  Scale and bias are read once for both pixels, from the quad-ordered copy: the four
-// floats of channels 8*j + 4*i .. + 3 of a 32-channel block sit at 32*block + 16*i + 4*j, so that the four lanes of a
-// pixel read one contiguous 64-byte piece per load (channel order would put neighbouring lanes on the same banks).
-template <bool kInt8, bool kPrelu>
-__device__ __forceinline__ void epi_quad_rows(const EpiParams& e, const float* q_scale, const float* q_bias, int cl, int cq,
-                                              int pa, int pb, bool add_res, const uint4& ra, const uint4& rb,
-                                              const uint32_t (&raw)[16]) {
-    float va[8], vb[8];
-    const float4* sc = reinterpret_cast<const float4*>(q_scale + (cl & ~31) + 4 * cq);
-    const float4* bi = reinterpret_cast<const float4*>(q_bias + (cl & ~31) + 4 * cq);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float4 s4 = sc[4 * i], b4 = bi[4 * i];
-        va[4 * i + 0] = epi_value<kInt8>(raw[8 * i + 0], s4.x, b4.x);
-        va[4 * i + 1] = epi_value<kInt8>(raw[8 * i + 1], s4.y, b4.y);
-        va[4 * i + 2] = epi_value<kInt8>(raw[8 * i + 4], s4.z, b4.z);
-        va[4 * i + 3] = epi_value<kInt8>(raw[8 * i + 5], s4.w, b4.w);
-        vb[4 * i + 0] = epi_value<kInt8>(raw[8 * i + 2], s4.x, b4.x);
-        vb[4 * i + 1] = epi_value<kInt8>(raw[8 * i + 3], s4.y, b4.y);
-        vb[4 * i + 2] = epi_value<kInt8>(raw[8 * i + 6], s4.z, b4.z);
-        vb[4 * i + 3] = epi_value<kInt8>(raw[8 * i + 7], s4.w, b4.w);
-    }
-    if (add_res) {
-        const __half2* ha = reinterpret_cast<const __half2*>(&ra);
-        const __half2* hb = reinterpret_cast<const __half2*>(&rb);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 fa = __half22float2(ha[i]), fb = __half22float2(hb[i]);
-            va[2 * i] += fa.x;
-            va[2 * i + 1] += fa.y;
-            vb[2 * i] += fb.x;
-            vb[2 * i + 1] += fb.y;
-        }
-    }
-    if constexpr (kPrelu) {
-        const float4 l0 = __ldg(reinterpret_cast<const float4*>(e.slope + cl)), l1 = __ldg(reinterpret_cast<const float4*>(e.slope + cl) + 1);
-        const float sl[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            va[i] = va[i] >= 0.f ? va[i] : va[i] * sl[i];
-            vb[i] = vb[i] >= 0.f ? vb[i] : vb[i] * sl[i];
-        }
-    } else {
-        apply_act_vec(va, e.act);
-        apply_act_vec(vb, e.act);
-    }
-    if (pa >= 0) {
-        const int64_t off = (int64_t)pa * e.y_pitch + cl;
-        epi_store_vec8(e.y, e.out_dtype, off, va, e.out_scale);
-        if (e.out2_dtype >= 0) epi_store_vec8(e.y2, e.out2_dtype, off, va, e.out2_scale);
-    }
-    if (pb >= 0) {
-        const int64_t off = (int64_t)pb * e.y_pitch + cl;
-        epi_store_vec8(e.y, e.out_dtype, off, vb, e.out_scale);
-        if (e.out2_dtype >= 0) epi_store_vec8(e.y2, e.out2_dtype, off, vb, e.out2_scale);
-    }
-}
-
-// The lean form of the same for the outputs that layers have in earnest: fp16, alone or with an int8 copy, behind no
-// activation, ReLU, ReLU6 or SiLU.  What bounds short reductions is the instruction stream of the epilogue warps (16
-// instructions per value in the general form: dispatch on activation and types per vector, 64-bit addresses per store), so
-// everything that can be is known at compile time, sums are formed two at a time, clamps act on packed halves (rounding is
-// monotone and 0 and 6 are halves: the same results), and the accumulator is handed back after the last load instead of after
-// the last store.  Measured against the general form: 32 -> 160 int8 1x1 + ReLU6 at 64 x 56 x 56 29.5 -> 19.8 us, 32 -> 96 at
-// 64 x 112 x 112 59.5 -> 40.2 (4.5 TB/s), 64 -> 64 fp16 1x1 + SiLU at 16 x 160 x 160 37.5 -> 30.4, 128 -> 128 + SiLU at
-// 16 x 80 x 80 23.2 -> 18.2.  Loading fragment f + 1 while f is worked on needs more than the 96 registers (5.8 KB spilled).
-enum QuadAct { kQuadNone = 0, kQuadRelu = 1, kQuadRelu6 = 2, kQuadSilu = 3 };
-template <int kAct>
-using QuadActC = std::integral_constant<int, kAct>;
-
-// activation | residual << 2 | int8 copy << 3, or -1 where the general form is needed
-__device__ __forceinline__ int quad_variant(const ConvTcParams& p) {
-    if (p.e.out_dtype != EXB_F16 || (p.e.out2_dtype >= 0 && p.e.out2_dtype != EXB_I8)) return -1;
-    const int more = (p.has_res ? 4 : 0) | (p.e.out2_dtype >= 0 ? 8 : 0);
-    if (p.e.act == EXB_ACT_NONE) return kQuadNone | more;
-    if (p.e.act == EXB_ACT_RELU) return kQuadRelu | more;
-    if (more) return -1;
-    return p.e.act == EXB_ACT_RELU6 ? kQuadRelu6 : p.e.act == EXB_ACT_SILU ? kQuadSilu : -1;
-}
-
-template <bool kInt8>
-__device__ __forceinline__ f32x2 quad_value(uint32_t r0, uint32_t r1, f32x2 scale, f32x2 bias) {
-    return fma2(kInt8 ? pack2((float)(int)r0, (float)(int)r1) : pack2(__uint_as_float(r0), __uint_as_float(r1)), scale, bias);
-}
-
-// One pixel's 8 consecutive channels, first[i] and first[i] + 1 the accumulators of pair i.
-template <bool kInt8, int kAct, bool kRes, bool kOut2, int kFirst>
-__device__ __forceinline__ void quad_pixel(const uint32_t (&raw)[16], const f32x2 (&sc)[4], const f32x2 (&bi)[4], const uint4& res, bool store,
-                                           __half* y, int8_t* y2, f32x2 out2_scale) {
-    uint32_t o[4];
-    int qv[8];
-    const uint32_t rr[4] = {res.x, res.y, res.z, res.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f32x2 v = quad_value<kInt8>(raw[4 * i + kFirst], raw[4 * i + kFirst + 1], sc[i], bi[i]);
-        if (kRes) v = add2(v, cvt2(rr[i]));
-        float a, b;
-        unpack2(v, a, b);
-        if (kAct == kQuadSilu) {
-            a *= sigmoid_fast(a);
-            b *= sigmoid_fast(b);
-        }
-        if (kOut2 && kAct == kQuadRelu) {      // the copy is quantised from the fp32 value
-            a = fmaxf(a, 0.f);
-            b = fmaxf(b, 0.f);
-        }
-        __half2 h = __floats2half2_rn(a, b);
-        if ((kAct == kQuadRelu && !kOut2) || kAct == kQuadRelu6) h = __hmax2(h, __half2half2(__ushort_as_half(0)));
-        if (kAct == kQuadRelu6) h = __hmin2(h, __half2half2(__ushort_as_half(0x4600)));      // 6
-        o[i] = *reinterpret_cast<const uint32_t*>(&h);
-        if (kOut2) {
-            float qa, qb;
-            unpack2(mul2(pack2(a, b), out2_scale), qa, qb);
-            qv[2 * i] = __float2int_rn(qa);
-            qv[2 * i + 1] = __float2int_rn(qb);
-        }
-    }
-    if (!store) return;
-    *reinterpret_cast<uint4*>(y) = make_uint4(o[0], o[1], o[2], o[3]);
-    if (kOut2) *reinterpret_cast<uint2*>(y2) = make_uint2(sat_pack4(qv[0], qv[1], qv[2], qv[3]), sat_pack4(qv[4], qv[5], qv[6], qv[7]));
-}
-
 // The MMAs of one row-box unit, fully unrolled: tap s reads the box s pixels further in (kSteps 32-byte K steps per
 // pixel) against the weight block of that tap.  The issuing warp retires one instruction every few cycles, so
 // every address computed at run time shows in the MMA rate of narrow tiles.
@@ -474,7 +350,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
     for (int c = threadIdx.x; c < p.n_tiles * p.BN; c += kThreads) {
         const bool in = c < p.cout_pad;
         // quad epilogue: channel 32*b + 8*j + 4*i + k is kept at 32*b + 16*i + 4*j + k (see epi_quad_rows)
-        const int at = kEpi == kEpiQuad || kEpi == kEpiMapped ? ((c & ~31) | ((c & 4) << 2) | ((c & 24) >> 1) | (c & 3)) : c;
+        const int at = kEpi == kEpiQuad || kEpi == kEpiMapped ? quad_order(c) : c;
         s_scale[at] = in ? p.e.scale[c] : 0.f;
         s_bias[at] = in ? p.e.bias[c] : 0.f;
     }
@@ -922,7 +798,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                 return (n * (p.OH >> 1) + (oh >> 1)) * (p.OW >> 1) + (ow >> 1);
             };
             const bool want_res = p.has_res != 0;
-            const int lean = kPrelu ? -1 : quad_variant(p);
+            const int lean = kPrelu ? -1 : quad_variant(p.e, want_res);
             TileCursor cur(p, first_unit + grp * unit_step, p.epi_groups * unit_step);
             for (int t = first_unit + grp * unit_step; t < total_tiles && ok; t += p.epi_groups * unit_step, ti += p.epi_groups) {
                 const TileCoord tc = tile_of(cur);
@@ -989,9 +865,10 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                     }
                 };
                 // Lean form (see quad_pixel)
-                auto drain = [&](auto act, auto with_res, auto with_out2) __attribute__((always_inline)) {
+                auto drain = [&](auto act, auto with_res, auto outputs) __attribute__((always_inline)) {
                     constexpr int kAct = decltype(act)::value;
-                    constexpr bool kRes = decltype(with_res)::value, kOut2 = decltype(with_out2)::value;
+                    constexpr bool kRes = decltype(with_res)::value;
+                    constexpr int kOut = decltype(outputs)::value;
                     const f32x2 out2_scale = pack2(p.e.out2_scale, p.e.out2_scale);
 #pragma unroll 1
                     for (int f = 0; f < nfrag; ++f) {
@@ -1002,15 +879,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                         uint4 na = make_uint4(0, 0, 0, 0), nb = na;
                         if (kRes) res_load(f + 1, na, nb);
                         f32x2 sc[4], bi[4];
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const int at = (cl & ~31) + 4 * cq + 16 * i;
-                            const ulonglong2 s = *reinterpret_cast<const ulonglong2*>(s_scale + at), c = *reinterpret_cast<const ulonglong2*>(s_bias + at);
-                            sc[2 * i] = s.x;
-                            sc[2 * i + 1] = s.y;
-                            bi[2 * i] = c.x;
-                            bi[2 * i + 1] = c.y;
-                        }
+                        quad_scales(s_scale, s_bias, cl, cq, sc, bi);
                         ptx::tmem_ld_wait(raw);
                         if (f + 1 == nfrag) release();
                         int pa = second ? pa1 : pa0, pb = second ? pb1 : pb0;
@@ -1019,25 +888,13 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                         const int64_t oa = (int64_t)(pa + shift) * p.e.y_pitch + cl, ob = (int64_t)(pb + shift) * p.e.y_pitch + cl;
                         __half* const y = static_cast<__half*>(p.e.y);
                         int8_t* const y2 = static_cast<int8_t*>(p.e.y2);
-                        quad_pixel<kInt8, kAct, kRes, kOut2, 0>(raw, sc, bi, ra, sa, y + oa, y2 + oa, out2_scale);
-                        quad_pixel<kInt8, kAct, kRes, kOut2, 2>(raw, sc, bi, rb, sb, y + ob, y2 + ob, out2_scale);
+                        quad_pixel<kInt8, kAct, kRes, kOut, 0>(raw, sc, bi, ra, sa, y + oa, y2 + oa, out2_scale);
+                        quad_pixel<kInt8, kAct, kRes, kOut, 2>(raw, sc, bi, rb, sb, y + ob, y2 + ob, out2_scale);
                         ra = na;
                         rb = nb;
                     }
                 };
-                using std::false_type;
-                using std::true_type;
-                if (lean == kQuadRelu6) drain(QuadActC<kQuadRelu6>(), false_type(), false_type());
-                else if (lean == kQuadSilu) drain(QuadActC<kQuadSilu>(), false_type(), false_type());
-                else if (lean == kQuadRelu) drain(QuadActC<kQuadRelu>(), false_type(), false_type());
-                else if (lean == kQuadNone) drain(QuadActC<kQuadNone>(), false_type(), false_type());
-                else if (lean == (kQuadRelu | 4)) drain(QuadActC<kQuadRelu>(), true_type(), false_type());
-                else if (lean == (kQuadNone | 4)) drain(QuadActC<kQuadNone>(), true_type(), false_type());
-                else if (lean == (kQuadRelu | 8)) drain(QuadActC<kQuadRelu>(), false_type(), true_type());
-                else if (lean == (kQuadNone | 8)) drain(QuadActC<kQuadNone>(), false_type(), true_type());
-                else if (lean == (kQuadRelu | 12)) drain(QuadActC<kQuadRelu>(), true_type(), true_type());
-                else if (lean == (kQuadNone | 12)) drain(QuadActC<kQuadNone>(), true_type(), true_type());
-                else {
+                if (!quad_dispatch<false>(lean, drain)) {
 #pragma unroll 1
                 for (int f = 0; f < nfrag; ++f) {
                     const bool second = f >= nblk;
@@ -1596,30 +1453,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     if (!patch)
         if (int rc = encode_input_views(g, fold, x, p.kb_elems, sw, p.rowbox ? p.TW + g.kw - 1 : p.TW, p.TH, p.TN, p.tmA)) return rc;
     p.b_perm = quad ? 1 : 0;
-    {
-        const int K = g.kh * w->kw_pack * w->cin_pad;
-        CUresult r;
-        if (quad) {
-            // Rows of the packed matrix [cout][K] seen as (e: 2, j: 4, g: 4, block) with row = 32*block + 8*j + 2*g + e,
-            // traversed e, j, g, block: shared-memory row (= accumulator column) 8*g + 2*j + e of a block holds
-            // output channel 8*j + 2*g + e.
-            const cuuint64_t kb = (cuuint64_t)K * es;
-            cuuint64_t dims[5] = {(cuuint64_t)K, 2, 4, 4, (cuuint64_t)(w->cout_pad / 32)};
-            cuuint64_t strides[4] = {kb, 8 * kb, 2 * kb, 32 * kb};
-            cuuint32_t box[5] = {(cuuint32_t)p.kb_elems, 2, 4, 4, (cuuint32_t)((pair ? p.BN / 2 : p.BN) / 32)};
-            cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-            r = encode(&p.tmB, dt, 5, w->d_w, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        } else {
-            cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)w->cout_pad};
-            cuuint64_t strides[1] = {(cuuint64_t)K * es};
-            cuuint32_t box[2] = {(cuuint32_t)p.kb_elems, (cuuint32_t)(pair ? p.BN / 2 : p.BN)};
-            cuuint32_t estr[2] = {1, 1};
-            r = encode(&p.tmB, dt, 2, w->d_w, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        }
-        if (r != CUDA_SUCCESS) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled(B) failed with %d", (int)r);
-    }
+    if (int rc = encode_weights(g, w, p.kb_elems, sw, pair ? p.BN / 2 : p.BN, quad, &p.tmB)) return rc;
 
     const int units = p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;      // tiles, or pairs of them (clusters of two CTAs)
     const int max_units = pair ? ctx->sm_count / 2 : ctx->sm_count * (two ? 2 : 1);

@@ -39,14 +39,12 @@ inline PixelBox search_pixel_box(int N, int OH, int OW) {
     return b;
 }
 
-// The same, searched once per shape (the search is some 500 candidates, 4 us of every eager call): the last shape that
-// fell into each of 256 slots is kept.
+// The same, searched once per shape and thread (the search is some 500 candidates, 4 us of every eager call): the last shape
+// that fell into each of 256 slots is kept.
 inline PixelBox choose_pixel_box(int N, int OH, int OW) {
-    static std::mutex mutex;
-    static PixelBox kept[256];
+    static thread_local PixelBox kept[256];
     uint32_t h = 2166136261u;
     for (int v : {N, OH, OW}) h = (h ^ (uint32_t)v) * 16777619u;
-    std::lock_guard<std::mutex> lock(mutex);
     PixelBox& e = kept[(h ^ (h >> 16)) & 255u];
     if (e.N != N || e.OH != OH || e.OW != OW) e = search_pixel_box(N, OH, OW);
     return e;
@@ -87,6 +85,25 @@ inline int encode_input_views(const ConvGeom& g, const FoldPlan& fold, const voi
         if (r != CUDA_SUCCESS) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled(A view %d) failed with %d", v, (int)r);
     }
     return EXB_OK;
+}
+
+// Tensor map of the packed weights [cout][K], boxes of `rows` rows and a K block.  `quad`: in the column order of the quad
+// epilogue (rows in whole 32-channel blocks).  Row 32*block + 8*j + 2*g + e is seen as (e: 2, j: 4, g: 4, block) and traversed
+// e, j, g, block: shared-memory row (= accumulator column) 8*g + 2*j + e of a block holds output channel 8*j + 2*g + e.
+inline int encode_weights(const ConvGeom& g, const exb_conv_weights* w, int kb_elems, CUtensorMapSwizzle sw, int rows, bool quad, CUtensorMap* map) {
+    auto encode = tensor_map_encoder();
+    const bool int8 = g.in_dtype == EXB_I8;
+    const int K = g.kh * w->kw_pack * w->cin_pad;
+    const cuuint64_t kb = (cuuint64_t)K * (int8 ? 1 : 2);
+    const cuuint64_t dims2[2] = {(cuuint64_t)K, (cuuint64_t)w->cout_pad}, strides2[1] = {kb};
+    const cuuint32_t box2[2] = {(cuuint32_t)kb_elems, (cuuint32_t)rows};
+    const cuuint64_t dims5[5] = {(cuuint64_t)K, 2, 4, 4, (cuuint64_t)(weight_rows(w->cout_pad) / 32)}, strides5[4] = {kb, 8 * kb, 2 * kb, 32 * kb};
+    const cuuint32_t box5[5] = {(cuuint32_t)kb_elems, 2, 4, 4, (cuuint32_t)(rows / 32)};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = encode(map, int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, quad ? 5 : 2, w->d_w, quad ? dims5 : dims2,
+                              quad ? strides5 : strides2, quad ? box5 : box2, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? EXB_OK : fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled(B) failed with %d", (int)r);
 }
 
 }  // namespace exb

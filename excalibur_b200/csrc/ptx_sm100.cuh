@@ -224,6 +224,16 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The two halves by themselves: what lies between them overlaps the other CTAs' arrival.  The arrival orders no memory (a
+// release waits for every access under way): barriers are published by their own fence, data by mbarriers.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Bytes of this CTA's shared memory into that of a CTA of the cluster, counted on that CTA's barrier (`dst` and `bar` are
+// shared::cluster addresses; addresses and size multiples of 16).
+__device__ __forceinline__ void copy_to_cta(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
 // shared::cluster address of the same shared-memory offset in the CTA of the given rank
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
     uint32_t r;

@@ -694,3 +694,30 @@ def test_lean_quad_epilogue(ctx, case, i8):
                         ok = ~torch.isnan(want)
                         assert torch.equal(y2[ok], (want * 0.7).round().clamp(-128, 127).to(torch.int8)[ok]), (act, res, out2)
     ctx.sync_check()
+
+
+# Reductions that are not divided, and the exchange of those that are, with boxes of fewer pixels than a tile has rows and rings
+# smaller than the tile that takes their place; channel counts with and without whole 32-channel blocks.
+@pytest.mark.parametrize("case", [(15, 32, 11, 11, 176, 1, 2), (15, 32, 11, 11, 192, 1, 2), (1, 64, 6, 6, 48, 1, 1), (3, 64, 5, 5, 64, 1, 1), (2, 512, 5, 7, 208, 3, 1),
+                                  (1, 1024, 3, 3, 512, 1, 1), (7, 128, 9, 13, 128, 3, 1), (1, 256, 13, 11, 256, 3, 1)])
+@pytest.mark.parametrize("i8", [True, False])
+def test_split_tiles_of_few_pixels(ctx, case, i8):
+    import torch
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s = case
+    names = _route(ctx, case, i8, capi.EXB_I8 if i8 else capi.EXB_F16, 0)
+    assert len(names) == 1 and "conv_split_kernel" in names[0], names
+    r = rng(sum(case) + i8)
+    wq = r.integers(-4, 5, (Cout, Cin, k, k)).astype(np.int8)
+    x = dev(r.integers(-4, 5, (N, H, W, Cin)).astype(np.int8 if i8 else np.float16))
+    got = []
+    for impl in (0, 2):        # whole numbers: exact whatever the order of the sums
+        d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8 if i8 else capi.EXB_F16, capi.EXB_F16, capi.EXB_I8, res=True, act=1,
+                                out2_scale=0.01, impl=impl)
+        oh, ow = capi.conv_out_dims(d)
+        skip = dev(rng(7).integers(-50, 50, (N, oh, ow, Cout)).astype(np.float16))
+        p = capi.ConvWeights(ctx, d, wq, None, np.ones(Cout, np.float32), 1.0) if i8 else capi.ConvWeights(ctx, d, wq.astype(np.float32))
+        got.append(capi.conv2d(ctx, d, x, p, residual=skip))
+        ctx.sync_check()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
