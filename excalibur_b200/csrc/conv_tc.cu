@@ -283,86 +283,109 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
     // Let the next kernel of the stream be scheduled as soon as SMs free up (it waits for this
     // grid's completion at its own griddepcontrol.wait before it reads or writes global memory).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (threadIdx.x == 0) {
-        abort_flag = 0;
-        for (int i = 0; i < kMaxAccBufs; ++i) pool_fail[i] = 0;
-        for (int s = 0; s < p.stages; ++s) {
-            ptx::mbar_init(&full_bar[s], 1);
-            ptx::mbar_init(&empty_bar[s], 1);
+    // Each role prepares what it alone needs, so that none waits for another's global loads: with one CTA per SM nothing of this
+    // overlaps the previous kernel's last tiles.  Warp 0 initialises the barriers and goes on to its table of K units and the
+    // weights without waiting for the block (bar.arrive); warp 1 allocates TMEM; the epilogue warps stage scale and bias and
+    // meet at a barrier of their own.  In a captured chain 64 -> 64 fp16 3x3 at 4 x 120 x 184 13.0 -> 11.6 us, 128 -> 128 int8 3x3
+    // at 32 x 28 x 28 10.9 -> 9.1, 64 -> 384 int8 1x1 at 64 x 14 x 14 7.3 -> 6.6.
+    if (warp == 0) {
+        // (one lane per barrier: 33 of them one after the other are half a microsecond)
+        if (lane < p.stages) {
+            ptx::mbar_init(&full_bar[lane], 1);
+            ptx::mbar_init(&empty_bar[lane], 1);
         }
-        for (int i = 0; i < p.acc_bufs; ++i) {
-            ptx::mbar_init(&tfull_bar[i], 1);
-            ptx::mbar_init(&tempty_bar[i], (kPair ? 2 : 1) * (kEpiWarps / p.epi_groups));   // pair: both CTAs' warps arrive at rank 0
+        if (lane < p.acc_bufs) {
+            ptx::mbar_init(&tfull_bar[lane], 1);
+            ptx::mbar_init(&tempty_bar[lane], (kPair ? 2 : 1) * (kEpiWarps / p.epi_groups));   // pair: both CTAs' warps arrive at rank 0
         }
-        ptx::mbar_init(&bres_bar, 1);
+        if (kEpi == kEpiPool && lane < kMaxAccBufs) pool_fail[lane] = 0;
+        if (lane == 0) {
+            ptx::mbar_init(&bres_bar, 1);
+            abort_flag = 0;
+            ptx::tma_prefetch_desc(&p.tmB);
+            ptx::tma_prefetch_desc(&p.tmA[0]);
+        }
         ptx::fence_mbar_init();
-        ptx::tma_prefetch_desc(&p.tmA[0]);
-        ptx::tma_prefetch_desc(&p.tmB);
-    }
-    if (warp == 1) {
-        if (kPair) {
-            ptx::tmem_alloc_pair(&tmem_base_smem, (uint32_t)p.tmem_cols);
-            ptx::tmem_relinquish_pair();
-        } else {
-            ptx::tmem_alloc(&tmem_base_smem, (uint32_t)p.tmem_cols);
-            ptx::tmem_relinquish();
+        __syncwarp();
+        if (kPair) ptx::cluster_arrive();
+        // (not barrier 0: this warp may be at the end before the others are here)
+        asm volatile("bar.arrive 4, 64;" ::: "memory");
+        asm volatile("bar.arrive 3, %0;" ::"n"(kThreads) : "memory");
+        for (int it = lane; it < k_iters; it += 32) {
+            if (p.fold) {   // one K block per kernel row: the box starts at the output column itself
+                const int oh_ = it - p.pad_t;
+                const int ph = p.stride == 2 ? (oh_ & 1) : 0;
+                k_tab[it] = make_int4(0, 0, p.stride == 2 ? ((oh_ - ph) >> 1) : oh_, (it * p.kb_elems) | ((ph * 2) << 28));
+                continue;
+            }
+            if (p.rowbox) {  // one unit per (kernel row, channel block): the box starts pad_l pixels left of the tile
+                const int r = it / p.cblks, cb = it - r * p.cblks;
+                k_tab[it] = make_int4(cb * p.kb_elems, -p.pad_l, r - p.pad_t, r * p.kw * p.cin_pad + cb * p.kb_elems);
+                continue;
+            }
+            const int tap = it / p.cblks, cb = it - tap * p.cblks;
+            const int r = tap / p.kw, sx = tap - r * p.kw;
+            int view = 0, dw, dh;
+            if (p.stride == 1) {
+                dw = sx - p.pad_l;
+                dh = r - p.pad_t;
+            } else {
+                const int ow_ = sx - p.pad_l, oh_ = r - p.pad_t;
+                const int pw = ow_ & 1, ph = oh_ & 1;
+                dw = (ow_ - pw) >> 1;
+                dh = (oh_ - ph) >> 1;
+                view = ph * 2 + pw;
+            }
+            k_tab[it] = make_int4(cb * p.kb_elems, dw, dh, (tap * p.cin_pad + cb * p.kb_elems) | (view << 28));
         }
-    }
-    for (int it = threadIdx.x; it < k_iters; it += kThreads) {
-        if (p.fold) {   // one K block per kernel row: the box starts at the output column itself
-            const int oh_ = it - p.pad_t;
-            const int ph = p.stride == 2 ? (oh_ & 1) : 0;
-            k_tab[it] = make_int4(0, 0, p.stride == 2 ? ((oh_ - ph) >> 1) : oh_, (it * p.kb_elems) | ((ph * 2) << 28));
-            continue;
+        __syncwarp();
+        if (kPair) ptx::cluster_wait();      // the peer's barriers are initialised before anything signals them
+    } else {
+        if (kPair) ptx::cluster_arrive();
+        if (warp == 1) {
+            if (kPair) {
+                ptx::tmem_alloc_pair(&tmem_base_smem, (uint32_t)p.tmem_cols);
+                ptx::tmem_relinquish_pair();
+            } else {
+                ptx::tmem_alloc(&tmem_base_smem, (uint32_t)p.tmem_cols);
+                ptx::tmem_relinquish();
+            }
         }
-        if (p.rowbox) {  // one unit per (kernel row, channel block): the box starts pad_l pixels left of the tile
-            const int r = it / p.cblks, cb = it - r * p.cblks;
-            k_tab[it] = make_int4(cb * p.kb_elems, -p.pad_l, r - p.pad_t, r * p.kw * p.cin_pad + cb * p.kb_elems);
-            continue;
+        if (p.patch && warp >= kFirstEpiWarp) {
+            // Weights into the un-swizzled canonical K-major layout: for kernel row r, 16-byte K
+            // chunk j, output channel n: r*(BN*64) + j*(BN*16) + (n/8)*128 + (n%8)*16.
+            const uint4* src = static_cast<const uint4*>(p.w_global);
+            const int total = p.kh * p.BN * 4;
+            for (int i = (int)threadIdx.x - 32 * kFirstEpiWarp; i < total; i += 32 * kEpiWarps) {
+                const int j = i & 3, n = (i >> 2) % p.BN, r = (i >> 2) / p.BN;
+                const uint4 v = n < p.cout_pad ? src[((size_t)n * p.kh + r) * 4 + j] : make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(smem_b + r * (p.BN * 64) + j * (p.BN * 16) + (n >> 3) * 128 + (n & 7) * 16) = v;
+            }
+            ptx::fence_proxy_async();   // generic-proxy writes, read by the tensor core through the async proxy
         }
-        const int tap = it / p.cblks, cb = it - tap * p.cblks;
-        const int r = tap / p.kw, sx = tap - r * p.kw;
-        int view = 0, dw, dh;
-        if (p.stride == 1) {
-            dw = sx - p.pad_l;
-            dh = r - p.pad_t;
-        } else {
-            const int ow_ = sx - p.pad_l, oh_ = r - p.pad_t;
-            const int pw = ow_ & 1, ph = oh_ & 1;
-            dw = (ow_ - pw) >> 1;
-            dh = (oh_ - ph) >> 1;
-            view = ph * 2 + pw;
+        if (warp >= kFirstEpiWarp) {
+            for (int c = (int)threadIdx.x - 32 * kFirstEpiWarp; c < p.n_tiles * p.BN; c += 32 * kEpiWarps) {
+                const bool in = c < p.cout_pad;
+                // quad epilogue: channel 32*b + 8*j + 4*i + k is kept at 32*b + 16*i + 4*j + k (see epi_quad_rows)
+                const int at = kEpi == kEpiQuad || kEpi == kEpiMapped ? quad_order(c) : c;
+                s_scale[at] = in ? p.e.scale[c] : 0.f;
+                s_bias[at] = in ? p.e.bias[c] : 0.f;
+            }
         }
-        k_tab[it] = make_int4(cb * p.kb_elems, dw, dh, (tap * p.cin_pad + cb * p.kb_elems) | (view << 28));
-    }
-    if (p.patch) {
-        // Weights into the un-swizzled canonical K-major layout: for kernel row r, 16-byte K
-        // chunk j, output channel n: r*(BN*64) + j*(BN*16) + (n/8)*128 + (n%8)*16.
-        const uint4* src = static_cast<const uint4*>(p.w_global);
-        const int total = p.kh * p.BN * 4;
-        for (int i = threadIdx.x; i < total; i += kThreads) {
-            const int j = i & 3, n = (i >> 2) % p.BN, r = (i >> 2) / p.BN;
-            const uint4 v = n < p.cout_pad ? src[((size_t)n * p.kh + r) * 4 + j] : make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4*>(smem_b + r * (p.BN * 64) + j * (p.BN * 16) + (n >> 3) * 128 + (n & 7) * 16) = v;
-        }
-        ptx::fence_proxy_async();   // generic-proxy writes, read by the tensor core through the async proxy
-    }
-    for (int c = threadIdx.x; c < p.n_tiles * p.BN; c += kThreads) {
-        const bool in = c < p.cout_pad;
-        // quad epilogue: channel 32*b + 8*j + 4*i + k is kept at 32*b + 16*i + 4*j + k (see epi_quad_rows)
-        const int at = kEpi == kEpiQuad || kEpi == kEpiMapped ? quad_order(c) : c;
-        s_scale[at] = in ? p.e.scale[c] : 0.f;
-        s_bias[at] = in ? p.e.bias[c] : 0.f;
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        // the issuing warp waits for the barriers only, unless the epilogue warps copied its weights
+        if (warp == 1 && !p.patch) asm volatile("bar.arrive 3, %0;" ::"n"(kThreads) : "memory");
+        else asm volatile("bar.sync 3, %0;" ::"n"(kThreads) : "memory");
+        if (warp == 1) asm volatile("bar.sync 4, 64;" ::: "memory");
+        if (kPair) ptx::cluster_wait();
+        ptx::tc_fence_after_sync();
     }
     // Programmatic dependent launch: everything up to a role's own griddepcontrol.wait touches only this launch's
     // parameters, constant weights and on-chip state, so it may run while the previous kernel of the stream is still
     // draining.  The producer waits before its first activation load, the epilogue before it reads or writes global
     // memory; the weights of the first stages (or all of them, resident) are on their way by then.
-    ptx::tc_fence_before_sync();
-    __syncthreads();
-    if (kPair) ptx::cluster_sync();      // the peer's barriers are initialised before anything signals them
-    ptx::tc_fence_after_sync();
-    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
+    const uint32_t tmem_base = warp == 0 ? 0u : __shfl_sync(0xffffffffu, tmem_base_smem, 0);
 
     if (warp == 0) {
         // ------------------------------- TMA producer --------------------------------------
@@ -382,29 +405,29 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
         const bool bres = p.b_resident != 0;
         const bool bperm = p.b_perm != 0;
         const uint32_t tx = (uint32_t)(p.a_tx_bytes + (bres ? 0 : p.taps * p.b_bytes));
-        if (bres && lane == 0) {
+        if (bres) {
             // Weights stay resident: the slice [BN x K] is loaded once (n_tiles == 1 here), one block per tap and
             // channel block in tap-major order (row-box mode: unit (r, cb) holds taps (r, 0..kw-1)).
             // pair mode: each CTA keeps its half of the rows; both halves complete on the rank-0 CTA's barrier
             const uint32_t rb = kPair ? ptx::map_to_cta(ptx::smem_u32(&bres_bar), 0) : ptx::smem_u32(&bres_bar);
-            if (!kPair || cta_rank == 0)
+            if (lane == 0 && (!kPair || cta_rank == 0))
                 ptx::mbar_arrive_expect_tx_u32(ptx::smem_u32(&bres_bar), (uint32_t)((kPair ? 2 : 1) * k_iters * p.taps * p.b_bytes));
             const int nrow = kPair ? (int)cta_rank * (p.BN >> 1) : 0;
-            for (int it = 0; it < k_iters; ++it) {
+            for (int i = lane; i < k_iters * p.taps; i += 32) {
+                const int it = i / p.taps, sx = i - it * p.taps;
                 const int r = it / p.cblks, cb = it - r * p.cblks;
-                for (int sx = 0; sx < p.taps; ++sx) {
-                    const int blk = p.rowbox ? (r * p.kw + sx) * p.cblks + cb : it;
-                    const uint32_t dst = ptx::smem_u32(smem_b) + (uint32_t)(blk * p.b_bytes);
-                    const int kc = (k_tab[it].w & 0x0fffffff) + sx * p.cin_pad;
-                    if (kPair) {
-                        if (bperm) ptx::tma_load_5d_pair(dst, mapB, rb, kc, 0, 0, 0, nrow >> 5);
-                        else ptx::tma_load_2d_pair(dst, mapB, rb, kc, nrow);
-                    } else {
-                        if (bperm) ptx::tma_load_5d_u32(dst, mapB, rb, kc, 0, 0, 0, 0);
-                        else ptx::tma_load_2d_u32(dst, mapB, rb, kc, 0);
-                    }
+                const int blk = p.rowbox ? (r * p.kw + sx) * p.cblks + cb : it;
+                const uint32_t dst = ptx::smem_u32(smem_b) + (uint32_t)(blk * p.b_bytes);
+                const int kc = (k_tab[it].w & 0x0fffffff) + sx * p.cin_pad;
+                if (kPair) {
+                    if (bperm) ptx::tma_load_5d_pair(dst, mapB, rb, kc, 0, 0, 0, nrow >> 5);
+                    else ptx::tma_load_2d_pair(dst, mapB, rb, kc, nrow);
+                } else {
+                    if (bperm) ptx::tma_load_5d_u32(dst, mapB, rb, kc, 0, 0, 0, 0);
+                    else ptx::tma_load_2d_u32(dst, mapB, rb, kc, 0);
                 }
             }
+            __syncwarp();
         }
         auto load_b = [&](uint32_t fb, int stage_, int w, int ncoord) {
             for (int sx = 0; sx < p.taps; ++sx) {
@@ -426,8 +449,9 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
         };
         // streamed weights: the first tile's, as far as the ring reaches
         int early = 0;
+        TileCursor cur(p, first_unit, unit_step);      // ahead of the wait for the previous kernel: eight divisions
         if (!p.patch && !bres && lane < G && first_unit < total_tiles) {
-            const int ncoord = tile_of(TileCursor(p, first_unit, unit_step)).ntile * p.BN + (kPair ? (int)cta_rank * (p.BN >> 1) : 0);
+            const int ncoord = cur.nt * p.BN + (kPair ? (int)cta_rank * (p.BN >> 1) : 0);
             for (int it0 = 0; it0 < k_iters && early < p.stages; it0 += G, ++early) {
                 const int nb = min(G, k_iters - it0);
                 expect(early, nb);
@@ -438,7 +462,6 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
         if (p.patch) {
             if (lane == 0) {
                 const uint32_t bytes = (uint32_t)(p.patch_rows * p.patch_pitch);
-                TileCursor cur(p, first_unit, unit_step);
                 for (int t = first_unit; t < total_tiles && ok; t += unit_step, cur.advance(p)) {
                     const TileCoord tc = tile_of(cur);
                     // Fused pooling: patch ring and accumulator ring have the same length and tile i uses slot i % length
@@ -467,7 +490,6 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                 if (!ok) ptx::give_up(p.error, 1);
             }
         } else if (lane < G) {
-            TileCursor cur(p, first_unit, unit_step);
             for (int t = first_unit; t < total_tiles && ok; t += unit_step, cur.advance(p)) {
                 const TileCoord tc = tile_of(cur);
                 // pair mode: this CTA loads its half of the N tile's weight rows
@@ -657,7 +679,6 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
         // Tile i of this CTA's sequence is accumulated in buffer i % acc_bufs (use number i / acc_bufs of that
         // buffer gives the barrier parity) and drained by group i % epi_groups.  A group has kEpiWarps /
         // epi_groups warps: one or two per TMEM lane quarter; two share the quarter's work.
-        pdl_wait();
         const int e = warp - kFirstEpiWarp;
         const int q = warp & 3;                 // TMEM lane quarter: a warp can only reach lanes 32*(warp%4)..+31
         const int nsub = kEpiWarps / 4 / p.epi_groups;
@@ -677,6 +698,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
             uint8_t* stg = pool_stage + grp * (kTileM * 128);
             volatile int* failed = &pool_fail[grp];
             TileCursor cur(p, first_unit + grp * unit_step, p.epi_groups * unit_step);
+            pdl_wait();
             for (int t = first_unit + grp * unit_step; t < total_tiles; t += p.epi_groups * unit_step, ti += p.epi_groups, cur.advance(p)) {
                 const TileCoord tc = tile_of(cur);
                 const int ow = tc.ow0 + tw, oh = tc.oh0 + th;
@@ -800,6 +822,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
             const bool want_res = p.has_res != 0;
             const int lean = kPrelu ? -1 : quad_variant(p.e, want_res);
             TileCursor cur(p, first_unit + grp * unit_step, p.epi_groups * unit_step);
+            pdl_wait();
             for (int t = first_unit + grp * unit_step; t < total_tiles && ok; t += p.epi_groups * unit_step, ti += p.epi_groups) {
                 const TileCoord tc = tile_of(cur);
                 cur.advance(p);            // from here on: this group's next tile
@@ -932,6 +955,7 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                               (p.e.y_pitch & 31) == 0 && ((n_chunks / nsub) & 1) == 0;
             const float lean_lo = p.e.act == EXB_ACT_RELU ? 0.f : -INFINITY;
             TileCursor cur(p, first_unit + grp * unit_step, p.epi_groups * unit_step);
+            pdl_wait();
             for (int t = first_unit + grp * unit_step; t < total_tiles && ok; t += p.epi_groups * unit_step, ti += p.epi_groups) {
                 const TileCoord tc = tile_of(cur);
                 cur.advance(p);            // from here on: this group's next tile
@@ -1417,6 +1441,10 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
         p.stages = p.acc_bufs;
     }
     p.epi_groups = two ? 2 : (p.acc_bufs >= 4 ? 4 : 2);
+    // One tile per CTA: nothing overlaps its epilogue, and two warps per lane quarter drain it in half the time.
+    const int units = p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;      // tiles, or pairs of them (clusters of two CTAs)
+    const int max_units = pair ? ctx->sm_count / 2 : ctx->sm_count * (two ? 2 : 1);
+    if (units <= max_units && p.BN % 64 == 0 && !p.pool) p.epi_groups = two ? 1 : 2;
     int cols = 32;
     while (cols < p.acc_bufs * p.BN) cols *= 2;
     p.tmem_cols = cols;
@@ -1455,8 +1483,6 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     p.b_perm = quad ? 1 : 0;
     if (int rc = encode_weights(g, w, p.kb_elems, sw, pair ? p.BN / 2 : p.BN, quad, &p.tmB)) return rc;
 
-    const int units = p.tiles_w * p.tiles_h * p.tiles_nb * p.n_tiles;      // tiles, or pairs of them (clusters of two CTAs)
-    const int max_units = pair ? ctx->sm_count / 2 : ctx->sm_count * (two ? 2 : 1);
     const int grid = (units < max_units ? units : max_units) * (pair ? 2 : 1);
     const size_t smem = (size_t)p.stages * p.kgroup * p.a_bytes + p.b_region + 1024 + epi_bytes;
     const bool prelu = p.e.act == EXB_ACT_PRELU;
