@@ -8,10 +8,12 @@
 namespace glasssix {
 namespace excalibur {
 
+constexpr double kBodyPower = 0.85;
+
 // The division of n images whose modelled time is shortest, or {n} where none promises 3 % and 20 us.  Copies to the
 // device, kernels and copies back are three lanes that run side by side; a sub-batch passes through them one after the
 // other.  in_us and out_us: the copies of the whole batch; the kernels of a share s of the images take
-// fixed_us + body_us * s^0.8 (small sub-batches fill the chip less).  Divisions are looked for among all ways to put 16
+// fixed_us + body_us * s^kBodyPower (small sub-batches fill the chip less).  Divisions are looked for among all ways to put 16
 // units together, n units of one image below 16 images, in at most eight parts.
 inline std::vector<int> divide_batch(int n, double in_us, double out_us, double fixed_us, double body_us) {
     constexpr int kUnits = 16, kParts = 8;
@@ -19,7 +21,7 @@ inline std::vector<int> divide_batch(int n, double in_us, double out_us, double 
     if (n < 2) return undivided;
     const int units = std::min(n, kUnits);
     double kernels[kUnits + 1];
-    for (int u = 0; u <= units; ++u) kernels[u] = fixed_us + body_us * std::pow(u / (double)units, 0.8);
+    for (int u = 0; u <= units; ++u) kernels[u] = fixed_us + body_us * std::pow(u / (double)units, kBodyPower);
     const double whole = in_us + kernels[units] + out_us;
     double best = std::min(0.97 * whole, whole - 20.0);
     std::vector<int> parts, best_parts;

@@ -1742,9 +1742,9 @@ double fused_plan::run_resident(int iters, bool use_graph) {
     return ms;
 }
 
-// How a forward is divided when the caller leaves it open (see divide_batch): kernels are taken as 4.6 us a launch and a
-// body from the plan's own traffic and arithmetic, within 15 % of the measured time of the benchmark networks from 4 images
-// on.  Copies move 53 GB/s.
+// How a forward is divided when the caller leaves it open (see divide_batch): kernels are taken as 23 us, 2.8 us a launch and a
+// body that grows with the 0.85th power of the plan's own traffic and arithmetic, on average within 4 % of 58 measured times of
+// the benchmark networks (1 to 256 images of the classifiers, 1 to 32 of the detectors).  Copies move 53 GB/s.
 std::vector<int> fused_plan::choose_slices(bool f16_src) {
     const program& prog = program_for({N_}, f16_src);
     if (N_ < 2) return {N_};
@@ -1759,8 +1759,8 @@ std::vector<int> fused_plan::choose_slices(bool f16_src) {
     }
     for (auto& kv : host_out_) out_bytes += 4.0 * kv.second->count();
     const double in_us = (double)N_ * C_ * H_ * W_ * (f16_src ? 2 : 4) / 53e3, out_us = out_bytes / 53e3;
-    const double fixed = 4.6 * prog.launches();
-    const double body = 2 * bytes / 4.5e6 + prog.flops_i8 / 1.2e9 + prog.flops_f16 / 0.6e9;
+    const double fixed = 23.0 + 2.78 * prog.launches();
+    const double body = std::pow(1.715 * bytes / 1e6 + 1.19 * prog.flops_i8 / 1e9 + 2.43 * prog.flops_f16 / 1e9, kBodyPower);
     return divide_batch(N_, in_us, out_us, fixed, body);
 }
 
