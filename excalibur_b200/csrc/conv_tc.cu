@@ -12,7 +12,7 @@
 // 18 warps for wider ones.
 //   warp 0   TMA producer (lane g issues K block g of a stage) - fills a ring of shared-memory stages
 //   warp 1   MMA issuer (uniform, one lane elected) + TMEM owner - tcgen05.mma, fp32 / int32 accumulators
-//                                                                 in as many TMEM buffers as fit (2-4)
+//                                                                 in as many TMEM buffers as fit (2-8)
 //   warps 2+ epilogue, in groups of four warps (one per TMEM     - tile i uses buffer i % buffers and
 //            lane quarter)                                        group i % groups
 //
@@ -71,7 +71,7 @@ struct ConvTcParams {
     int a_tx_bytes;         // bytes one A box delivers
     int tmem_cols;
     int acc_bufs;     // accumulator buffers in TMEM (2 to kMaxAccBufs)
-    int epi_groups;   // epilogue warp groups (2 or 4); group g drains tiles g, g + epi_groups, ... of the CTA
+    int epi_groups;   // epilogue warp groups (1, 2 or 4); group g drains tiles g, g + epi_groups, ... of the CTA
     int cout_pad;     // entries of the scale / bias arrays
     uint32_t idesc;
     int has_res;
@@ -228,7 +228,7 @@ __device__ __forceinline__ void rowbox_unit(uint32_t d_tmem, uint32_t a_lo, uint
     }
 }
 
-// kEpiWarps = 16: one CTA per SM (all of shared memory and TMEM, 2-4 accumulator buffers).
+// kEpiWarps = 16: one CTA per SM (all of shared memory and TMEM, 2-8 accumulator buffers).
 // kEpiWarps = 8:  two CTAs per SM for layers with narrow N tiles: two MMA issuers and two producers per SM;
 //                 each CTA takes half the shared memory and at most 256 TMEM columns.
 // kEpi: which epilogue (see the head of the file); each is its own instantiation so that the others keep
