@@ -1186,13 +1186,18 @@ ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64
     return t;
 }
 
-int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_conv_weights* w,
-                   const void* residual, void* y, void* y2, cudaStream_t st) {
-    auto encode = tensor_map_encoder();
-    if (!encode) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+// What a launch of the persistent kernel chooses beside its parameters.
+struct ConvTcForm {
+    bool two, pair, quad, patch, mapped;      // two CTAs per SM, CTA pairs, epilogue, stem on 8-byte pixels, mapped epilogue
+    FoldPlan fold;
+    int units, max_units;                     // tiles (or pairs of them) and how many run at a time
+    int epi_bytes;                            // shared memory of the tables
+};
+
+// Tiles, modes and shared memory of a launch: every parameter that does not depend on pointers.
+static int conv_tc_layout(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w, ConvTcParams& p, ConvTcForm& f) {
     const bool int8 = g.in_dtype == EXB_I8;
     const int es = int8 ? 1 : 2;
-    ConvTcParams p;
     memset(&p, 0, sizeof(p));
     p.N = g.N; p.OH = g.OH; p.OW = g.OW;
     {
@@ -1451,6 +1456,23 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     p.idesc = ptx::make_idesc(int8, pair ? 2 * kTileM : kTileM, (uint32_t)p.BN);
     p.cout_pad = w->cout_pad;
     p.has_res = g.has_res;
+    p.b_perm = quad ? 1 : 0;
+    f.two = two; f.pair = pair; f.quad = quad; f.patch = patch; f.mapped = mapped;
+    f.fold = fold;
+    f.units = units; f.max_units = max_units;
+    f.epi_bytes = epi_bytes;
+    return EXB_OK;
+}
+
+int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_conv_weights* w,
+                   const void* residual, void* y, void* y2, cudaStream_t st) {
+    auto encode = tensor_map_encoder();
+    if (!encode) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    const bool int8 = g.in_dtype == EXB_I8;
+    const int es = int8 ? 1 : 2;
+    ConvTcParams p;
+    ConvTcForm f;
+    if (int rc = conv_tc_layout(ctx, g, w, p, f)) return rc;
     p.e.scale = w->d_scale; p.e.bias = w->d_bias; p.e.slope = w->d_slope; p.e.residual = static_cast<const __half*>(residual);
     p.e.y = y; p.e.y2 = y2; p.e.out_dtype = g.out_dtype; p.e.out2_dtype = g.out2_dtype; p.e.act = g.act;
     p.e.out_scale = g.out_scale; p.e.out2_scale = g.out2_scale; p.e.cout_stride = g.cout_stride; p.e.y_pitch = g.y_pitch;
@@ -1466,51 +1488,50 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
     const CUtensorMapSwizzle sw = swizzle_for(p.kb_bytes);
     const size_t px_bytes = (size_t)g.cin_stride * es;
     const size_t row_pitch = (size_t)g.w_pitch * px_bytes;
-    if (patch) {
+    if (f.patch) {
         // One map: whole padded rows as the innermost dimension, box = 24 pixels x patch_rows.
         cuuint64_t dims[3] = {(cuuint64_t)g.w_pitch * g.cin_stride, (cuuint64_t)g.H, (cuuint64_t)g.N};
         cuuint64_t strides[2] = {(cuuint64_t)row_pitch, (cuuint64_t)g.H * row_pitch};
         cuuint32_t box[3] = {(cuuint32_t)(p.patch_pitch / es), (cuuint32_t)p.patch_rows, 1};
         cuuint32_t estr[3] = {1, 1, 1};
-        void* base = const_cast<char*>(static_cast<const char*>(x)) + (size_t)(g.w_pad - fold.pl_eff) * px_bytes;
+        void* base = const_cast<char*>(static_cast<const char*>(x)) + (size_t)(g.w_pad - f.fold.pl_eff) * px_bytes;
         CUresult r = encode(&p.tmA[0], dt, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled(patch) failed with %d", (int)r);
     }
-    if (!patch)
-        if (int rc = encode_input_views(g, fold, x, p.kb_elems, sw, p.rowbox ? p.TW + g.kw - 1 : p.TW, p.TH, p.TN, p.tmA)) return rc;
-    p.b_perm = quad ? 1 : 0;
-    if (int rc = encode_weights(g, w, p.kb_elems, sw, pair ? p.BN / 2 : p.BN, quad, &p.tmB)) return rc;
+    if (!f.patch)
+        if (int rc = encode_input_views(g, f.fold, x, p.kb_elems, sw, p.rowbox ? p.TW + g.kw - 1 : p.TW, p.TH, p.TN, p.tmA)) return rc;
+    if (int rc = encode_weights(g, w, p.kb_elems, sw, f.pair ? p.BN / 2 : p.BN, f.quad, &p.tmB)) return rc;
 
-    const int grid = (units < max_units ? units : max_units) * (pair ? 2 : 1);
-    const size_t smem = (size_t)p.stages * p.kgroup * p.a_bytes + p.b_region + 1024 + epi_bytes;
+    const int grid = (f.units < f.max_units ? f.units : f.max_units) * (f.pair ? 2 : 1);
+    const size_t smem = (size_t)p.stages * p.kgroup * p.a_bytes + p.b_region + 1024 + f.epi_bytes;
     const bool prelu = p.e.act == EXB_ACT_PRELU;
     void (*kern)(const ConvTcParams);
     if (p.pool) kern = conv_tc_kernel<false, 8, kEpiPool>;
-    else if (mapped)
-        kern = int8 ? (two ? conv_tc_kernel<true, 8, kEpiMapped> : conv_tc_kernel<true, 16, kEpiMapped>)
-                    : (two ? conv_tc_kernel<false, 8, kEpiMapped> : conv_tc_kernel<false, 16, kEpiMapped>);
-    else if (pair && !prelu)
-        kern = int8 ? (quad ? conv_tc_kernel<true, 16, kEpiQuad, false, true> : conv_tc_kernel<true, 16, kEpiRow, false, true>)
-                    : (quad ? conv_tc_kernel<false, 16, kEpiQuad, false, true> : conv_tc_kernel<false, 16, kEpiRow, false, true>);
-    else if (quad && !prelu)
-        kern = int8 ? (two ? conv_tc_kernel<true, 8, kEpiQuad> : conv_tc_kernel<true, 16, kEpiQuad>)
-                    : (two ? conv_tc_kernel<false, 8, kEpiQuad> : conv_tc_kernel<false, 16, kEpiQuad>);
-    else if (quad)
-        kern = int8 ? (two ? conv_tc_kernel<true, 8, kEpiQuad, true> : conv_tc_kernel<true, 16, kEpiQuad, true>)
-                    : (two ? conv_tc_kernel<false, 8, kEpiQuad, true> : conv_tc_kernel<false, 16, kEpiQuad, true>);
+    else if (f.mapped)
+        kern = int8 ? (f.two ? conv_tc_kernel<true, 8, kEpiMapped> : conv_tc_kernel<true, 16, kEpiMapped>)
+                    : (f.two ? conv_tc_kernel<false, 8, kEpiMapped> : conv_tc_kernel<false, 16, kEpiMapped>);
+    else if (f.pair && !prelu)
+        kern = int8 ? (f.quad ? conv_tc_kernel<true, 16, kEpiQuad, false, true> : conv_tc_kernel<true, 16, kEpiRow, false, true>)
+                    : (f.quad ? conv_tc_kernel<false, 16, kEpiQuad, false, true> : conv_tc_kernel<false, 16, kEpiRow, false, true>);
+    else if (f.quad && !prelu)
+        kern = int8 ? (f.two ? conv_tc_kernel<true, 8, kEpiQuad> : conv_tc_kernel<true, 16, kEpiQuad>)
+                    : (f.two ? conv_tc_kernel<false, 8, kEpiQuad> : conv_tc_kernel<false, 16, kEpiQuad>);
+    else if (f.quad)
+        kern = int8 ? (f.two ? conv_tc_kernel<true, 8, kEpiQuad, true> : conv_tc_kernel<true, 16, kEpiQuad, true>)
+                    : (f.two ? conv_tc_kernel<false, 8, kEpiQuad, true> : conv_tc_kernel<false, 16, kEpiQuad, true>);
     else if (!prelu)
-        kern = int8 ? (two ? conv_tc_kernel<true, 8, kEpiRow> : conv_tc_kernel<true, 16, kEpiRow>)
-                    : (two ? conv_tc_kernel<false, 8, kEpiRow> : conv_tc_kernel<false, 16, kEpiRow>);
+        kern = int8 ? (f.two ? conv_tc_kernel<true, 8, kEpiRow> : conv_tc_kernel<true, 16, kEpiRow>)
+                    : (f.two ? conv_tc_kernel<false, 8, kEpiRow> : conv_tc_kernel<false, 16, kEpiRow>);
     else
-        kern = int8 ? (two ? conv_tc_kernel<true, 8, kEpiRow, true> : conv_tc_kernel<true, 16, kEpiRow, true>)
-                    : (two ? conv_tc_kernel<false, 8, kEpiRow, true> : conv_tc_kernel<false, 16, kEpiRow, true>);
+        kern = int8 ? (f.two ? conv_tc_kernel<true, 8, kEpiRow, true> : conv_tc_kernel<true, 16, kEpiRow, true>)
+                    : (f.two ? conv_tc_kernel<false, 8, kEpiRow, true> : conv_tc_kernel<false, 16, kEpiRow, true>);
     if (int rc = raise_smem_limit(ctx, kern)) return rc;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)((kFirstEpiWarp + (two ? 8 : 16)) * 32));
+    cfg.blockDim = dim3((unsigned)((kFirstEpiWarp + (f.two ? 8 : 16)) * 32));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -1520,7 +1541,7 @@ int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_con
         attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
         ++n_attr;
     }
-    if (pair) {
+    if (f.pair) {
         attr[n_attr].id = cudaLaunchAttributeClusterDimension;
         attr[n_attr].val.clusterDim.x = 2;
         attr[n_attr].val.clusterDim.y = 1;
