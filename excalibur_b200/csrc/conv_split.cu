@@ -447,15 +447,45 @@ __global__ void __launch_bounds__(kSplitThreads) conv_split_kernel(const __grid_
 
 }  // namespace
 
-// Which kernel, and how a tile is divided: modelled time in us of both kernels in a captured chain, fitted to 590 layers (batch
-// 1 to 256, 1x1 and 3x3, 16 to 1024 -> 16 to 1280 channels, maps of 4 x 4 to 80 x 80; every split of 32 and 64 channels).
-// Split kernel: a constant, what the exchange costs by the number of parts and by the bytes a CTA receives, then K blocks and
-// epilogue of a tile one after the other, stretched by the tiles per SM once there are more than SMs.  Persistent kernel: a
-// constant and rounds of tiles.  The constants are regression weights, not times of parts.  On those layers the pick is 2 %
-// slower than the fastest of all of them on average and 5 % or more slower in one of eight (at worst 68 %: 304 -> 288 fp16 3x3
-// stride 2 at 31 x 13 x 14).  Against the kernels with parts summed out of the other CTAs' shared memory, and their constants, 220
-// of the layers took 0.83 of the time on average.
-ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
+// Shared memory of a launch.
+struct SplitRing {
+    int stages, a_bytes, b_bytes;
+    int part;      // of all CTAs of a cluster for one's slice
+};
+static SplitRing split_ring(const exb_ctx* ctx, int rows, int kb_bytes, int bn, int splits, int k_iters, int grid) {
+    SplitRing r;
+    r.a_bytes = round_up(rows * kb_bytes, 1024);      // the MMA reads 128 rows whatever the box holds: unused ones from what follows
+    r.b_bytes = bn * kb_bytes;
+    r.part = splits == 1 ? 0 : (rows + splits - 1) / splits * splits * (bn * 4 + 16);
+    // two CTAs of neighbouring launches fit an SM side by side (programmatic launch): half of the shared memory each, and all
+    // of it where the neighbours find SMs of their own
+    const int room = 2 * grid <= ctx->sm_count ? ctx->smem_optin - 6 * 1024 : 109 * 1024;
+    const int units = (k_iters + splits - 1) / splits;
+    r.stages = (room - (kTileM * kb_bytes - r.a_bytes) - r.part) / (r.a_bytes + r.b_bytes);
+    if (r.stages > kSplitStages) r.stages = kSplitStages;
+    if (r.stages > units) r.stages = units;
+    return r;
+}
+
+// Which kernel, and how a tile is divided: modelled time in us of both kernels, fitted to 1200 layers (batch 1 to 256, 1x1 and
+// 3x3, 16 to 1280 -> 16 to 1280 channels, maps of 4 x 4 to 160 x 160, those of the benchmark networks among them; every split of
+// 32 and 64 channels).  A layer's time is the mean of two measurements, a captured chain of its own launches and one in which
+// they alternate with another layer's: the persistent kernel loses 1.2 to 1.6 us between launches of other kernels,
+// the split kernel 0 to 0.5.  The constants are regression weights, not times of parts.
+//  - Split kernel: a constant, what the exchange costs by the number of parts, the chain of a CTA (K blocks, of which those that
+//    the ring does not hold wait for their loads, the epilogue, the volume of the exchange) and, beyond one CTA per SM, what they
+//    take from each other.  Two run side by side on an SM, fewer where clusters of four and eight do not fill the SMs that
+//    are wired together (at 1.9 and 1.8 per SM times jump by half); beyond that the chain is walked once more.
+//  - Persistent kernel: conv_tc_time, from the layout that its launch would have (row boxes, resident weights, pairs).
+// Up to one CTA per SM a division's time depends on K and the N tile alone, not on the pixels: a small call gives an fp16
+// result of the same bits whether its images come in one batch or in several (a cost by the pixels of a box and the fill of
+// the chip would pick 0.5 % better on average).  Parts of one K block are left out for the same end: of 304 drawn layers they
+// were the fastest choice of twelve, by 2 to 10 %, each of a few small maps.
+// On 600 layers outside the fit the pick is 1.7 % slower than the fastest of all of them on average and 5 % or more slower in
+// one of eight, at worst 37 %.  A model by N tile alone, with CTAs beyond one per SM as a common factor, was 3.5 %, one of five
+// and 101 % off: 512 -> 32 fp16 3x3 at 5 x 56 x 56 ran undivided in 21.7 us (in two parts 14.9), 288 -> 192 int8 3x3 stride 2 at
+// 8 x 56 x 56 in 23.5 (15.8).
+static ConvSplit search_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
     const ConvSplit none = {0, 0, 0, 0, 0};
     if (g.pool || g.out_dtype == EXB_I32 || (g.cout_stride & 7) || (g.y_pitch & 7) || conv_fold_plan(g).on) return none;
     const int row_bytes = g.cin_stride * (g.in_dtype == EXB_I8 ? 1 : 2);
@@ -466,44 +496,50 @@ ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
     if (m_tiles > 8.0 * ctx->sm_count) return none;
     ConvSplit best = {0, 0, box.TW, box.TH, box.TN};
     double best_t = 1e30;
-    static const double kParts[4] = {0.0, 1.0, 0.53, 0.46};      // an exchange of 1, 2, 4, 8 parts beside its volume
-    const double unit = kb == 128 ? 0.218 : kb == 64 ? 0.209 : 0.192;
+    static const double kParts[4] = {0.0, 1.347, 0.899, 1.002};      // an exchange of 1, 2, 4, 8 parts beside its volume
+    static const double kPlaces[4] = {2.0, 2.0, 1.9, 1.8};           // CTAs per SM of one wave
+    const double unit = kb == 128 ? 0.1487 : kb == 64 ? 0.1923 : 0.1965, shared = kb == 128 ? 0.0679 : kb == 64 ? 0.0343 : 0.0341;
     for (int bn = 32; bn <= 64; bn *= 2)
         for (int sp = 1, i = 0; sp <= kSplitMaxParts && (sp == 1 || 2 * sp <= k_iters); sp *= 2, ++i) {      // two K blocks a part
-            const double ctas = m_tiles * ((w->cout_pad + bn - 1) / bn) * sp;
-            const double stretch = ctas > 1.02 * ctx->sm_count ? ctas / (1.02 * ctx->sm_count) : 1.0;
-            const double units = (k_iters + sp - 1) / sp;
-            const double volume = box.TW * box.TH * box.TN * bn * (sp - 1) / (sp * 8192.0);
-            const double t = 0.8 + kParts[i] + 1.29 * volume +
-                             stretch * (units * unit * (bn == 32 ? 0.962 : 1.0) + (bn == 32 ? 1.40 : 1.52) + 1.31 * volume - (sp > 1 ? 0.36 : 0.0));
+            const double per_sm = m_tiles * ((w->cout_pad + bn - 1) / bn) * sp / ctx->sm_count, full = per_sm / kPlaces[i];
+            const int units = (k_iters + sp - 1) / sp, stages = split_ring(ctx, kTileM, kb, bn, sp, k_iters, ctx->sm_count).stages;
+            const double epi = (bn == 32 ? 0.696 : 0.915) + 0.670 * bn * (sp - 1) / (sp * 64.0);
+            const double chain = units * unit + 0.445 * (units - stages) / stages + epi;
+            const double t = 1.663 + kParts[i] + chain * (full <= 1 ? 1.0 : 0.116 * full + 0.884 * ceil(full)) +
+                             (per_sm > 1 ? per_sm - 1 : 0.0) * (units * shared * (bn == 32 ? 1.105 : 1.0) + 1.548 * epi);
             if (t < best_t) {
                 best_t = t;
                 best.BN = bn;
                 best.splits = sp;
             }
         }
-    const ConvNTile nt = conv_n_tile(ctx, g, w->cout_pad, (int64_t)m_tiles);
-    const int bn = nt.BN;
-    const bool two = bn <= 128 && !nt.paired;
-    const double tiles = m_tiles * nt.n_tiles, slots = (double)ctx->sm_count * (two ? 2 : 1);
-    const double rounds = tiles <= slots ? 1.0 : ceil(tiles / slots);
-    double share = 1.0;      // two CTAs of an SM share its tensor pipe
-    if (two && tiles > ctx->sm_count) share += 0.35 * (tiles < 2 * ctx->sm_count ? tiles / ctx->sm_count - 1 : 1.0);
-    double step = 0.292, rest = 1.45;       // one CTA (or pair) per SM, more than 128 channels
-    if (two) {
-        step = bn <= 64 ? 0.216 : 0.304;
-        rest = bn <= 64 ? 0.0 : 1.09;
-    } else if (nt.paired) {
-        step = 0.207;
-        rest = 1.71;
+    return best_t < 0.98 * conv_tc_time(ctx, g, w) ? best : none;      // near a tie the kernel that does not divide
+}
+
+// The same, searched once per layer and thread (0.2 us of every eager call): a pure function of the values that are compared,
+// and the last layer that fell into each of 64 slots is kept.
+ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
+    struct Layer {
+        ConvGeom g;
+        int cout_pad, cin_pad, kw_pack, sm_count, smem_optin;
+    };
+    struct Kept {
+        Layer layer;
+        ConvSplit plan;
+        bool used;
+    };
+    static thread_local Kept kept[64];
+    static_assert(sizeof(Layer) == sizeof(ConvGeom) + 5 * sizeof(int) && sizeof(ConvGeom) % sizeof(int) == 0, "compared by its bytes");
+    const Layer layer = {g, w->cout_pad, w->cin_pad, w->kw_pack, ctx->sm_count, ctx->smem_optin};
+    uint32_t h = 2166136261u;
+    for (int v : {g.N, g.OH, g.OW, g.cin_stride, w->cout_pad, g.kh, g.has_res}) h = (h ^ (uint32_t)v) * 16777619u;
+    Kept& k = kept[(h ^ (h >> 16)) & 63u];
+    if (!k.used || memcmp(&k.layer, &layer, sizeof(Layer)) != 0) {
+        k.plan = search_split_plan(ctx, g, w);
+        memcpy(&k.layer, &layer, sizeof(Layer));
+        k.used = true;
     }
-    step *= kb == 128 ? 1.0 : kb == 64 ? 0.65 : 0.56;
-    double body = rounds * (k_iters * step + rest + (g.has_res ? 1.5 : 0.0)) * share;
-    // int8 tiles of a short K, more of them than fit the SMs as clusters; an int8 result alone has a loop of its own in the row
-    // epilogue (96 -> 320 1x1 at 8 x 40 x 40: int8 7.8 us, undivided tiles of this kernel 7.6; fp16 8.3 and 7.6)
-    if (two && g.in_dtype == EXB_I8 && k_iters * kb <= 256 && m_tiles * ((w->cout_pad + 63) / 64) > ctx->sm_count)
-        body *= g.out_dtype == EXB_I8 && g.out2_dtype < 0 ? 0.8 : 1.28;
-    return best_t < 3.92 + body ? best : none;
+    return k.plan;
 }
 
 int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, const void* x, const exb_conv_weights* w, const void* residual,
@@ -530,19 +566,13 @@ int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, cons
     p.rows = p.TW * p.TH * p.TN;
     p.slice = (p.rows + p.splits - 1) / p.splits;
     p.a_tx_bytes = p.TW * p.TH * p.TN * p.kb_bytes;
-    p.a_bytes = round_up(p.a_tx_bytes, 1024);      // the MMA reads 128 rows whatever the box holds: unused ones from what follows
-    p.b_bytes = p.BN * p.kb_bytes;
-    const int overread = kTileM * p.kb_bytes - p.a_bytes;
-    const int units = (p.k_iters + p.splits - 1) / p.splits;
     const bool direct = p.splits == 1;
     const int grid = p.tiles_w * p.tiles_h * tiles_nb * p.n_tiles * p.splits;
-    const int part = p.slice * p.splits * (p.BN * 4 + 16);      // of all CTAs of a cluster for one's slice
-    // two CTAs of neighbouring launches fit an SM side by side (programmatic launch): half of the shared memory each, and all
-    // of it where the neighbours find SMs of their own
-    const int room = 2 * grid <= ctx->sm_count ? ctx->smem_optin - 6 * 1024 : 109 * 1024;
-    p.stages = (room - overread - (direct ? 0 : part)) / (p.a_bytes + p.b_bytes);
-    if (p.stages > kSplitStages) p.stages = kSplitStages;
-    if (p.stages > units) p.stages = units;
+    const SplitRing ring = split_ring(ctx, p.rows, p.kb_bytes, p.BN, p.splits, p.k_iters, grid);
+    p.stages = ring.stages;
+    p.a_bytes = ring.a_bytes;
+    p.b_bytes = ring.b_bytes;
+    const int overread = kTileM * p.kb_bytes - p.a_bytes;
     p.tmem_cols = p.BN <= 32 ? 32 : 64;
     p.cout_pad = w->cout_pad;
     p.has_res = g.has_res;
@@ -558,9 +588,9 @@ int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, cons
     if (int rc = encode_weights(g, w, p.kb_elems, sw, p.BN, direct, &p.tmB)) return rc;
     size_t smem = (size_t)p.stages * (p.a_bytes + p.b_bytes) + (overread > p.b_bytes ? overread - p.b_bytes : 0);
     if (!direct) {
-        if (smem < (size_t)part) smem = part;      // the box's rows take the ring's place
+        if (smem < (size_t)ring.part) smem = ring.part;      // the box's rows take the ring's place
         p.recv = (int)((smem + 15) / 16 * 16);
-        smem = (size_t)p.recv + part;
+        smem = (size_t)p.recv + ring.part;
     }
     smem += 1024;
     const bool prelu = g.act == EXB_ACT_PRELU;

@@ -35,6 +35,8 @@
 // per-channel PReLU activation.
 // All mbarrier waits are bounded; when one runs out the kernel raises the context's error
 // word, every role leaves its loop, TMEM is freed and the launch returns normally.
+#include <math.h>
+
 #include "conv_tc_host.cuh"
 #include "conv_quad.cuh"
 #include "ptx_sm100.cuh"
@@ -1149,6 +1151,12 @@ static bool conv_pairable(const exb_ctx* ctx, const ConvGeom& g) {
     return ctx->sm_count >= 2 && g.act != EXB_ACT_PRELU && !g.res_half && g.rh * g.rw == 1 && !g.pool && !conv_fold_plan(g).on;
 }
 
+// N tiles: how many, of how many channels, and whether they were chosen to run as CTA pairs.
+struct ConvNTile {
+    int n_tiles, BN;
+    bool paired;
+};
+
 // The N tile: 256 channels, or 128 where that is the faster one.
 //  - Below 512 bytes of K, and up to 1152 in the first round of tiles (two of them for two N tiles), the epilogue sets the
 //    pace, and two CTAs of 128 channels per SM drain more than one of 256: 96 -> 576 int8 1x1 at 256 x 14 x 14 23.8 ->
@@ -1162,7 +1170,7 @@ static bool conv_pairable(const exb_ctx* ctx, const ConvGeom& g) {
 //    of one of 256 (half the MMA time, but the same activations): 128 where its rounds of pairs come to less.
 //    512 -> 512 3x3 fp16 at 64 x 7 x 7: 26 pairs of 256 on 74 places 30.9 us, 52 of 128 24.0; 256 -> 256 int8 at
 //    100 x 14 x 14: two rounds 21.8, three of 128 19.4; 256 -> 256 fp16 at 64 x 14 x 14: one round 22.3, two of 128 23.5.
-ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64_t m_tiles) {
+static ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64_t m_tiles) {
     auto tile = [&](int most) {
         const int n = (cout_pad + most - 1) / most;
         return ConvNTile{n, round_up((cout_pad + n - 1) / n, 16), false};
@@ -1462,6 +1470,38 @@ static int conv_tc_layout(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
     f.units = units; f.max_units = max_units;
     f.epi_bytes = epi_bytes;
     return EXB_OK;
+}
+
+// Modelled time of a launch in us (see search_split_plan): a constant; for every round of tiles a chain of K blocks, of which
+// those that the ring does not hold wait for their loads; and what each tile takes from its SM (operand bytes, values of the
+// epilogue).  A layout that cannot be launched takes for ever.
+double conv_tc_time(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
+    ConvTcParams p;
+    ConvTcForm f;
+    if (conv_tc_layout(ctx, g, w, p, f) != EXB_OK) return 1e30;
+    auto size_of = [](int dtype) { return dtype == EXB_I8 ? 1 : dtype == EXB_F16 ? 2 : 4; };
+    const int out_bytes = size_of(g.out_dtype) + (g.out2_dtype >= 0 ? size_of(g.out2_dtype) : 0);
+    const bool lone_i8 = g.in_dtype == EXB_I8 && out_bytes == 1;
+    const bool with_more = g.has_res || g.out2_dtype >= 0;      // beside ReLU6 and the like: the general quad epilogue
+    const bool lean = g.act == EXB_ACT_NONE || g.act == EXB_ACT_RELU || !with_more;
+    const double form = f.quad ? (lean ? 1.0 : 1.336) : lone_i8 ? 2.826 : 1.507;
+    const double epi = 1e-2 * p.BN * (0.323 * out_bytes + (g.has_res ? 0.357 : 0.0)) * form;
+    const int ring = p.stages * p.kgroup;
+    const double block = (p.kb_bytes == 128 ? 0.0810 : p.kb_bytes == 64 ? 0.1075 : 0.1193) * (p.rowbox ? 0.802 * p.taps : 1.0);
+    const double sms = (double)f.units * (f.pair ? 2 : 1) / ctx->sm_count;
+    const double wait = 0.303 + 0.552 * (sms < 1 ? sms : 1.0);      // a load's, longer the more of the chip loads
+    const double chain = p.k_iters * block + (p.k_iters > ring ? wait * (p.k_iters - ring) / ring : 0.0);
+    const double kbytes = p.k_iters / 1024.0 * (p.a_bytes + (p.b_resident ? 0 : p.taps * p.b_bytes));
+    const double full = (double)f.units / f.max_units;
+    const double rounds = full <= 1 ? 1.0 : 0.425 * full + 0.575 * ceil(full);
+    const double per_sm = ceil((double)f.units / (f.pair ? f.max_units : ctx->sm_count));
+    const double t = (f.two ? 3.977 : f.pair ? 3.852 : 3.086) + rounds * (chain + 0.615 * epi) + per_sm * (0.0025 * kbytes + epi);
+    // Short int8 reductions with an int8 result alone have a loop of their own in the row epilogue, which pays where launches
+    // like them follow each other: 96 -> 320 1x1 at 8 x 40 x 40 7.1 us, undivided tiles of the split kernel 7.6 (between launches of
+    // other layers 9.1 and 7.9).
+    if (!f.two || !lone_i8 || p.k_iters * p.kb_bytes > 256) return t;
+    const double more = f.units * (p.BN / 64.0) / ctx->sm_count - 1.0;
+    return t * (1.0 - 0.2 * (more < 0.0 ? 0.0 : more < 1.0 ? more : 1.0));
 }
 
 int conv_tc_launch(exb_ctx* ctx, const ConvGeom& g, const void* x, const exb_conv_weights* w,

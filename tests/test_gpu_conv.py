@@ -643,6 +643,30 @@ def test_short_int8_reductions_are_divided_only_when_few(ctx, case, split):
     assert len(names) == 1 and ("conv_split_kernel" in names[0]) == split, names
 
 
+# Reductions that are divided although undivided tiles would just fit the SMs: 512 -> 32 3x3 at 5 x 56 x 56 takes 14.9 us in
+# two parts and 21.7 undivided, 304 -> 288 stride 2 at 31 x 13 x 14 16.6 in four and 27.8 in two, 288 -> 192 int8 stride 2 at
+# 8 x 56 x 56 15.8 in two and 23.5 undivided.
+@pytest.mark.parametrize("case,i8,kernel,ctas", [((5, 512, 56, 56, 32, 3, 1), False, "conv_split_kernel<false, false, false>", 266),
+                                                 ((31, 304, 13, 14, 288, 3, 2), False, "conv_split_kernel<false, false, false>", 280),
+                                                 ((8, 288, 56, 56, 192, 3, 2), True, "conv_split_kernel<true, false, false>", 294)])
+def test_long_reductions_of_one_tile_per_sm(ctx, case, i8, kernel, ctas):
+    import torch
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s = case
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8 if i8 else capi.EXB_F16, capi.EXB_F16, impl=0)
+    r = rng(sum(case))
+    wq = r.integers(-4, 5, (Cout, Cin, k, k)).astype(np.int8)
+    x = r.integers(-2, 3, (N, H, W, Cin)).astype(np.int8)
+    p = capi.ConvWeights(ctx, d, wq, None, np.ones(Cout, np.float32), 1.0) if i8 else capi.ConvWeights(ctx, d, wq.astype(np.float32))
+    xd = dev(x if i8 else x.astype(np.float16))
+    launches = [l for l in kernels_of(lambda: capi.conv2d(ctx, d, xd, p)) if "conv_" in l[0]]
+    assert len(launches) == 1 and kernel in launches[0][0] and launches[0][1][0] == ctas, launches
+    y, _ = capi.conv2d(ctx, d, xd, p)
+    ctx.sync_check()
+    want = O.conv2d_i8_acc(x[-1:].transpose(0, 3, 1, 2), wq, s, k // 2)[0].astype(np.float16)
+    np.testing.assert_array_equal(host(y[-1]).transpose(2, 0, 1), want)
+
+
 # The lean quad epilogue (fp16 result, alone or with an int8 copy) against the same kernel's fp32 result, which is read from the
 # general form: whole-number operands, so the sums are exact whatever their order, and scale, bias, residual, activation and
 # rounding are repeated here in the same fp32 steps.  N tiles of one, two, three and five blocks, a tile that ends inside its
