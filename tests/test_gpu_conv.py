@@ -669,15 +669,23 @@ def test_long_reductions_of_one_tile_per_sm(ctx, case, i8, kernel, ctas):
 
 # The lean quad epilogue (fp16 result, alone or with an int8 copy) against the same kernel's fp32 result, which is read from the
 # general form: whole-number operands, so the sums are exact whatever their order, and scale, bias, residual, activation and
-# rounding are repeated here in the same fp32 steps.  N tiles of one, two, three and five blocks, a tile that ends inside its
-# last block, one CTA per SM and two, pairs, three and eight accumulators in flight; infinities and NaN.
-LEAN_CASES = [(5, 32, 17, 13, 32, 1, 1), (3, 64, 9, 7, 72, 1, 1), (2, 32, 11, 13, 160, 1, 1), (40, 64, 28, 28, 96, 1, 1), (3, 96, 8, 8, 64, 3, 2),
-              (50, 64, 24, 24, 64, 3, 1), (9, 32, 30, 30, 320, 1, 1)]
+# rounding are repeated here in the same fp32 steps; infinities and NaN.  With each case the kernel that it is there for, fp16 and
+# int8: epilogue warps, q(uad) or r(ow) epilogue, p(airs).
+LEAN_CASES = [((5, 32, 17, 13, 32, 1, 1), "8q", "8q"), ((3, 64, 9, 7, 72, 1, 1), "8r", "8r"), ((2, 32, 11, 13, 160, 1, 1), "16q", "16q"),
+              ((40, 64, 28, 28, 96, 1, 1), "8q", "8q"), ((3, 96, 8, 8, 64, 3, 2), "8q", "8q"), ((50, 64, 24, 24, 64, 3, 1), "8q", "8q"),
+              ((9, 32, 30, 30, 320, 1, 1), "16q", "8r"),
+              # channels that end inside the last block
+              ((5, 32, 17, 13, 24, 1, 1), "8q", "8q"), ((3, 64, 9, 7, 56, 1, 1), "8q", "8q"), ((5, 64, 12, 9, 88, 3, 1), "8q", "8q"),
+              # more tiles per CTA than its eight, three and four accumulators
+              ((100, 32, 56, 56, 32, 1, 1), "8q", "8q"), ((19, 32, 56, 56, 160, 1, 1), "16q", "16q"), ((50, 64, 56, 56, 64, 1, 1), "8q", "8q"),
+              # pairs: row boxes, tap loop, one and several tiles each
+              ((50, 128, 28, 28, 64, 3, 1), "16qp", "16qp"), ((3, 64, 15, 15, 128, 3, 1), "16qp", "16qp"), ((2, 128, 9, 9, 384, 3, 1), "16qp", "8q"),
+              ((40, 256, 14, 14, 512, 3, 1), "16qp", "16qp")]
 
 
 @pytest.mark.parametrize("i8", [True, False])
-@pytest.mark.parametrize("case", LEAN_CASES)
-def test_lean_quad_epilogue(ctx, case, i8):
+@pytest.mark.parametrize("case,f16_kernel,i8_kernel", LEAN_CASES)
+def test_lean_quad_epilogue(ctx, case, f16_kernel, i8_kernel, i8):
     import torch
     capi = _capi()
     N, Cin, H, W, Cout, k, s = case
@@ -698,6 +706,9 @@ def test_lean_quad_epilogue(ctx, case, i8):
     v = capi.conv2d(ctx, d0, xd, p)[0]
     oh, ow = capi.conv_out_dims(d0)
     skip = dev(r.standard_normal((N, oh, ow, Cout)).astype(np.float16))
+    name = [n for n, _, _ in kernels_of(lambda: capi.conv2d(ctx, desc(capi.EXB_F16, -1, 1, False), xd, p)) if "conv_" in n][0]
+    warps, epi, pair = re.search(r"conv_tc_kernel<\w+, (\d+), \D*(\d), \w+, (\w+)>", name).groups()
+    assert warps + {"0": "r", "1": "q"}[epi] + ("p" if pair == "true" else "") == (i8_kernel if i8 else f16_kernel), name
     for act in (0, 1, 103, 104):
         for res in (False, True):
             for out2 in (-1, capi.EXB_I8):
@@ -730,7 +741,8 @@ def test_split_tiles_of_few_pixels(ctx, case, i8):
     capi = _capi()
     N, Cin, H, W, Cout, k, s = case
     names = _route(ctx, case, i8, capi.EXB_I8 if i8 else capi.EXB_F16, 0)
-    assert len(names) == 1 and "conv_split_kernel" in names[0], names
+    undivided = "true" if Cin * k * k <= 64 else "false"
+    assert len(names) == 1 and re.search(r"conv_split_kernel<\w+, \w+, %s>" % undivided, names[0]), names
     r = rng(sum(case) + i8)
     wq = r.integers(-4, 5, (Cout, Cin, k, k)).astype(np.int8)
     x = dev(r.integers(-4, 5, (N, H, W, Cin)).astype(np.int8 if i8 else np.float16))
@@ -745,3 +757,49 @@ def test_split_tiles_of_few_pixels(ctx, case, i8):
         ctx.sync_check()
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+# Undivided tiles, which go from TMEM to the result in a loop of their own: every activation, residual and output against the
+# persistent kernel on whole-number operands.  Channel counts with and without whole 32-channel blocks, N tiles beyond the first,
+# boxes of fewer pixels than a tile has rows; int8 alone behind a residual and no activation, PReLU and fp32 take the general form.
+DIRECT_CASES = [(15, 32, 11, 11, 176, 1, 2), (1, 64, 12, 10, 256, 1, 1), (3, 64, 6, 4, 72, 1, 1), (40, 128, 14, 14, 96, 1, 1)]
+
+
+@pytest.mark.parametrize("i8", [True, False])
+@pytest.mark.parametrize("case", DIRECT_CASES)
+def test_split_undivided_tiles(ctx, case, i8):
+    import torch
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s = case
+    r = rng(sum(case) + i8)
+    wq = r.integers(-3, 4, (Cout, Cin, k, k)).astype(np.int8)
+    bias = r.integers(-40, 40, Cout).astype(np.float32) / 8
+    x = dev(r.integers(-4, 5, (N, H, W, Cin)).astype(np.int8 if i8 else np.float16))
+    slopes = r.integers(1, 8, Cout).astype(np.float32) / 8
+
+    def desc(out, out2, act, res, impl):
+        d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8 if i8 else capi.EXB_F16, out, out2, res=res != 0, act=act,
+                                out_scale=0.7, out2_scale=0.3, impl=impl)
+        d.res_half = int(res == 2)
+        return d
+    d0 = desc(capi.EXB_F16, -1, 0, 0, 0)
+    p = capi.ConvWeights(ctx, d0, wq, bias, np.exp2(r.integers(2, 6, Cout)).astype(np.float32), 0.25) if i8 else \
+        capi.ConvWeights(ctx, d0, wq.astype(np.float32), bias)
+    p.set_slopes(ctx, slopes)
+    oh, ow = capi.conv_out_dims(d0)
+    full = dev(r.standard_normal((N, oh, ow, Cout)).astype(np.float16))
+    half = dev(r.standard_normal((N, oh // 2, ow // 2, Cout)).astype(np.float16))
+    halves = oh % 2 == 0 and ow % 2 == 0 and Cout % 32 == 0
+    for act in (0, 1, 103, 104, capi.ACT_PRELU):
+        for res in (0, 1, 2) if halves else (0, 1):
+            for out, out2 in ((capi.EXB_F16, -1), (capi.EXB_F16, capi.EXB_I8), (capi.EXB_I8, -1), (capi.EXB_F32, -1)):
+                if res == 2 and (out == capi.EXB_I8 or act == capi.ACT_PRELU):
+                    continue
+                run = lambda impl: capi.conv2d(ctx, desc(out, out2, act, res, impl), x, p, residual=(None, full, half)[res])
+                if out == capi.EXB_F16:
+                    names = [n for n, _, _ in kernels_of(lambda: run(0)) if "conv_" in n]
+                    assert len(names) == 1 and re.search(r"conv_split_kernel<\w+, \w+, true>", names[0]), names
+                (a, a2), (b, b2) = run(0), run(2)
+                assert torch.equal(a, b), (act, res, out, out2)
+                assert a2 is None or torch.equal(a2, b2), (act, res, out, out2)
+    ctx.sync_check()
