@@ -669,23 +669,15 @@ def test_long_reductions_of_one_tile_per_sm(ctx, case, i8, kernel, ctas):
 
 # The lean quad epilogue (fp16 result, alone or with an int8 copy) against the same kernel's fp32 result, which is read from the
 # general form: whole-number operands, so the sums are exact whatever their order, and scale, bias, residual, activation and
-# rounding are repeated here in the same fp32 steps; infinities and NaN.  With each case the kernel that it is there for, fp16 and
-# int8: epilogue warps, q(uad) or r(ow) epilogue, p(airs).
-LEAN_CASES = [((5, 32, 17, 13, 32, 1, 1), "8q", "8q"), ((3, 64, 9, 7, 72, 1, 1), "8r", "8r"), ((2, 32, 11, 13, 160, 1, 1), "16q", "16q"),
-              ((40, 64, 28, 28, 96, 1, 1), "8q", "8q"), ((3, 96, 8, 8, 64, 3, 2), "8q", "8q"), ((50, 64, 24, 24, 64, 3, 1), "8q", "8q"),
-              ((9, 32, 30, 30, 320, 1, 1), "16q", "8r"),
-              # channels that end inside the last block
-              ((5, 32, 17, 13, 24, 1, 1), "8q", "8q"), ((3, 64, 9, 7, 56, 1, 1), "8q", "8q"), ((5, 64, 12, 9, 88, 3, 1), "8q", "8q"),
-              # more tiles per CTA than its eight, three and four accumulators
-              ((100, 32, 56, 56, 32, 1, 1), "8q", "8q"), ((19, 32, 56, 56, 160, 1, 1), "16q", "16q"), ((50, 64, 56, 56, 64, 1, 1), "8q", "8q"),
-              # pairs: row boxes, tap loop, one and several tiles each
-              ((50, 128, 28, 28, 64, 3, 1), "16qp", "16qp"), ((3, 64, 15, 15, 128, 3, 1), "16qp", "16qp"), ((2, 128, 9, 9, 384, 3, 1), "16qp", "8q"),
-              ((40, 256, 14, 14, 512, 3, 1), "16qp", "16qp")]
+# rounding are repeated here in the same fp32 steps.  N tiles of one, two, three and five blocks, a tile that ends inside its
+# last block, one CTA per SM and two, pairs, three and eight accumulators in flight; infinities and NaN.
+LEAN_CASES = [(5, 32, 17, 13, 32, 1, 1), (3, 64, 9, 7, 72, 1, 1), (2, 32, 11, 13, 160, 1, 1), (40, 64, 28, 28, 96, 1, 1), (3, 96, 8, 8, 64, 3, 2),
+              (50, 64, 24, 24, 64, 3, 1), (9, 32, 30, 30, 320, 1, 1)]
 
 
 @pytest.mark.parametrize("i8", [True, False])
-@pytest.mark.parametrize("case,f16_kernel,i8_kernel", LEAN_CASES)
-def test_lean_quad_epilogue(ctx, case, f16_kernel, i8_kernel, i8):
+@pytest.mark.parametrize("case", LEAN_CASES)
+def test_lean_quad_epilogue(ctx, case, i8):
     import torch
     capi = _capi()
     N, Cin, H, W, Cout, k, s = case
@@ -706,9 +698,6 @@ def test_lean_quad_epilogue(ctx, case, f16_kernel, i8_kernel, i8):
     v = capi.conv2d(ctx, d0, xd, p)[0]
     oh, ow = capi.conv_out_dims(d0)
     skip = dev(r.standard_normal((N, oh, ow, Cout)).astype(np.float16))
-    name = [n for n, _, _ in kernels_of(lambda: capi.conv2d(ctx, desc(capi.EXB_F16, -1, 1, False), xd, p)) if "conv_" in n][0]
-    warps, epi, pair = re.search(r"conv_tc_kernel<\w+, (\d+), \D*(\d), \w+, (\w+)>", name).groups()
-    assert warps + {"0": "r", "1": "q"}[epi] + ("p" if pair == "true" else "") == (i8_kernel if i8 else f16_kernel), name
     for act in (0, 1, 103, 104):
         for res in (False, True):
             for out2 in (-1, capi.EXB_I8):
@@ -731,6 +720,34 @@ def test_lean_quad_epilogue(ctx, case, f16_kernel, i8_kernel, i8):
     ctx.sync_check()
 
 
+# The same where each case is sure to run in the quad epilogue (q; r: row epilogue) of so many warps, in pairs (p), fp16 and int8.
+LEAN_KERNELS = [((5, 32, 17, 13, 32, 1, 1), "8q", "8q"), ((3, 64, 9, 7, 72, 1, 1), "8r", "8r"), ((2, 32, 11, 13, 160, 1, 1), "16q", "16q"),
+                ((40, 64, 28, 28, 96, 1, 1), "8q", "8q"), ((3, 96, 8, 8, 64, 3, 2), "8q", "8q"), ((50, 64, 24, 24, 64, 3, 1), "8q", "8q"),
+                ((9, 32, 30, 30, 320, 1, 1), "16q", "8r"),
+                # channels that end inside the last block
+                ((5, 32, 17, 13, 24, 1, 1), "8q", "8q"), ((3, 64, 9, 7, 56, 1, 1), "8q", "8q"), ((5, 64, 12, 9, 88, 3, 1), "8q", "8q"),
+                # more tiles per CTA than its eight, three and four accumulators
+                ((100, 32, 56, 56, 32, 1, 1), "8q", "8q"), ((19, 32, 56, 56, 160, 1, 1), "16q", "16q"), ((50, 64, 56, 56, 64, 1, 1), "8q", "8q"),
+                # pairs: row boxes, tap loop, one and several tiles each
+                ((50, 128, 28, 28, 64, 3, 1), "16qp", "16qp"), ((3, 64, 15, 15, 128, 3, 1), "16qp", "16qp"),
+                ((2, 128, 9, 9, 384, 3, 1), "16qp", "8q"), ((40, 256, 14, 14, 512, 3, 1), "16qp", "16qp")]
+
+
+@pytest.mark.parametrize("i8", [True, False])
+@pytest.mark.parametrize("case,f16_kernel,i8_kernel", LEAN_KERNELS)
+def test_lean_quad_kernels(ctx, case, f16_kernel, i8_kernel, i8):
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s = case
+    d = capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_I8 if i8 else capi.EXB_F16, capi.EXB_F16, act=1, impl=2)
+    w = np.ones((Cout, Cin, k, k), np.int8 if i8 else np.float32)
+    p = capi.ConvWeights(ctx, d, w, None, np.ones(Cout, np.float32), 1.0) if i8 else capi.ConvWeights(ctx, d, w)
+    x = dev(np.zeros((N, H, W, Cin), np.int8 if i8 else np.float16))
+    name = [n for n, _, _ in kernels_of(lambda: capi.conv2d(ctx, d, x, p)) if "conv_" in n][0]
+    warps, epi, pair = re.search(r"conv_tc_kernel<\w+, (\d+), \D*(\d), \w+, (\w+)>", name).groups()
+    assert warps + {"0": "r", "1": "q"}[epi] + ("p" if pair == "true" else "") == (i8_kernel if i8 else f16_kernel), name
+    test_lean_quad_epilogue(ctx, case, i8)
+
+
 # Reductions that are not divided, and the exchange of those that are, with boxes of fewer pixels than a tile has rows and rings
 # smaller than the tile that takes their place; channel counts with and without whole 32-channel blocks.
 @pytest.mark.parametrize("case", [(15, 32, 11, 11, 176, 1, 2), (15, 32, 11, 11, 192, 1, 2), (1, 64, 6, 6, 48, 1, 1), (3, 64, 5, 5, 64, 1, 1), (2, 512, 5, 7, 208, 3, 1),
@@ -741,8 +758,7 @@ def test_split_tiles_of_few_pixels(ctx, case, i8):
     capi = _capi()
     N, Cin, H, W, Cout, k, s = case
     names = _route(ctx, case, i8, capi.EXB_I8 if i8 else capi.EXB_F16, 0)
-    undivided = "true" if Cin * k * k <= 64 else "false"
-    assert len(names) == 1 and re.search(r"conv_split_kernel<\w+, \w+, %s>" % undivided, names[0]), names
+    assert len(names) == 1 and "conv_split_kernel" in names[0], names
     r = rng(sum(case) + i8)
     wq = r.integers(-4, 5, (Cout, Cin, k, k)).astype(np.int8)
     x = dev(r.integers(-4, 5, (N, H, W, Cin)).astype(np.int8 if i8 else np.float16))
@@ -757,6 +773,16 @@ def test_split_tiles_of_few_pixels(ctx, case, i8):
         ctx.sync_check()
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("case,undivided", [((15, 32, 11, 11, 176, 1, 2), True), ((15, 32, 11, 11, 192, 1, 2), True), ((1, 64, 6, 6, 48, 1, 1), True),
+                                            ((3, 64, 5, 5, 64, 1, 1), True), ((2, 512, 5, 7, 208, 3, 1), False), ((1, 1024, 3, 3, 512, 1, 1), False),
+                                            ((7, 128, 9, 13, 128, 3, 1), False), ((1, 256, 13, 11, 256, 3, 1), False)])
+@pytest.mark.parametrize("i8", [True, False])
+def test_form_of_split_tiles_of_few_pixels(ctx, case, undivided, i8):
+    capi = _capi()
+    names = _route(ctx, case, i8, capi.EXB_I8 if i8 else capi.EXB_F16, 0)
+    assert len(names) == 1 and re.search(r"conv_split_kernel<\w+, \w+, %s>" % ("true" if undivided else "false"), names[0]), names
 
 
 # Undivided tiles, which go from TMEM to the result in a loop of their own: every activation, residual and output against the
