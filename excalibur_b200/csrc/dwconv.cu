@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kRowThreads, 2)
         ++o;
         yo += ypitch;
     };
-    row_stream_run<S, 3, RS, kDwStages>(
+    row_stream_run<S, 3, RS, kDwStages, S == 1 && std::is_same<TOut, int8_t>::value>(
         map, p, ring, full, &abort_flag,
         [&](const RowTile& tile) {
             t = tile;

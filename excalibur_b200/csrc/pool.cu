@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kRowThreads, 2)
         ++o;
         off += ypitch;
     };
-    row_stream_run<S, K, kind.RS, kind.NS>(
+    row_stream_run<S, K, kind.RS, kind.NS, false>(
         map, p, ring, full, &abort_flag,
         [&](const RowTile& tile) {
             t = tile;

@@ -54,7 +54,7 @@ struct RowTile {
 
 // Runs the CTA's tiles.  tile(t) is called at the start of each tile, row(index within the stage as a constant, the
 // thread's input of that row: IN vectors of 4 channels) for every input row, in order.  Returns after the last tile or when a bounded wait ran out (error word set).
-template <int S, int K, int RS, int NS, class Tile, class Row>
+template <int S, int K, int RS, int NS, bool kSharedPlace, class Tile, class Row>
 __device__ __forceinline__ void row_stream_run(const CUtensorMap& map, const RowStreamParams& p, uint8_t* ring, uint64_t* full, int* abort_flag,
                                                Tile tile_fn, Row row_fn) {
     constexpr int IN = (kRowCols - 1) * S + K;
@@ -63,26 +63,41 @@ __device__ __forceinline__ void row_stream_run(const CUtensorMap& map, const Row
     const int slab0 = (int)(blockIdx.x % p.slabs) * p.slab;
     const int u = tid % p.units, g = tid / p.units;
     // Thread 0: next stage to request.  The tile's place is worked out once per tile: six divisions in front of every stage held
-    // its warp, and at the barrier behind the stage all others, up (160 channels @56 x 56 stride 2, 64 images 17.4 -> 16.9 us, 144
-    // channels @56 x 56, 256 images 82.7 -> 81.1).
-    int it_tile = (int)blockIdx.x, it_stage = 0, it_x = 0, it_y = 0, it_n = 0;
+    // its warp, and at the barrier behind the stage all others, up (fp16 144 channels @56 x 56, 256 images 82.8 -> 81.0 us, 16 channels
+    // @103 x 10 stride 2, 98 images 11.2 -> 9.5).  Every thread carries what one of them needs through the arithmetic, unless it
+    // stands in shared memory: taken where that arithmetic has no register left for it (depthwise int8 results at stride 1, all
+    // 128: 192 channels @28 x 28, 256 images 44.7 us with divisions per stage, 47.2 with the place in registers, 46.0 in shared
+    // memory; 160 @56 x 56, 64 images 42.6, 44.1, 43.0; 144 @56 x 56, 256 images 92.0, 91.3, 89.0; 576 @14 x 14 34.8, 32.8, 32.2).
+    __shared__ __align__(16) int4 shared_place;
+    __shared__ int shared_tile;
+    int4 own_place;
+    int own_tile;
+    int4& place = kSharedPlace ? shared_place : own_place;      // x, y, image, stage of the tile
+    int& next_tile = kSharedPlace ? shared_tile : own_tile;
+    if (!kSharedPlace || tid == 0) {
+        next_tile = (int)blockIdx.x;
+        place = make_int4(0, 0, 0, 0);
+    }
     auto request = [&](int slot) {
-        if (it_tile >= p.tiles) return;
-        if (it_stage == 0) {
-            int t = it_tile / p.slabs;
-            it_x = t % p.tiles_w * (p.groups * kRowCols * S) + p.x0;
+        const int tile = next_tile;
+        if (tile >= p.tiles) return;
+        int4 at = place;
+        if (at.w == 0) {
+            int t = tile / p.slabs;
+            at.x = t % p.tiles_w * (p.groups * kRowCols * S) + p.x0;
             t /= p.tiles_w;
-            it_y = t % p.bands * (p.R * S) + p.y0;
-            it_n = t / p.bands;
+            at.y = t % p.bands * (p.R * S) + p.y0;
+            at.z = t / p.bands;
         }
         const uint32_t bar = ptx::smem_u32(&full[slot]);
         ptx::mbar_arrive_expect_tx_u32(bar, (uint32_t)(RS * p.row_bytes));
-        ptx::tma_load_4d_u32(ptx::smem_u32(ring + (size_t)slot * p.slot_bytes), reinterpret_cast<uint64_t>(&map), bar, slab0, it_x, it_y, it_n);
-        it_y += RS;
-        if (++it_stage == p.stages) {
-            it_stage = 0;
-            it_tile += gridDim.x;
+        ptx::tma_load_4d_u32(ptx::smem_u32(ring + (size_t)slot * p.slot_bytes), reinterpret_cast<uint64_t>(&map), bar, slab0, at.x, at.y, at.z);
+        at.y += RS;
+        if (++at.w == p.stages) {
+            at.w = 0;
+            next_tile = tile + gridDim.x;
         }
+        place = at;
     };
     if (tid == 0)
         for (int i = 0; i < NS - 1; ++i) request(i);

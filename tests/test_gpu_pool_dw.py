@@ -172,6 +172,30 @@ def test_dwconv_stream_edges(ctx, case, out_i8):
         np.testing.assert_allclose(y, ref, rtol=2e-3, atol=2e-3)
 
 
+# CTAs of several tiles and slabs: the int8 kernel of stride 1 keeps the place of the next tile elsewhere than the others.  Whole
+# numbers, whose fp16 result is exact.
+@pytest.mark.parametrize("case", [(64, 160, 56, 56, 1, 1), (130, 192, 28, 28, 1, 1), (300, 528, 9, 21, 1, 0), (1100, 16, 17, 30, 1, 1), (64, 96, 57, 40, 2, 1)])
+def test_dwconv_stream_of_many_tiles(ctx, case):
+    import torch
+    capi = _capi()
+    N, Cc, H, W, s, pad = case
+    g = torch.Generator("cuda").manual_seed(sum(case))
+    x = torch.randint(-4, 5, (N, H, W, Cc), generator=g, device="cuda").half()
+    r = rng(sum(case))
+    w, b = r.integers(-2, 3, (Cc, 1, 3, 3)).astype(np.float32), r.integers(-9, 10, Cc).astype(np.float32)
+    y = []
+    for out in (capi.EXB_F16, capi.EXB_I8):
+        d = capi.make_dw_desc(N, H, W, Cc, 3, s, pad, capi.EXB_F16, out, 1, out_scale=1.0)
+        run = lambda p=capi.DwWeights(ctx, d, w, b): capi.dwconv2d(ctx, d, x, p)
+        (name, _, _), = kernels_of(run)
+        assert "dw3x3_stream_kernel" in name
+        y.append(run())
+    ctx.sync_check()
+    assert torch.equal(y[0].clamp(max=127).to(torch.int8), y[1])
+    ref = O.dwconv2d_f32(to_nchw(host(x[-1:].float())), w, b, s, pad, 1)
+    np.testing.assert_array_equal(to_nchw(host(y[0][-1:].float())), ref)
+
+
 # Edges of the streaming pooling kernel: windows hanging over every border of maps smaller than a thread's four columns,
 # negative values next to padding (a maximum must not see the fill), channel counts around one CTA's, ceil mode, the
 # int8 second output; below 32 channels stride 2 takes the other kernel.
