@@ -675,10 +675,10 @@ def yolo_strong_scaling(host, torch, local_rank, rank, world, barrier, max_over_
 # launch per layer shape at batch 256, weighted by how often each shape occurs among the int8 conv launches of a step.
 # It is a constant of the kernel version named in TRAFFIC_SOURCE, not re-measured by this script (ncu cannot run
 # inside the timed program); lower than the algorithmic bytes because small outputs stay in L2.
-TRAFFIC_FROM_NCU = 63.2e6
+TRAFFIC_FROM_NCU = 62.9e6
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch per layer shape at batch 256 (bench_layers.py "
                   "--iters 1 --warmup 0), weighted over the 19 int8 conv launches of a step; captured on the kernel with "
-                  "uniform MMA issue, N tiles by rounds and CTA pairs of 64 to 256 channels")
+                  "lean epilogues and roles that prepare what they alone need")
 
 
 def main():
