@@ -211,8 +211,15 @@ struct ConvSplit {
     int TW, TH, TN;
 };
 ConvSplit conv_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w);
-// Modelled time of the persistent kernel in us.
-double conv_tc_time(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w);
+// N tiles of the persistent kernel: how many, of how many channels, and whether they were chosen to run as CTA pairs.
+struct ConvNTile {
+    int n_tiles, BN;
+    bool paired;
+};
+ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64_t m_tiles);
+// Modelled time of the persistent kernel in us.  tap_order: it sums tap after tap, all channels of each (row boxes of several
+// channel blocks go through the taps of a kernel row block by block).
+double conv_tc_time(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w, bool* tap_order);
 int conv_split_launch(exb_ctx* ctx, const ConvGeom& g, const ConvSplit& sp, const void* x, const exb_conv_weights* w, const void* residual,
                       void* y, void* y2, cudaStream_t st);
 // True when the tcgen05 kernel can run this geometry.

@@ -68,12 +68,10 @@ __device__ __forceinline__ void epi_quad_rows(const EpiParams& e, const float* q
 
 // The lean form of the same for the outputs that layers have in earnest: fp16, alone or with an int8 copy, behind no
 // activation, ReLU, ReLU6 or SiLU.  What bounds short reductions is the instruction stream of the epilogue warps (16
-// instructions per value in the general form: dispatch on activation and types per vector, 64-bit addresses per store), so
-// everything that can be is known at compile time, sums are formed two at a time, clamps act on packed halves (rounding is
-// monotone and 0 and 6 are halves: the same results), and the accumulator is handed back after the last load instead of after
-// the last store.  Measured against the general form: 32 -> 160 int8 1x1 + ReLU6 at 64 x 56 x 56 29.5 -> 19.8 us, 32 -> 96 at
-// 64 x 112 x 112 59.5 -> 40.2 (4.5 TB/s), 64 -> 64 fp16 1x1 + SiLU at 16 x 160 x 160 37.5 -> 30.4, 128 -> 128 + SiLU at
-// 16 x 80 x 80 23.2 -> 18.2.  Loading fragment f + 1 while f is worked on needs more than the 96 registers (5.8 KB spilled).
+// instructions per value in the general form), so everything that can be is known at compile time, sums are formed two at a
+// time, clamps act on packed halves (rounding is monotone and 0 and 6 are halves: the same results), and the accumulator is
+// handed back after the last load.  32 -> 160 int8 1x1 + ReLU6 at 64 x 56 x 56 29.5 -> 19.8 us, 64 -> 64 fp16 1x1 + SiLU at
+// 16 x 160 x 160 37.5 -> 30.4.
 enum QuadAct { kQuadNone = 0, kQuadRelu = 1, kQuadRelu6 = 2, kQuadSilu = 3 };
 template <int kAct>
 using QuadActC = std::integral_constant<int, kAct>;
@@ -141,7 +139,7 @@ __device__ __forceinline__ f32x2 quad_value(uint32_t r0, uint32_t r1, f32x2 scal
     return fma2(kInt8 ? pack2((float)(int)r0, (float)(int)r1) : pack2(__uint_as_float(r0), __uint_as_float(r1)), scale, bias);
 }
 
-// One pixel's 8 consecutive channels, first[i] and first[i] + 1 the accumulators of pair i.
+// One pixel's 8 consecutive channels; raw[4 * i + kFirst] and the next are the accumulators of pair i.
 template <bool kInt8, int kAct, bool kRes, int kOut, int kFirst>
 __device__ __forceinline__ void quad_pixel(const uint32_t (&raw)[16], const f32x2 (&sc)[4], const f32x2 (&bi)[4], const uint4& res, bool store,
                                            __half* y, int8_t* y2, f32x2 out2_scale) {

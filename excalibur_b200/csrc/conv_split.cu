@@ -11,13 +11,9 @@
 // MMAs of a few K blocks, the exchange and the store.  int8 sums are exact whatever the split; fp16 ones are fp32 sums of at
 // most eight partial sums.  An undivided tile goes from TMEM to the result directly, in the column order of the quad epilogue.
 //
-// Such launches are chains of latencies.  Time stamps of the roles showed 2.2 to 3 us behind the last MMA: 0.6 until the parts
-// lay in shared memory behind a cluster barrier, 1.2 to sum them out of the other CTAs' shared memory item after item and to
-// store, 0.3-0.7 for the barrier that kept every CTA until its neighbours had read; undivided tiles took the same way through
-// shared memory.  Per layer of a captured chain, before and after: undivided 64 -> 384 fp16 1x1 at 9 x 13 x 12 3.46 -> 2.26 us,
-// 256 -> 256 int8 3x3 at 32 x 14 x 14 9.6 -> 8.3; divided 512 -> 512 int8 3x3 at 7 x 7 5.6 -> 4.6, 256 -> 256 at 14 x 14 5.4 -> 4.6.
-// Copies between CTAs move some 14 bytes per cycle and SM, so only the box's rows are sent.  Tried: st.async of 16 bytes
-// per lane straight from registers (1 us to issue, 1 more to arrive: every packet is counted by itself).
+// Such launches are chains of latencies: per layer of a captured chain 2.6 us undivided (64 -> 384 fp16 1x1 at 9 x 13 x 12), 4.2 and 4.4
+// in eight parts (512 -> 512 int8 3x3 at 7 x 7, 256 -> 256 at 14 x 14); with parts summed out of the other CTAs' shared memory
+// between cluster barriers 3.6, 5.8 and 5.5.  Copies between CTAs move some 14 bytes per cycle and SM, so only the box's rows are sent.
 #include "conv_quad.cuh"
 #include "conv_tc_host.cuh"
 #include "ptx_sm100.cuh"
@@ -458,62 +454,132 @@ static SplitRing split_ring(const exb_ctx* ctx, int rows, int kb_bytes, int bn, 
     r.b_bytes = bn * kb_bytes;
     r.part = splits == 1 ? 0 : (rows + splits - 1) / splits * splits * (bn * 4 + 16);
     // two CTAs of neighbouring launches fit an SM side by side (programmatic launch): half of the shared memory each, and all
-    // of it where the neighbours find SMs of their own
-    const int room = 2 * grid <= ctx->sm_count ? ctx->smem_optin - 6 * 1024 : 109 * 1024;
+    // of it where the neighbours find SMs of their own, or where one CTA per SM walks through more than two such rings (not
+    // larger clusters: at one CTA per SM those of eight reach some 130 SMs, and 144 CTAs took two waves, 8.5 -> 12.2 us on
+    // 512 -> 136 fp16 3x3 at 2 x 26 x 13)
     const int units = (k_iters + splits - 1) / splits;
-    r.stages = (room - (kTileM * kb_bytes - r.a_bytes) - r.part) / (r.a_bytes + r.b_bytes);
+    const auto stages = [&](int room) { return (room - (kTileM * kb_bytes - r.a_bytes) - r.part) / (r.a_bytes + r.b_bytes); };
+    r.stages = stages(109 * 1024);
+    if (2 * grid <= ctx->sm_count || (grid <= ctx->sm_count && splits <= 2 && units > 2 * r.stages)) r.stages = stages(ctx->smem_optin - 6 * 1024);
     if (r.stages > kSplitStages) r.stages = kSplitStages;
     if (r.stages > units) r.stages = units;
     return r;
 }
 
-// Which kernel, and how a tile is divided: modelled time in us of both kernels, fitted to 1200 layers (batch 1 to 256, 1x1 and
-// 3x3, 16 to 1280 -> 16 to 1280 channels, maps of 4 x 4 to 160 x 160, those of the benchmark networks among them; every split of
-// 32 and 64 channels).  A layer's time is the mean of two measurements, a captured chain of its own launches and one in which
-// they alternate with another layer's: the persistent kernel loses 1.2 to 1.6 us between launches of other kernels,
-// the split kernel 0 to 0.5.  The constants are regression weights, not times of parts.
-//  - Split kernel: a constant, what the exchange costs by the number of parts, the chain of a CTA (K blocks, of which those that
-//    the ring does not hold wait for their loads, the epilogue, the volume of the exchange) and, beyond one CTA per SM, what they
-//    take from each other.  Two run side by side on an SM, fewer where clusters of four and eight do not fill the SMs that
-//    are wired together (at 1.9 and 1.8 per SM times jump by half); beyond that the chain is walked once more.
-//  - Persistent kernel: conv_tc_time, from the layout that its launch would have (row boxes, resident weights, pairs).
-// Up to one CTA per SM a division's time depends on K and the N tile alone, not on the pixels: a small call gives an fp16
-// result of the same bits whether its images come in one batch or in several (a cost by the pixels of a box and the fill of
-// the chip would pick 0.5 % better on average).  Parts of one K block are left out for the same end: of 304 drawn layers they
-// were the fastest choice of twelve, by 2 to 10 %, each of a few small maps.
-// On 600 layers outside the fit the pick is 1.7 % slower than the fastest of all of them on average and 5 % or more slower in
-// one of eight, at worst 37 %.  A model by N tile alone, with CTAs beyond one per SM as a common factor, was 3.5 %, one of five
-// and 101 % off: 512 -> 32 fp16 3x3 at 5 x 56 x 56 ran undivided in 21.7 us (in two parts 14.9), 288 -> 192 int8 3x3 stride 2 at
-// 8 x 56 x 56 in 23.5 (15.8).
-static ConvSplit search_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
-    const ConvSplit none = {0, 0, 0, 0, 0};
-    if (g.pool || g.out_dtype == EXB_I32 || (g.cout_stride & 7) || (g.y_pitch & 7) || conv_fold_plan(g).on) return none;
-    const int row_bytes = g.cin_stride * (g.in_dtype == EXB_I8 ? 1 : 2);
-    const int kb = row_bytes % 128 == 0 ? 128 : (row_bytes % 64 == 0 ? 64 : 32);
-    const int k_iters = g.kh * g.kw * (row_bytes / kb);
-    const PixelBox box = choose_pixel_box(g.N, g.OH, g.OW);
-    const double m_tiles = (double)((g.OW + box.TW - 1) / box.TW) * ((g.OH + box.TH - 1) / box.TH) * ((g.N + box.TN - 1) / box.TN);
-    if (m_tiles > 8.0 * ctx->sm_count) return none;
-    ConvSplit best = {0, 0, box.TW, box.TH, box.TN};
+// What both models of the launch of a layer read.
+struct SplitProblem {
+    PixelBox box;
+    double m_tiles;
+    int kb, k_iters;      // bytes of a K block, K blocks of a tile
+};
+
+// The pick of the first model: both kernels' times in a captured chain, fitted to 590 layers before the layouts of their launches
+// were modelled.  splits = 0: the persistent kernel.
+static ConvSplit first_pick(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w, const SplitProblem& q) {
+    ConvSplit best = {0, 0, q.box.TW, q.box.TH, q.box.TN};
     double best_t = 1e30;
-    static const double kParts[4] = {0.0, 1.347, 0.899, 1.002};      // an exchange of 1, 2, 4, 8 parts beside its volume
-    static const double kPlaces[4] = {2.0, 2.0, 1.9, 1.8};           // CTAs per SM of one wave
-    const double unit = kb == 128 ? 0.1487 : kb == 64 ? 0.1923 : 0.1965, shared = kb == 128 ? 0.0679 : kb == 64 ? 0.0343 : 0.0341;
+    static const double kParts[4] = {0.0, 1.0, 0.53, 0.46};      // an exchange of 1, 2, 4, 8 parts beside its volume
+    const double unit = q.kb == 128 ? 0.218 : q.kb == 64 ? 0.209 : 0.192;
     for (int bn = 32; bn <= 64; bn *= 2)
-        for (int sp = 1, i = 0; sp <= kSplitMaxParts && (sp == 1 || 2 * sp <= k_iters); sp *= 2, ++i) {      // two K blocks a part
-            const double per_sm = m_tiles * ((w->cout_pad + bn - 1) / bn) * sp / ctx->sm_count, full = per_sm / kPlaces[i];
-            const int units = (k_iters + sp - 1) / sp, stages = split_ring(ctx, kTileM, kb, bn, sp, k_iters, ctx->sm_count).stages;
-            const double epi = (bn == 32 ? 0.696 : 0.915) + 0.670 * bn * (sp - 1) / (sp * 64.0);
-            const double chain = units * unit + 0.445 * (units - stages) / stages + epi;
-            const double t = 1.663 + kParts[i] + chain * (full <= 1 ? 1.0 : 0.116 * full + 0.884 * ceil(full)) +
-                             (per_sm > 1 ? per_sm - 1 : 0.0) * (units * shared * (bn == 32 ? 1.105 : 1.0) + 1.548 * epi);
+        for (int sp = 1, i = 0; sp <= kSplitMaxParts && (sp == 1 || 2 * sp <= q.k_iters); sp *= 2, ++i) {      // two K blocks a part
+            const double ctas = q.m_tiles * ((w->cout_pad + bn - 1) / bn) * sp;
+            const double stretch = ctas > 1.02 * ctx->sm_count ? ctas / (1.02 * ctx->sm_count) : 1.0;
+            const double units = (q.k_iters + sp - 1) / sp;
+            const double volume = q.box.TW * q.box.TH * q.box.TN * bn * (sp - 1) / (sp * 8192.0);
+            const double t = 0.8 + kParts[i] + 1.29 * volume +
+                             stretch * (units * unit * (bn == 32 ? 0.962 : 1.0) + (bn == 32 ? 1.40 : 1.52) + 1.31 * volume - (sp > 1 ? 0.36 : 0.0));
             if (t < best_t) {
                 best_t = t;
                 best.BN = bn;
                 best.splits = sp;
             }
         }
-    return best_t < 0.98 * conv_tc_time(ctx, g, w) ? best : none;      // near a tie the kernel that does not divide
+    const ConvNTile nt = conv_n_tile(ctx, g, w->cout_pad, (int64_t)q.m_tiles);
+    const bool two = nt.BN <= 128 && !nt.paired;
+    const double tiles = q.m_tiles * nt.n_tiles, slots = (double)ctx->sm_count * (two ? 2 : 1);
+    const double rounds = tiles <= slots ? 1.0 : ceil(tiles / slots);
+    double share = 1.0, step = 0.292, rest = 1.45;      // one CTA per SM
+    if (two) {
+        if (tiles > ctx->sm_count) share += 0.35 * (tiles < 2 * ctx->sm_count ? tiles / ctx->sm_count - 1 : 1.0);
+        step = nt.BN <= 64 ? 0.216 : 0.304;
+        rest = nt.BN <= 64 ? 0.0 : 1.09;
+    } else if (nt.paired) {
+        step = 0.207;
+        rest = 1.71;
+    }
+    step *= q.kb == 128 ? 1.0 : q.kb == 64 ? 0.65 : 0.56;
+    double body = rounds * (q.k_iters * step + rest + (g.has_res ? 1.5 : 0.0)) * share;
+    // int8 tiles of a short K, more of them than fit the SMs as clusters
+    if (two && g.in_dtype == EXB_I8 && q.k_iters * q.kb <= 256 && q.m_tiles * ((w->cout_pad + 63) / 64) > ctx->sm_count)
+        body *= g.out_dtype == EXB_I8 && g.out2_dtype < 0 ? 0.8 : 1.28;
+    if (best_t >= 3.92 + body) best.splits = 0;
+    return best;
+}
+
+// Modelled time of a launch of the split kernel in us, fitted like conv_tc_time to 1200 layers (batch 1 to 256, 1x1 and 3x3, 16 to
+// 1280 -> 16 to 1280 channels, maps of 4 x 4 to 160 x 160; every split of 32 and 64 channels).  A layer's time is the mean of
+// two measurements, a captured chain of its own launches and one in which they alternate with another layer's: the persistent
+// kernel loses 1.2 to 1.6 us between launches of other kernels, the split kernel 0 to 0.5.  The constants are regression
+// weights, not times of parts: a constant, what the exchange costs by the number of parts, the chain of a CTA (K blocks, of
+// which those that the ring does not hold wait for their loads, the epilogue, the volume of the exchange) and, beyond one CTA
+// per SM, what they take from each other.  Two run side by side on an SM, fewer where clusters of four and eight do not fill
+// the SMs that are wired together (at 1.9 and 1.8 per SM times jump by half); beyond that the chain is walked once more.
+static double split_time(const exb_ctx* ctx, const exb_conv_weights* w, const SplitProblem& q, int bn, int sp) {
+    static const double kParts[4] = {0.0, 1.347, 0.899, 1.002}, kPlaces[4] = {2.0, 2.0, 1.9, 1.8};      // CTAs per SM of one wave
+    const int i = sp == 1 ? 0 : sp == 2 ? 1 : sp == 4 ? 2 : 3;
+    const double unit = q.kb == 128 ? 0.1487 : q.kb == 64 ? 0.1923 : 0.1965, shared = q.kb == 128 ? 0.0679 : q.kb == 64 ? 0.0343 : 0.0341;
+    const double ctas = q.m_tiles * ((w->cout_pad + bn - 1) / bn) * sp, per_sm = ctas / ctx->sm_count, full = per_sm / kPlaces[i];
+    const int grid = per_sm > 0.5 && per_sm <= 1 ? (int)ctas : ctx->sm_count + 1;      // (small grids were fitted with half a ring)
+    const int units = (q.k_iters + sp - 1) / sp, stages = split_ring(ctx, kTileM, q.kb, bn, sp, q.k_iters, grid).stages;
+    const double epi = (bn == 32 ? 0.696 : 0.915) + 0.670 * bn * (sp - 1) / (sp * 64.0);
+    const double chain = units * unit + 0.445 * (units - stages) / stages + epi;
+    return 1.663 + kParts[i] + chain * (full <= 1 ? 1.0 : 0.116 * full + 0.884 * ceil(full)) +
+           (per_sm > 1 ? per_sm - 1 : 0.0) * (units * shared * (bn == 32 ? 1.105 : 1.0) + 1.548 * epi);
+}
+
+// Which kernel, and how a tile is divided.  Two models have to agree: the first one's pick stays unless the second, which knows
+// the layouts, promises 7 % more: of 118 drawn layers it promised less in five, four of which it made 10 to 32 % slower, and
+// more in nine, of which seven were 7 to 33 % faster and two 2 % slower; of 110 others 0.985 of the first pick's time.
+// fp16 layers keep the order of their sums, whose last bits, rounded through the layers of a network, show in its results
+// (1e-4): the number of parts stays the first model's, undivided tiles and a persistent kernel that goes through the taps in
+// the same order are exchanged for each other.  int8 sums are exact whatever the order.
+// 288 -> 192 int8 3x3 stride 2 at 8 x 56 x 56, whose undivided tiles just fit the SMs, 23.4 -> 15.7 us in two parts; 48 -> 264 fp16 3x3
+// at 2 x 64 x 50 11.8 -> 10.2.
+static ConvSplit search_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
+    const ConvSplit none = {0, 0, 0, 0, 0};
+    if (g.pool || g.out_dtype == EXB_I32 || (g.cout_stride & 7) || (g.y_pitch & 7) || conv_fold_plan(g).on) return none;
+    const int row_bytes = g.cin_stride * (g.in_dtype == EXB_I8 ? 1 : 2);
+    SplitProblem q;
+    q.kb = row_bytes % 128 == 0 ? 128 : (row_bytes % 64 == 0 ? 64 : 32);
+    q.k_iters = g.kh * g.kw * (row_bytes / q.kb);
+    q.box = choose_pixel_box(g.N, g.OH, g.OW);
+    q.m_tiles = (double)((g.OW + q.box.TW - 1) / q.box.TW) * ((g.OH + q.box.TH - 1) / q.box.TH) * ((g.N + q.box.TN - 1) / q.box.TN);
+    if (q.m_tiles > 8.0 * ctx->sm_count) return none;
+    const ConvSplit first = first_pick(ctx, g, w, q);
+    bool tap_order;      // as undivided tiles sum
+    const double persistent = conv_tc_time(ctx, g, w, &tap_order);
+    const double limit = 0.93 * (first.splits ? split_time(ctx, w, q, first.BN, first.splits) : persistent);
+    const bool exact = g.in_dtype == EXB_I8;
+    ConvSplit best = first;
+    double best_t = limit;
+    // between launches of other kernels the persistent one loses twice what its modelled time holds (32 -> 160 fp16 1x1 at
+    // 9 x 50 x 45 in a network: 9 us, undivided tiles 7)
+    if (first.splits && persistent + 0.7 < best_t && (exact || (first.splits == 1 && tap_order))) {
+        best_t = persistent;
+        best.splits = 0;
+    }
+    if (first.splits || exact || tap_order)      // (a persistent launch that has no layout is refused)
+        for (int bn = 32; bn <= 64 && (first.splits || persistent < 1e30); bn *= 2)
+            for (int sp = 1; sp <= kSplitMaxParts && (sp == 1 || 2 * sp <= q.k_iters); sp *= 2) {
+                if (!exact && sp != (first.splits ? first.splits : 1)) continue;
+                const double t = split_time(ctx, w, q, bn, sp);
+                if (t < best_t) {
+                    best_t = t;
+                    best.BN = bn;
+                    best.splits = sp;
+                }
+            }
+    return best.splits ? best : none;
 }
 
 // The same, searched once per layer and thread (0.2 us of every eager call): a pure function of the values that are compared,

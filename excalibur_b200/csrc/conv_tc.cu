@@ -288,8 +288,8 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
     // Each role prepares what it alone needs, so that none waits for another's global loads: with one CTA per SM nothing of this
     // overlaps the previous kernel's last tiles.  Warp 0 initialises the barriers and goes on to its table of K units and the
     // weights without waiting for the block (bar.arrive); warp 1 allocates TMEM; the epilogue warps stage scale and bias and
-    // meet at a barrier of their own.  In a captured chain 64 -> 64 fp16 3x3 at 4 x 120 x 184 13.0 -> 11.6 us, 128 -> 128 int8 3x3
-    // at 32 x 28 x 28 10.9 -> 9.1, 64 -> 384 int8 1x1 at 64 x 14 x 14 7.3 -> 6.6.
+    // meet at a barrier of their own.  With tiles that all warps drain where a CTA has one, in a captured chain: 64 -> 64 fp16 3x3 at
+    // 4 x 120 x 184 14.2 -> 11.6 us, 128 -> 128 int8 3x3 at 32 x 28 x 28 11.1 -> 9.2, 64 -> 384 int8 1x1 at 64 x 14 x 14 7.6 -> 6.4.
     if (warp == 0) {
         // (one lane per barrier: 33 of them one after the other are half a microsecond)
         if (lane < p.stages) {
@@ -1151,12 +1151,6 @@ static bool conv_pairable(const exb_ctx* ctx, const ConvGeom& g) {
     return ctx->sm_count >= 2 && g.act != EXB_ACT_PRELU && !g.res_half && g.rh * g.rw == 1 && !g.pool && !conv_fold_plan(g).on;
 }
 
-// N tiles: how many, of how many channels, and whether they were chosen to run as CTA pairs.
-struct ConvNTile {
-    int n_tiles, BN;
-    bool paired;
-};
-
 // The N tile: 256 channels, or 128 where that is the faster one.
 //  - Below 512 bytes of K, and up to 1152 in the first round of tiles (two of them for two N tiles), the epilogue sets the
 //    pace, and two CTAs of 128 channels per SM drain more than one of 256: 96 -> 576 int8 1x1 at 256 x 14 x 14 23.8 ->
@@ -1170,7 +1164,7 @@ struct ConvNTile {
 //    of one of 256 (half the MMA time, but the same activations): 128 where its rounds of pairs come to less.
 //    512 -> 512 3x3 fp16 at 64 x 7 x 7: 26 pairs of 256 on 74 places 30.9 us, 52 of 128 24.0; 256 -> 256 int8 at
 //    100 x 14 x 14: two rounds 21.8, three of 128 19.4; 256 -> 256 fp16 at 64 x 14 x 14: one round 22.3, two of 128 23.5.
-static ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64_t m_tiles) {
+ConvNTile conv_n_tile(const exb_ctx* ctx, const ConvGeom& g, int cout_pad, int64_t m_tiles) {
     auto tile = [&](int most) {
         const int n = (cout_pad + most - 1) / most;
         return ConvNTile{n, round_up((cout_pad + n - 1) / n, 16), false};
@@ -1329,7 +1323,8 @@ static int conv_tc_layout(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
         if (rb.one_cta) two = false;
     }
     // Quad epilogue: N tiles of whole 32-channel blocks, every channel group of 8 either fully inside the output or
-    // fully outside, weights stored in whole 32-row blocks (the permuting map walks rows 32 at a time).  Taken when
+    // fully outside (channel counts that end inside a block would run here too, their weights are stored in whole blocks;
+    // they are left in the row epilogue, where they were measured).  Taken when
     // the epilogue moves fp16 / fp32 data (an fp16 output or residual): there its whole-sector accesses are worth
     // 15-20 % of the layer; a lone int8 output is as fast from the thread-per-pixel epilogue (measured on the
     // ResNet-18-style layers at batch 256), which needs fewer TMEM loads.
@@ -1475,10 +1470,12 @@ static int conv_tc_layout(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
 // Modelled time of a launch in us (see search_split_plan): a constant; for every round of tiles a chain of K blocks, of which
 // those that the ring does not hold wait for their loads; and what each tile takes from its SM (operand bytes, values of the
 // epilogue).  A layout that cannot be launched takes for ever.
-double conv_tc_time(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {
+double conv_tc_time(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w, bool* tap_order) {
     ConvTcParams p;
     ConvTcForm f;
+    *tap_order = false;
     if (conv_tc_layout(ctx, g, w, p, f) != EXB_OK) return 1e30;
+    *tap_order = !p.rowbox || p.cblks == 1;
     auto size_of = [](int dtype) { return dtype == EXB_I8 ? 1 : dtype == EXB_F16 ? 2 : 4; };
     const int out_bytes = size_of(g.out_dtype) + (g.out2_dtype >= 0 ? size_of(g.out2_dtype) : 0);
     const bool lone_i8 = g.in_dtype == EXB_I8 && out_bytes == 1;

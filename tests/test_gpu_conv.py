@@ -643,11 +643,8 @@ def test_short_int8_reductions_are_divided_only_when_few(ctx, case, split):
     assert len(names) == 1 and ("conv_split_kernel" in names[0]) == split, names
 
 
-# Reductions that are divided although undivided tiles would just fit the SMs: 512 -> 32 3x3 at 5 x 56 x 56 takes 14.9 us in
-# two parts and 21.7 undivided, 304 -> 288 stride 2 at 31 x 13 x 14 16.6 in four and 27.8 in two, 288 -> 192 int8 stride 2 at
-# 8 x 56 x 56 15.8 in two and 23.5 undivided.
-@pytest.mark.parametrize("case,i8,kernel,ctas", [((5, 512, 56, 56, 32, 3, 1), False, "conv_split_kernel<false, false, false>", 266),
-                                                 ((31, 304, 13, 14, 288, 3, 2), False, "conv_split_kernel<false, false, false>", 280),
+# Long reductions whose undivided tiles just fit the SMs: int8 ones are divided, fp16 ones keep the order of their sums.
+@pytest.mark.parametrize("case,i8,kernel,ctas", [((5, 512, 56, 56, 32, 3, 1), False, "conv_split_kernel<false, false, true>", 133),
                                                  ((8, 288, 56, 56, 192, 3, 2), True, "conv_split_kernel<true, false, false>", 294)])
 def test_long_reductions_of_one_tile_per_sm(ctx, case, i8, kernel, ctas):
     import torch
@@ -665,6 +662,25 @@ def test_long_reductions_of_one_tile_per_sm(ctx, case, i8, kernel, ctas):
     ctx.sync_check()
     want = O.conv2d_i8_acc(x[-1:].transpose(0, 3, 1, 2), wq, s, k // 2)[0].astype(np.float16)
     np.testing.assert_array_equal(host(y[-1]).transpose(2, 0, 1), want)
+
+
+# Whichever kernel the plan picks, an fp16 layer's sums keep their order, to the last bit of an fp32 result: undivided tiles and the
+# persistent kernel's tap loop (and its row boxes of one channel block) sum alike.
+@pytest.mark.parametrize("case", [(1, 80, 66, 50, 400, 3, 1), (2, 48, 64, 50, 264, 3, 1), (9, 64, 13, 12, 384, 1, 1), (4, 320, 21, 77, 344, 1, 2), (20, 64, 30, 25, 128, 3, 1),
+                                  (16, 32, 40, 40, 64, 3, 1)])
+def test_undivided_sums_keep_their_order(ctx, case):
+    import torch
+    capi = _capi()
+    N, Cin, H, W, Cout, k, s = case
+    r = rng(sum(case))
+    w = r.standard_normal((Cout, Cin, k, k)).astype(np.float32)
+    x = dev(r.standard_normal((N, H, W, Cin)).astype(np.float16))
+    desc = lambda impl: capi.make_conv_desc(N, H, W, Cin, Cout, k, s, k // 2, capi.EXB_F16, capi.EXB_F32, impl=impl)
+    p = capi.ConvWeights(ctx, desc(0), w)
+    names = [n for n, _, _ in kernels_of(lambda: capi.conv2d(ctx, desc(0), x, p)) if "conv_" in n]
+    assert len(names) == 1 and re.search(r"conv_split_kernel<\w+, \w+, true>", names[0]), names
+    assert torch.equal(capi.conv2d(ctx, desc(0), x, p)[0], capi.conv2d(ctx, desc(2), x, p)[0])
+    ctx.sync_check()
 
 
 # The lean quad epilogue (fp16 result, alone or with an int8 copy) against the same kernel's fp32 result, which is read from the
