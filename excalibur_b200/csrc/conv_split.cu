@@ -542,7 +542,9 @@ static double split_time(const exb_ctx* ctx, const exb_conv_weights* w, const Sp
 // more in nine, of which seven were 7 to 33 % faster and two 2 % slower; of 110 others 0.985 of the first pick's time.
 // fp16 layers keep the order of their sums, whose last bits, rounded through the layers of a network, show in its results
 // (1e-4): the number of parts stays the first model's, undivided tiles and a persistent kernel that goes through the taps in
-// the same order are exchanged for each other.  int8 sums are exact whatever the order.
+// the same order are exchanged for each other.  int8 sums are exact whatever the order.  A part has two K blocks at least:
+// parts of one were the fastest choice of 12 of 304 drawn layers, by 2 to 10 %, and without them small batches of the same
+// image more often keep one order.
 // 288 -> 192 int8 3x3 stride 2 at 8 x 56 x 56, whose undivided tiles just fit the SMs, 23.4 -> 15.7 us in two parts; 48 -> 264 fp16 3x3
 // at 2 x 64 x 50 11.8 -> 10.2.
 static ConvSplit search_split_plan(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w) {

@@ -1467,7 +1467,7 @@ static int conv_tc_layout(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_
     return EXB_OK;
 }
 
-// Modelled time of a launch in us (see search_split_plan): a constant; for every round of tiles a chain of K blocks, of which
+// Modelled time of a launch in us (fitted like split_time of conv_split.cu): a constant; for every round of tiles a chain of K blocks, of which
 // those that the ring does not hold wait for their loads; and what each tile takes from its SM (operand bytes, values of the
 // epilogue).  A layout that cannot be launched takes for ever.
 double conv_tc_time(const exb_ctx* ctx, const ConvGeom& g, const exb_conv_weights* w, bool* tap_order) {
