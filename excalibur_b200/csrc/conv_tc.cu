@@ -1065,8 +1065,12 @@ __global__ void __launch_bounds__((kFirstEpiWarp + kEpiWarps) * 32, kEpiWarps ==
                                 }
                             }
                             if constexpr (kPrelu) {
+                                // two vector loads instead of eight behind a comparison each: 128 -> 200 fp16 1x1 at 64 x 28 x 28
+                                // 24.3 -> 20.7 us, int8 18.0 -> 16.2
+                                const float4 l0 = __ldg(reinterpret_cast<const float4*>(p.e.slope + c8)), l1 = __ldg(reinterpret_cast<const float4*>(p.e.slope + c8) + 1);
+                                const float sl[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
 #pragma unroll
-                                for (int i = 0; i < 8; ++i) v[i] = v[i] >= 0.f ? v[i] : v[i] * __ldg(p.e.slope + c8 + i);
+                                for (int i = 0; i < 8; ++i) v[i] = v[i] >= 0.f ? v[i] : v[i] * sl[i];
                             } else {
                                 apply_act_vec(v, p.e.act);
                             }
